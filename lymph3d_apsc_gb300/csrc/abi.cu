@@ -20,13 +20,11 @@
 
 // kernels (setup.cu, step.cu)
 int lymph_dev_geometry(lymph_ctx* c);
-int lymph_dev_assemble(lymph_ctx* c, int which, void* out, int out_fp32, bool write_mass);
-int lymph_dev_assemble_list(lymph_ctx* c, int which, void* out, int out_fp32, bool write_mass, const int64_t* list,
-                            int64_t n_list, int64_t out_stride);
+int lymph_dev_assemble(lymph_ctx* c, int which, double* out, bool write_mass);
 int lymph_mf_setup(lymph_ctx* c, const RefTables& R);
 int lymph_dev_cholesky(lymph_ctx* c);
 int lymph_dev_damping(lymph_ctx* c, bool assemble);
-int lymph_dev_mass(lymph_ctx* c, const int64_t* self_list);
+int lymph_dev_mass(lymph_ctx* c);
 int lymph_dev_self_tc(lymph_ctx* c, float* out, bool block_csr);
 int lymph_dev_nb_tc(lymph_ctx* c, float* out, const int64_t* list, int64_t n_list);
 int lymph_dev_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scale, double* out);
@@ -493,17 +491,8 @@ static int make_mf_matrices(lymph_ctx* c) {
         c->d_K = pK;
         c->device_bytes += (int64_t)(nK * sizeof(float));
     }
-    std::vector<int64_t> self(np);
-    for (int P = 0; P < np; ++P) self[P] = c->h_row_ptr[P];
-    int64_t* d_list = nullptr;
-    LYMPH_CUDA_TRY(cudaMalloc(&d_list, sizeof(int64_t) * (size_t)np));
-    int rc = cudaMemcpy(d_list, self.data(), sizeof(int64_t) * (size_t)np, cudaMemcpyHostToDevice) == cudaSuccess
-                 ? LYMPH_OK : LYMPH_ERR_CUDA;
-    if (rc == LYMPH_OK) rc = lymph_dev_mass(c, d_list);
-    if (rc == LYMPH_OK) rc = lymph_dev_self_tc(c, (float*)c->d_K, false);
-    if (rc == LYMPH_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = LYMPH_ERR_CUDA;
-    cudaFree(d_list);
-    LYMPH_TRY(rc);
+    LYMPH_TRY(lymph_dev_mass(c));
+    LYMPH_TRY(lymph_dev_self_tc(c, (float*)c->d_K, false));
     RefTables R;
     if (!build_ref_tables(c->p, R)) { lymph_set_error("lymph_make_matrices: no quadrature for this degree"); return LYMPH_ERR_INVALID; }
     return lymph_mf_setup(c, R);
@@ -513,18 +502,17 @@ static int make_mf_matrices(lymph_ctx* c) {
 // tensor cores, the mass matrices in FP64.
 static int make_mixed_blocks(lymph_ctx* c) {
     const int np = c->n_poly;
-    std::vector<int64_t> lists;
+    std::vector<int64_t> lists;  // the neighbour blocks
     lists.reserve((size_t)c->n_blocks);
-    for (int P = 0; P < np; ++P) lists.push_back(c->h_row_ptr[P]);
     for (int P = 0; P < np; ++P)
         for (int64_t k = (int64_t)c->h_row_ptr[P] + 1; k < c->h_row_ptr[P + 1]; ++k) lists.push_back(k);
-    const int64_t n_nb = (int64_t)lists.size() - np;
+    const int64_t n_nb = (int64_t)lists.size();
     int64_t* d_lists = nullptr;
-    LYMPH_CUDA_TRY(cudaMalloc(&d_lists, sizeof(int64_t) * lists.size()));
+    LYMPH_CUDA_TRY(cudaMalloc(&d_lists, sizeof(int64_t) * (lists.size() + 1)));
     int rc = cudaMemcpy(d_lists, lists.data(), sizeof(int64_t) * lists.size(), cudaMemcpyHostToDevice) == cudaSuccess
                  ? LYMPH_OK : LYMPH_ERR_CUDA;
-    if (rc == LYMPH_OK) rc = lymph_dev_mass(c, d_lists);
-    if (rc == LYMPH_OK && n_nb > 0) rc = lymph_dev_nb_tc(c, (float*)c->d_K, d_lists + np, n_nb);
+    if (rc == LYMPH_OK) rc = lymph_dev_mass(c);
+    if (rc == LYMPH_OK && n_nb > 0) rc = lymph_dev_nb_tc(c, (float*)c->d_K, d_lists, n_nb);
     if (rc == LYMPH_OK) rc = lymph_dev_self_tc(c, (float*)c->d_K, true);
     if (rc == LYMPH_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = LYMPH_ERR_CUDA;
     cudaFree(d_lists);
@@ -576,7 +564,7 @@ int lymph_make_matrices(lymph_ctx* c) {
     c->k32_valid = false;  // an FP32 copy made from earlier blocks is stale
     c->rhs_version++;      // and so is any cached M^-1 F
     if (c->precision == LYMPH_MIXED) LYMPH_TRY(make_mixed_blocks(c));
-    else LYMPH_TRY(lymph_dev_assemble(c, LYMPH_BLOCKS_K, c->d_K, 0, true));
+    else LYMPH_TRY(lymph_dev_assemble(c, LYMPH_BLOCKS_K, (double*)c->d_K, true));
     LYMPH_TRY(lymph_dev_cholesky(c));
     LYMPH_TRY(lymph_dev_damping(c, true));
     LYMPH_TRY(lymph_sync_status(c, "lymph_make_matrices"));
@@ -909,7 +897,7 @@ int lymph_error_dg(lymph_ctx* c, int s_uh, int s_uex, double* sumsq) {
         lymph_set_error("lymph_error_dg: cannot allocate the A_dg blocks");
         return LYMPH_ERR_OOM;
     }
-    int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_ADG, A, 0, false);
+    int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_ADG, A, false);
     if (rc == LYMPH_OK) rc = lymph_dev_error_dg(c, A, lymph_slot_ptr(c, s_uh), lymph_slot_ptr(c, s_uex), c->d_scalar);
     if (rc == LYMPH_OK && cudaMemcpyAsync(sumsq, c->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
         rc = LYMPH_ERR_CUDA;
@@ -974,7 +962,7 @@ int lymph_get_blocks(lymph_ctx* c, int which, double* vals) {
         // every block (the neighbour blocks are not stored in this mode)
         double* A = nullptr;
         if (cudaMalloc(&A, nK * sizeof(double)) != cudaSuccess) { lymph_set_error("lymph_get_blocks: out of memory"); return LYMPH_ERR_OOM; }
-        int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_K, A, 0, false);
+        int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_K, A, false);
         if (rc == LYMPH_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = LYMPH_ERR_CUDA;
         if (rc == LYMPH_OK && cudaMemcpy(tmp.data(), A, nK * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) rc = LYMPH_ERR_CUDA;
         cudaFree(A);
@@ -988,7 +976,7 @@ int lymph_get_blocks(lymph_ctx* c, int which, double* vals) {
     } else {
         double* A = nullptr;
         if (cudaMalloc(&A, nK * sizeof(double)) != cudaSuccess) { lymph_set_error("lymph_get_blocks: out of memory"); return LYMPH_ERR_OOM; }
-        int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_ADG, A, 0, false);
+        int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_ADG, A, false);
         if (rc == LYMPH_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = LYMPH_ERR_CUDA;
         if (rc == LYMPH_OK && cudaMemcpy(tmp.data(), A, nK * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) rc = LYMPH_ERR_CUDA;
         cudaFree(A);

@@ -4,26 +4,16 @@
 //
 // Assembly design.  The reference builds every (3Np)^2 block entry by entry
 // at every quadrature point (MAKE_STIFFNESS_VOLUME, assemble_element.f90:24-77;
-// MAKE_STIFFNESS_FACE, :404-661).  Here each CTA owns one block and
-// accumulates, per pair of basis functions (m,n), a handful of scalar
-// moments over the quadrature points, then folds them into the 9 component
-// entries with the material and face constants:
-//   volume:  G_kl(m,n) = sum_q w|J| d_k phi_m d_l phi_n,
-//            V_ij = lambda G_ij + mu G_ji + delta_ij mu (G_11+G_22+G_33)
-//   faces:   P(a,b) = sum W phi_a phi_b', H_k(a,b) = sum W d_k phi_a phi_b',
-//            HT_k(a,b) = sum W phi_a d_k phi_b'  (W = weight * area)
-//            S  = sigma T_ij P,  T_ii = n_i^2 + (n_j^2 + n_k^2)/2,  T_ij = n_i n_j / 2
-//            I(i,j) = c [lambda n_j H_i + mu n_i H_j + delta_ij mu n.H]
-// which is algebraically the reference's sum, with 9x fewer FP64 products.
+// MAKE_STIFFNESS_FACE, :404-661).  Here a CTA owns one block and forms, per
+// pair of basis functions, plain mass moments over the quadrature points (one
+// multiply-add per point), sums them over the tetrahedra or triangles with
+// their material and normal factors, and applies the derivatives once per
+// block through the Legendre expansion of phi' (k_assemble_self,
+// k_assemble_nb): algebraically the reference's sum.
 
 #include "common.cuh"
 
 namespace {
-
-constexpr int ASM_THREADS = 256;
-// AsmArgs::which for the mass matrices alone (the self blocks of the
-// mixed operators come from the tensor-core assembly in selftc.cu)
-constexpr int ASM_MASS_ONLY = 2;
 
 template <int P> struct Deg {
     static constexpr int NP = (P + 1) * (P + 2) * (P + 3) / 6;
@@ -128,7 +118,63 @@ __device__ inline void tet_point(const double* fk, const RefTables* ref, int q, 
     }
 }
 
+// Shape of the assembly CTAs per degree.  The moments of a self block are
+// symmetric, so a CTA owns the NS = Np (Np + 1) / 2 pairs a <= b (packed:
+// pair (a, b) at b (b + 1) / 2 + a); a neighbour block owns all Np^2 pairs.
+// The thread counts fill whole rounds of pairs with FP64 lanes (the pipe
+// retires 2 lanes per clock and SM whether they are used or not): p = 4,
+// 630 of 640 and 1225 of 1280 lanes; p = 3, 210 of 224 and 400 of 416.
+template <int PD> struct AsmShape {
+    using D = Deg<PD>;
+    static constexpr int NP = D::NP, L1 = PD + 1;
+    static constexpr int NS = NP * (NP + 1) / 2;
+    static constexpr int T = PD == 4 ? 320 : (PD == 3 ? 224 : (PD == 2 ? 64 : 32));       // self blocks
+    static constexpr int PPT = (NS + T - 1) / T;
+    static constexpr int R = PD == 4 ? 50 : (PD == 3 ? 64 : (PD == 2 ? 27 : 8));          // tabulated points at once
+    static constexpr int FB = R / D::NQ2;                                                 // faces at once
+    static constexpr int TN = PD == 4 ? 320 : (PD == 3 ? 416 : (PD == 2 ? 64 : 32));      // neighbour blocks
+    static constexpr int PPTN = (D::NPAIR + TN - 1) / TN;
+    static_assert(FB >= 1, "one face per table at least");
+};
+
+// Position of basis function (x, y, z) in the reference's order, and the
+// Legendre expansion of the derivatives: with phi_n the scaled Legendre
+// polynomial of degree n on an interval of half width h,
+//     phi_n' = (1/h) sum_{m = n-1, n-3, ..} (2m + 1) phi_m,
+// at most two terms for n <= 4.  idx[f][k][t] is the basis function of term
+// t of d_k phi_f, w[n][t] the weight (2m + 1) (0: no such term).
+template <int PD> struct DerTab {
+    short idx[Deg<PD>::NP][3][2];
+    signed char deg[Deg<PD>::NP][3];
+    constexpr DerTab() : idx(), deg() {
+        constexpr Blist<PD> BL{};
+        int pos[PD + 1][PD + 1][PD + 1] = {};
+        for (int f = 0; f < Deg<PD>::NP; ++f) pos[BL.d[f][0]][BL.d[f][1]][BL.d[f][2]] = f;
+        for (int f = 0; f < Deg<PD>::NP; ++f)
+            for (int k = 0; k < 3; ++k) {
+                deg[f][k] = (signed char)BL.d[f][k];
+                for (int t = 0; t < 2; ++t) {
+                    int q[3] = {BL.d[f][0], BL.d[f][1], BL.d[f][2]};
+                    q[k] -= 1 + 2 * t;
+                    idx[f][k][t] = (short)(q[k] >= 0 ? pos[q[0]][q[1]][q[2]] : 0);
+                }
+            }
+    }
+};
+template <int PD> __device__ const DerTab<PD> g_der{};
+// Its copy in shared memory (the threads of a warp read different functions).
+template <int PD> __device__ __forceinline__ void load_der(DerTab<PD>* dst) {
+    static_assert(sizeof(DerTab<PD>) % sizeof(short) == 0, "copied as shorts");
+    const short* src = reinterpret_cast<const short*>(&g_der<PD>);
+    for (int i = threadIdx.x; i < (int)(sizeof(DerTab<PD>) / sizeof(short)); i += blockDim.x)
+        reinterpret_cast<short*>(dst)[i] = src[i];
+}
+__device__ __forceinline__ double der_weight(int n, int t) {  // (2m + 1) for m = n - 1 - 2t
+    return n - 1 - 2 * t >= 0 ? (double)(2 * (n - 1 - 2 * t) + 1) : 0.0;
+}
+
 struct AsmArgs {
+    const int32_t* row_ptr;
     const int32_t* blk_row;
     const int32_t* col;
     const int64_t* bf_ptr;
@@ -147,324 +193,487 @@ struct AsmArgs {
     const double* hk;
     const RefTables* ref;
     double alpha, theta;
-    int which;        // LYMPH_BLOCKS_K or LYMPH_BLOCKS_ADG
-    int out_fp32;     // store FP32 blocks
-    void* out;        // [n][out_stride] blocks, each [ND][ND] column-major
-    const int64_t* list;  // blocks to assemble (null: all, in order); output slot = position in the list
-    int64_t out_stride;   // elements from one output block to the next (>= ND*ND)
-    double* M;        // [n_poly][NP][NP] rho-weighted mass (self blocks only; may be null)
+    double* out;      // [n_blocks][ND][ND], each block column-major
+    double* M;        // [n_poly][NP][NP] rho-weighted mass (may be null)
     double* Mm;       // unweighted (modal) mass
-    int64_t block0;   // first block of this launch
+    int64_t block0;   // first block of this launch (neighbour blocks)
 };
 
-// One CTA per operator block (row polyhedron P, column polyhedron Q).
+// Interval constants of a bounding box per coordinate, as legendre_1d forms them.
+struct BoxC {
+    double mb[3], hb[3], sh[3];
+};
+__device__ __forceinline__ void box_consts(const double* bb, BoxC* B, int d) {
+    B->hb[d] = (bb[2 * d + 1] - bb[2 * d]) / 2.0;
+    B->mb[d] = (bb[2 * d + 1] + bb[2 * d]) / 2.0;
+    B->sh[d] = sqrt(B->hb[d]);
+}
+// The scaled Legendre values of degrees 0..PD at coordinate x of direction d:
+// legendre_1d's values, with the interval's constants and the normalised
+// coordinate formed once for all degrees.
 template <int PD>
-__global__ void __launch_bounds__(ASM_THREADS) k_assemble(AsmArgs A) {
+__device__ __forceinline__ void legendre_vals(const BoxC* B, int d, double x, double* v) {
+    const double xp = (x - B->mb[d]) / B->hb[d], sh = B->sh[d];
+#pragma unroll
+    for (int n = 0; n <= PD; ++n) v[n] = lp_nonnorm(xp, n) / sh;
+}
+
+// Coordinate j of the affine map of face f of a tetrahedron: cm[l] =
+// (Fk node_maps(:,:,f))(j, l), as face_point forms it.
+__device__ __forceinline__ double face_map(const double* fk, const RefTables* ref, int f, int j, int l) {
+    const double* nm = &ref->node_maps[f * 16];
+    double tmp = 0.0;
+    for (int m = 0; m < 4; ++m) tmp = tmp + fk[j * 4 + m] * nm[m * 4 + l];
+    return tmp;
+}
+
+// The 12 factors of a face's moments P(a, b) = sum_q W phi_a phi_b, W =
+// weight * area: c lambda n_j, c mu n_j (j = 0..2) and sigma T_ij for (i, j)
+// = 00, 11, 22, 01, 02, 12 (T_ii = n_i^2 + (n_j^2 + n_k^2) / 2, T_ij =
+// n_i n_j / 2).
+constexpr int FACE_F = 12;
+__device__ __forceinline__ void face_factors(const AsmArgs& A, int code, int P, int Qn, double c, double pdeg2, double* o) {
+    const int t = code >> 2, f = code & 3;
+    const int mid = A.tet_mat[t];
+    const double lam = A.mat[mid * 3 + 1], mu = A.mat[mid * 3 + 2];
+    const double* n = &A.nrm[t * 12 + f * 3];
+    const double h1 = A.hk[P];
+    const double sigma = A.alpha * pdeg2 / (Qn < 0 ? h1 : fmin(h1, A.hk[Qn])) * (lam + 2 * mu);
+    const double n2[3] = {n[0] * n[0], n[1] * n[1], n[2] * n[2]};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        o[j] = c * lam * n[j];
+        o[3 + j] = c * mu * n[j];
+        o[6 + j] = sigma * (n2[j] + 0.5 * n2[(j + 1) % 3] + 0.5 * n2[(j + 2) % 3]);
+    }
+    o[9] = sigma * (0.5 * n[0] * n[1]);
+    o[10] = sigma * (0.5 * n[0] * n[2]);
+    o[11] = sigma * (0.5 * n[1] * n[2]);
+}
+
+enum { ASM_MASS = 0, ASM_K = 1, ASM_ADG = 2 };
+
+// The self block of each polyhedron (stiffness or DG-norm block) and its two
+// mass matrices, one CTA per polyhedron.
+//
+// FP64-pipe bound, so the design removes FP64 operations.  Derivatives of
+// Legendre products are sums of at most two lower ones per direction, so
+// every term follows from plain mass moments: per tetrahedron M_t(a, b) =
+// sum_q w phi_a phi_b (needed for the mass matrices anyway), per face
+// P(a, b) = sum_q W phi_a phi_b, each weighted with its material and normal
+// factors and summed over the tetrahedra or faces; only then the derivative
+// expansion is applied, once per block:
+//     volume  V_ij = D_i (sum lambda M_t) D_j^T + D_j (sum mu M_t) D_i^T + delta_ij sum_k D_k (sum mu M_t) D_k^T
+//     faces   S = sum sigma T_ij P,  H-terms D_i (sum c lambda n_j P), ...
+// A quadrature point of a pair then costs one multiply-add instead of ten
+// (volume) or seven (faces).  All moments are symmetric, so only a <= b is
+// formed.  The mass matrices keep legendre_1d's values and the sums' order
+// (products and sums rounded separately), because their inverses amplify a
+// change of rounding by the condition number (up to 1e7).
+template <int PD, int WHICH>
+__global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
     using D = Deg<PD>;
-    constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = D::NQ2;
-    constexpr int PPT = (D::NPAIR + ASM_THREADS - 1) / ASM_THREADS;
-    constexpr int QC = NQ3 < 32 ? NQ3 : 32;
+    using S = AsmShape<PD>;
+    constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = D::NQ2, NS = S::NS, T = S::T, PPT = S::PPT, R = S::R,
+                  L1 = S::L1, FB = S::FB;
+    constexpr int NMAT = WHICH == ASM_MASS ? 0 : 14;   // lambda M, mu M, c lambda n_j P (3), c mu n_j P (3), sigma T P (6)
     extern __shared__ double sm[];
-    double* acc = sm;                   // [ND][ND] row-major
-    double* tab = acc + ND * ND;        // tabulation area
-    const int tid = threadIdx.x;
-    const int64_t slot = A.block0 + blockIdx.x;
-    const int64_t k = A.list ? A.list[slot] : slot;
-    const int P = A.blk_row[k];
-    const int Qc = A.col[k];
-    const bool self = (Qc == P);
-    const double pdeg2 = (double)(PD * PD);
-
-    const bool mass_only = (A.which == ASM_MASS_ONLY);
-    if (!mass_only)
-        for (int i = tid; i < ND * ND; i += ASM_THREADS) acc[i] = 0.0;
-
-    if (self) {
-        // ---- volume terms and mass matrices over the sub-tetrahedra ----
-        double* tphi = tab;                 // [QC][NP]
-        double* tdphi = tphi + QC * NP;     // [QC][3][NP]
-        double* tw = tdphi + QC * 3 * NP;   // [QC]
-        double* ttl = tw + QC;              // [QC][3][p+1] (value, derivative) pairs
-        double msum[PPT], mrho[PPT];
+    double* mats = sm;                    // [NMAT][NS]
+    double* tphi = mats + NMAT * NS;      // [R][NP]
+    double* twphi = tphi + R * NP;        // [R][NP]
+    double* tleg = twphi + R * NP;        // [R][3][L1]
+    double* tw = tleg + R * 3 * L1;       // [R]
+    double* ffac = tw + R;                // [FB][FACE_F]
+    double* fmap = ffac + FB * FACE_F;    // [FB][3][4]
+    __shared__ BoxC box;
+    __shared__ DerTab<PD> der;
+    const int tid = threadIdx.x, P = blockIdx.x;
+    load_der<PD>(&der);
+    if (tid < 3) box_consts(&A.bbox[P * 6], &box, tid);
+    int pm[PPT], pn[PPT];                 // this thread's pairs m <= n
 #pragma unroll
-        for (int u = 0; u < PPT; ++u) { msum[u] = 0.0; mrho[u] = 0.0; }
-        const double* bb = &A.bbox[P * 6];
-        for (int kt = A.poly_ptr[P]; kt < A.poly_ptr[P + 1]; ++kt) {
-            const int t = A.poly_tets[kt];
-            const double* fk = &A.fk[t * 12];
-            const int mid = A.tet_mat[t];
-            const double rho = A.mat[mid * 3 + 0], lam = A.mat[mid * 3 + 1], mu = A.mat[mid * 3 + 2];
-            const double aj = fabs(A.jdet[t]);
-            double G[PPT][9], Mt[PPT];
-#pragma unroll
-            for (int u = 0; u < PPT; ++u) {
-                Mt[u] = 0.0;
-#pragma unroll
-                for (int e = 0; e < 9; ++e) G[u][e] = 0.0;
-            }
-            for (int q0 = 0; q0 < NQ3; q0 += QC) {
-                __syncthreads();
-                if (mass_only) {
-                    // phi alone, from one table of the 1-D factors per point
-                    // (3 (p+1) legendre_1d calls instead of 3 Np), multiplied
-                    // in basis_eval's order, and w phi_m once per (q, m): the
-                    // same values and sums as the full assembly, bit for bit
-                    constexpr int L1 = PD + 1;
-                    double* tleg = tdphi;               // [QC][3][L1]
-                    double* twphi = tdphi + QC * 3 * L1; // [QC][NP]
-                    for (int it = tid; it < QC * 3 * L1; it += ASM_THREADS) {
-                        const int qq = it / (3 * L1), r = it % (3 * L1), d = r / L1, deg = r % L1, q = q0 + qq;
-                        if (q < NQ3) {
-                            double pt[3], v, dv;
-                            tet_point(fk, A.ref, q, pt);
-                            legendre_1d(pt[d], deg, bb[2 * d], bb[2 * d + 1], &v, &dv);
-                            tleg[it] = v;
-                            if (r == 0) tw[qq] = A.ref->weitet3[q] * aj;
-                        }
-                    }
-                    __syncthreads();
-                    for (int it = tid; it < QC * NP; it += ASM_THREADS) {
-                        const int qq = it / NP, f = it % NP, q = q0 + qq;
-                        if (q < NQ3) {
-                            const int* bl = &A.ref->blist[f * 3];
-                            const double* tq = tleg + qq * 3 * L1;
-                            const double ph = tq[bl[0]] * tq[L1 + bl[1]] * tq[2 * L1 + bl[2]];
-                            tphi[qq * NP + f] = ph;
-                            twphi[qq * NP + f] = tw[qq] * ph;
-                        }
-                    }
-                    __syncthreads();
-                    const int nq = (NQ3 - q0) < QC ? (NQ3 - q0) : QC;
-#pragma unroll
-                    for (int u = 0; u < PPT; ++u) {
-                        const int pr = tid + u * ASM_THREADS;
-                        if (pr < D::NPAIR) {
-                            const int m = pr / NP, n = pr % NP;
-                            for (int qq = 0; qq < nq; ++qq) Mt[u] += twphi[qq * NP + m] * tphi[qq * NP + n];
-                        }
-                    }
-                    continue;
-                }
-                // basis_eval's 1-D factors (value, derivative) per point,
-                // coordinate and degree, then their products in its order:
-                // the same bits at 3 (p+1) legendre_1d calls per point
-                // instead of 3 Np
-                constexpr int L1 = PD + 1;
-                for (int it = tid; it < QC * 3 * L1; it += ASM_THREADS) {
-                    const int qq = it / (3 * L1), r = it % (3 * L1), d = r / L1, deg = r % L1, q = q0 + qq;
-                    if (q < NQ3) {
-                        double pt[3];
-                        tet_point(fk, A.ref, q, pt);
-                        legendre_1d(pt[d], deg, bb[2 * d], bb[2 * d + 1], &ttl[2 * it], &ttl[2 * it + 1]);
-                        if (r == 0) tw[qq] = A.ref->weitet3[q] * aj;
-                    }
-                }
-                __syncthreads();
-                for (int it = tid; it < QC * NP; it += ASM_THREADS) {
-                    const int qq = it / NP, f = it % NP, q = q0 + qq;
-                    if (q < NQ3) {
-                        const int* bl = &A.ref->blist[f * 3];
-                        const double* tq = ttl + 2 * qq * 3 * L1;
-                        const double vx = tq[2 * bl[0]], dx = tq[2 * bl[0] + 1];
-                        const double vy = tq[2 * (L1 + bl[1])], dy = tq[2 * (L1 + bl[1]) + 1];
-                        const double vz = tq[2 * (2 * L1 + bl[2])], dz = tq[2 * (2 * L1 + bl[2]) + 1];
-                        tphi[qq * NP + f] = vx * vy * vz;
-                        tdphi[(qq * 3 + 0) * NP + f] = dx * vy * vz;
-                        tdphi[(qq * 3 + 1) * NP + f] = vx * dy * vz;
-                        tdphi[(qq * 3 + 2) * NP + f] = vx * vy * dz;
-                    }
-                }
-                __syncthreads();
-                const int nq = (NQ3 - q0) < QC ? (NQ3 - q0) : QC;
-#pragma unroll
-                for (int u = 0; u < PPT; ++u) {
-                    const int pr = tid + u * ASM_THREADS;
-                    if (pr < D::NPAIR) {
-                        const int m = pr / NP, n = pr % NP;
-                        for (int qq = 0; qq < nq; ++qq) {
-                            const double w = tw[qq];
-                            const double a0 = w * tdphi[(qq * 3 + 0) * NP + m];
-                            const double a1 = w * tdphi[(qq * 3 + 1) * NP + m];
-                            const double a2 = w * tdphi[(qq * 3 + 2) * NP + m];
-                            const double b0 = tdphi[(qq * 3 + 0) * NP + n];
-                            const double b1 = tdphi[(qq * 3 + 1) * NP + n];
-                            const double b2 = tdphi[(qq * 3 + 2) * NP + n];
-                            G[u][0] += a0 * b0; G[u][1] += a0 * b1; G[u][2] += a0 * b2;
-                            G[u][3] += a1 * b0; G[u][4] += a1 * b1; G[u][5] += a1 * b2;
-                            G[u][6] += a2 * b0; G[u][7] += a2 * b1; G[u][8] += a2 * b2;
-                            Mt[u] += (w * tphi[qq * NP + m]) * tphi[qq * NP + n];
-                        }
-                    }
-                }
-            }
-            // fold V_t = lambda G_ij + mu G_ji + delta_ij mu tr G into the block
-#pragma unroll
-            for (int u = 0; u < PPT; ++u) {
-                const int pr = tid + u * ASM_THREADS;
-                if (pr < D::NPAIR) {
-                    const int m = pr / NP, n = pr % NP;
-                    const double tr = G[u][0] + G[u][4] + G[u][8];
-                    if (!mass_only) {
-#pragma unroll
-                        for (int i = 0; i < 3; ++i)
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) {
-                                double v = lam * G[u][i * 3 + j] + mu * G[u][j * 3 + i];
-                                if (i == j) v += mu * tr;
-                                acc[(i * NP + m) * ND + j * NP + n] += v;
-                            }
-                    }
-                    msum[u] += Mt[u];
-                    mrho[u] += Mt[u] * rho;
-                }
-            }
+    for (int u = 0; u < PPT; ++u) {
+        const int e = tid + u * T;
+        int n = 0;
+        while ((n + 1) * (n + 2) / 2 <= e) ++n;
+        pn[u] = n < NP ? n : NP - 1;
+        pm[u] = n < NP ? e - n * (n + 1) / 2 : 0;
+    }
+    // products of the 1-D factors at r0 points, in basis_eval's order
+    auto products = [&](int r0) {
+        for (int it = tid; it < r0 * NP; it += T) {
+            const int q = it / NP, f = it - q * NP;
+            const double* tq = tleg + q * 3 * L1;
+            const double ph = tq[der.deg[f][0]] * tq[L1 + der.deg[f][1]] * tq[2 * L1 + der.deg[f][2]];
+            tphi[it] = ph;
+            twphi[it] = tw[q] * ph;
         }
-        if (A.M != nullptr) {
+    };
+    // ---- mass moments of the sub-tetrahedra ----
+    double msum[PPT], mrho[PPT], mlam[PPT], mmu[PPT];
 #pragma unroll
-            for (int u = 0; u < PPT; ++u) {
-                const int pr = tid + u * ASM_THREADS;
-                if (pr < D::NPAIR) {
-                    A.M[(int64_t)P * D::NPAIR + pr] = mrho[u];
-                    A.Mm[(int64_t)P * D::NPAIR + pr] = msum[u];
-                }
+    for (int u = 0; u < PPT; ++u) msum[u] = mrho[u] = mlam[u] = mmu[u] = 0.0;
+    for (int kt = A.poly_ptr[P]; kt < A.poly_ptr[P + 1]; ++kt) {
+        const int t = A.poly_tets[kt];
+        const double* fk = &A.fk[t * 12];
+        const int mid = A.tet_mat[t];
+        const double rho = A.mat[mid * 3 + 0], lam = A.mat[mid * 3 + 1], mu = A.mat[mid * 3 + 2];
+        const double aj = fabs(A.jdet[t]);
+        double Mt[PPT];
+#pragma unroll
+        for (int u = 0; u < PPT; ++u) Mt[u] = 0.0;
+        for (int q0 = 0; q0 < NQ3; q0 += R) {
+            const int nq = (NQ3 - q0) < R ? (NQ3 - q0) : R;
+            __syncthreads();
+            for (int it = tid; it < nq * 3; it += T) {
+                const int qq = it / 3, d = it - qq * 3;
+                const double* nt = &A.ref->nodtet3[(q0 + qq) * 4];
+                double x = 0.0;
+                for (int l = 0; l < 4; ++l) x = x + fk[d * 4 + l] * nt[l];
+                legendre_vals<PD>(&box, d, x, tleg + it * L1);
+                if (d == 0) tw[qq] = A.ref->weitet3[q0 + qq] * aj;
+            }
+            __syncthreads();
+            products(nq);
+            __syncthreads();
+            for (int qq = 0; qq < nq; ++qq)
+#pragma unroll
+                for (int u = 0; u < PPT; ++u) Mt[u] += twphi[qq * NP + pm[u]] * tphi[qq * NP + pn[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < PPT; ++u) {
+            msum[u] += Mt[u];
+            mrho[u] += Mt[u] * rho;
+            if (WHICH != ASM_MASS) {
+                mlam[u] = fma(Mt[u], lam, mlam[u]);
+                mmu[u] = fma(Mt[u], mu, mmu[u]);
             }
         }
     }
-
-    if (mass_only) return;
-
-    // ---- face terms ----
-    {
-        double* fpt = tab;                        // [NQ2][3]
-        double* fphi = fpt + NQ2 * 3;             // [2][NQ2][NP]
-        double* fdphi = fphi + 2 * NQ2 * NP;      // [2][NQ2][3][NP]
-        double* ftl = fdphi + 2 * NQ2 * 3 * NP;   // [2][NQ2][3][p+1] (value, derivative) pairs
-        const double* bbp = &A.bbox[P * 6];
-        for (int64_t e = A.bf_ptr[k]; e < A.bf_ptr[k + 1]; ++e) {
-            const int code = A.bf[e];
-            const int t = code >> 2, f = code & 3;
-            const int E2 = A.neigh[code];
-            const bool dir = (E2 == LYMPH_BC_DIRI);
-            const int Qn = dir ? -1 : A.tet_poly[E2];
-            const double* fk = &A.fk[t * 12];
-            const int mid = A.tet_mat[t];
-            const double lam = A.mat[mid * 3 + 1], mu = A.mat[mid * 3 + 2];
-            const double n0 = A.nrm[t * 12 + f * 3 + 0], n1 = A.nrm[t * 12 + f * 3 + 1], n2 = A.nrm[t * 12 + f * 3 + 2];
-            const double ar = A.area[t * 4 + f];
-            const double Dbar = lam + 2 * mu;
-            const double hk1 = A.hk[P];
-            const double sigma = dir ? A.alpha * pdeg2 / hk1 * Dbar : A.alpha * pdeg2 / fmin(hk1, A.hk[Qn]) * Dbar;
-            const double cI = dir ? 1.0 : 0.5;
-            const int nside = self ? 1 : 2;
-            __syncthreads();
-            for (int q = tid; q < NQ2; q += ASM_THREADS) face_point(fk, A.ref, f, q, &fpt[q * 3]);
-            __syncthreads();
-            constexpr int L1 = PD + 1;
-            for (int it = tid; it < nside * NQ2 * 3 * L1; it += ASM_THREADS) {
-                const int s = it / (NQ2 * 3 * L1), rem = it % (NQ2 * 3 * L1), q = rem / (3 * L1);
-                const int d = (rem % (3 * L1)) / L1, deg = rem % L1;
-                const double* bb = (s == 0) ? bbp : &A.bbox[Qn * 6];
-                legendre_1d(fpt[q * 3 + d], deg, bb[2 * d], bb[2 * d + 1], &ftl[2 * it], &ftl[2 * it + 1]);
-            }
-            __syncthreads();
-            for (int it = tid; it < nside * NQ2 * NP; it += ASM_THREADS) {
-                const int s = it / (NQ2 * NP), rem = it % (NQ2 * NP), q = rem / NP, fb = rem % NP;
-                const int* bl = &A.ref->blist[fb * 3];
-                const double* tq = ftl + 2 * (s * NQ2 + q) * 3 * L1;
-                const double vx = tq[2 * bl[0]], dx = tq[2 * bl[0] + 1];
-                const double vy = tq[2 * (L1 + bl[1])], dy = tq[2 * (L1 + bl[1]) + 1];
-                const double vz = tq[2 * (2 * L1 + bl[2])], dz = tq[2 * (2 * L1 + bl[2]) + 1];
-                fphi[(s * NQ2 + q) * NP + fb] = vx * vy * vz;
-                fdphi[((s * NQ2 + q) * 3 + 0) * NP + fb] = dx * vy * vz;
-                fdphi[((s * NQ2 + q) * 3 + 1) * NP + fb] = vx * dy * vz;
-                fdphi[((s * NQ2 + q) * 3 + 2) * NP + fb] = vx * vy * dz;
-            }
-            __syncthreads();
-            const double nv[3] = {n0, n1, n2};
-            const double T00 = fabs(n0) * fabs(n0) + 0.5 * (fabs(n1) * fabs(n1)) + 0.5 * (fabs(n2) * fabs(n2));
-            const double T11 = fabs(n1) * fabs(n1) + 0.5 * (fabs(n0) * fabs(n0)) + 0.5 * (fabs(n2) * fabs(n2));
-            const double T22 = fabs(n2) * fabs(n2) + 0.5 * (fabs(n0) * fabs(n0)) + 0.5 * (fabs(n1) * fabs(n1));
-            const int sb = self ? 0 : 1;  // side of the trial functions (column polyhedron)
 #pragma unroll
-            for (int u = 0; u < PPT; ++u) {
-                const int pr = tid + u * ASM_THREADS;
-                if (pr >= D::NPAIR) continue;
-                const int a = pr / NP, b = pr % NP;
-                // Pab = sum W phi+_a phi^s_b ; H_k = sum W d_k phi+_a phi^s_b ;
-                // HT_k = sum W phi+_a d_k phi^s_b
-                double Pab = 0, H0 = 0, H1 = 0, H2 = 0, T0 = 0, T1 = 0, T2 = 0;
-                for (int q = 0; q < NQ2; ++q) {
-                    const double W = A.ref->weitria2[q] * ar;
-                    const double pa = fphi[q * NP + a];
-                    const double pb = fphi[(sb * NQ2 + q) * NP + b];
-                    const double wa = W * pa, wb = W * pb;
-                    Pab += wa * pb;
-                    H0 += wb * fdphi[(q * 3 + 0) * NP + a];
-                    H1 += wb * fdphi[(q * 3 + 1) * NP + a];
-                    H2 += wb * fdphi[(q * 3 + 2) * NP + a];
-                    T0 += wa * fdphi[((sb * NQ2 + q) * 3 + 0) * NP + b];
-                    T1 += wa * fdphi[((sb * NQ2 + q) * 3 + 1) * NP + b];
-                    T2 += wa * fdphi[((sb * NQ2 + q) * 3 + 2) * NP + b];
+    for (int u = 0; u < PPT; ++u) {
+        const int e = tid + u * T;
+        if (e < NS) {
+            if (A.M != nullptr) {
+                double* M = A.M + (int64_t)P * D::NPAIR;
+                double* Mm = A.Mm + (int64_t)P * D::NPAIR;
+                M[pm[u] * NP + pn[u]] = M[pn[u] * NP + pm[u]] = mrho[u];
+                Mm[pm[u] * NP + pn[u]] = Mm[pn[u] * NP + pm[u]] = msum[u];
+            }
+            if (WHICH != ASM_MASS) {
+                mats[e] = mlam[u];
+                mats[NS + e] = mmu[u];
+            }
+        }
+    }
+    if constexpr (WHICH != ASM_MASS) {
+        // ---- face moments ----
+        const int64_t k = A.row_ptr[P];   // the self block comes first in its row
+        double acc[PPT][FACE_F];
+#pragma unroll
+        for (int u = 0; u < PPT; ++u)
+#pragma unroll
+            for (int j = 0; j < FACE_F; ++j) acc[u][j] = 0.0;
+        const int64_t e0 = A.bf_ptr[k], e1 = A.bf_ptr[k + 1];
+        for (int64_t eb = e0; eb < e1; eb += FB) {
+            const int nf = (int)((e1 - eb) < FB ? (e1 - eb) : FB);
+            __syncthreads();
+            for (int it = tid; it < nf * 12; it += T) {
+                const int fi = it / 12, jl = it - fi * 12, code = A.bf[eb + fi];
+                fmap[it] = face_map(&A.fk[(code >> 2) * 12], A.ref, code & 3, jl / 4, jl & 3);
+            }
+            for (int fi = tid; fi < nf; fi += T) {
+                const int code = A.bf[eb + fi], e2 = A.neigh[code];
+                const bool dir = e2 == LYMPH_BC_DIRI;
+                face_factors(A, code, P, dir ? -1 : A.tet_poly[e2], dir ? 1.0 : 0.5, (double)(PD * PD), ffac + fi * FACE_F);
+            }
+            __syncthreads();
+            for (int it = tid; it < nf * NQ2 * 3; it += T) {
+                const int qq = it / 3, d = it - qq * 3, fi = qq / NQ2, q = qq - fi * NQ2;
+                const double* cm = fmap + fi * 12 + d * 4;
+                const double* nt = &A.ref->nodtria2[q * 4];
+                double x = 0.0;
+                for (int l = 0; l < 4; ++l) x = x + cm[l] * nt[l];
+                legendre_vals<PD>(&box, d, x, tleg + it * L1);
+                if (d == 0) tw[qq] = A.ref->weitria2[q] * A.area[A.bf[eb + fi]];
+            }
+            __syncthreads();
+            products(nf * NQ2);
+            __syncthreads();
+            for (int fi = 0; fi < nf; ++fi) {
+                double p[PPT];
+#pragma unroll
+                for (int u = 0; u < PPT; ++u) p[u] = 0.0;
+                for (int q = fi * NQ2; q < (fi + 1) * NQ2; ++q)
+#pragma unroll
+                    for (int u = 0; u < PPT; ++u) p[u] = fma(twphi[q * NP + pm[u]], tphi[q * NP + pn[u]], p[u]);
+#pragma unroll
+                for (int u = 0; u < PPT; ++u)
+#pragma unroll
+                    for (int j = (WHICH == ASM_ADG ? 6 : 0); j < FACE_F; ++j)
+                        acc[u][j] = fma(ffac[fi * FACE_F + j], p[u], acc[u][j]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PPT; ++u) {
+            const int e = tid + u * T;
+            if (e < NS)
+#pragma unroll
+                for (int j = (WHICH == ASM_ADG ? 6 : 0); j < FACE_F; ++j) mats[(2 + j) * NS + e] = acc[u][j];
+        }
+        __syncthreads();
+        // ---- the block from the moments, written column-major ----
+        const double* ML = mats;
+        const double* MM = mats + NS;
+        const double* PL = mats + 2 * NS;    // [3][NS]
+        const double* PM = mats + 5 * NS;    // [3][NS]
+        const double* SP = mats + 8 * NS;    // [6][NS]
+        auto sym = [](int a, int b) { return a <= b ? b * (b + 1) / 2 + a : a * (a + 1) / 2 + b; };
+        double* o = A.out + k * ND * ND;
+        for (int pr = tid; pr < D::NPAIR; pr += T) {
+            const int b = pr / NP, a = pr - b * NP;
+            int ia[3][2], ib[3][2];
+            double wa[3][2], wb[3][2];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    ia[d][t] = der.idx[a][d][t];
+                    ib[d][t] = der.idx[b][d][t];
+                    wa[d][t] = der_weight(der.deg[a][d], t) / box.hb[d];
+                    wb[d][t] = der_weight(der.deg[b][d], t) / box.hb[d];
                 }
-                const double H[3] = {H0, H1, H2}, HT[3] = {T0, T1, T2};
-                const double nH = n0 * H0 + n1 * H1 + n2 * H2;
-                const double nHT = n0 * T0 + n1 * T1 + n2 * T2;
+            double V[3][3], tr = 0.0;        // lambda D_i M D_j^T + mu D_j M D_i^T
+            double Gm[3][3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    double gl = 0.0, gm = 0.0;
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const double w = wa[i][t] * wb[j][s];
+                            if (w != 0.0) {
+                                const int x = sym(ia[i][t], ib[j][s]);
+                                gl = fma(w, ML[x], gl);
+                                gm = fma(w, MM[x], gm);
+                            }
+                        }
+                    V[i][j] = gl;
+                    Gm[i][j] = gm;
+                }
+            tr = Gm[0][0] + Gm[1][1] + Gm[2][2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) V[i][j] += Gm[j][i] + (i == j ? tr : 0.0);
+            const int e = sym(a, b);
+            const double s01 = SP[3 * NS + e], s02 = SP[4 * NS + e], s12 = SP[5 * NS + e];
+            V[0][0] += SP[e]; V[1][1] += SP[NS + e]; V[2][2] += SP[2 * NS + e];
+            V[0][1] += s01; V[1][0] += s01;
+            V[0][2] += s02; V[2][0] += s02;
+            V[1][2] += s12; V[2][1] += s12;
+            if (WHICH == ASM_K) {
+                // theta I(i,j,a,b) - I(j,i,b,a), I(i,j) = D_i PL_j + D_j PM_i + delta_ij sum_k D_k PM_k
+                double tL = 0.0, tR = 0.0;
+                double L[3][3], Rr[3][3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) L[i][j] = Rr[i][j] = 0.0;
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        if (wa[i][t] != 0.0) {
+                            const int x = sym(ia[i][t], b);
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) {
+                                L[i][j] = fma(wa[i][t], PL[j * NS + x], L[i][j]);
+                                L[j][i] = fma(wa[i][t], PM[j * NS + x], L[j][i]);
+                            }
+                            tL = fma(wa[i][t], PM[i * NS + x], tL);
+                        }
+                        if (wb[i][t] != 0.0) {
+                            const int x = sym(a, ib[i][t]);
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) {
+                                Rr[j][i] = fma(wb[i][t], PL[j * NS + x], Rr[j][i]);
+                                Rr[i][j] = fma(wb[i][t], PM[j * NS + x], Rr[i][j]);
+                            }
+                            tR = fma(wb[i][t], PM[i * NS + x], tR);
+                        }
+                    }
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
 #pragma unroll
                     for (int j = 0; j < 3; ++j) {
-                        const double Tij = (i == j) ? (i == 0 ? T00 : (i == 1 ? T11 : T22)) : 0.5 * nv[i] * nv[j];
-                        const double S = sigma * Tij * Pab;
-                        double v;
-                        if (self) {
-                            if (A.which == LYMPH_BLOCKS_ADG) {
-                                v = S;
-                            } else {
-                                // S_E1 + theta I_E1(i,j,a,b) - I_E1(j,i,b,a)
-                                double I = lam * nv[j] * H[i] + mu * nv[i] * H[j] + (i == j ? mu * nH : 0.0);
-                                double IT = lam * nv[i] * HT[j] + mu * nv[j] * HT[i] + (i == j ? mu * nHT : 0.0);
-                                v = S + A.theta * cI * I - cI * IT;
-                            }
-                        } else {
-                            if (A.which == LYMPH_BLOCKS_ADG) {
-                                v = -S;
-                            } else {
-                                // theta I_E2 + S_E2 - IT_E2 (IT_E2 carries the reference's index
-                                // order, assemble_element.f90:610-616)
-                                double I = lam * nv[j] * H[i] + mu * nv[i] * H[j] + (i == j ? mu * nH : 0.0);
-                                double IT = lam * nv[j] * HT[i] + mu * nv[i] * HT[j] + (i == j ? mu * nHT : 0.0);
-                                v = -0.5 * A.theta * I - S - 0.5 * IT;
-                            }
-                        }
-                        acc[(i * NP + a) * ND + j * NP + b] += v;
+                        double l = L[i][j], r = Rr[i][j];
+                        if (i == j) { l += tL; r += tR; }
+                        V[i][j] += A.theta * l - r;
                     }
             }
-        }
-    }
-    __syncthreads();
-    // write the block column-major (entry (r,c) at c*ND + r)
-    const int64_t base = slot * A.out_stride;
-    if (A.out_fp32) {
-        float* o = (float*)A.out;
-        for (int i = tid; i < ND * ND; i += ASM_THREADS) {
-            const int c = i / ND, r = i % ND;
-            o[base + i] = (float)acc[r * ND + c];
-        }
-    } else {
-        double* o = (double*)A.out;
-        for (int i = tid; i < ND * ND; i += ASM_THREADS) {
-            const int c = i / ND, r = i % ND;
-            o[base + i] = acc[r * ND + c];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) o[(int64_t)(j * NP + b) * ND + i * NP + a] = V[i][j];
         }
     }
 }
 
-template <int PD> size_t asm_smem() {
+// One neighbour block K_PQ = -theta/2 I - S - IT/2 per CTA (or the DG norm's
+// -S), from the moments P(a, b) = sum_q W phi^P_a phi^Q_b of the triangles P
+// shares with Q, as in k_assemble_self: 25 multiply-adds per triangle and
+// pair for the moment (p = 4), 12 for its weighted sums, and the derivative
+// expansion once per block,
+//     I(i,j)  = D_i PL_j + D_j PM_i + delta_ij sum_k D_k PM_k,
+//     IT(i,j) = PL_j D_i^T + PM_i D_j^T + delta_ij sum_k PM_k D_k^T
+// (IT carries the reference's index order, assemble_element.f90:610-616),
+// PL_j = sum lambda n_j P, PM_j = sum mu n_j P, D on the left in P's basis and
+// on the right in Q's.
+template <int PD, int WHICH>
+__global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_nb(AsmArgs A) {
     using D = Deg<PD>;
-    constexpr int QC = D::NQ3 < 32 ? D::NQ3 : 32;
-    size_t vol = (size_t)QC * D::NP * 4 + QC + (size_t)QC * 3 * (PD + 1) * 2;
-    size_t face = (size_t)D::NQ2 * 3 + 2 * (size_t)D::NQ2 * D::NP * 4 + 2 * (size_t)D::NQ2 * 3 * (PD + 1) * 2;
-    return sizeof(double) * ((size_t)D::ND * D::ND + (vol > face ? vol : face));
+    using S = AsmShape<PD>;
+    constexpr int NP = D::NP, ND = D::ND, NQ2 = D::NQ2, NPAIR = D::NPAIR, T = S::TN, PPT = S::PPTN, L1 = S::L1;
+    extern __shared__ double sm[];
+    double* PL = sm;                                     // [3][NPAIR], pair (a, b) at b NP + a
+    double* PM = PL + (WHICH == ASM_K ? 3 * NPAIR : 0);  // [3][NPAIR]
+    double* fphi = PM + (WHICH == ASM_K ? 3 * NPAIR : 0);   // [2][NQ2][NP]; Q's side carries W
+    double* tleg = fphi + 2 * NQ2 * NP;                  // [2][NQ2][3][L1]
+    double* ffac = tleg + 2 * NQ2 * 3 * L1;              // [FACE_F]
+    double* fmap = ffac + FACE_F;                        // [3][4]
+    __shared__ BoxC box[2];
+    const int tid = threadIdx.x;
+    const int64_t k = A.block0 + blockIdx.x;
+    const int P = A.blk_row[k], Q = A.col[k];
+    if (P == Q) return;                                  // self blocks: k_assemble_self
+    __shared__ DerTab<PD> der;
+    load_der<PD>(&der);
+    if (tid < 6) box_consts(&A.bbox[(tid < 3 ? P : Q) * 6], &box[tid / 3], tid % 3);
+    double SP[PPT][6];
+#pragma unroll
+    for (int u = 0; u < PPT; ++u)
+#pragma unroll
+        for (int j = 0; j < 6; ++j) SP[u][j] = 0.0;
+    const int64_t e0 = A.bf_ptr[k], e1 = A.bf_ptr[k + 1];
+    for (int64_t e = e0; e < e1; ++e) {
+        const int code = A.bf[e];
+        __syncthreads();
+        if (tid < 12) fmap[tid] = face_map(&A.fk[(code >> 2) * 12], A.ref, code & 3, tid / 4, tid & 3);
+        if (tid == T - 1) face_factors(A, code, P, Q, 1.0, (double)(PD * PD), ffac);
+        __syncthreads();
+        for (int it = tid; it < 2 * NQ2 * 3; it += T) {
+            const int s = it / (NQ2 * 3), r = it - s * NQ2 * 3, q = r / 3, d = r - q * 3;
+            const double* cm = fmap + d * 4;
+            const double* nt = &A.ref->nodtria2[q * 4];
+            double x = 0.0;
+            for (int l = 0; l < 4; ++l) x = x + cm[l] * nt[l];
+            legendre_vals<PD>(&box[s], d, x, tleg + it * L1);
+        }
+        __syncthreads();
+        const double ar = A.area[code];
+        for (int it = tid; it < 2 * NQ2 * NP; it += T) {
+            const int s = it / (NQ2 * NP), r = it - s * NQ2 * NP, q = r / NP, f = r - q * NP;
+            const double* tq = tleg + (s * NQ2 + q) * 3 * L1;
+            double ph = tq[der.deg[f][0]] * tq[L1 + der.deg[f][1]] * tq[2 * L1 + der.deg[f][2]];
+            if (s == 1) ph *= A.ref->weitria2[q] * ar;
+            fphi[it] = ph;
+        }
+        __syncthreads();
+        double p[PPT];
+#pragma unroll
+        for (int u = 0; u < PPT; ++u) p[u] = 0.0;
+        int ra[PPT], rb[PPT];
+#pragma unroll
+        for (int u = 0; u < PPT; ++u) {
+            const int pr = tid + u * T < NPAIR ? tid + u * T : NPAIR - 1;
+            rb[u] = pr / NP;
+            ra[u] = pr - rb[u] * NP;
+        }
+        for (int q = 0; q < NQ2; ++q)
+#pragma unroll
+            for (int u = 0; u < PPT; ++u) p[u] = fma(fphi[q * NP + ra[u]], fphi[(NQ2 + q) * NP + rb[u]], p[u]);
+#pragma unroll
+        for (int u = 0; u < PPT; ++u) {
+            const int pr = tid + u * T;
+            if (pr >= NPAIR) continue;
+            if (WHICH == ASM_K) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    // each thread owns its pairs, so the sums over the triangles need no barrier
+                    PL[j * NPAIR + pr] = e == e0 ? ffac[j] * p[u] : fma(ffac[j], p[u], PL[j * NPAIR + pr]);
+                    PM[j * NPAIR + pr] = e == e0 ? ffac[3 + j] * p[u] : fma(ffac[3 + j], p[u], PM[j * NPAIR + pr]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 6; ++j) SP[u][j] = fma(ffac[6 + j], p[u], SP[u][j]);
+        }
+    }
+    __syncthreads();
+    double* o = A.out + k * ND * ND;
+    const double mth = -0.5 * A.theta;
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+        const int pr = tid + u * T;
+        if (pr >= NPAIR) continue;
+        const int b = pr / NP, a = pr - b * NP;
+        double V[3][3];
+        V[0][0] = -SP[u][0]; V[1][1] = -SP[u][1]; V[2][2] = -SP[u][2];
+        V[0][1] = V[1][0] = -SP[u][3];
+        V[0][2] = V[2][0] = -SP[u][4];
+        V[1][2] = V[2][1] = -SP[u][5];
+        if (WHICH == ASM_K) {
+            double tr = 0.0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const double w = der_weight(der.deg[a][i], t);
+                    if (w != 0.0) {
+                        const double wl = mth * (w / box[0].hb[i]);
+                        const int x = b * NP + der.idx[a][i][t];
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            V[i][j] = fma(wl, PL[j * NPAIR + x], V[i][j]);
+                            V[j][i] = fma(wl, PM[j * NPAIR + x], V[j][i]);
+                        }
+                        tr = fma(wl, PM[i * NPAIR + x], tr);
+                    }
+                    const double w2 = der_weight(der.deg[b][i], t);
+                    if (w2 != 0.0) {
+                        const double wr = -0.5 * (w2 / box[1].hb[i]);
+                        const int x = der.idx[b][i][t] * NP + a;
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            V[i][j] = fma(wr, PL[j * NPAIR + x], V[i][j]);
+                            V[j][i] = fma(wr, PM[j * NPAIR + x], V[j][i]);
+                        }
+                        tr = fma(wr, PM[i * NPAIR + x], tr);
+                    }
+                }
+            V[0][0] += tr; V[1][1] += tr; V[2][2] += tr;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) o[(int64_t)(j * NP + b) * ND + i * NP + a] = V[i][j];
+    }
+}
+
+template <int PD, int WHICH> size_t asm_self_smem() {
+    using S = AsmShape<PD>;
+    constexpr int nmat = WHICH == ASM_MASS ? 0 : 14;
+    return sizeof(double) * ((size_t)nmat * S::NS + 2 * (size_t)S::R * S::NP + (size_t)S::R * 3 * S::L1 + S::R +
+                             S::FB * (FACE_F + 12));
+}
+template <int PD, int WHICH> size_t asm_nb_smem() {
+    using S = AsmShape<PD>;
+    constexpr int NQ2 = Deg<PD>::NQ2;
+    return sizeof(double) * ((WHICH == ASM_K ? 6 * (size_t)Deg<PD>::NPAIR : 0) + 2 * (size_t)NQ2 * S::NP +
+                             2 * (size_t)NQ2 * 3 * S::L1 + FACE_F + 12);
 }
 
 // cholesky (vet_mat_operations.f90:84-120) of the NP x NP matrix of every
@@ -903,29 +1112,44 @@ __global__ void k_double_couple(int Np, int nq3, int t, int P, const double* __r
     for (int i = 0; i < 3; ++i) rhs[base + i * Np + m] += acc[i];
 }
 
-template <int PD>
-int launch_assemble(lymph_ctx* c, int which, void* out, int out_fp32, bool write_mass, const int64_t* list,
-                    int64_t n_list, int64_t out_stride) {
-    size_t smem = asm_smem<PD>();
-    LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_assemble<PD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+template <int PD, int WHICH>
+int launch_assemble(lymph_ctx* c, double* out, bool write_mass) {
     AsmArgs A;
-    A.blk_row = c->d_blk_row; A.col = c->d_col; A.bf_ptr = c->d_bf_ptr; A.bf = c->d_bf;
+    A.row_ptr = c->d_row_ptr; A.blk_row = c->d_blk_row; A.col = c->d_col; A.bf_ptr = c->d_bf_ptr; A.bf = c->d_bf;
     A.poly_ptr = c->d_poly_ptr; A.poly_tets = c->d_poly_tets; A.tet_poly = c->d_tet_poly; A.tet_mat = c->d_tet_mat;
     A.neigh = c->d_neigh; A.mat = c->d_mat; A.fk = c->d_fk; A.jdet = c->d_jdet; A.nrm = c->d_normal; A.area = c->d_area;
-    A.bbox = c->d_bbox; A.hk = c->d_hk; A.ref = c->d_ref; A.alpha = c->alpha; A.theta = c->theta;
-    A.which = which; A.out_fp32 = out_fp32; A.out = out;
+    A.bbox = c->d_bbox; A.hk = c->d_hk; A.ref = c->d_ref; A.alpha = c->alpha; A.theta = c->theta; A.out = out;
     A.M = write_mass ? c->d_M : nullptr; A.Mm = write_mass ? c->d_Mm : nullptr;
-    A.list = list; A.out_stride = out_stride;
-    const int64_t n = list ? n_list : c->n_blocks;
-    const int64_t chunk = 1 << 20;
-    for (int64_t b0 = 0; b0 < n; b0 += chunk) {
-        A.block0 = b0;
-        int64_t nb = n - b0 < chunk ? n - b0 : chunk;
-        k_assemble<PD><<<(unsigned)nb, ASM_THREADS, smem, c->stream>>>(A);
-        c->launches++;
-        LYMPH_CUDA_TRY(cudaGetLastError());
+    A.block0 = 0;
+    const size_t sself = asm_self_smem<PD, WHICH>();
+    LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_assemble_self<PD, WHICH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sself));
+    k_assemble_self<PD, WHICH><<<c->n_poly, AsmShape<PD>::T, sself, c->stream>>>(A);
+    c->launches++;
+    LYMPH_CUDA_TRY(cudaGetLastError());
+    if constexpr (WHICH != ASM_MASS) {
+        const size_t snb = asm_nb_smem<PD, WHICH>();
+        LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_assemble_nb<PD, WHICH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)snb));
+        const int64_t chunk = 1 << 20;
+        for (int64_t b0 = 0; b0 < c->n_blocks; b0 += chunk) {
+            A.block0 = b0;
+            const int64_t nb = c->n_blocks - b0 < chunk ? c->n_blocks - b0 : chunk;
+            k_assemble_nb<PD, WHICH><<<(unsigned)nb, AsmShape<PD>::TN, snb, c->stream>>>(A);
+            c->launches++;
+            LYMPH_CUDA_TRY(cudaGetLastError());
+        }
     }
     return LYMPH_OK;
+}
+
+template <int WHICH>
+int assemble_degree(lymph_ctx* c, double* out, bool write_mass) {
+    switch (c->p) {
+        case 1: return launch_assemble<1, WHICH>(c, out, write_mass);
+        case 2: return launch_assemble<2, WHICH>(c, out, write_mass);
+        case 3: return launch_assemble<3, WHICH>(c, out, write_mass);
+        case 4: return launch_assemble<4, WHICH>(c, out, write_mass);
+        default: lymph_set_error("degree not supported on the device"); return LYMPH_ERR_INVALID;
+    }
 }
 
 template <int PD>
@@ -967,29 +1191,14 @@ int lymph_dev_geometry(lymph_ctx* c) {
     return LYMPH_OK;
 }
 
-// Blocks list[0..n_list) (all blocks in order when list is null) into
-// consecutive output slots out_stride elements apart.
-int lymph_dev_assemble_list(lymph_ctx* c, int which, void* out, int out_fp32, bool write_mass, const int64_t* list,
-                            int64_t n_list, int64_t out_stride) {
-    switch (c->p) {
-        case 1: return launch_assemble<1>(c, which, out, out_fp32, write_mass, list, n_list, out_stride);
-        case 2: return launch_assemble<2>(c, which, out, out_fp32, write_mass, list, n_list, out_stride);
-        case 3: return launch_assemble<3>(c, which, out, out_fp32, write_mass, list, n_list, out_stride);
-        case 4: return launch_assemble<4>(c, which, out, out_fp32, write_mass, list, n_list, out_stride);
-        default: lymph_set_error("degree not supported on the device"); return LYMPH_ERR_INVALID;
-    }
-}
+// The rho-weighted and the plain mass matrix of every polyhedron (what the
+// mixed operators need of the FP64 assembly).
+int lymph_dev_mass(lymph_ctx* c) { return assemble_degree<ASM_MASS>(c, nullptr, true); }
 
-// The rho-weighted and the plain mass matrix of every polyhedron (the
-// self-block CTAs of k_assemble with the stiffness and face terms skipped:
-// the same sums in the same order, so M and Mm have the bits a full assembly
-// gives them).
-int lymph_dev_mass(lymph_ctx* c, const int64_t* self_list) {
-    return lymph_dev_assemble_list(c, ASM_MASS_ONLY, nullptr, 0, true, self_list, c->n_poly, 0);
-}
-
-int lymph_dev_assemble(lymph_ctx* c, int which, void* out, int out_fp32, bool write_mass) {
-    return lymph_dev_assemble_list(c, which, out, out_fp32, write_mass, nullptr, 0, (int64_t)c->nd * c->nd);
+// Every FP64 block of the operator (LYMPH_BLOCKS_K) or of the DG norm
+// (LYMPH_BLOCKS_ADG) into out; with write_mass also the mass matrices.
+int lymph_dev_assemble(lymph_ctx* c, int which, double* out, bool write_mass) {
+    return which == LYMPH_BLOCKS_ADG ? assemble_degree<ASM_ADG>(c, out, write_mass) : assemble_degree<ASM_K>(c, out, write_mass);
 }
 
 int lymph_dev_cholesky(lymph_ctx* c) {

@@ -1,0 +1,53 @@
+"""The FP64 block assembly from mass moments (k_assemble_self, k_assemble_nb)
+at the forms the shared parity meshes do not reach: theta = 0 and 1, and a
+polyhedron of 162 tetrahedra and 108 shared triangles (many rounds of the
+tetrahedron and face tables).  Every block of K and A_dg against the oracle,
+normwise <= 1e-12 over the mesh (the bar of the other set-up data: sums of at
+most ~1e4 products of O(1) condition, eps * 1e4 = 2e-12 worst case, ~1e-14
+expected), and M exactly symmetric.
+"""
+import math
+
+import numpy as np
+import pytest
+
+from lymph3d_apsc_gb300 import MatrixFree, _lib, mesh as M
+from oracle.oracle_py import Oracle
+from test_gpu_mf import _big_polyhedron_mesh
+
+pytestmark = pytest.mark.gpu
+
+
+def _blocks_close(m, p, theta):
+    o = Oracle(m, p, 1e-3, theta=theta)
+    o.make_matrices()
+    with MatrixFree(m, p, 1e-3, theta=theta) as g:
+        g.MAKE_MATRICES_FREE()
+        rp, col = g.pattern()
+        for which in (_lib.BLOCKS_K, _lib.BLOCKS_ADG):
+            vals, ref = g.blocks(which), o.block_dict(which)
+            num = den = 0.0
+            for P in range(g.n_poly):
+                for k in range(rp[P], rp[P + 1]):
+                    r = ref[(P, int(col[k]))]
+                    num += float(np.sum((vals[k] - r) ** 2))
+                    den += float(np.sum(r ** 2))
+            assert math.sqrt(num / den) <= 1e-12, (which, math.sqrt(num / den))
+        for which in (0, 1):
+            mm = g.mass(which)
+            assert np.array_equal(mm, mm.transpose(0, 2, 1))
+    o.close()
+
+
+@pytest.mark.parametrize("theta", [0.0, 1.0])
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+def test_blocks_of_other_penalty_forms(require_gpu, p, theta):
+    m = M.cube(2, bc="reference", agglomeration="bfs", seed=3, group=(4, 12), jitter=0.2)
+    mats = M.lognormal_materials(m.n_poly, seed=3)
+    m.mat, m.tet_mat = mats, m.tet_poly.copy()
+    _blocks_close(m, p, theta)
+
+
+@pytest.mark.parametrize("p", [1, 2, 4])
+def test_blocks_of_a_large_polyhedron(require_gpu, p):
+    _blocks_close(_big_polyhedron_mesh(), p, -1.0)
