@@ -108,16 +108,6 @@ __device__ inline void face_point(const double* fk, const RefTables* ref, int f,
     }
 }
 
-// Physical point of tetrahedron quadrature node q (basis, :471-479).
-__device__ inline void tet_point(const double* fk, const RefTables* ref, int q, double pt[3]) {
-    const double* nt = &ref->nodtet3[q * 4];
-    for (int j = 0; j < 3; ++j) {
-        double s = 0.0;
-        for (int l = 0; l < 4; ++l) s = s + fk[j * 4 + l] * nt[l];
-        pt[j] = s;
-    }
-}
-
 // Shape of the assembly CTAs per degree.  The moments of a self block are
 // symmetric, so a CTA owns the NS = Np (Np + 1) / 2 pairs a <= b (packed:
 // pair (a, b) at b (b + 1) / 2 + a); a neighbour block owns all Np^2 pairs.
@@ -734,32 +724,36 @@ __global__ void k_mass_inverse(int n_poly, int NP, const double* __restrict__ R,
 }
 
 // ---- data functions (problem_data_and_properties.f90) ----
-__device__ inline void dev_u_space(const double p[3], double r[3]) {
-    const double PI = 3.141592653589793;
-    r[0] = cos(PI * p[0]) * sin(PI * p[1]) * sin(PI * p[2]);
-    r[1] = sin(PI * p[0]) * cos(PI * p[1]) * sin(PI * p[2]);
-    r[2] = sin(PI * p[0]) * sin(PI * p[1]) * cos(PI * p[2]);
+// Each takes sn[d] = sin(pi x_d), cs[d] = cos(pi x_d) of the point, formed
+// once per point and coordinate; the products keep the reference's order.
+constexpr double DATA_PI = 3.141592653589793;
+
+__device__ inline void dev_u_space(const double* sn, const double* cs, double r[3]) {
+    r[0] = cs[0] * sn[1] * sn[2];
+    r[1] = sn[0] * cs[1] * sn[2];
+    r[2] = sn[0] * sn[1] * cs[2];
 }
 
-__device__ inline void dev_forcing(int id, double lam, double mu, const double p[3], double rho, double r[3]) {
-    const double PI = 3.141592653589793;
+__device__ inline void dev_forcing(int id, double lam, double mu, double rho, const double* sn, const double* cs,
+                                   double r[3]) {
+    const double PI = DATA_PI;
     if (id == LYMPH_F_TIME) {
         const double c = (-2.0 * rho + 3.0 * (lam + 2.0 * mu)) * PI * PI;
-        r[0] = c * cos(PI * p[0]) * sin(PI * p[1]) * sin(PI * p[2]);
-        r[1] = c * sin(PI * p[0]) * cos(PI * p[1]) * sin(PI * p[2]);
-        r[2] = c * sin(PI * p[0]) * sin(PI * p[1]) * cos(PI * p[2]);
+        r[0] = c * cs[0] * sn[1] * sn[2];
+        r[1] = c * sn[0] * cs[1] * sn[2];
+        r[2] = c * sn[0] * sn[1] * cs[2];
     } else if (id == LYMPH_F_STAT) {
-        r[0] = 3 * PI * PI * cos(PI * p[0]) * sin(PI * p[1]) * sin(PI * p[2]) * (lam + 2 * mu);
-        r[1] = 3 * PI * PI * cos(PI * p[1]) * sin(PI * p[0]) * sin(PI * p[2]) * (lam + 2 * mu);
-        r[2] = 3 * PI * PI * cos(PI * p[2]) * sin(PI * p[0]) * sin(PI * p[1]) * (lam + 2 * mu);
+        r[0] = 3 * PI * PI * cs[0] * sn[1] * sn[2] * (lam + 2 * mu);
+        r[1] = 3 * PI * PI * cs[1] * sn[0] * sn[2] * (lam + 2 * mu);
+        r[2] = 3 * PI * PI * cs[2] * sn[0] * sn[1] * (lam + 2 * mu);
     } else {
         r[0] = r[1] = r[2] = 0.0;
     }
 }
 
-__device__ inline void dev_dirichlet(int id, const double p[3], int tag, double r[3]) {
+__device__ inline void dev_dirichlet(int id, int tag, const double* sn, const double* cs, double r[3]) {
     if (id == LYMPH_GD) {
-        if (tag == 1 || tag == 2 || tag == 3) dev_u_space(p, r);
+        if (tag == 1 || tag == 2 || tag == 3) dev_u_space(sn, cs, r);
         else r[0] = r[1] = r[2] = 0.0;
     } else if (id == LYMPH_GD_STAT) {
         r[0] = r[1] = r[2] = 2.0;
@@ -768,29 +762,29 @@ __device__ inline void dev_dirichlet(int id, const double p[3], int tag, double 
     }
 }
 
-__device__ inline void dev_neumann(int id, double lam, double mu, const double n[3], const double p[3], int tag,
-                                   double r[3]) {
-    const double PI = 3.141592653589793;
+__device__ inline void dev_neumann(int id, double lam, double mu, const double n[3], int tag, const double* sn,
+                                   const double* cs, double r[3]) {
+    const double PI = DATA_PI;
     r[0] = r[1] = r[2] = 0.0;
     if (id != LYMPH_GN || !(tag == 1 || tag == 2 || tag == 3)) return;
     double s[3][3];
-    const double d = -PI * sin(PI * p[0]) * sin(PI * p[1]) * sin(PI * p[2]) * (3.0 * lam + 2.0 * mu);
+    const double d = -PI * sn[0] * sn[1] * sn[2] * (3.0 * lam + 2.0 * mu);
     s[0][0] = d; s[1][1] = d; s[2][2] = d;
-    s[0][1] = 2.0 * mu * PI * cos(PI * p[0]) * cos(PI * p[1]) * sin(PI * p[2]); s[1][0] = s[0][1];
-    s[0][2] = 2.0 * mu * PI * cos(PI * p[0]) * cos(PI * p[2]) * sin(PI * p[1]); s[2][0] = s[0][2];
-    s[1][2] = 2.0 * mu * PI * cos(PI * p[1]) * cos(PI * p[2]) * sin(PI * p[0]); s[2][1] = s[1][2];
+    s[0][1] = 2.0 * mu * PI * cs[0] * cs[1] * sn[2]; s[1][0] = s[0][1];
+    s[0][2] = 2.0 * mu * PI * cs[0] * cs[2] * sn[1]; s[2][0] = s[0][2];
+    s[1][2] = 2.0 * mu * PI * cs[1] * cs[2] * sn[0]; s[2][1] = s[1][2];
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) r[i] = r[i] + s[i][j] * n[j];
 }
 
-__device__ inline void dev_analytic(int id, const double p[3], double r[3]) {
-    const double PI = 3.141592653589793, SQ2 = 1.4142135623730951;
+__device__ inline void dev_analytic(int id, const double* sn, const double* cs, double r[3]) {
+    const double PI = DATA_PI, SQ2 = 1.4142135623730951;
     if (id == LYMPH_FUN_IC_VELOCITY) {
-        r[0] = SQ2 * PI * cos(PI * p[0]) * sin(PI * p[1]) * sin(PI * p[2]);
-        r[1] = SQ2 * PI * sin(PI * p[0]) * cos(PI * p[1]) * sin(PI * p[2]);
-        r[2] = SQ2 * PI * sin(PI * p[0]) * sin(PI * p[1]) * cos(PI * p[2]);
+        r[0] = SQ2 * PI * cs[0] * sn[1] * sn[2];
+        r[1] = SQ2 * PI * sn[0] * cs[1] * sn[2];
+        r[2] = SQ2 * PI * sn[0] * sn[1] * cs[2];
     } else if (id == LYMPH_FUN_UEX) {
-        dev_u_space(p, r);
+        dev_u_space(sn, cs, r);
     } else {
         r[0] = r[1] = r[2] = 0.0;
     }
@@ -819,7 +813,15 @@ struct VecArgs {
     double* out;         // [n_poly][ND]
 };
 
-constexpr int VEC_THREADS = 128;
+constexpr int VEC_THREADS = 128;   // k_damping
+
+// Shape of k_vector per degree: T threads (the rows ND and the 3 R tasks per
+// round of points fill them), R tabulated points at once.
+template <int PD> struct VecShape {
+    static constexpr int T = PD >= 3 ? 128 : (PD == 2 ? 96 : 32);
+    static constexpr int R = PD == 4 ? 64 : Deg<PD>::NQ3;
+    static_assert(R >= Deg<PD>::NQ2, "a face's points fit the table");
+};
 
 // solve_LU(R^T, R, b) (vet_mat_operations.f90:123-153) in the reference's
 // operation order, one lane: forward substitution y_i = (b_i - sum_{j<i}
@@ -843,121 +845,146 @@ __device__ inline void lane_solve_rtr(int NP, const double* __restrict__ R, doub
 // MAKE_RHS_FREE (matrix_free.f90:467-843) with MAKE_RHS_VOLUME / MAKE_RHS_FACE
 // (assemble_element.f90:171-390), or COMPUTE_MODAL_COEFFICIENTS_FREE
 // (matrix_free.f90:847-997): one CTA per polyhedron.
+//
+// FP64-pipe bound: the sine and cosine of each quadrature coordinate, the
+// Legendre values and the sums over the points.  So each coordinate of a point
+// is one task (its interval map, every degree's value and its sine and cosine
+// formed once), the weight is multiplied into the data once per point and
+// component, and data functions that are zero everywhere (f_null,
+// ic_displacement, uex_stat) do no quadrature.  Values and sums keep
+// legendre_1d's and the reference's order: the projection's solve amplifies a
+// change of rounding by the condition number of the mass matrix.
 template <int PD>
-__global__ void __launch_bounds__(VEC_THREADS) k_vector(VecArgs A) {
+__global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
     using D = Deg<PD>;
-    constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = D::NQ2;
+    constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = D::NQ2, T = VecShape<PD>::T, R = VecShape<PD>::R, L1 = PD + 1;
     extern __shared__ double vsm[];
     double* s_acc = vsm;                  // [ND]
-    double* s_phi = s_acc + ND;           // [NQ3][NP]
-    double* s_dphi = s_phi + NQ3 * NP;    // [NQ2][3][NP]
-    double* s_dat = s_dphi + NQ2 * 3 * NP;// [NQ3][3]
-    double* s_w = s_dat + NQ3 * 3;        // [NQ3]
-    double* s_pt = s_w + NQ3;             // [NQ2][3]
-    // 1-D factors of basis_eval (legendre_1d of each coordinate and degree):
-    // volume [NQ3][3][L1] values, faces [NQ2][3][L1] (value, derivative)
-    // pairs; the basis values are their products in basis_eval's order, so
-    // they are the same bits at 3 (p+1) instead of 3 Np legendre_1d calls
-    constexpr int L1 = PD + 1;
-    static_assert(NQ3 >= 2 * NQ2, "the face table fits the volume table's space");
-    double* s_tab = s_pt + NQ2 * 3;
+    double* s_phi = s_acc + ND;           // [R][NP]
+    double* s_leg = s_phi + R * NP;       // [R][3][L1]
+    double* s_sc = s_leg + R * 3 * L1;    // [R][3] sines, [R][3] cosines
+    double* s_wd = s_sc + R * 6;          // [R][3] data (times weight in the volume)
+    double* s_dphi = s_wd + R * 3;        // faces: [NQ2][3][NP]
+    double* s_dleg = s_dphi + NQ2 * 3 * NP;   // faces: [NQ2][3][L1] derivatives
+    __shared__ BoxC box;
+    __shared__ DerTab<PD> der;
     const int tid = threadIdx.x, P = blockIdx.x;
-    const double* bb = &A.bbox[P * 6];
-    for (int i = tid; i < ND; i += VEC_THREADS) s_acc[i] = 0.0;
-    for (int kt = A.poly_ptr[P]; kt < A.poly_ptr[P + 1]; ++kt) {
+    load_der<PD>(&der);
+    if (tid < 3) box_consts(&A.bbox[P * 6], &box, tid);
+    for (int i = tid; i < ND; i += T) s_acc[i] = 0.0;
+    const bool vol = A.mode == 0 ? A.fid != LYMPH_F_NULL
+                                 : (A.fid == LYMPH_FUN_IC_VELOCITY || A.fid == LYMPH_FUN_UEX);
+    const bool bnd = A.mode == 0 && (A.did != LYMPH_GD_NULL || A.nid == LYMPH_GN);
+    const int k1 = vol || bnd ? A.poly_ptr[P + 1] : A.poly_ptr[P];
+    for (int kt = A.poly_ptr[P]; kt < k1; ++kt) {
         const int t = A.poly_tets[kt];
         const double* fk = &A.fk[t * 12];
         const int mid = A.tet_mat[t];
         const double rho = A.mat[mid * 3 + 0], lam = A.mat[mid * 3 + 1], mu = A.mat[mid * 3 + 2];
         const double aj = fabs(A.jdet[t]);
-        __syncthreads();
-        for (int it = tid; it < NQ3 * 3 * L1; it += VEC_THREADS) {
-            const int q = it / (3 * L1), rr = it % (3 * L1), d = rr / L1, deg = rr % L1;
-            double pt[3], v, dv;
-            tet_point(fk, A.ref, q, pt);
-            legendre_1d(pt[d], deg, bb[2 * d], bb[2 * d + 1], &v, &dv);
-            s_tab[it] = v;
-            if (rr == 0) {
-                double r[3];
-                if (A.mode == 0) dev_forcing(A.fid, lam, mu, pt, rho, r);
-                else dev_analytic(A.fid, pt, r);
-                s_dat[q * 3 + 0] = r[0]; s_dat[q * 3 + 1] = r[1]; s_dat[q * 3 + 2] = r[2];
-                s_w[q] = aj * A.ref->weitet3[q];
+        // RHS: per-tetrahedron integral added to the polyhedron's vector
+        // (MAKE_RHS_VOLUME then the row copy, matrix_free.f90:711-717);
+        // projection: one running integral over all sub-tetrahedra
+        // (uex_integral, matrix_free.f90:960-972)
+        double s = 0.0;   // this thread's row (T >= ND)
+        static_assert(T >= ND, "one thread per row");
+        if (vol) {
+            if (A.mode != 0 && tid < ND) s = s_acc[tid];
+            for (int q0 = 0; q0 < NQ3; q0 += R) {
+                const int nq = (NQ3 - q0) < R ? (NQ3 - q0) : R;
+                __syncthreads();
+                for (int it = tid; it < nq * 3; it += T) {
+                    const int qq = it / 3, d = it - qq * 3;
+                    const double* nt = &A.ref->nodtet3[(q0 + qq) * 4];
+                    double x = 0.0;
+                    for (int l = 0; l < 4; ++l) x = x + fk[d * 4 + l] * nt[l];
+                    legendre_vals<PD>(&box, d, x, s_leg + it * L1);
+                    s_sc[it] = sin(DATA_PI * x);
+                    s_sc[R * 3 + it] = cos(DATA_PI * x);
+                }
+                __syncthreads();
+                for (int qq = tid; qq < nq; qq += T) {
+                    double r[3];
+                    const double *sn = &s_sc[qq * 3], *cs = &s_sc[R * 3 + qq * 3];
+                    if (A.mode == 0) dev_forcing(A.fid, lam, mu, rho, sn, cs, r);
+                    else dev_analytic(A.fid, sn, cs, r);
+                    const double w = aj * A.ref->weitet3[q0 + qq];
+                    s_wd[qq * 3 + 0] = w * r[0]; s_wd[qq * 3 + 1] = w * r[1]; s_wd[qq * 3 + 2] = w * r[2];
+                }
+                for (int it = tid; it < nq * NP; it += T) {
+                    const int q = it / NP, f = it - q * NP;
+                    const double* tq = s_leg + q * 3 * L1;
+                    s_phi[it] = tq[der.deg[f][0]] * tq[L1 + der.deg[f][1]] * tq[2 * L1 + der.deg[f][2]];
+                }
+                __syncthreads();
+                if (tid < ND) {
+                    const int i = tid / NP, m = tid - i * NP;
+#pragma unroll 4
+                    for (int q = 0; q < nq; ++q) s = s + s_wd[q * 3 + i] * s_phi[q * NP + m];
+                }
+            }
+            if (tid < ND) {
+                if (A.mode == 0) s_acc[tid] += s;
+                else s_acc[tid] = s;
             }
         }
-        __syncthreads();
-        for (int it = tid; it < NQ3 * NP; it += VEC_THREADS) {
-            const int q = it / NP, f = it % NP;
-            const int* bl = &A.ref->blist[f * 3];
-            const double* tq = s_tab + q * 3 * L1;
-            s_phi[q * NP + f] = tq[bl[0]] * tq[L1 + bl[1]] * tq[2 * L1 + bl[2]];
-        }
-        __syncthreads();
-        for (int r = tid; r < ND; r += VEC_THREADS) {
-            const int i = r / NP, m = r % NP;
-            // RHS: per-tetrahedron integral added to the polyhedron's vector
-            // (MAKE_RHS_VOLUME then the row copy, matrix_free.f90:711-717);
-            // projection: one running integral over all sub-tetrahedra
-            // (uex_integral, matrix_free.f90:960-972)
-            double s = (A.mode == 0) ? 0.0 : s_acc[r];
-            for (int q = 0; q < NQ3; ++q) s = s + s_w[q] * s_dat[q * 3 + i] * s_phi[q * NP + m];
-            if (A.mode == 0) s_acc[r] += s;
-            else s_acc[r] = s;
-        }
-        if (A.mode != 0) continue;
+        if (!bnd) continue;
         // boundary faces of this tetrahedron (only boundary faces are added, :809-819)
         for (int f = 0; f < 4; ++f) {
             const int E2 = A.neigh[t * 4 + f];
             if (E2 != LYMPH_BC_DIRI && E2 != LYMPH_BC_NEUM) continue;
+            if (E2 == LYMPH_BC_DIRI ? A.did == LYMPH_GD_NULL : A.nid != LYMPH_GN) continue;   // zero data
             const int tag = A.fun_tag ? A.fun_tag[t * 4 + f] : 1;
             const double nv[3] = {A.nrm[t * 12 + f * 3], A.nrm[t * 12 + f * 3 + 1], A.nrm[t * 12 + f * 3 + 2]};
             const double ar = A.area[t * 4 + f];
             __syncthreads();
-            for (int q = tid; q < NQ2; q += VEC_THREADS) {
-                face_point(fk, A.ref, f, q, &s_pt[q * 3]);
-                // data points as MAKE_RHS_FACE forms them (assemble_element.f90:313-320)
-                double pq[3];
-                const double* nm = &A.ref->node_maps[f * 16];
+            for (int it = tid; it < NQ2 * 3; it += T) {
+                const int q = it / 3, j = it - q * 3;
+                // the basis point (basis_boundary, basis_function.f90:560-577)
                 const double* nt = &A.ref->nodtria2[q * 4];
-                for (int j = 0; j < 3; ++j) {
-                    double s = 0.0;
-                    for (int kk = 0; kk < 4; ++kk)
-                        for (int tt = 0; tt < 4; ++tt) s = s + fk[j * 4 + kk] * nm[kk * 4 + tt] * nt[tt];
-                    pq[j] = s;
+                double x = 0.0;
+                for (int l = 0; l < 4; ++l) x = x + face_map(fk, A.ref, f, j, l) * nt[l];
+                double dv;
+                for (int n = 0; n <= PD; ++n) {
+                    legendre_1d(x, n, A.bbox[P * 6 + 2 * j], A.bbox[P * 6 + 2 * j + 1], &s_leg[it * L1 + n], &dv);
+                    s_dleg[it * L1 + n] = dv;
                 }
+                // the data point as MAKE_RHS_FACE forms it (assemble_element.f90:313-320)
+                const double* nm = &A.ref->node_maps[f * 16];
+                double y = 0.0;
+                for (int kk = 0; kk < 4; ++kk)
+                    for (int tt = 0; tt < 4; ++tt) y = y + fk[j * 4 + kk] * nm[kk * 4 + tt] * nt[tt];
+                s_sc[it] = sin(DATA_PI * y);
+                s_sc[R * 3 + it] = cos(DATA_PI * y);
+            }
+            __syncthreads();
+            for (int q = tid; q < NQ2; q += T) {
                 double g[3];
-                if (E2 == LYMPH_BC_DIRI) dev_dirichlet(A.did, pq, tag, g);
-                else dev_neumann(A.nid, lam, mu, nv, pq, tag, g);
-                s_dat[q * 3 + 0] = g[0]; s_dat[q * 3 + 1] = g[1]; s_dat[q * 3 + 2] = g[2];
+                const double *sn = &s_sc[q * 3], *cs = &s_sc[R * 3 + q * 3];
+                if (E2 == LYMPH_BC_DIRI) dev_dirichlet(A.did, tag, sn, cs, g);
+                else dev_neumann(A.nid, lam, mu, nv, tag, sn, cs, g);
+                s_wd[q * 3 + 0] = g[0]; s_wd[q * 3 + 1] = g[1]; s_wd[q * 3 + 2] = g[2];
             }
-            __syncthreads();
-            for (int it = tid; it < NQ2 * 3 * L1; it += VEC_THREADS) {
-                const int q = it / (3 * L1), rr = it % (3 * L1), d = rr / L1, deg = rr % L1;
-                legendre_1d(s_pt[q * 3 + d], deg, bb[2 * d], bb[2 * d + 1], &s_tab[2 * it], &s_tab[2 * it + 1]);
-            }
-            __syncthreads();
-            for (int it = tid; it < NQ2 * NP; it += VEC_THREADS) {
-                const int q = it / NP, fb = it % NP;
-                const int* bl = &A.ref->blist[fb * 3];
-                const double* tq = s_tab + 2 * q * 3 * L1;
-                const double vx = tq[2 * bl[0]], dx = tq[2 * bl[0] + 1];
-                const double vy = tq[2 * (L1 + bl[1])], dy = tq[2 * (L1 + bl[1]) + 1];
-                const double vz = tq[2 * (2 * L1 + bl[2])], dz = tq[2 * (2 * L1 + bl[2]) + 1];
-                s_phi[q * NP + fb] = vx * vy * vz;
-                s_dphi[(q * 3 + 0) * NP + fb] = dx * vy * vz;
-                s_dphi[(q * 3 + 1) * NP + fb] = vx * dy * vz;
-                s_dphi[(q * 3 + 2) * NP + fb] = vx * vy * dz;
+            for (int it = tid; it < NQ2 * NP; it += T) {
+                const int q = it / NP, fb = it - q * NP;
+                const double *tv = s_leg + q * 3 * L1, *td = s_dleg + q * 3 * L1;
+                const int bx = der.deg[fb][0], by = L1 + der.deg[fb][1], bz = 2 * L1 + der.deg[fb][2];
+                const double vx = tv[bx], vy = tv[by], vz = tv[bz];
+                s_phi[it] = vx * vy * vz;
+                s_dphi[(q * 3 + 0) * NP + fb] = td[bx] * vy * vz;
+                s_dphi[(q * 3 + 1) * NP + fb] = vx * td[by] * vz;
+                s_dphi[(q * 3 + 2) * NP + fb] = vx * vy * td[bz];
             }
             __syncthreads();
             const double sigma = A.alpha * (double)(PD * PD) / A.hk[P] * (lam + 2 * mu);
             const double n0 = nv[0], n1 = nv[1], n2 = nv[2];
             const double a0 = fabs(n0) * fabs(n0), a1 = fabs(n1) * fabs(n1), a2 = fabs(n2) * fabs(n2);
-            for (int r = tid; r < ND; r += VEC_THREADS) {
+            for (int r = tid; r < ND; r += T) {
                 const int i = r / NP, m = r % NP;
                 double rf = 0.0;
                 for (int q = 0; q < NQ2; ++q) {
                     const double w = A.ref->weitria2[q];
-                    const double* gd = &s_dat[q * 3];
+                    const double* gd = &s_wd[q * 3];
                     const double ph = s_phi[q * NP + m];
                     if (E2 == LYMPH_BC_DIRI) {
                         const double g0 = s_dphi[(q * 3 + 0) * NP + m], g1 = s_dphi[(q * 3 + 1) * NP + m],
@@ -987,13 +1014,13 @@ __global__ void __launch_bounds__(VEC_THREADS) k_vector(VecArgs A) {
     }
     __syncthreads();
     if (A.mode == 0) {
-        for (int r = tid; r < ND; r += VEC_THREADS) A.out[(int64_t)P * ND + r] = s_acc[r];
+        for (int r = tid; r < ND; r += T) A.out[(int64_t)P * ND + r] = s_acc[r];
         return;
     }
     // L2 projection: solve_LU(R^T, R) per component with the modal factor
-    if (tid < 3) lane_solve_rtr(NP, A.R + (int64_t)P * NP * NP, &s_acc[tid * NP]);
+    if (vol && tid < 3) lane_solve_rtr(NP, A.R + (int64_t)P * NP * NP, &s_acc[tid * NP]);
     __syncthreads();
-    for (int r = tid; r < ND; r += VEC_THREADS) A.out[(int64_t)P * ND + r] = s_acc[r] * A.scale;
+    for (int r = tid; r < ND; r += T) A.out[(int64_t)P * ND + r] = s_acc[r] * A.scale;
 }
 
 // MAKE_DAMPING_FACE (assemble_element.f90:666-731) summed over the absorbing
@@ -1160,11 +1187,11 @@ int launch_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scal
     A.area = c->d_area; A.bbox = c->d_bbox; A.hk = c->d_hk; A.ref = c->d_ref; A.alpha = c->alpha; A.theta = c->theta;
     A.mode = mode; A.fid = fid; A.did = did; A.nid = nid; A.R = c->d_Rm; A.RT = c->d_RmT; A.scale = scale; A.out = out;
     using D = Deg<PD>;
-    // + the 1-D factor table (NQ3 * 3 (p+1) >= NQ2 * 3 (p+1) * 2 doubles)
-    size_t smem = sizeof(double) * ((size_t)D::ND + D::NQ3 * D::NP + D::NQ2 * 3 * D::NP + D::NQ3 * 3 + D::NQ3 + D::NQ2 * 3 +
-                                    (size_t)D::NQ3 * 3 * (PD + 1));
+    using V = VecShape<PD>;
+    const size_t face = (size_t)D::NQ2 * 3 * (D::NP + PD + 1);   // gradient tables of a boundary face (RHS only)
+    const size_t smem = sizeof(double) * ((size_t)D::ND + (size_t)V::R * (D::NP + 3 * (PD + 1) + 9) + (mode == 0 ? face : 0));
     LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_vector<PD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_vector<PD><<<c->n_poly, VEC_THREADS, smem, c->stream>>>(A);
+    k_vector<PD><<<c->n_poly, V::T, smem, c->stream>>>(A);
     c->launches++;
     LYMPH_CUDA_TRY(cudaGetLastError());
     return LYMPH_OK;

@@ -51,3 +51,27 @@ def test_blocks_of_other_penalty_forms(require_gpu, p, theta):
 @pytest.mark.parametrize("p", [1, 2, 4])
 def test_blocks_of_a_large_polyhedron(require_gpu, p):
     _blocks_close(_big_polyhedron_mesh(), p, -1.0)
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+def test_rhs_of_every_data_combination(require_gpu, p):
+    """Every forcing / Dirichlet / Neumann id together (zero functions do no
+    quadrature): normwise <= 1e-12 of the oracle's vector, exactly zero where
+    all three are zero; projections of zero functions exactly zero."""
+    m = M.cube(2, bc="reference", agglomeration="bfs", seed=5, group=(4, 12), jitter=0.2, material=(1.0, 2.0, 1.0))
+    o = Oracle(m, p, 1e-3)
+    o.make_matrices()
+    with MatrixFree(m, p, 1e-3) as g:
+        g.MAKE_MATRICES_FREE()
+        for f in range(3):
+            for d in range(3):
+                for n in range(3):
+                    g.MAKE_RHS_FREE(_lib.RHS_DYN, f, d, n)
+                    o.make_rhs(1, f, d, n)
+                    ref, got = o.rhs(1), g.rhs(_lib.RHS_DYN)
+                    assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref), (f, d, n)
+        for fun in (_lib.FUN_IC_DISPLACEMENT, _lib.FUN_UEX_STAT):
+            g.set_state(_lib.SLOT_UEX, np.ones((g.n_poly, g.nd)))
+            g.COMPUTE_MODAL_COEFFICIENTS_FREE(fun, _lib.SLOT_UEX, 0.5)
+            assert not g.get_state(_lib.SLOT_UEX).any()
+    o.close()
