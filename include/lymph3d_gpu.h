@@ -262,8 +262,8 @@ int lymph_checkpoint_load(lymph_ctx* ctx, const char* path, double* t, int64_t* 
 int lymph_error_l2(lymph_ctx* ctx, int slot_uh, int slot_uex, double* sumsq);
 
 /* COMPUTE_ERROR_DG_MATRIX_FREE (src/matrix_free.f90:1421-1504): sum over
- * polyhedra of du_P^T (A_PP du_P + sum_Q A_PQ du_Q).  Assembles the A_dg
- * blocks into a temporary device buffer for the duration of the call. */
+ * polyhedra of du_P^T (A_PP du_P + sum_Q A_PQ du_Q), evaluated from the
+ * quadrature without forming the A_dg blocks (no device allocation). */
 int lymph_error_dg(lymph_ctx* ctx, int slot_uh, int slot_uex, double* sumsq);
 
 /* L2 error without any device allocation.  No counterpart in the reference:

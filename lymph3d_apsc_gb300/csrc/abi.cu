@@ -36,7 +36,7 @@ int lymph_dev_double_couple(lymph_ctx* c, int t, int P, const double moment[9], 
 int lymph_dev_power_iteration(lymph_ctx* c, double* x, double* y, double* d_ss, int iters);
 int lymph_dev_point_source(lymph_ctx* c, int P, const double x0[3], const double dir[3], double* out);
 int lymph_dev_bump(lymph_ctx* c);
-int lymph_dev_error_dg(lymph_ctx* c, const void* blocks, const double* uh, const double* uex, double* d_out);
+int lymph_dev_error_dg(lymph_ctx* c, const double* uh, const double* uex, double* d_out);
 int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double* d_out);
 int lymph_dev_energy(lymph_ctx* c, const double* ua, const double* ub, double* d_out);
 
@@ -891,19 +891,8 @@ int lymph_error_l2(lymph_ctx* c, int s_uh, int s_uex, double* sumsq) {
 int lymph_error_dg(lymph_ctx* c, int s_uh, int s_uex, double* sumsq) {
     if (!c || !sumsq || !valid_slot(s_uh) || !valid_slot(s_uex)) return LYMPH_ERR_INVALID;
     if (!c->have_matrices) { lymph_set_error("lymph_error_dg: call lymph_make_matrices first"); return LYMPH_ERR_ORDER; }
-    size_t nK = (size_t)c->n_blocks * c->nd * c->nd;
-    double* A = nullptr;
-    if (cudaMalloc(&A, nK * sizeof(double)) != cudaSuccess) {
-        lymph_set_error("lymph_error_dg: cannot allocate the A_dg blocks");
-        return LYMPH_ERR_OOM;
-    }
-    int rc = lymph_dev_assemble(c, LYMPH_BLOCKS_ADG, A, false);
-    if (rc == LYMPH_OK) rc = lymph_dev_error_dg(c, A, lymph_slot_ptr(c, s_uh), lymph_slot_ptr(c, s_uex), c->d_scalar);
-    if (rc == LYMPH_OK && cudaMemcpyAsync(sumsq, c->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
-        rc = LYMPH_ERR_CUDA;
-    cudaStreamSynchronize(c->stream);
-    cudaFree(A);
-    LYMPH_TRY(rc);
+    LYMPH_TRY(lymph_dev_error_dg(c, lymph_slot_ptr(c, s_uh), lymph_slot_ptr(c, s_uex), c->d_scalar));
+    LYMPH_CUDA_TRY(cudaMemcpyAsync(sumsq, c->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     return lymph_sync_status(c, "lymph_error_dg");
 }
 

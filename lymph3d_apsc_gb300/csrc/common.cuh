@@ -216,23 +216,35 @@ inline int np_of(int p) { return (p + 1) * (p + 2) * (p + 3) / 6; }
 // COMPUTE_ERROR_L2_MATRIX_FREE's body for polyhedron P
 // (src/matrix_free.f90:1388-1418): sum_i du_i^T M du_i with du = uh - uex,
 // M the Np x Np modal mass matrix, rows and columns in the reference's order.
+// One CTA of L2_THREADS threads per polyhedron; the result is returned in thread 0.
+// M comes into shared memory in coalesced reads (a thread per polyhedron read
+// it at a stride of Np^2 doubles), a thread forms one row's t = M du, and one
+// thread per component adds the rows up in order.
+constexpr int L2_THREADS = 128;
+static_assert(3 * MAX_NP <= L2_THREADS, "one thread per row");
 __device__ __forceinline__ double l2_partial_poly(int P, int NP, const double* __restrict__ Mm,
                                                   const double* __restrict__ uh, const double* __restrict__ uex) {
-    const int ND = 3 * NP;
-    double err = 0.0;
+    __shared__ double s_M[MAX_NP * MAX_NP], s_du[3 * MAX_NP], s_t[3 * MAX_NP];
+    const int ND = 3 * NP, tid = threadIdx.x;
     const double* M = Mm + (int64_t)P * NP * NP;
-    for (int i = 0; i < 3; ++i) {
-        double e = 0.0;
-        for (int rr = 0; rr < NP; ++rr) {
-            double t = 0.0;
-            for (int c = 0; c < NP; ++c) {
-                const int64_t qc = (int64_t)P * ND + i * NP + c;
-                t = t + M[rr * NP + c] * (uh[qc] - uex[qc]);
-            }
-            const int64_t qr = (int64_t)P * ND + i * NP + rr;
-            e = e + (uh[qr] - uex[qr]) * t;
-        }
-        err = err + e;
+    for (int i = tid; i < NP * NP; i += L2_THREADS) s_M[i] = M[i];
+    if (tid < ND) s_du[tid] = uh[(int64_t)P * ND + tid] - uex[(int64_t)P * ND + tid];
+    __syncthreads();
+    if (tid < ND) {
+        const int i = tid / NP, rr = tid - i * NP;
+        double t = 0.0;
+        for (int c = 0; c < NP; ++c) t = fma(s_M[rr * NP + c], s_du[i * NP + c], t);
+        s_t[tid] = t;
+    }
+    __syncthreads();
+    double e = 0.0;
+    if (tid < 3)
+        for (int rr = 0; rr < NP; ++rr) e = fma(s_du[tid * NP + rr], s_t[tid * NP + rr], e);
+    double err = 0.0;
+    if (tid < 32) {
+        err = err + __shfl_sync(0xffffffffu, e, 0);
+        err = err + __shfl_sync(0xffffffffu, e, 1);
+        err = err + __shfl_sync(0xffffffffu, e, 2);
     }
     return err;
 }

@@ -32,11 +32,218 @@ __global__ void __launch_bounds__(Shape<PD>::T, Shape<PD>::MINB) k_step(StepArgs
 __global__ void k_bump(int64_t* idx) { *idx += 1; }
 
 // COMPUTE_ERROR_L2_MATRIX_FREE body per polyhedron: sum_i du_i^T M du_i.
-__global__ void k_l2_partial(int n_poly, int NP, const double* __restrict__ Mm, const double* __restrict__ uh,
-                             const double* __restrict__ uex, double* partial) {
-    const int P = blockIdx.x * blockDim.x + threadIdx.x;
-    if (P >= n_poly) return;
-    partial[P] = l2_partial_poly(P, NP, Mm, uh, uex);
+__global__ void __launch_bounds__(L2_THREADS) k_l2_partial(int NP, const double* __restrict__ Mm,
+                                                           const double* __restrict__ uh, const double* __restrict__ uex,
+                                                           double* partial) {
+    const double e = l2_partial_poly(blockIdx.x, NP, Mm, uh, uex);
+    if (threadIdx.x == 0) partial[blockIdx.x] = e;
+}
+
+// ---- COMPUTE_ERROR_DG_MATRIX_FREE ----
+
+struct DgArgs {
+    const int32_t* row_ptr;
+    const int64_t* bf_ptr;
+    const int32_t* bf;
+    const int32_t* poly_ptr;
+    const int32_t* poly_tets;
+    const int32_t* tet_poly;
+    const int32_t* tet_mat;
+    const int32_t* neigh;
+    const double *mat, *fk, *jdet, *nrm, *area, *bbox, *hk;
+    const RefTables* ref;
+    const double *uh, *uex;
+    double alpha;
+    double* partial;   // [n_poly]
+};
+
+// Position of basis function (a, b, c) in the reference's order.
+template <int PD> struct BasisPos {
+    int i[PD + 1][PD + 1][PD + 1];
+    constexpr BasisPos() : i() {
+        constexpr Blist<PD> BL{};
+        for (int k = 0; k < Deg<PD>::NP; ++k) i[BL.d[k][0]][BL.d[k][1]][BL.d[k][2]] = k;
+    }
+};
+
+// Legendre polynomials and derivatives of degrees 0..PD at x (recurrences).
+template <int PD> __device__ __forceinline__ void legendre_rec(double x, double* L, double* dL) {
+    L[0] = 1.0;
+    dL[0] = 0.0;
+    L[1] = x;
+    dL[1] = 1.0;
+#pragma unroll
+    for (int n = 1; n < PD; ++n) {
+        L[n + 1] = ((2 * n + 1) * x * L[n] - n * L[n - 1]) * (1.0 / (n + 1));
+        dL[n + 1] = dL[n - 1] + (2 * n + 1) * L[n];
+    }
+}
+
+// The three components of sum_m u_m phi_m at a point, unscaled, by sum
+// factorisation over the degree triples; at(m, j): coefficient m of component j.
+template <int PD, typename At>
+__device__ __forceinline__ void field_sf(At at, const double* X, const double* Y, const double* Z, double (&v)[3]) {
+    constexpr BasisPos<PD> BP{};
+    v[0] = v[1] = v[2] = 0.0;
+#pragma unroll
+    for (int a = 0; a <= PD; ++a) {
+        double r[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int b = 0; b <= PD - a; ++b) {
+            double w[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int c = 0; c <= PD - a - b; ++c)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) w[j] = fma(at(BP.i[a][b][c], j), Z[c], w[j]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) r[j] = fma(w[j], Y[b], r[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) v[j] = fma(r[j], X[a], v[j]);
+    }
+}
+
+constexpr int DG_THREADS = 128;
+
+// du_P . (A_PP du_P + sum_Q A_PQ du_Q), du = uh - uex, of the DG-norm blocks
+// the reference assembles (strain energy of P's tetrahedra, penalty of the
+// jumps on its faces), straight from the quadrature: a thread per point
+// evaluates the gradient (volume) or the two sides' values (faces) of du by
+// sum factorisation,
+//     sum_q w (lambda (tr g)^2 + mu g : (g + g^T)) + sum_q W sigma v_P . T (v_P - v_Q),
+// T z = n (n . z) / 2 + |n|^2 z / 2 and v_Q = 0 on a Dirichlet face.  FP64-pipe
+// bound.  No block is formed: a tetrahedron costs (p+1)^3 evaluations instead
+// of Np^2 moments per point, and no operator-sized buffer is needed.
+template <int PD>
+__global__ void __launch_bounds__(DG_THREADS, 4) k_dg_partial(const __grid_constant__ DgArgs A) {
+    constexpr int NP = Deg<PD>::NP, ND = Deg<PD>::ND, NQ3 = (PD + 1) * (PD + 1) * (PD + 1), NQ2 = (PD + 1) * (PD + 1);
+    constexpr BasisPos<PD> BP{};
+    __shared__ double s_du[ND], s_red[DG_THREADS / 32];
+    const int tid = threadIdx.x, P = blockIdx.x;
+    for (int i = tid; i < ND; i += DG_THREADS) s_du[i] = A.uh[(int64_t)P * ND + i] - A.uex[(int64_t)P * ND + i];
+    double mid[3], ih[3], hp = 1.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double lo = A.bbox[P * 6 + 2 * d], hi = A.bbox[P * 6 + 2 * d + 1];
+        mid[d] = 0.5 * (lo + hi);
+        ih[d] = 2.0 / (hi - lo);
+        hp *= ih[d];
+    }
+    const double sc = sqrt(hp);   // phi = sc L_a L_b L_c
+    __syncthreads();
+    const int p0 = A.poly_ptr[P], n_vol = (A.poly_ptr[P + 1] - p0) * NQ3;
+    double acc = 0.0;
+    for (int it = tid; it < n_vol; it += DG_THREADS) {
+        // the coefficients are read from shared memory at each point: hoisted
+        // out of the loop, all 3 Np of them spill
+        asm volatile("" ::: "memory");
+        const int kt = it / NQ3, q = it - kt * NQ3, t = A.poly_tets[p0 + kt];
+        const double* fk = &A.fk[(int64_t)t * 12];
+        const double* nt = &A.ref->nodtet3[q * 4];
+        double L[3][PD + 1], dL[3][PD + 1];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double x = fma(fk[d * 4], nt[0], fma(fk[d * 4 + 1], nt[1], fma(fk[d * 4 + 2], nt[2], fk[d * 4 + 3])));
+            legendre_rec<PD>((x - mid[d]) * ih[d], L[d], dL[d]);
+        }
+        double g[3][3] = {};   // g[k][j] = d_k du_j
+#pragma unroll
+        for (int a = 0; a <= PD; ++a) {
+            double r0[3] = {}, r1[3] = {}, r2[3] = {};
+#pragma unroll
+            for (int b = 0; b <= PD - a; ++b) {
+                double w0[3] = {}, w1[3] = {};
+#pragma unroll
+                for (int c = 0; c <= PD - a - b; ++c)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const double u = s_du[j * NP + BP.i[a][b][c]];
+                        w0[j] = fma(u, L[2][c], w0[j]);
+                        w1[j] = fma(u, dL[2][c], w1[j]);
+                    }
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    r0[j] = fma(w0[j], L[1][b], r0[j]);
+                    r1[j] = fma(w0[j], dL[1][b], r1[j]);
+                    r2[j] = fma(w1[j], L[1][b], r2[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                g[0][j] = fma(r0[j], dL[0][a], g[0][j]);
+                g[1][j] = fma(r1[j], L[0][a], g[1][j]);
+                g[2][j] = fma(r2[j], L[0][a], g[2][j]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) g[k][j] *= sc * ih[k];
+        const int m = A.tet_mat[t];
+        const double tr = g[0][0] + g[1][1] + g[2][2];
+        double gg = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) gg = fma(g[k][j], g[k][j] + g[j][k], gg);
+        acc = fma(A.ref->weitet3[q] * fabs(A.jdet[t]), A.mat[m * 3 + 1] * (tr * tr) + A.mat[m * 3 + 2] * gg, acc);
+    }
+    // faces that carry a term: the self block's list, first in P's row
+    const int64_t e0 = A.bf_ptr[A.row_ptr[P]];
+    const int n_face = (int)(A.bf_ptr[A.row_ptr[P] + 1] - e0) * NQ2;
+    for (int it = tid; it < n_face; it += DG_THREADS) {
+        asm volatile("" ::: "memory");
+        const int fi = it / NQ2, q = it - fi * NQ2, code = A.bf[e0 + fi], t = code >> 2, e2 = A.neigh[code];
+        const bool dir = e2 == LYMPH_BC_DIRI;
+        const int Q = dir ? P : A.tet_poly[e2];
+        const double* fk = &A.fk[(int64_t)t * 12];
+        const double* nm = &A.ref->node_maps[(code & 3) * 16];
+        const double* nt = &A.ref->nodtria2[q * 4];
+        double rc[3], x[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            rc[r] = fma(nm[r * 4], nt[0], fma(nm[r * 4 + 1], nt[1], fma(nm[r * 4 + 2], nt[2], nm[r * 4 + 3] * nt[3])));
+        double L[3][PD + 1], dL[PD + 1], v[3], z[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            x[d] = fma(fk[d * 4], rc[0], fma(fk[d * 4 + 1], rc[1], fma(fk[d * 4 + 2], rc[2], fk[d * 4 + 3])));
+            legendre_rec<PD>((x[d] - mid[d]) * ih[d], L[d], dL);
+        }
+        field_sf<PD>([&](int m, int j) { return s_du[j * NP + m]; }, L[0], L[1], L[2], v);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) z[j] = v[j] = v[j] * sc;
+        if (!dir) {
+            double hq = 1.0, w[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double lo = A.bbox[Q * 6 + 2 * d], hi = A.bbox[Q * 6 + 2 * d + 1], i2 = 2.0 / (hi - lo);
+                hq *= i2;
+                legendre_rec<PD>((x[d] - 0.5 * (lo + hi)) * i2, L[d], dL);
+            }
+            const double *uh = A.uh + (int64_t)Q * ND, *ue = A.uex + (int64_t)Q * ND;
+            field_sf<PD>([&](int m, int j) { return uh[j * NP + m] - ue[j * NP + m]; }, L[0], L[1], L[2], w);
+            const double sq = sqrt(hq);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) z[j] = fma(-sq, w[j], z[j]);
+        }
+        const double* n = &A.nrm[(int64_t)t * 12 + (code & 3) * 3];
+        const int m = A.tet_mat[t];
+        const double h = dir ? A.hk[P] : fmin(A.hk[P], A.hk[Q]);
+        const double sigma = A.alpha * (double)(PD * PD) / h * (A.mat[m * 3 + 1] + 2.0 * A.mat[m * 3 + 2]);
+        const double nv = n[0] * v[0] + n[1] * v[1] + n[2] * v[2], nz = n[0] * z[0] + n[1] * z[1] + n[2] * z[2];
+        const double nn = n[0] * n[0] + n[1] * n[1] + n[2] * n[2], vz = v[0] * z[0] + v[1] * z[1] + v[2] * z[2];
+        acc = fma(A.ref->weitria2[q] * A.area[code] * sigma, 0.5 * (nv * nz + nn * vz), acc);
+    }
+    // a fixed tree over the threads
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((tid & 31) == 0) s_red[tid >> 5] = acc;
+    __syncthreads();
+    if (tid == 0) {
+        double e = 0.0;
+        for (int w = 0; w < DG_THREADS / 32; ++w) e += s_red[w];
+        A.partial[P] = e;
+    }
 }
 
 // Deterministic sum of n values (one CTA of 1024 threads).
@@ -224,15 +431,23 @@ int lymph_dev_first_step(lymph_ctx* c) {
     return launch_ctx<MODE_FIRST>(c, A);
 }
 
-// du . (A du) per polyhedron with FP64 A_dg blocks in `blocks`, then the sum.
-int lymph_dev_error_dg(lymph_ctx* c, const void* blocks, const double* uh, const double* uex, double* d_out) {
-    StepArgs A = base_args(c);
-    A.K = blocks;
-    A.u0 = uh;
-    A.un = uex;
-    LYMPH_TRY(launch_step_mode<MODE_DG>(c, A, false));
+// du . (A_dg du) per polyhedron by quadrature, then the sum.
+int lymph_dev_error_dg(lymph_ctx* c, const double* uh, const double* uex, double* d_out) {
+    DgArgs A;
+    A.row_ptr = c->d_row_ptr; A.bf_ptr = c->d_bf_ptr; A.bf = c->d_bf; A.poly_ptr = c->d_poly_ptr;
+    A.poly_tets = c->d_poly_tets; A.tet_poly = c->d_tet_poly; A.tet_mat = c->d_tet_mat; A.neigh = c->d_neigh;
+    A.mat = c->d_mat; A.fk = c->d_fk; A.jdet = c->d_jdet; A.nrm = c->d_normal; A.area = c->d_area;
+    A.bbox = c->d_bbox; A.hk = c->d_hk; A.ref = c->d_ref; A.uh = uh; A.uex = uex; A.alpha = c->alpha;
+    A.partial = c->d_partial;
+    switch (c->p) {
+        case 1: k_dg_partial<1><<<c->n_poly, DG_THREADS, 0, c->stream>>>(A); break;
+        case 2: k_dg_partial<2><<<c->n_poly, DG_THREADS, 0, c->stream>>>(A); break;
+        case 3: k_dg_partial<3><<<c->n_poly, DG_THREADS, 0, c->stream>>>(A); break;
+        case 4: k_dg_partial<4><<<c->n_poly, DG_THREADS, 0, c->stream>>>(A); break;
+        default: lymph_set_error("degree not supported on the device"); return LYMPH_ERR_INVALID;
+    }
     k_sum<<<1, 1024, 0, c->stream>>>(c->n_poly, c->d_partial, d_out);
-    c->launches++;
+    c->launches += 2;
     LYMPH_CUDA_TRY(cudaGetLastError());
     return LYMPH_OK;
 }
@@ -240,7 +455,7 @@ int lymph_dev_error_dg(lymph_ctx* c, const void* blocks, const double* uh, const
 // Leapfrog energy terms: d_out[0] = |ub - ua|^2_M (rho-weighted mass),
 // d_out[1] = ub . K ua.
 int lymph_dev_energy(lymph_ctx* c, const double* ua, const double* ub, double* d_out) {
-    k_l2_partial<<<(c->n_poly + 127) / 128, 128, 0, c->stream>>>(c->n_poly, c->Np, c->d_M, ub, ua, c->d_partial);
+    k_l2_partial<<<c->n_poly, L2_THREADS, 0, c->stream>>>(c->Np, c->d_M, ub, ua, c->d_partial);
     k_sum<<<1, 1024, 0, c->stream>>>(c->n_poly, c->d_partial, d_out);
     StepArgs A = base_args(c);
     A.u0 = ua;
@@ -253,7 +468,7 @@ int lymph_dev_energy(lymph_ctx* c, const double* ua, const double* ub, double* d
 }
 
 int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double* d_out) {
-    k_l2_partial<<<(c->n_poly + 127) / 128, 128, 0, c->stream>>>(c->n_poly, c->Np, c->d_Mm, uh, uex, c->d_partial);
+    k_l2_partial<<<c->n_poly, L2_THREADS, 0, c->stream>>>(c->Np, c->d_Mm, uh, uex, c->d_partial);
     k_sum<<<1, 1024, 0, c->stream>>>(c->n_poly, c->d_partial, d_out);
     c->launches += 2;
     LYMPH_CUDA_TRY(cudaGetLastError());

@@ -26,7 +26,7 @@ constexpr int NBB = 16;   // neighbour blocks staged in shared memory at once
 // MODE_APPLY: out = M^-1 K u (power iteration for the CFL bound)
 // MODE_BILIN: partial[P] = un_P . (K u0)_P (the bilinear form of the leapfrog energy)
 // MODE_KU:    out = K u (the operator apply alone, before M^-1)
-enum { MODE_STEP = 0, MODE_FIRST = 1, MODE_DG = 2, MODE_APPLY = 3, MODE_BILIN = 4, MODE_KU = 5 };
+enum { MODE_STEP = 0, MODE_FIRST = 1, MODE_APPLY = 3, MODE_BILIN = 4, MODE_KU = 5 };
 
 struct StepArgs {
     const int32_t* row_ptr;
@@ -37,11 +37,11 @@ struct StepArgs {
     const double* rhs_dyn;
     const double* gvals;       // time-function values
     const int64_t* step_idx;   // index into gvals (device counter)
-    const double* u0;          // u^{n-1} (MODE_STEP), u^0 (MODE_FIRST), u_h (MODE_DG)
-    const double* un;          // u^n (MODE_STEP, MODE_APPLY), v^0 (MODE_FIRST), u_ex (MODE_DG)
+    const double* u0;          // u^{n-1} (MODE_STEP), u^0 (MODE_FIRST)
+    const double* un;          // u^n (MODE_STEP, MODE_APPLY), v^0 (MODE_FIRST)
     double* out;               // u^{n+1} (MODE_STEP: may alias u0), u^1 (MODE_FIRST), M^-1 K u (MODE_APPLY),
                                // K u (MODE_KU)
-    double* partial;           // MODE_DG: per-polyhedron du . (A du)
+    double* partial;           // MODE_BILIN: per-polyhedron sums
     const int32_t* abs_idx;    // per polyhedron its index among those with absorbing faces, -1 for the
                                // others; null when the mesh has no absorbing face
     const double* Dabs;        // [n_abs][ND][ND] damping blocks (symmetric)
@@ -66,7 +66,7 @@ template <int PD, typename KT, int S_ = Shape<PD>::S> struct SmemSize {
 
 // The end of one polyhedron's step once thread tid < ND holds y = (K u)_tid
 // of row tid in FP64: the right-hand side, the mass-matrix inverse and the
-// leapfrog update (or the bilinear/DG partial sum).  The mass-matrix inverse is
+// leapfrog update (or the bilinear partial sum).  The mass-matrix inverse is
 // applied in FP64 as a dense Np x Np product per component (precomputed from
 // the Cholesky factor), which replaces the reference's two triangular solves
 // per component with a parallel product of the same value.  s_b holds ND
@@ -76,14 +76,14 @@ template <int PD, int MODE>
 __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, double* s_b) {
     constexpr int NP = Deg<PD>::NP, ND = Deg<PD>::ND;
     const int tid = threadIdx.x;
-    if (MODE == MODE_DG || MODE == MODE_BILIN) {
+    if (MODE == MODE_BILIN) {
         if (tid < ND) s_b[tid] = y;
         __syncthreads();
         if (tid == 0) {
             double e = 0.0;
             for (int rr = 0; rr < ND; ++rr) {
                 const int64_t q = (int64_t)P * ND + rr;
-                e = e + (MODE == MODE_DG ? (A.u0[q] - A.un[q]) : A.un[q]) * s_b[rr];
+                e = e + A.un[q] * s_b[rr];
             }
             A.partial[P] = e;
         }
@@ -179,7 +179,7 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
 // degree's shape only help with the gather.
 template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S>
 __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) {
-    constexpr int NP = Deg<PD>::NP, ND = Deg<PD>::ND, S = S_;
+    constexpr int ND = Deg<PD>::ND, S = S_;
     constexpr int CPT = (ND + S - 1) / S;
     using AT = KT;  // FP64 blocks accumulate in FP64, FP32 blocks in FP32
     AT* s_u = (AT*)smem;
@@ -200,11 +200,7 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
         for (int i = tid; i < nb * ND; i += nthr) {
             const int bb = i / ND, c = i % ND;
             const int64_t q = (int64_t)A.col[b0 + bb] * ND + c;
-            double v;
-            if (MODE == MODE_STEP || MODE == MODE_APPLY || MODE == MODE_KU) v = A.un[q];
-            else if (MODE == MODE_FIRST || MODE == MODE_BILIN) v = A.u0[q];
-            else v = A.u0[q] - A.un[q];
-            s_u[i] = (AT)v;
+            s_u[i] = (AT)((MODE == MODE_FIRST || MODE == MODE_BILIN) ? A.u0[q] : A.un[q]);
         }
         __syncthreads();
         if (act) {

@@ -75,3 +75,39 @@ def test_rhs_of_every_data_combination(require_gpu, p):
             g.COMPUTE_MODAL_COEFFICIENTS_FREE(fun, _lib.SLOT_UEX, 0.5)
             assert not g.get_state(_lib.SLOT_UEX).any()
     o.close()
+
+
+@pytest.mark.parametrize("kind", ["one_poly", "tet_ref_jitter", "bfs_lognormal", "big"])
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+def test_error_norms_of_rough_states(require_gpu, kind, p):
+    """The DG norm by quadrature and the L2 norm, of random coefficients (no
+    cancellation between the terms of the quadratic forms): 1e-11 relative of
+    the oracle's assembled forms (block entries of ~1e4 rounded terms each,
+    1e4 eps = 2e-12, and their mild cancellation in the forms)."""
+    from test_gpu_parity import _mesh
+    m = _big_polyhedron_mesh() if kind == "big" else _mesh(kind)
+    o = Oracle(m, p, 1e-3)
+    o.make_matrices()
+    rng = np.random.default_rng(p)
+    with MatrixFree(m, p, 1e-3) as g:
+        g.MAKE_MATRICES_FREE()
+        for slot in (_lib.SLOT_UN, _lib.SLOT_UEX):
+            u = rng.standard_normal((g.n_poly, g.nd))
+            g.set_state(slot, u)
+            o.set_state(slot, u)
+        for got, ref in ((g.COMPUTE_ERROR_L2_MATRIX_FREE(), o.error_l2(1, 3)), (g.COMPUTE_ERROR_DG_MATRIX_FREE(), o.error_dg(1, 3))):
+            assert abs(got - ref) <= 1e-11 * abs(ref), (got, ref)
+    o.close()
+
+
+@pytest.mark.parametrize("p", [1, 4])
+def test_geometry_of_a_large_polyhedron(require_gpu, p):
+    """Boxes and diameters (a polyhedron of 648 vertex entries reads them from
+    device memory): the oracle's boxes, diameters to the last bit or two."""
+    m = _big_polyhedron_mesh()
+    o = Oracle(m, p, 1e-3)
+    with MatrixFree(m, p, 1e-3) as g:
+        (bb, hk), (rb, rk) = g.poly_geometry(), o.poly_geometry()
+        assert np.array_equal(bb, rb)
+        assert np.abs(hk / rk - 1.0).max() <= 1e-15
+    o.close()
