@@ -276,12 +276,12 @@ int lymph_destroy(lymph_ctx* c) {
     void* ptrs[] = {c->d_coords, c->d_tet_vert, c->d_tet_poly, c->d_tet_mat, c->d_neigh, c->d_fun_tag, c->d_mat,
                     c->d_ref, c->d_fk, c->d_jdet, c->d_normal, c->d_area, c->d_bbox, c->d_hk, c->d_poly_ptr,
                     c->d_poly_tets, c->d_row_ptr, c->d_col, c->d_blk_row, c->d_bf_ptr, c->d_bf, c->d_K, c->d_K32, c->d_M,
-                    c->d_Mm, c->d_R, c->d_Rm, c->d_RT, c->d_RmT, c->d_Minv, c->d_rhs_stat, c->d_rhs_dyn, c->d_buf[0], c->d_buf[1],
+                    c->d_Mm, c->d_R, c->d_Rm, c->d_Minv, c->d_rhs_stat, c->d_rhs_dyn, c->d_buf[0], c->d_buf[1],
                     c->d_v0, c->d_uex, c->d_gvals, c->d_step_idx, c->d_partial, c->d_scalar, c->d_status,
                     c->d_mf_tri, c->d_mf_poly, c->d_mf_u32, c->d_mf_range, c->d_layout};
     for (void* p : ptrs) dfree(p);
     dfree(c->d_layout2);
-    void* absp[] = {c->d_abs_idx, c->d_abs_poly, c->d_abs_ptr, c->d_abs_faces, c->d_Dabs, c->d_Wabs, c->d_Rw, c->d_RwT,
+    void* absp[] = {c->d_abs_idx, c->d_abs_poly, c->d_abs_ptr, c->d_abs_faces, c->d_Dabs, c->d_Wabs, c->d_Rw,
                     c->d_Winv};
     for (void* p : absp) dfree(p);
     if (c->h_status) cudaFreeHost(c->h_status);
@@ -433,7 +433,6 @@ int lymph_create(const lymph_mesh_desc* m, const lymph_params* prm, lymph_ctx** 
         if ((rc = dalloc(c, &c->d_Dabs, nd2))) return fail(rc);
         if ((rc = dalloc(c, &c->d_Wabs, nd2))) return fail(rc);
         if ((rc = dalloc(c, &c->d_Rw, nd2))) return fail(rc);
-        if ((rc = dalloc(c, &c->d_RwT, nd2))) return fail(rc);
         if ((rc = dalloc(c, &c->d_Winv, nd2))) return fail(rc);
     }
     if ((rc = dalloc(c, &c->d_fk, 12 * (size_t)nt))) return fail(rc);
@@ -528,9 +527,7 @@ int lymph_make_matrices(lymph_ctx* c) {
             LYMPH_TRY(dalloc(c, &c->d_M, nm));
             LYMPH_TRY(dalloc(c, &c->d_Mm, nm));
             LYMPH_TRY(dalloc(c, &c->d_R, nm));
-            LYMPH_TRY(dalloc(c, &c->d_RT, nm));
             LYMPH_TRY(dalloc(c, &c->d_Rm, nm));
-            LYMPH_TRY(dalloc(c, &c->d_RmT, nm));
             LYMPH_TRY(dalloc(c, &c->d_Minv, nm));
         }
         c->rhs_version++;
@@ -556,9 +553,7 @@ int lymph_make_matrices(lymph_ctx* c) {
         LYMPH_TRY(dalloc(c, &c->d_M, nm));
         LYMPH_TRY(dalloc(c, &c->d_Mm, nm));
         LYMPH_TRY(dalloc(c, &c->d_R, nm));
-        LYMPH_TRY(dalloc(c, &c->d_RT, nm));
         LYMPH_TRY(dalloc(c, &c->d_Rm, nm));
-        LYMPH_TRY(dalloc(c, &c->d_RmT, nm));
         LYMPH_TRY(dalloc(c, &c->d_Minv, nm));
     }
     c->k32_valid = false;  // an FP32 copy made from earlier blocks is stale

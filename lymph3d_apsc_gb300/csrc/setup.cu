@@ -65,30 +65,56 @@ __global__ void k_geometry(int n_tet, const double* __restrict__ X, const int32_
 }
 
 // CREATE_BBOX_EL (MAKE_PARTITION_AND_MPI_FILES.f90:1510-1580): bounding box
-// and diameter (largest vertex distance) of every polyhedron.
-__global__ void k_bbox(int n_poly, const int32_t* __restrict__ pptr, const int32_t* __restrict__ ptets,
-                       const int32_t* __restrict__ tv, const double* __restrict__ X, double* bbox, double* hk) {
-    int P = blockIdx.x * blockDim.x + threadIdx.x;
+// and diameter (largest vertex distance) of every polyhedron, a warp each.
+// The vertices are gathered once (up to BBOX_V of them, else read again for
+// each pair); the root is taken of the largest squared distance, which is the
+// largest root since the correctly rounded root is monotone.  A thread per
+// polyhedron took 1.17 ms on 11^3 x 6 tets: one dependent chain of loads and
+// roots per polyhedron.
+constexpr int BBOX_WARPS = 4, BBOX_V = 128;
+__global__ void __launch_bounds__(32 * BBOX_WARPS) k_bbox(int n_poly, const int32_t* __restrict__ pptr,
+                                                          const int32_t* __restrict__ ptets,
+                                                          const int32_t* __restrict__ tv, const double* __restrict__ X,
+                                                          double* bbox, double* hk) {
+    __shared__ double s_v[BBOX_WARPS][BBOX_V][3];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, P = blockIdx.x * BBOX_WARPS + wid;
     if (P >= n_poly) return;
-    int t0 = pptr[P], t1 = pptr[P + 1];
+    const int t0 = pptr[P], nv = 4 * (pptr[P + 1] - t0);
+    const bool fits = nv <= BBOX_V;
     double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    int nv = 4 * (t1 - t0);
-    for (int a = 0; a < nv; ++a) {
+    for (int a = lane; a < nv; a += 32) {
         const double* c = &X[tv[ptets[t0 + a / 4] * 4 + (a & 3)] * 3];
-        for (int d = 0; d < 3; ++d) { mn[d] = fmin(mn[d], c[d]); mx[d] = fmax(mx[d], c[d]); }
-    }
-    double h = 0.0;
-    for (int a = 0; a < nv; ++a) {
-        const double* ca = &X[tv[ptets[t0 + a / 4] * 4 + (a & 3)] * 3];
-        for (int b = a + 1; b < nv; ++b) {
-            const double* cb = &X[tv[ptets[t0 + b / 4] * 4 + (b & 3)] * 3];
-            double dist = sqrt((ca[0] - cb[0]) * (ca[0] - cb[0]) + (ca[1] - cb[1]) * (ca[1] - cb[1]) +
-                               (ca[2] - cb[2]) * (ca[2] - cb[2]));
-            if (dist > h) h = dist;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double v = c[d];
+            mn[d] = fmin(mn[d], v);
+            mx[d] = fmax(mx[d], v);
+            if (fits) s_v[wid][a][d] = v;
         }
     }
-    for (int d = 0; d < 3; ++d) { bbox[P * 6 + 2 * d] = mn[d]; bbox[P * 6 + 2 * d + 1] = mx[d]; }
-    hk[P] = h;
+    __syncwarp();
+    double h2 = 0.0;
+    for (int a = lane; a < nv; a += 32) {
+        const double* ca = fits ? s_v[wid][a] : &X[tv[ptets[t0 + a / 4] * 4 + (a & 3)] * 3];
+        const double a0 = ca[0], a1 = ca[1], a2 = ca[2];
+        for (int b = 0; b < a; ++b) {
+            const double* cb = fits ? s_v[wid][b] : &X[tv[ptets[t0 + b / 4] * 4 + (b & 3)] * 3];
+            h2 = fmax(h2, (a0 - cb[0]) * (a0 - cb[0]) + (a1 - cb[1]) * (a1 - cb[1]) + (a2 - cb[2]) * (a2 - cb[2]));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        h2 = fmax(h2, __shfl_xor_sync(0xffffffffu, h2, o));
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
+            mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+        }
+    }
+    if (lane == 0) {
+        for (int d = 0; d < 3; ++d) { bbox[P * 6 + 2 * d] = mn[d]; bbox[P * 6 + 2 * d + 1] = mx[d]; }
+        hk[P] = sqrt(h2);
+    }
 }
 
 // Physical quadrature points of face f of tetrahedron t as basis_boundary
@@ -667,8 +693,8 @@ template <int PD, int WHICH> size_t asm_nb_smem() {
 }
 
 // cholesky (vet_mat_operations.f90:84-120) of the NP x NP matrix of every
-// polyhedron, one warp each; writes R (row-major upper) and R^T.
-__global__ void k_cholesky(int n_poly, int NP, const double* __restrict__ A, double* R, double* RT, int* status) {
+// polyhedron, one warp each; writes R (row-major upper).
+__global__ void k_cholesky(int n_poly, int NP, const double* __restrict__ A, double* R, int* status) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n_poly) return;
     extern __shared__ double shm[];
@@ -678,35 +704,73 @@ __global__ void k_cholesky(int n_poly, int NP, const double* __restrict__ A, dou
     __syncwarp();
     bool ok = true;
     for (int j = 0; j < NP; ++j) {
-        double sum = a[j * NP + j];
-        for (int kk = 0; kk < j; ++kk) sum = sum - r[kk * NP + j] * r[kk * NP + j];
-        if (!(sum > 0.0)) { ok = false; sum = 1.0; }
-        const double rjj = sqrt(sum);
-        for (int i = j + 1 + lane; i < NP; i += 32) {
-            double s = a[j * NP + i];
-            for (int kk = 0; kk < j; ++kk) s = s - r[kk * NP + j] * r[kk * NP + i];
-            r[j * NP + i] = s / rjj;
+        // row j's sums, the diagonal's (lane 0 of the first round) beside the
+        // others: alone, it doubled the chain of FP64 operations
+        double rjj = 1.0;
+        for (int i0 = j; i0 < NP; i0 += 32) {
+            const int i = i0 + lane;
+            double s = i < NP ? a[j * NP + i] : 1.0;
+            if (i < NP)
+                for (int kk = 0; kk < j; ++kk) s = s - r[kk * NP + j] * r[kk * NP + i];
+            if (i0 == j) {
+                double sum = __shfl_sync(0xffffffffu, s, 0);
+                if (!(sum > 0.0)) { ok = false; sum = 1.0; }
+                rjj = sqrt(sum);
+            }
+            if (i < NP) r[j * NP + i] = i == j ? rjj : s / rjj;
         }
-        if (lane == 0) r[j * NP + j] = rjj;
         __syncwarp();
     }
     if (!ok && lane == 0) atomicOr(status, ST_NOT_SPD);
-    for (int i = lane; i < NP * NP; i += 32) {
-        const int row = i / NP, c = i % NP;
-        R[(int64_t)warp * NP * NP + i] = r[i];
-        RT[(int64_t)warp * NP * NP + c * NP + row] = r[i];
+    for (int i = lane; i < NP * NP; i += 32) R[(int64_t)warp * NP * NP + i] = r[i];
+}
+
+// Inverse from a Cholesky factor: column k of the inverse is solve_LU(R^T, R,
+// e_k) (vet_mat_operations.f90:123-153, reference operation order), one lane
+// per column.  Stored column-major: inv[c*NP + r], so that lane r of a warp
+// reads consecutive addresses when applying it.  INV_MATS factors per CTA
+// come into shared memory with the columns being solved (NP <= MAX_NP); a
+// fifth warp solves the columns beyond 31 of all of them, which otherwise
+// cost each matrix a second pass of the whole chain for three lanes.
+constexpr int INV_MATS = 4, INV_THREADS = 32 * (INV_MATS + 1);
+__global__ void __launch_bounds__(INV_THREADS) k_mass_inverse(int n_poly, int NP, const double* __restrict__ R, double* Minv) {
+    extern __shared__ double shm[];
+    const int NP2 = NP * NP, tid = threadIdx.x, P0 = blockIdx.x * INV_MATS;
+    const int nm = n_poly - P0 < INV_MATS ? n_poly - P0 : INV_MATS;
+    double *s_r = shm, *s_x = shm + INV_MATS * NP2;   // factors; columns as [row][column]
+    for (int i = tid; i < nm * NP2; i += INV_THREADS) s_r[i] = R[(int64_t)P0 * NP2 + i];
+    __syncthreads();
+    const int wid = tid >> 5, lane = tid & 31, rest = NP > 32 ? NP - 32 : 0;
+    const int mat = wid < INV_MATS ? wid : (rest ? lane / rest : INV_MATS);
+    const int k = wid < INV_MATS ? lane : (rest ? 32 + lane % rest : NP);
+    if (mat < nm && k < NP) {
+        const double* r = s_r + mat * NP2;
+        double* x = s_x + mat * NP2 + k;
+        for (int i = 0; i < NP; ++i) {
+            double y = (i == k) ? 1.0 : 0.0;
+            for (int j = 0; j < i; ++j) y = y - r[j * NP + i] * x[j * NP];
+            x[i * NP] = y / r[i * NP + i];
+        }
+        for (int i = NP - 1; i >= 0; --i) {
+            double v = x[i * NP];
+            for (int j = i + 1; j < NP; ++j) v = v - r[i * NP + j] * x[j * NP];
+            x[i * NP] = v / r[i * NP + i];
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < nm * NP2; i += INV_THREADS) {
+        const int m = i / NP2, e = i - m * NP2, c = e / NP, row = e - c * NP;
+        Minv[(int64_t)P0 * NP2 + i] = s_x[m * NP2 + row * NP + c];
     }
 }
 
-// Inverse of the mass matrix from its Cholesky factor: column k of M^-1 is
-// solve_LU(R^T, R, e_k) (vet_mat_operations.f90:123-153, reference operation
-// order), one lane per column.  Stored column-major: Minv[c*NP + r] = (M^-1)(r,c),
-// so that lane r of a warp reads consecutive addresses when applying it.
-__global__ void k_mass_inverse(int n_poly, int NP, const double* __restrict__ R, double* Minv) {
+// The same for the larger factors of the absorbing polyhedra (size 3 Np): the
+// columns are solved in place in device memory.
+__global__ void k_inverse_columns(int n, int NP, const double* __restrict__ R, double* inv) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n_poly) return;
+    if (warp >= n) return;
     const double* r = R + (int64_t)warp * NP * NP;
-    double* out = Minv + (int64_t)warp * NP * NP;
+    double* out = inv + (int64_t)warp * NP * NP;
     for (int k = lane; k < NP; k += 32) {
         double* x = out + (int64_t)k * NP;  // column k, solved in place
         for (int i = 0; i < NP; ++i) x[i] = (i == k) ? 1.0 : 0.0;
@@ -808,7 +872,6 @@ struct VecArgs {
     int mode;            // 0 = RHS (MAKE_RHS_FREE), 1 = L2 projection
     int fid, did, nid;   // data function ids
     const double* R;     // modal factor (projection only)
-    const double* RT;
     double scale;
     double* out;         // [n_poly][ND]
 };
@@ -1185,7 +1248,7 @@ int launch_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scal
     A.poly_ptr = c->d_poly_ptr; A.poly_tets = c->d_poly_tets; A.tet_mat = c->d_tet_mat; A.neigh = c->d_neigh;
     A.fun_tag = c->d_fun_tag; A.mat = c->d_mat; A.fk = c->d_fk; A.jdet = c->d_jdet; A.nrm = c->d_normal;
     A.area = c->d_area; A.bbox = c->d_bbox; A.hk = c->d_hk; A.ref = c->d_ref; A.alpha = c->alpha; A.theta = c->theta;
-    A.mode = mode; A.fid = fid; A.did = did; A.nid = nid; A.R = c->d_Rm; A.RT = c->d_RmT; A.scale = scale; A.out = out;
+    A.mode = mode; A.fid = fid; A.did = did; A.nid = nid; A.R = c->d_Rm; A.scale = scale; A.out = out;
     using D = Deg<PD>;
     using V = VecShape<PD>;
     const size_t face = (size_t)D::NQ2 * 3 * (D::NP + PD + 1);   // gradient tables of a boundary face (RHS only)
@@ -1210,7 +1273,7 @@ int lymph_dev_geometry(lymph_ctx* c) {
         LYMPH_CUDA_TRY(cudaGetLastError());
     }
     if (c->n_poly > 0) {
-        k_bbox<<<(c->n_poly + 127) / 128, 128, 0, c->stream>>>(c->n_poly, c->d_poly_ptr, c->d_poly_tets, c->d_tet_vert,
+        k_bbox<<<(c->n_poly + BBOX_WARPS - 1) / BBOX_WARPS, 32 * BBOX_WARPS, 0, c->stream>>>(c->n_poly, c->d_poly_ptr, c->d_poly_tets, c->d_tet_vert,
                                                               c->d_coords, c->d_bbox, c->d_hk);
         c->launches++;
         LYMPH_CUDA_TRY(cudaGetLastError());
@@ -1232,9 +1295,13 @@ int lymph_dev_cholesky(lymph_ctx* c) {
     const int warps_per_block = 4;
     size_t smem = sizeof(double) * warps_per_block * c->Np * c->Np;
     unsigned grid = (unsigned)((c->n_poly + warps_per_block - 1) / warps_per_block);
-    k_cholesky<<<grid, 32 * warps_per_block, smem, c->stream>>>(c->n_poly, c->Np, c->d_M, c->d_R, c->d_RT, c->d_status);
-    k_cholesky<<<grid, 32 * warps_per_block, smem, c->stream>>>(c->n_poly, c->Np, c->d_Mm, c->d_Rm, c->d_RmT, c->d_status);
-    k_mass_inverse<<<grid, 32 * warps_per_block, 0, c->stream>>>(c->n_poly, c->Np, c->d_R, c->d_Minv);
+    k_cholesky<<<grid, 32 * warps_per_block, smem, c->stream>>>(c->n_poly, c->Np, c->d_M, c->d_R, c->d_status);
+    k_cholesky<<<grid, 32 * warps_per_block, smem, c->stream>>>(c->n_poly, c->Np, c->d_Mm, c->d_Rm, c->d_status);
+    const size_t smem_inv = sizeof(double) * 2 * INV_MATS * c->Np * c->Np;
+    // raise (never lower) the dynamic shared-memory limit: other contexts may launch with a larger Np
+    LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_mass_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(sizeof(double) * 2 * INV_MATS * MAX_NP * MAX_NP)));
+    k_mass_inverse<<<(c->n_poly + INV_MATS - 1) / INV_MATS, INV_THREADS, smem_inv, c->stream>>>(c->n_poly, c->Np, c->d_R, c->d_Minv);
     c->launches += 3;
     LYMPH_CUDA_TRY(cudaGetLastError());
     return LYMPH_OK;
@@ -1266,8 +1333,8 @@ int lymph_dev_damping(lymph_ctx* c, bool assemble) {
     // factorisation launches it with up to 4 Np^2 doubles per block
     const size_t lim = smem > (size_t)48 * 1024 ? smem : (size_t)48 * 1024;
     LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
-    k_cholesky<<<c->n_abs, 32, smem, c->stream>>>(c->n_abs, ND, c->d_Wabs, c->d_Rw, c->d_RwT, c->d_status);
-    k_mass_inverse<<<(unsigned)((c->n_abs + 3) / 4), 128, 0, c->stream>>>(c->n_abs, ND, c->d_Rw, c->d_Winv);
+    k_cholesky<<<c->n_abs, 32, smem, c->stream>>>(c->n_abs, ND, c->d_Wabs, c->d_Rw, c->d_status);
+    k_inverse_columns<<<(unsigned)((c->n_abs + 3) / 4), 128, 0, c->stream>>>(c->n_abs, ND, c->d_Rw, c->d_Winv);
     c->launches += 3;
     c->winv_dt = c->dt;
     LYMPH_CUDA_TRY(cudaGetLastError());
