@@ -286,6 +286,7 @@ template <int PD> struct MfSmem {
         double b[S::ND];               // the right-hand side of the M^-1 apply (beside red: the
                                        // last reads of red and the writes of b are not separated
                                        // by a barrier)
+        double x[finish_scratch(S::ND, MF_THREADS)];   // finish_poly's scratch, right behind b
     };
     union Work {
         Loop loop;
@@ -305,6 +306,9 @@ template <int PD> constexpr bool mf_smem_aligned() {
     return offsetof(MfSmem<PD>, uQ) % 16 == 0 && offsetof(MfSmem<PD>, tri) % 16 == 0 &&
            offsetof(MfSmem<PD>, polyQ) % 16 == 0 && sizeof(MfTri) % 16 == 0 && sizeof(MfPoly) % 16 == 0;
 }
+static_assert(offsetof(MfSmem<4>::Fin, x) == offsetof(MfSmem<4>::Fin, b) + sizeof(double) * MfShape<4>::ND &&
+                  offsetof(MfSmem<1>::Fin, x) == offsetof(MfSmem<1>::Fin, b) + sizeof(double) * MfShape<1>::ND,
+              "finish_poly's scratch follows the right-hand side");
 static_assert(mf_smem_aligned<1>() && mf_smem_aligned<2>() && mf_smem_aligned<3>() && mf_smem_aligned<4>(),
               "cp.async destinations must be 16-byte aligned");
 
@@ -335,6 +339,14 @@ __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, int
         if (MODE == MODE_STEP || MODE == MODE_FIRST) {
             prefetch_l2(sa.rhs_stat, sb, sa.rhs_stat + (int64_t)P * ND, vb);
             prefetch_l2(sa.rhs_dyn, sb, sa.rhs_dyn + (int64_t)P * ND, vb);
+        }
+        if ((MODE == MODE_STEP || MODE == MODE_FIRST) && sa.abs_idx) {
+            const int ai = sa.abs_idx[P];
+            if (ai >= 0) {
+                const int64_t db = (int64_t)ND * ND * 8;
+                prefetch_l2(sa.Dabs, (ai + 1) * db, sa.Dabs + (int64_t)ai * ND * ND, db);
+                if (MODE == MODE_STEP) prefetch_l2(sa.Winv, (ai + 1) * db, sa.Winv + (int64_t)ai * ND * ND, db);
+            }
         }
         prefetch_l2(sa.u0, sb, sa.u0 + (int64_t)P * ND, vb);
         prefetch_l2(sa.un, sb, sa.un + (int64_t)P * ND, vb);
