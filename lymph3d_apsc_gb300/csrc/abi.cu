@@ -28,14 +28,15 @@ int lymph_dev_mass(lymph_ctx* c);
 int lymph_dev_self_tc(lymph_ctx* c, float* out, bool block_csr);
 int lymph_dev_nb_tc(lymph_ctx* c, float* out, const int64_t* list, int64_t n_list);
 int lymph_dev_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scale, double* out);
-int lymph_dev_step(lymph_ctx* c, bool bump);
-int lymph_dev_first_step(lymph_ctx* c);
+int lymph_dev_step(lymph_ctx* c, int off, double g, bool fresh);
+int lymph_dev_run_start(lymph_ctx* c);
+int lymph_dev_first_step(lymph_ctx* c, double g);
 int lymph_dev_apply(lymph_ctx* c, const double* u, double* out);
 int lymph_dev_ku(lymph_ctx* c, const double* u, double* out);
 int lymph_dev_double_couple(lymph_ctx* c, int t, int P, const double moment[9], double* out);
 int lymph_dev_power_iteration(lymph_ctx* c, double* x, double* y, double* d_ss, int iters);
 int lymph_dev_point_source(lymph_ctx* c, int P, const double x0[3], const double dir[3], double* out);
-int lymph_dev_bump(lymph_ctx* c);
+int lymph_dev_bump(lymph_ctx* c, int n);
 int lymph_dev_error_dg(lymph_ctx* c, const double* uh, const double* uex, double* d_out);
 int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double* d_out);
 int lymph_dev_energy(lymph_ctx* c, const double* ua, const double* ub, double* d_out);
@@ -146,12 +147,6 @@ void dfree(void* p) {
 
 double time_function(double t) { return std::sin(std::sqrt(2.0) * PI * t); }  // problem_data_and_properties.f90:14-23
 
-int set_g(lymph_ctx* c, double g) {
-    LYMPH_CUDA_TRY(cudaMemcpyAsync(c->d_gvals, &g, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    LYMPH_CUDA_TRY(cudaMemsetAsync(c->d_step_idx, 0, sizeof(int64_t), c->stream));
-    return LYMPH_OK;
-}
-
 bool valid_slot(int s) { return s >= 0 && s < LYMPH_NUM_SLOTS; }
 
 // FNV-1a (64-bit) over byte ranges: identifies the mesh a checkpoint belongs to.
@@ -243,9 +238,9 @@ double* lymph_slot_ptr(lymph_ctx* c, int slot) {
 int status_rc(lymph_ctx* c, int st, const char* where);
 
 int lymph_sync_status(lymph_ctx* c, const char* where) {
-    LYMPH_CUDA_TRY(cudaStreamSynchronize(c->stream));
     int st = 0;
-    LYMPH_CUDA_TRY(cudaMemcpy(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+    LYMPH_CUDA_TRY(cudaMemcpyAsync(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    LYMPH_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return status_rc(c, st, where);
 }
 
@@ -278,7 +273,7 @@ int lymph_destroy(lymph_ctx* c) {
                     c->d_poly_tets, c->d_row_ptr, c->d_col, c->d_blk_row, c->d_bf_ptr, c->d_bf, c->d_K, c->d_K32, c->d_M,
                     c->d_Mm, c->d_R, c->d_Rm, c->d_Minv, c->d_rhs_stat, c->d_rhs_dyn, c->d_buf[0], c->d_buf[1],
                     c->d_v0, c->d_uex, c->d_gvals, c->d_step_idx, c->d_partial, c->d_scalar, c->d_status,
-                    c->d_mf_tri, c->d_mf_poly, c->d_mf_u32, c->d_mf_range, c->d_layout};
+                    c->d_mf_tri, c->d_mf_poly, c->d_mf_u32[0], c->d_mf_u32[1], c->d_mf_range, c->d_layout};
     for (void* p : ptrs) dfree(p);
     dfree(c->d_layout2);
     void* absp[] = {c->d_abs_idx, c->d_abs_poly, c->d_abs_ptr, c->d_abs_faces, c->d_Dabs, c->d_Wabs, c->d_Rw,
@@ -595,8 +590,7 @@ int lymph_first_step(lymph_ctx* c, double t) {
     NvtxRange nvtx_("lymph_first_step");
     if (!c) return LYMPH_ERR_INVALID;
     if (!c->have_matrices) { lymph_set_error("lymph_first_step: call lymph_make_matrices first"); return LYMPH_ERR_ORDER; }
-    LYMPH_TRY(set_g(c, time_function(t)));
-    LYMPH_TRY(lymph_dev_first_step(c));
+    LYMPH_TRY(lymph_dev_first_step(c, time_function(t)));
     return lymph_sync_status(c, "lymph_first_step");
 }
 
@@ -604,8 +598,7 @@ int lymph_step(lymph_ctx* c, double t) {
     NvtxRange nvtx_("lymph_step");
     if (!c) return LYMPH_ERR_INVALID;
     if (!c->have_matrices) { lymph_set_error("lymph_step: call lymph_make_matrices first"); return LYMPH_ERR_ORDER; }
-    LYMPH_TRY(set_g(c, time_function(t)));
-    LYMPH_TRY(lymph_dev_step(c, false));
+    LYMPH_TRY(lymph_dev_step(c, -1, time_function(t), false));
     c->cur ^= 1;
     return lymph_sync_status(c, "lymph_step");
 }
@@ -636,8 +629,7 @@ int lymph_time_step_host(lymph_ctx* c, double t, const double* u0, const double*
     if (fort) LYMPH_TRY(transpose(c, c->d_layout, d_un, c->nd, c->n_poly, c->stream));
     LYMPH_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->ev_copy, 0));
     // TIME_STEP_MATRIX_FREE
-    LYMPH_TRY(set_g(c, time_function(t)));
-    LYMPH_TRY(lymph_dev_step(c, false));
+    LYMPH_TRY(lymph_dev_step(c, -1, time_function(t), false));
     c->cur ^= 1;
     // u^{n+1} down and the status word, then one synchronisation
     const double* d_out = lymph_slot_ptr(c, LYMPH_SLOT_UN);
@@ -654,16 +646,14 @@ int lymph_time_step_host(lymph_ctx* c, double t, const double* u0, const double*
 int lymph_first_step_g(lymph_ctx* c, double g) {
     if (!c || !std::isfinite(g)) return LYMPH_ERR_INVALID;
     if (!c->have_matrices) { lymph_set_error("lymph_first_step_g: call lymph_make_matrices first"); return LYMPH_ERR_ORDER; }
-    LYMPH_TRY(set_g(c, g));
-    LYMPH_TRY(lymph_dev_first_step(c));
+    LYMPH_TRY(lymph_dev_first_step(c, g));
     return lymph_sync_status(c, "lymph_first_step_g");
 }
 
 int lymph_step_g(lymph_ctx* c, double g) {
     if (!c || !std::isfinite(g)) return LYMPH_ERR_INVALID;
     if (!c->have_matrices) { lymph_set_error("lymph_step_g: call lymph_make_matrices first"); return LYMPH_ERR_ORDER; }
-    LYMPH_TRY(set_g(c, g));
-    LYMPH_TRY(lymph_dev_step(c, false));
+    LYMPH_TRY(lymph_dev_step(c, -1, g, false));
     c->cur ^= 1;
     return lymph_sync_status(c, "lymph_step_g");
 }
@@ -697,7 +687,7 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
     cudaEvent_t e0, e1;
     LYMPH_CUDA_TRY(cudaEventCreate(&e0));
     LYMPH_CUDA_TRY(cudaEventCreate(&e1));
-    int rc = LYMPH_OK;
+    int rc = lymph_dev_run_start(c);
     if (ms_kernel) {
         // per-launch events around every step kernel (no graph)
         std::vector<cudaEvent_t> ev(2 * n);
@@ -705,9 +695,9 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
         cudaEventRecord(e0, c->stream);
         for (int64_t i = 0; i < n && rc == LYMPH_OK; ++i) {
             cudaEventRecord(ev[2 * i], c->stream);
-            rc = lymph_dev_step(c, false);
+            rc = lymph_dev_step(c, 0, 0.0, true);
             cudaEventRecord(ev[2 * i + 1], c->stream);
-            if (rc == LYMPH_OK) rc = lymph_dev_bump(c);
+            if (rc == LYMPH_OK) rc = lymph_dev_bump(c, 1);
             c->cur ^= 1;
         }
         cudaEventRecord(e1, c->stream);
@@ -720,7 +710,7 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
         }
         *ms_kernel = sum;
         for (auto& e : ev) cudaEventDestroy(e);
-    } else {
+    } else if (rc == LYMPH_OK) {
         const int R = 16;  // steps per graph (even: returns to the same buffer parity)
         if (c->graph_exec && (c->graph_steps != R || c->graph_parity != c->cur)) {
             cudaGraphExecDestroy(c->graph_exec);
@@ -735,9 +725,10 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
                 LYMPH_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
                 int64_t l0 = c->launches;
                 for (int j = 0; j < R; ++j) {
-                    lymph_dev_step(c, true);
+                    lymph_dev_step(c, j, 0.0, true);
                     c->cur ^= 1;
                 }
+                lymph_dev_bump(c, R);
                 c->graph_launches = c->launches - l0;
                 c->launches = l0;
                 cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
@@ -757,8 +748,8 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
                 c->launches += c->graph_launches;
             }
         }
-        for (; i < n; ++i) {
-            LYMPH_TRY(lymph_dev_step(c, true));
+        for (int off = 0; i < n; ++i, ++off) {  // the rest: step_idx stands at a multiple of R
+            LYMPH_TRY(lymph_dev_step(c, off, 0.0, true));
             c->cur ^= 1;
         }
         cudaEventRecord(e1, c->stream);

@@ -7,10 +7,11 @@
 // into one work list.  A persistent grid of CTAs pulls items from an atomic
 // queue and runs the same per-polyhedron body as the single-problem kernel
 // (step_body.cuh) with the degree of the item's problem, so results are
-// bit-identical to stepping each context alone.  A 1-thread kernel after
-// each step advances the step counter (which selects each problem's buffer
-// parity and time-function value) and resets the queue; the loop is launched
-// as CUDA graphs of 16 steps.  The grid size and the item order (largest
+// bit-identical to stepping each context alone.  A step's index (which selects
+// each problem's buffer parity and time-function value) is the step counter
+// plus its place in the graph; a 1-thread kernel beside each step clears the
+// next one's queue and the graph's last one moves the counter on.  The loop is
+// launched as CUDA graphs of 16 steps.  The grid size and the item order (largest
 // cost first or problem-major) are picked by a timing autotuner whose choice
 // is cached per batch signature.  The autotuner also picks the tile shape:
 // the number of column slices S per degree (kBatchShapes).  Shape 0, the
@@ -18,8 +19,8 @@
 // bit-identical to stepping each context alone; the other shapes group the
 // row's partial sums differently (deterministic, equal to rounding).  On the
 // matrix-free path (mf.cu) the items are grouped by degree and each degree
-// present gets its own persistent launch per step, so every degree runs
-// with its own register and shared-memory budget.
+// present gets its own persistent launch per step, side by side, so every
+// degree runs with its own register and shared-memory budget.
 
 #include <algorithm>
 #include <cstdlib>
@@ -39,8 +40,11 @@ using namespace stepk;
 size_t lymph_mf_batch_problem_bytes();
 int lymph_mf_batch_ctas_per_sm(int p);
 void lymph_mf_batch_problem(const lymph_ctx* c, int* status, void* out);
-int lymph_mf_batch_step(cudaStream_t st, const int* grid, const void* probs, const int2* items, const int* off,
-                        int* queue, const int64_t* step_idx, const double* gvals, int64_t g_stride, int* launched);
+int lymph_mf_batch_u32(cudaStream_t st, const void* probs, const int2* items, int n_items, const int64_t* step_idx,
+                       int step_off);
+int lymph_mf_batch_step(const cudaStream_t* st, const int* grid, const void* probs, const int2* items, const int* off,
+                        int* queue, const int64_t* step_idx, int step_off, const double* gvals, int64_t g_stride,
+                        int* launched);
 
 namespace {
 
@@ -76,10 +80,10 @@ static_assert(Deg<1>::ND * kBatchShapes[2][1] <= BATCH_THREADS && Deg<2>::ND * k
 template <typename KT, int V>
 __global__ void __launch_bounds__(BATCH_THREADS, BATCH_MINB)
 k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ items, int n_items, int* queue,
-             const int64_t* step_idx, const double* gvals, int64_t g_stride) {
+             const int64_t* step_idx, int off, const double* gvals, int64_t g_stride) {
     __shared__ __align__(16) char smem[BatchSmem<KT>::bytes];
     __shared__ int s_item;
-    const int64_t k = *step_idx;
+    const int64_t k = *step_idx + off;   // off: the step's place in the graph
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
         __syncthreads();
@@ -94,6 +98,7 @@ k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ it
         A.out = probs[w.x].buf[cur ^ 1];
         A.gvals = gvals + (int64_t)w.x * g_stride;
         A.step_idx = step_idx;
+        A.step_off = off;
         switch (probs[w.x].p) {
             case 1: step_poly<1, KT, MODE_STEP, kBatchShapes[V][1]>(A, w.y, smem); break;
             case 2: step_poly<2, KT, MODE_STEP, kBatchShapes[V][2]>(A, w.y, smem); break;
@@ -103,8 +108,10 @@ k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ it
     }
 }
 
-__global__ void k_batch_bump(int64_t* idx, int* queue) {
-    *idx += 1;
+// Clears the item counters of the next step and moves the step counter on by n
+// (0 but at the end of a graph).
+__global__ void k_batch_bump(int64_t* idx, int n, int* queue) {
+    *idx += n;
     for (int i = 0; i < BATCH_QUEUES; ++i) queue[i] = 0;
 }
 
@@ -153,7 +160,12 @@ struct lymph_batch {
     int order = 0;       // 0 = largest cost first, 1 = problem-major
     int grid = 0;
     int shape = 0;       // tile shape (kBatchShapes row) of the FP64 / FP32-block kernel
-    int* d_queue = nullptr;          // BATCH_QUEUES item counters (one per degree on the matrix-free path)
+    int* d_queue = nullptr;          // two sets of BATCH_QUEUES item counters (one per degree on the matrix-free
+                                     // path), for the steps of even and odd place in a graph
+    // the passes of a step that run beside the first (degrees on the
+    // matrix-free path, the counters' reset) and what orders them
+    cudaStream_t side[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_join[4] = {nullptr, nullptr, nullptr, nullptr};
     int mf_off[5] = {0, 0, 0, 0, 0};  // matrix-free path: degree p's items are [mf_off[p - 1], mf_off[p])
     int mf_occ[4] = {1, 1, 1, 1};     // matrix-free path: CTAs per SM of each degree's kernel
     int64_t* d_step_idx = nullptr;
@@ -226,9 +238,9 @@ int refresh_problems(lymph_batch* b) {
 }
 
 template <typename KT>
-void launch_shape(lymph_batch* b, const BatchProblem* probs, int64_t g_stride) {
+void launch_shape(lymph_batch* b, const BatchProblem* probs, int off, int* queue, int64_t g_stride) {
     auto go = [&](auto kernel) {
-        kernel<<<b->grid, BATCH_THREADS, 0, b->stream>>>(probs, b->d_items, b->n_items, b->d_queue, b->d_step_idx,
+        kernel<<<b->grid, BATCH_THREADS, 0, b->stream>>>(probs, b->d_items, b->n_items, queue, b->d_step_idx, off,
                                                          b->d_gvals, g_stride);
     };
     switch (b->shape) {
@@ -238,25 +250,57 @@ void launch_shape(lymph_batch* b, const BatchProblem* probs, int64_t g_stride) {
     }
 }
 
-int launch_step(lymph_batch* b, int64_t g_stride) {
+// The step at place `off` of a graph (or of the steps launched one by one after
+// the last graph); bump: what the step counter moves on by after it.  The
+// passes of the degrees present run side by side, each on a stream of its own
+// (one after another, each left most SMs idle on small problems: 79 us a step
+// of 32 problems of 3^3..8^3 x 6 tetrahedra), and the item counters of the next
+// step are cleared beside them.
+int launch_step(lymph_batch* b, int64_t g_stride, int off, int bump) {
     const BatchProblem* probs = (const BatchProblem*)b->d_probs;
+    int* queue = b->d_queue + BATCH_QUEUES * (off & 1);
+    int* next = b->d_queue + BATCH_QUEUES * ((off + 1) & 1);
     int nl = 1;
-    if (b->precision == LYMPH_MIXED_MF) {
+    const bool mf = b->precision == LYMPH_MIXED_MF;
+    if (mf) LYMPH_TRY(lymph_mf_batch_u32(b->stream, b->d_probs, b->d_items, b->n_items, b->d_step_idx, off));
+    LYMPH_CUDA_TRY(cudaEventRecord(b->ev_fork, b->stream));
+    bool used[4] = {false, false, false, bump == 0};   // side[3] clears the counters unless the step counter moves
+    if (used[3]) {
+        LYMPH_CUDA_TRY(cudaStreamWaitEvent(b->side[3], b->ev_fork, 0));
+        k_batch_bump<<<1, 1, 0, b->side[3]>>>(b->d_step_idx, 0, next);
+    }
+    if (mf) {
         // per degree: the tuned grid, at most what the SMs hold of that
         // degree's kernel and at most one CTA per item
-        int grid[4];
+        int grid[4], n_side = 0;
+        cudaStream_t st[4];
+        bool first = true;
         for (int p = 1; p <= 4; ++p) {
             const int n = b->mf_off[p] - b->mf_off[p - 1];
             grid[p - 1] = std::min(std::min(b->grid, b->mf_occ[p - 1] * b->sms), n);
+            st[p - 1] = b->stream;
+            if (n <= 0) continue;
+            if (!first) {
+                used[n_side] = true;
+                st[p - 1] = b->side[n_side++];
+                LYMPH_CUDA_TRY(cudaStreamWaitEvent(st[p - 1], b->ev_fork, 0));
+            }
+            first = false;
         }
-        LYMPH_TRY(lymph_mf_batch_step(b->stream, grid, b->d_probs, b->d_items, b->mf_off, b->d_queue, b->d_step_idx,
-                                      b->d_gvals, g_stride, &nl));
+        LYMPH_TRY(lymph_mf_batch_step(st, grid, b->d_probs, b->d_items, b->mf_off, queue, b->d_step_idx, off, b->d_gvals,
+                                      g_stride, &nl));
+        ++nl;   // the FP32 copies
     } else if (b->precision == LYMPH_MIXED) {
-        launch_shape<float>(b, probs, g_stride);
+        launch_shape<float>(b, probs, off, queue, g_stride);
     } else {
-        launch_shape<double>(b, probs, g_stride);
+        launch_shape<double>(b, probs, off, queue, g_stride);
     }
-    k_batch_bump<<<1, 1, 0, b->stream>>>(b->d_step_idx, b->d_queue);
+    for (int i = 0; i < 4; ++i)
+        if (used[i]) {
+            LYMPH_CUDA_TRY(cudaEventRecord(b->ev_join[i], b->side[i]));
+            LYMPH_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join[i], 0));
+        }
+    if (bump) k_batch_bump<<<1, 1, 0, b->stream>>>(b->d_step_idx, bump, next);
     b->step_nl = nl + 1;
     b->launches += b->step_nl;
     LYMPH_CUDA_TRY(cudaGetLastError());
@@ -268,7 +312,7 @@ int launch_step(lymph_batch* b, int64_t g_stride) {
 int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, bool use_graph) {
     LYMPH_TRY(refresh_problems(b));
     LYMPH_CUDA_TRY(cudaMemsetAsync(b->d_step_idx, 0, sizeof(int64_t), b->stream));
-    LYMPH_CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, BATCH_QUEUES * sizeof(int), b->stream));
+    LYMPH_CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, 2 * BATCH_QUEUES * sizeof(int), b->stream));
     const int R = 16;
     int64_t i = 0;
     if (use_graph && n >= R) {
@@ -277,7 +321,7 @@ int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, bool use_graph) {
             cudaGraph_t g;
             LYMPH_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
             int64_t l0 = b->launches;
-            for (int j = 0; j < R; ++j) launch_step(b, g_stride);
+            for (int j = 0; j < R; ++j) launch_step(b, g_stride, j, j == R - 1 ? R : 0);
             b->launches = l0;
             cudaError_t e = cudaStreamEndCapture(b->stream, &g);
             if (e != cudaSuccess) { lymph_set_error(std::string("batch graph capture: ") + cudaGetErrorString(e)); return LYMPH_ERR_CUDA; }
@@ -291,7 +335,7 @@ int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, bool use_graph) {
             b->launches += (int64_t)b->step_nl * R;
         }
     }
-    for (; i < n; ++i) LYMPH_TRY(launch_step(b, g_stride));
+    for (int off = 0; i < n; ++i, ++off) LYMPH_TRY(launch_step(b, g_stride, off, 0));
     // each problem's buffers flipped n times
     if (n & 1)
         for (lymph_ctx* c : b->ctx) c->cur ^= 1;
@@ -343,6 +387,11 @@ int lymph_batch_create(lymph_ctx* const* ctxs, int32_t n, lymph_batch** out) {
     b->precision = ctxs[0]->precision;
     auto fail = [&](int rc) { lymph_batch_destroy(b); return rc; };
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) { delete b; lymph_set_error("lymph_batch_create: stream"); return LYMPH_ERR_CUDA; }
+    bool made = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; i < 4; ++i)
+        made = made && cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking) == cudaSuccess &&
+               cudaEventCreateWithFlags(&b->ev_join[i], cudaEventDisableTiming) == cudaSuccess;
+    if (!made) { lymph_set_error("lymph_batch_create: stream"); return fail(LYMPH_ERR_CUDA); }
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -368,7 +417,7 @@ int lymph_batch_create(lymph_ctx* const* ctxs, int32_t n, lymph_batch** out) {
     const size_t prob_bytes = b->precision == LYMPH_MIXED_MF ? lymph_mf_batch_problem_bytes() : sizeof(BatchProblem);
     if (cudaMalloc(&b->d_probs, prob_bytes * n) != cudaSuccess ||
         cudaMalloc(&b->d_items, sizeof(int2) * b->n_items) != cudaSuccess ||
-        cudaMalloc(&b->d_queue, BATCH_QUEUES * sizeof(int)) != cudaSuccess || cudaMalloc(&b->d_step_idx, sizeof(int64_t)) != cudaSuccess ||
+        cudaMalloc(&b->d_queue, 2 * BATCH_QUEUES * sizeof(int)) != cudaSuccess || cudaMalloc(&b->d_step_idx, sizeof(int64_t)) != cudaSuccess ||
         cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess) {
         lymph_set_error("lymph_batch_create: device allocation failed");
         return fail(LYMPH_ERR_OOM);
@@ -394,6 +443,11 @@ int lymph_batch_destroy(lymph_batch* b) {
     for (void* p : {(void*)b->d_probs, (void*)b->d_items, (void*)b->d_queue, (void*)b->d_step_idx, (void*)b->d_gvals,
                     (void*)b->d_status})
         if (p) cudaFree(p);
+    for (int i = 0; i < 4; ++i) {
+        if (b->side[i]) cudaStreamDestroy(b->side[i]);
+        if (b->ev_join[i]) cudaEventDestroy(b->ev_join[i]);
+    }
+    if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return LYMPH_OK;

@@ -108,7 +108,7 @@ struct lymph_ctx {
     // bounding box, mf_quad the triangle quadrature (xi, eta, w)
     void* d_mf_tri = nullptr;
     void* d_mf_poly = nullptr;
-    void* d_mf_u32 = nullptr;       // the operator input in FP32, [n_poly][Np] x 4
+    void* d_mf_u32[2] = {nullptr, nullptr};   // the operator input in FP32, [n_poly][Np] x 4: copies of d_buf[0], d_buf[1]
     void* d_mf_range = nullptr;     // per polyhedron: its triangles' range and neighbours (mf.cu k_mf_qrec)
     float mf_quad[3 * 25] = {};
     double *d_rhs_stat = nullptr, *d_rhs_dyn = nullptr;

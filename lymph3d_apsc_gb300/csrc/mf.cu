@@ -228,9 +228,7 @@ struct MfArgs {
     const int32_t* qrec;        // per polyhedron MF_REC ints: triangle range and neighbours (k_mf_qrec)
     const MfTri* tri;           // parallel to the block face lists
     const MfPoly* poly;         // [n_poly]
-    const float4* u32;          // operator input in FP32: [n_poly][Np] (u_0, u_1, u_2, 0)
-    int64_t kself_bytes;        // size of Kself
-    int64_t minv_bytes;         // size of the M^-1 array
+    const float4* u32;          // operator input in FP32 (k_mf)
     float quad[3 * MF_FACE_NQ_MAX];   // (xi, eta, w) of the triangle rule's nodes
     float theta;
 };
@@ -248,16 +246,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Prefetch [p, p + bytes) of an allocation [base, base + total) into L2 (one
-// bulk prefetch, range widened to 16-byte bounds inside the allocation).
-__device__ __forceinline__ void prefetch_l2(const void* base, int64_t total, const void* p, int64_t bytes) {
-    const uintptr_t b0 = (uintptr_t)base, lim = (b0 + (uintptr_t)total) & ~(uintptr_t)15;
-    uintptr_t s = (uintptr_t)p & ~(uintptr_t)15, e = ((uintptr_t)p + (uintptr_t)bytes + 15) & ~(uintptr_t)15;
-    if (e > lim) e = lim;
-    if (s < b0 || e <= s) return;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s), "r"((uint32_t)(e - s)) : "memory");
-}
 
 // One CTA per polyhedron P.  At the start the CTA reads P's record (its
 // triangles' range and neighbours, one coalesced load), and one thread
@@ -314,9 +302,10 @@ static_assert(mf_smem_aligned<1>() && mf_smem_aligned<2>() && mf_smem_aligned<3>
 
 // The pass of polyhedron P (every thread of the CTA calls it; it
 // synchronises): the per-problem tables come from A, the state, right-hand
-// sides and M^-1 from sa.
+// sides and M^-1 from sa, the operator input in FP32, [n_poly][Np]
+// (u_0, u_1, u_2, 0), from u32.
 template <int PD, int MODE>
-__device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, int P, char* smem) {
+__device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, const float4* u32, int P, char* smem) {
     using S = MfShape<PD>;
     constexpr int NP = S::NP, ND = S::ND, L = S::L, NQ2 = S::NQ2, CT = S::CT, NP2 = NP * NP;
     MfSmem<PD>& sm = *reinterpret_cast<MfSmem<PD>*>(smem);
@@ -332,28 +321,27 @@ __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, int
     // so the first chunk's staging waits on one global round trip, not three
     if (tid < MF_REC) sm.rec[tid] = A.qrec[(int64_t)P * MF_REC + tid];
     if (tid == 0) {
-        const int64_t nb = (int64_t)ND * ND * 4, vb = (int64_t)ND * 8;
-        prefetch_l2(A.Kself, A.kself_bytes, A.Kself + (int64_t)P * ND * ND, nb);
-        prefetch_l2(sa.Minv, A.minv_bytes, sa.Minv + (int64_t)P * NP2, (int64_t)NP2 * 8);
-        const int64_t sb = (int64_t)sa.n_poly * ND * 8;
+        const int64_t vb = (int64_t)ND * 8;
+        prefetch_inside(A.Kself + (int64_t)P * ND * ND, (int64_t)ND * ND * 4);
+        prefetch_inside(sa.Minv + (int64_t)P * NP2, (int64_t)NP2 * 8);
         if (MODE == MODE_STEP || MODE == MODE_FIRST) {
-            prefetch_l2(sa.rhs_stat, sb, sa.rhs_stat + (int64_t)P * ND, vb);
-            prefetch_l2(sa.rhs_dyn, sb, sa.rhs_dyn + (int64_t)P * ND, vb);
+            prefetch_inside(sa.rhs_stat + (int64_t)P * ND, vb);
+            prefetch_inside(sa.rhs_dyn + (int64_t)P * ND, vb);
         }
         if ((MODE == MODE_STEP || MODE == MODE_FIRST) && sa.abs_idx) {
             const int ai = sa.abs_idx[P];
             if (ai >= 0) {
-                const int64_t db = (int64_t)ND * ND * 8;
-                prefetch_l2(sa.Dabs, (ai + 1) * db, sa.Dabs + (int64_t)ai * ND * ND, db);
-                if (MODE == MODE_STEP) prefetch_l2(sa.Winv, (ai + 1) * db, sa.Winv + (int64_t)ai * ND * ND, db);
+                prefetch_inside(sa.Dabs + (int64_t)ai * ND * ND, (int64_t)ND * ND * 8);
+                if (MODE == MODE_STEP) prefetch_inside(sa.Winv + (int64_t)ai * ND * ND, (int64_t)ND * ND * 8);
             }
         }
-        prefetch_l2(sa.u0, sb, sa.u0 + (int64_t)P * ND, vb);
-        prefetch_l2(sa.un, sb, sa.un + (int64_t)P * ND, vb);
+        prefetch_inside(sa.u0 + (int64_t)P * ND, vb);
+        prefetch_inside(sa.un + (int64_t)P * ND, vb);
     }
     for (int i = tid; i < 3 * NQ2; i += MF_THREADS) s_quad[i] = A.quad[i];
+    if (MODE == MODE_STEP) pdl_wait();
     for (int i = tid; i < ND; i += MF_THREADS) {
-        const float4 w = A.u32[(int64_t)P * NP + i % NP];
+        const float4 w = u32[(int64_t)P * NP + i % NP];
         const int comp = i / NP;
         s_uP[i] = comp == 0 ? w.x : (comp == 1 ? w.y : w.z);
     }
@@ -370,7 +358,7 @@ __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, int
         for (int i = tid; i < nt; i += MF_THREADS) cp_async16(&s_polyQ[b][i], A.poly + getQ(c + i));
         for (int i = tid; i < nt * NP; i += MF_THREADS) {
             const int t = i / NP, bb = i - t * NP;
-            cp_async16(&s_uQ[b][t][bb], A.u32 + (int64_t)getQ(c + t) * NP + bb);
+            cp_async16(&s_uQ[b][t][bb], u32 + (int64_t)getQ(c + t) * NP + bb);
         }
         cp_async_commit();
     };
@@ -512,7 +500,7 @@ __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, int
         for (int kk = 0; kk < MF_SLOTS; ++kk) t += s_w.fin.red[kk][tid];
         y = (double)yself + (double)t;
     }
-    finish_poly<PD, MODE>(sa, P, y, s_b);
+    finish_poly<PD, MODE, true>(sa, P, y, s_b);
 }
 
 // CTAs per SM that the register budget is sized for, per degree (index p;
@@ -525,7 +513,7 @@ constexpr int MF_BATCH_MINB[5] = {5, 8, 8, 7, 5};   // the same for k_mf_batch<p
 template <int PD, int MODE>
 __global__ void __launch_bounds__(MF_THREADS, MF_MINB[PD]) k_mf(const __grid_constant__ MfArgs A) {
     __shared__ __align__(16) char smem[sizeof(MfSmem<PD>)];
-    mf_poly<PD, MODE>(A, A.s, blockIdx.x, smem);
+    mf_poly<PD, MODE>(A, A.s, A.u32, blockIdx.x, smem);
 }
 
 // ---- many problems in one persistent launch per step (lymph_batch) ----
@@ -542,13 +530,14 @@ struct MfBatchProblem {
 // so results equal stepping each problem alone.  One launch per degree
 // present, so each degree runs with its own register and shared-memory
 // budget (the CTAs per SM of k_mf).
+// off: the step's place in the graph (its index is *step_idx + off).
 template <int PD>
 __global__ void __launch_bounds__(MF_THREADS, MF_BATCH_MINB[PD])
 k_mf_batch(const MfBatchProblem* __restrict__ probs, const int2* __restrict__ items, int n_items, int* queue,
-           const int64_t* step_idx, const double* gvals, int64_t g_stride) {
+           const int64_t* step_idx, int off, const double* gvals, int64_t g_stride) {
     __shared__ __align__(16) char smem[sizeof(MfSmem<PD>)];
     __shared__ int s_item;
-    const int64_t k = *step_idx;
+    const int64_t k = *step_idx + off;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
         __syncthreads();
@@ -564,14 +553,15 @@ k_mf_batch(const MfBatchProblem* __restrict__ probs, const int2* __restrict__ it
         s.out = pb.buf[cur ^ 1];
         s.gvals = gvals + (int64_t)w.x * g_stride;
         s.step_idx = step_idx;
-        mf_poly<PD, MODE_STEP>(pb.a, s, w.y, smem);
+        s.step_off = off;
+        mf_poly<PD, MODE_STEP>(pb.a, s, pb.a.u32, w.y, smem);
     }
 }
 
 // The FP32 copies of every problem's u^n, a warp per (problem, polyhedron) item.
 __global__ void k_mf_u32_batch(const MfBatchProblem* __restrict__ probs, const int2* __restrict__ items, int n_items,
-                               const int64_t* step_idx) {
-    const int64_t k = *step_idx;
+                               const int64_t* step_idx, int off) {
+    const int64_t k = *step_idx + off;
     const int item = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (item >= n_items) return;
     const int2 w = items[item];
@@ -583,7 +573,8 @@ __global__ void k_mf_u32_batch(const MfBatchProblem* __restrict__ probs, const i
 }
 
 // u32[P][m] = (u[P][0][m], u[P][1][m], u[P][2][m], 0): the operator input in
-// FP32, converted once per pass instead of once per triangle that reads it.
+// FP32, converted once instead of once per triangle that reads it (before a
+// single pass and the first of a run; each step leaves the next one's copy).
 __global__ void k_mf_u32(int64_t n, int NP, const double* __restrict__ u, float4* __restrict__ u32) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t P = i / NP, m = i - P * NP;
@@ -685,35 +676,48 @@ MfArgs mf_args(const lymph_ctx* c, const StepArgs& s) {
     a.qrec = (const int32_t*)c->d_mf_range;
     a.tri = (const MfTri*)c->d_mf_tri;
     a.poly = (const MfPoly*)c->d_mf_poly;
-    a.u32 = (const float4*)c->d_mf_u32;
-    a.kself_bytes = (int64_t)c->n_poly * c->nd * c->nd * (int64_t)sizeof(float);
-    a.minv_bytes = (int64_t)c->n_poly * c->Np * c->Np * (int64_t)sizeof(double);
+    a.u32 = (const float4*)c->d_mf_u32[0];
     for (int i = 0; i < 3 * MF_FACE_NQ_MAX; ++i) a.quad[i] = c->mf_quad[i];
     a.theta = (float)c->theta;
     return a;
 }
 
-template <int PD, int MODE>
-int launch_mf_t(lymph_ctx* c, const StepArgs& s) {
-    const MfArgs a = mf_args(c, s);
-    k_mf<PD, MODE><<<c->n_poly, MF_THREADS, 0, c->stream>>>(a);
+int convert_u32(lymph_ctx* c, const double* u, void* u32) {
+    const int64_t n = (int64_t)c->n_poly * c->Np;
+    const int64_t nb = (n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096;
+    k_mf_u32<<<(unsigned)nb, 256, 0, c->stream>>>(n, c->Np, u, (float4*)u32);
     c->launches++;
     return LYMPH_OK;
 }
 
-template <int PD>
-int launch_mf_p(lymph_ctx* c, int mode, const StepArgs& s) {
-    const double* u = (mode == MODE_FIRST || mode == MODE_BILIN) ? s.u0 : s.un;
-    const int64_t n = (int64_t)c->n_poly * c->Np;
-    const int64_t nb = (n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096;
-    k_mf_u32<<<(unsigned)nb, 256, 0, c->stream>>>(n, c->Np, u, (float4*)c->d_mf_u32);
+template <int PD, int MODE>
+int launch_mf_t(lymph_ctx* c, const MfArgs& a) {
+    if (MODE == MODE_STEP) {
+        LYMPH_CUDA_TRY(launch_pdl(k_mf<PD, MODE>, (unsigned)c->n_poly, MF_THREADS, c->stream, a));
+    } else {
+        k_mf<PD, MODE><<<c->n_poly, MF_THREADS, 0, c->stream>>>(a);
+    }
     c->launches++;
+    return LYMPH_OK;
+}
+
+// The buffers alternate with the state's: d_mf_u32[b] is the copy of d_buf[b].
+template <int PD>
+int launch_mf_p(lymph_ctx* c, int mode, const StepArgs& s, bool fresh) {
+    MfArgs a = mf_args(c, s);
+    if (mode == MODE_STEP) {
+        a.u32 = (const float4*)c->d_mf_u32[c->cur];
+        a.s.u32_out = (float*)c->d_mf_u32[c->cur ^ 1];
+        if (!fresh) LYMPH_TRY(convert_u32(c, s.un, c->d_mf_u32[c->cur]));
+    } else {
+        LYMPH_TRY(convert_u32(c, (mode == MODE_FIRST || mode == MODE_BILIN) ? s.u0 : s.un, c->d_mf_u32[0]));
+    }
     switch (mode) {
-        case MODE_STEP: return launch_mf_t<PD, MODE_STEP>(c, s);
-        case MODE_FIRST: return launch_mf_t<PD, MODE_FIRST>(c, s);
-        case MODE_APPLY: return launch_mf_t<PD, MODE_APPLY>(c, s);
-        case MODE_BILIN: return launch_mf_t<PD, MODE_BILIN>(c, s);
-        case MODE_KU: return launch_mf_t<PD, MODE_KU>(c, s);
+        case MODE_STEP: return launch_mf_t<PD, MODE_STEP>(c, a);
+        case MODE_FIRST: return launch_mf_t<PD, MODE_FIRST>(c, a);
+        case MODE_APPLY: return launch_mf_t<PD, MODE_APPLY>(c, a);
+        case MODE_BILIN: return launch_mf_t<PD, MODE_BILIN>(c, a);
+        case MODE_KU: return launch_mf_t<PD, MODE_KU>(c, a);
         default: lymph_set_error("matrix-free neighbour terms: unsupported mode"); return LYMPH_ERR_INVALID;
     }
 }
@@ -737,9 +741,14 @@ int lymph_mf_setup(lymph_ctx* c, const RefTables& R) {
         LYMPH_CUDA_TRY(cudaMalloc(&p, sizeof(MfPoly) * (size_t)c->n_poly));
         c->d_mf_poly = p;
         c->device_bytes += (int64_t)(sizeof(MfPoly) * c->n_poly);
-        LYMPH_CUDA_TRY(cudaMalloc(&p, sizeof(float4) * (size_t)c->n_poly * c->Np));
-        c->d_mf_u32 = p;
-        c->device_bytes += (int64_t)(sizeof(float4) * c->n_poly * c->Np);
+        for (int b = 0; b < 2; ++b) {
+            const size_t bytes = sizeof(float4) * (size_t)c->n_poly * c->Np;
+            LYMPH_CUDA_TRY(cudaMalloc(&p, bytes));
+            c->d_mf_u32[b] = p;
+            c->device_bytes += (int64_t)bytes;
+            // a step writes three of a record's four floats
+            LYMPH_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, c->stream));
+        }
         LYMPH_CUDA_TRY(cudaMalloc(&p, sizeof(int32_t) * MF_REC * (size_t)c->n_poly));
         c->d_mf_range = p;
         c->device_bytes += (int64_t)(sizeof(int32_t) * MF_REC * c->n_poly);
@@ -761,15 +770,19 @@ int lymph_mf_setup(lymph_ctx* c, const RefTables& R) {
 }
 
 // The operator pass of one step mode with matrix-free neighbour terms.
-int lymph_dev_mf(lymph_ctx* c, int mode, const stepk::StepArgs& s) {
+// fresh (MODE_STEP): the step before left the FP32 copy of u^n.
+int lymph_dev_mf(lymph_ctx* c, int mode, const stepk::StepArgs& s, bool fresh) {
     switch (c->p) {
-        case 1: return launch_mf_p<1>(c, mode, s);
-        case 2: return launch_mf_p<2>(c, mode, s);
-        case 3: return launch_mf_p<3>(c, mode, s);
-        case 4: return launch_mf_p<4>(c, mode, s);
+        case 1: return launch_mf_p<1>(c, mode, s, fresh);
+        case 2: return launch_mf_p<2>(c, mode, s, fresh);
+        case 3: return launch_mf_p<3>(c, mode, s, fresh);
+        case 4: return launch_mf_p<4>(c, mode, s, fresh);
         default: lymph_set_error("degree not supported on the device"); return LYMPH_ERR_INVALID;
     }
 }
+
+// The FP32 copy of u^n for the first step of a run.
+int lymph_dev_mf_u32(lymph_ctx* c) { return convert_u32(c, c->d_buf[c->cur], c->d_mf_u32[c->cur]); }
 
 // ---- batch interface (batch.cu) ----
 
@@ -800,6 +813,9 @@ void lymph_mf_batch_problem(const lymph_ctx* c, int* status, void* out) {
     s.rhs_dyn = c->d_rhs_dyn;
     s.gvals = nullptr;
     s.step_idx = nullptr;
+    s.step_off = 0;
+    s.g = 0.0;
+    s.u32_out = nullptr;
     s.u0 = s.un = nullptr;
     s.out = nullptr;
     s.partial = nullptr;
@@ -818,30 +834,36 @@ void lymph_mf_batch_problem(const lymph_ctx* c, int* status, void* out) {
     std::memcpy(out, &pb, sizeof(pb));
 }
 
-// One batched leapfrog step: the FP32 copies of every problem's u^n, then one
-// persistent pass per degree over that degree's items, items[off[p - 1],
-// off[p]) with grid[p - 1] CTAs and queue counter queue[p - 1] (the caller
-// advances the step counter and clears the counters).  Returns the number of
-// kernels launched in *launched.
-int lymph_mf_batch_step(cudaStream_t st, const int* grid, const void* probs, const int2* items, const int* off,
-                        int* queue, const int64_t* step_idx, const double* gvals, int64_t g_stride, int* launched) {
+// The FP32 copies of every problem's u^n, before the passes of a batched step.
+int lymph_mf_batch_u32(cudaStream_t st, const void* probs, const int2* items, int n_items, const int64_t* step_idx,
+                       int step_off) {
+    k_mf_u32_batch<<<(unsigned)((n_items + 3) / 4), 128, 0, st>>>((const MfBatchProblem*)probs, items, n_items, step_idx,
+                                                                  step_off);
+    LYMPH_CUDA_TRY(cudaGetLastError());
+    return LYMPH_OK;
+}
+
+// One batched leapfrog step: one persistent pass per degree over that degree's
+// items, items[off[p - 1], off[p]), with grid[p - 1] CTAs on stream st[p - 1] and
+// the zeroed queue counter queue[p - 1].  No pass reads what another of the same
+// step writes (a problem has one degree), so they may run at the same time;
+// the caller orders the steps.  Returns the number of kernels launched.
+int lymph_mf_batch_step(const cudaStream_t* st, const int* grid, const void* probs, const int2* items, const int* off,
+                        int* queue, const int64_t* step_idx, int step_off, const double* gvals, int64_t g_stride,
+                        int* launched) {
     const MfBatchProblem* pb = (const MfBatchProblem*)probs;
-    const int n_all = off[4];
     int nl = 0;
-    if (n_all > 0) {
-        k_mf_u32_batch<<<(unsigned)((n_all + 3) / 4), 128, 0, st>>>(pb, items, n_all, step_idx);
-        ++nl;
-    }
     for (int p = 1; p <= 4; ++p) {
         const int n = off[p] - off[p - 1];
         if (n <= 0 || grid[p - 1] <= 0) continue;
         const int2* it = items + off[p - 1];
         int* q = queue + (p - 1);
+        const cudaStream_t s = st[p - 1];
         switch (p) {
-            case 1: k_mf_batch<1><<<grid[0], MF_THREADS, 0, st>>>(pb, it, n, q, step_idx, gvals, g_stride); break;
-            case 2: k_mf_batch<2><<<grid[1], MF_THREADS, 0, st>>>(pb, it, n, q, step_idx, gvals, g_stride); break;
-            case 3: k_mf_batch<3><<<grid[2], MF_THREADS, 0, st>>>(pb, it, n, q, step_idx, gvals, g_stride); break;
-            default: k_mf_batch<4><<<grid[3], MF_THREADS, 0, st>>>(pb, it, n, q, step_idx, gvals, g_stride); break;
+            case 1: k_mf_batch<1><<<grid[0], MF_THREADS, 0, s>>>(pb, it, n, q, step_idx, step_off, gvals, g_stride); break;
+            case 2: k_mf_batch<2><<<grid[1], MF_THREADS, 0, s>>>(pb, it, n, q, step_idx, step_off, gvals, g_stride); break;
+            case 3: k_mf_batch<3><<<grid[2], MF_THREADS, 0, s>>>(pb, it, n, q, step_idx, step_off, gvals, g_stride); break;
+            default: k_mf_batch<4><<<grid[3], MF_THREADS, 0, s>>>(pb, it, n, q, step_idx, step_off, gvals, g_stride); break;
         }
         ++nl;
     }

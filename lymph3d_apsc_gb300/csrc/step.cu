@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(Shape<PD>::T, Shape<PD>::MINB) k_step(StepArgs
     step_poly<PD, KT, MODE>(A, blockIdx.x, smem);
 }
 
-__global__ void k_bump(int64_t* idx) { *idx += 1; }
+__global__ void k_bump(int64_t* idx, int n) { *idx += n; }
 
 // COMPUTE_ERROR_L2_MATRIX_FREE body per polyhedron: sum_i du_i^T M du_i.
 __global__ void __launch_bounds__(L2_THREADS) k_l2_partial(int NP, const double* __restrict__ Mm,
@@ -274,7 +274,11 @@ __global__ void k_normalize(int64_t n, const double* __restrict__ y, const doubl
 
 template <int PD, typename KT, int MODE>
 int launch_step_t(lymph_ctx* c, const StepArgs& A) {
-    k_step<PD, KT, MODE><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
+    if (MODE == MODE_STEP) {
+        LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
+    } else {
+        k_step<PD, KT, MODE><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
+    }
     c->launches++;
     return LYMPH_OK;
 }
@@ -297,22 +301,26 @@ int launch_step_mode(lymph_ctx* c, const StepArgs& A, bool fp32) {
 
 }  // namespace
 
-int lymph_dev_mf(lymph_ctx* c, int mode, const stepk::StepArgs& A);
+int lymph_dev_mf(lymph_ctx* c, int mode, const stepk::StepArgs& A, bool fresh);
+
+int lymph_dev_mf_u32(lymph_ctx* c);
 
 namespace {
 
 // The operator pass of a step mode in the context's precision: the fused
 // block-CSR kernel (FP64 or FP32 blocks) or the matrix-free neighbour kernel.
+// fresh (matrix-free, MODE_STEP): the FP32 copy of u^n was left by the step before.
 template <int MODE>
-int launch_ctx(lymph_ctx* c, const StepArgs& A) {
-    if (c->precision == LYMPH_MIXED_MF) return lymph_dev_mf(c, MODE, A);
+int launch_ctx(lymph_ctx* c, const StepArgs& A, bool fresh = false) {
+    if (c->precision == LYMPH_MIXED_MF) return lymph_dev_mf(c, MODE, A, fresh);
     return launch_step_mode<MODE>(c, A, c->precision == LYMPH_MIXED);
 }
 
 StepArgs base_args(lymph_ctx* c) {
     StepArgs A;
     A.row_ptr = c->d_row_ptr; A.col = c->d_col; A.K = c->d_K; A.Minv = c->d_Minv;
-    A.rhs_stat = c->d_rhs_stat; A.rhs_dyn = c->d_rhs_dyn; A.gvals = c->d_gvals; A.step_idx = c->d_step_idx;
+    A.rhs_stat = c->d_rhs_stat; A.rhs_dyn = c->d_rhs_dyn; A.gvals = nullptr; A.step_idx = nullptr;
+    A.step_off = 0; A.g = 0.0; A.u32_out = nullptr;
     A.u0 = nullptr; A.un = nullptr; A.out = nullptr; A.partial = c->d_partial; A.dt = c->dt; A.status = c->d_status;
     A.n_poly = c->n_poly;
     A.abs_idx = c->n_abs > 0 ? c->d_abs_idx : nullptr;
@@ -324,25 +332,32 @@ StepArgs base_args(lymph_ctx* c) {
 }  // namespace
 
 // One leapfrog step on the context stream (no rotation): reads U0/UN buffers,
-// writes u^{n+1} over U0.  The caller flips c->cur afterwards.
-int lymph_dev_step(lymph_ctx* c, bool bump) {
+// writes u^{n+1} over U0.  The caller flips c->cur afterwards.  off >= 0: step
+// `off` of a run, its time-function value gvals[step_idx + off]; off < 0: the
+// value g.  fresh: directly after another step of the same run.
+int lymph_dev_step(lymph_ctx* c, int off, double g, bool fresh) {
     StepArgs A = base_args(c);
     A.u0 = c->d_buf[c->cur ^ 1];
     A.un = c->d_buf[c->cur];
     A.out = c->d_buf[c->cur ^ 1];
-    LYMPH_TRY(launch_ctx<MODE_STEP>(c, A));
-    if (bump) {
-        k_bump<<<1, 1, 0, c->stream>>>(c->d_step_idx);
-        c->launches++;
+    if (off >= 0) {
+        A.gvals = c->d_gvals;
+        A.step_idx = c->d_step_idx;
+        A.step_off = off;
     }
-    return LYMPH_OK;
+    A.g = g;
+    return launch_ctx<MODE_STEP>(c, A, fresh);
 }
 
-int lymph_dev_bump(lymph_ctx* c) {
-    k_bump<<<1, 1, 0, c->stream>>>(c->d_step_idx);
+// step_idx += n
+int lymph_dev_bump(lymph_ctx* c, int n) {
+    k_bump<<<1, 1, 0, c->stream>>>(c->d_step_idx, n);
     c->launches++;
     return LYMPH_OK;
 }
+
+// The FP32 copy of u^n that the first matrix-free step of a run reads.
+int lymph_dev_run_start(lymph_ctx* c) { return c->precision == LYMPH_MIXED_MF ? lymph_dev_mf_u32(c) : LYMPH_OK; }
 
 // out = M^-1 K u (u read from `u`), for the power iteration of the CFL bound.
 int lymph_dev_apply(lymph_ctx* c, const double* u, double* out) {
@@ -423,8 +438,9 @@ int lymph_dev_power_iteration(lymph_ctx* c, double* x, double* y, double* d_ss, 
     return LYMPH_OK;
 }
 
-int lymph_dev_first_step(lymph_ctx* c) {
+int lymph_dev_first_step(lymph_ctx* c, double g) {
     StepArgs A = base_args(c);
+    A.g = g;
     A.u0 = c->d_buf[c->cur ^ 1];
     A.un = c->d_v0;
     A.out = c->d_buf[c->cur];

@@ -21,6 +21,8 @@ template <int P> struct Shape {
     static constexpr int MINB = P == 1 ? 16 : (P == 4 ? 4 : 6);
 };
 
+constexpr int64_t STEP_PREFETCH = 32 * 1024;   // bytes of a row's blocks prefetched before its state is ready
+
 constexpr int NBB = 16;   // neighbour blocks staged in shared memory at once
 
 // Doubles of scratch finish_poly needs behind the right-hand side for polyhedra
@@ -40,8 +42,11 @@ struct StepArgs {
     const double* Minv;        // [n_poly][NP][NP] column-major inverse of M_loc
     const double* rhs_stat;
     const double* rhs_dyn;
-    const double* gvals;       // time-function values
-    const int64_t* step_idx;   // index into gvals (device counter)
+    const double* gvals;       // time-function values (null: the one value g)
+    const int64_t* step_idx;   // index into gvals: the device counter (steps of earlier graph launches) ...
+    int step_off;              // ... plus this step's place in the graph
+    double g;
+    float* u32_out;            // FP32 copy of u^{n+1} for the next matrix-free step, [n_poly][NP] x 4 (may be null)
     const double* u0;          // u^{n-1} (MODE_STEP), u^0 (MODE_FIRST)
     const double* un;          // u^n (MODE_STEP, MODE_APPLY), v^0 (MODE_FIRST)
     double* out;               // u^{n+1} (MODE_STEP: may alias u0), u^1 (MODE_FIRST), M^-1 K u (MODE_APPLY),
@@ -55,6 +60,35 @@ struct StepArgs {
     int* status;
     int n_poly;
 };
+
+// Programmatic dependent launch: a step kernel starts while the one before it
+// finishes, reads what no step writes, and waits for that kernel and its writes
+// before it touches a state.  A no-op on a plain launch.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a step kernel that may start before the stream's previous kernel ends.
+template <typename K, typename A>
+inline cudaError_t launch_pdl(K kernel, unsigned grid, unsigned block, cudaStream_t st, const A& arg) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, arg);
+}
+
+// One bulk prefetch into L2 of the whole 16-byte words inside [p, p + bytes).
+__device__ __forceinline__ void prefetch_inside(const void* p, int64_t bytes) {
+    const uintptr_t s = ((uintptr_t)p + 15) & ~(uintptr_t)15, e = ((uintptr_t)p + (uintptr_t)bytes) & ~(uintptr_t)15;
+    if (e > s) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s), "r"((uint32_t)(e - s)) : "memory");
+}
 
 __device__ __forceinline__ double ld_stream(const double* p) { return __ldcs(p); }
 __device__ __forceinline__ float ld_stream(const float* p) { return __ldcs(p); }
@@ -99,7 +133,9 @@ __device__ __forceinline__ double cta_matvec(const double* __restrict__ A, const
 // per component with a parallel product of the same value.  s_b holds ND
 // doubles, 16-byte aligned, then finish_scratch(ND, threads) more.  Every
 // thread of the CTA must call this (it synchronises).
-template <int PD, int MODE>
+// U32: also leave the FP32 copy of u^{n+1} (A.u32_out) for the next
+// matrix-free step.
+template <int PD, int MODE, bool U32 = false>
 __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, double* s_b) {
     constexpr int NP = Deg<PD>::NP, ND = Deg<PD>::ND;
     const int tid = threadIdx.x;
@@ -128,7 +164,7 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
         if (MODE == MODE_APPLY) {
             s_b[tid] = y;
         } else {
-            const double g = A.gvals[*A.step_idx];
+            const double g = A.gvals ? A.gvals[*A.step_idx + A.step_off] : A.g;
             s_b[tid] = -y + A.rhs_stat[q] + A.rhs_dyn[q] * g;
         }
     }
@@ -152,6 +188,7 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
                 const double v = x + 2.0 * A.un[q] - A.u0[q];
                 if (!isfinite(v)) atomicOr(A.status, ST_NONFINITE);
                 A.out[q] = v;
+                if (U32 && A.u32_out) A.u32_out[((int64_t)P * NP + tid % NP) * 4 + tid / NP] = (float)v;
             }
             return;
         }
@@ -181,6 +218,7 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
         }
         if (!isfinite(v)) atomicOr(A.status, ST_NONFINITE);
         A.out[q] = v;
+        if (U32 && MODE == MODE_STEP && A.u32_out) A.u32_out[((int64_t)P * NP + m) * 4 + i] = (float)v;
     }
 }
 
@@ -205,6 +243,14 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
     const bool act = tid < ND * S;
     const int rb = A.row_ptr[P], re = A.row_ptr[P + 1];
     const KT* Kbase = (const KT*)A.K;
+    if (MODE == MODE_STEP) {
+        if (tid == 0) {   // the head of the row's blocks and M^-1, while the previous step ends
+            const int64_t row = (int64_t)(re - rb) * ND * ND * (int64_t)sizeof(KT);
+            prefetch_inside(Kbase + (int64_t)rb * ND * ND, row < STEP_PREFETCH ? row : STEP_PREFETCH);
+            prefetch_inside(A.Minv + (int64_t)P * Deg<PD>::NP * Deg<PD>::NP, (int64_t)Deg<PD>::NP * Deg<PD>::NP * 8);
+        }
+        pdl_wait();
+    }
 
     AT acc0 = 0, acc1 = 0;
     for (int b0 = rb; b0 < re; b0 += NBB) {
