@@ -134,9 +134,11 @@ template <int PD> struct MfShape {
     static constexpr int NQ2 = MF_FACE_NQ[PD];    // quadrature points per triangle
     static constexpr int CT = MF_THREADS / NQ2;   // triangles per chunk
     static constexpr int NPT = CT * NQ2;          // points per chunk (one evaluating thread each)
-    // a point's (L, L') values of the three directions, padded to an odd
-    // number of 16-byte words so the points of a warp fall on distinct banks
-    static constexpr int LEGW = ((3 * L + 1) / 2 % 2 == 1) ? 2 * ((3 * L + 1) / 2) : 2 * ((3 * L + 1) / 2) + 2;
+    // a point's (L, L') values of degrees 1..p in the three directions (degree 0
+    // is (1, 0)), padded to an odd number of 16-byte words so the points of a
+    // warp fall on distinct banks
+    static constexpr int LW = (3 * PD + 1) / 2;
+    static constexpr int LEGW = 2 * (LW | 1);
     static_assert(ND <= MF_THREADS, "one thread per row of the self block");
 };
 
@@ -159,7 +161,8 @@ template <int PD> struct Bidx {
 // (u_0, u_1, u_2, 0) of basis function i.  Each w sum runs over c = p-a-b
 // down to 0 (the basis order), each r sum over b = 0.., each output over
 // a = 0..; one (a, b) group is live at a time, so the three components cost
-// no more registers than one did with every w_ab held.
+// no more registers than one did with every w_ab held.  L_0 = 1, L'_0 = 0 and
+// L'_1 = 1 are left out of the products (63 of 405 multiply-adds at p = 4).
 template <int PD>
 __device__ __forceinline__ void eval_sf3(const float4* uc, const float2* X, const float2* Y, const float2* Z,
                                          float (&o)[3][4]) {
@@ -180,23 +183,25 @@ __device__ __forceinline__ void eval_sf3(const float4* uc, const float2* X, cons
                 const float u3[3] = {uu.x, uu.y, uu.z};
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    w0[j] = fmaf(u3[j], Z[c].x, w0[j]);
-                    w1[j] = fmaf(u3[j], Z[c].y, w1[j]);
+                    w0[j] = c == 0 ? w0[j] + u3[j] : fmaf(u3[j], Z[c].x, w0[j]);
+                    if (c >= 1) w1[j] = c == 1 ? w1[j] + u3[j] : fmaf(u3[j], Z[c].y, w1[j]);
                 }
             }
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                r[j][0] = fmaf(w0[j], Y[b].x, r[j][0]);
-                r[j][1] = fmaf(w0[j], Y[b].y, r[j][1]);
-                r[j][2] = fmaf(w1[j], Y[b].x, r[j][2]);
+                r[j][0] = b == 0 ? r[j][0] + w0[j] : fmaf(w0[j], Y[b].x, r[j][0]);
+                if (b >= 1) r[j][1] = b == 1 ? r[j][1] + w0[j] : fmaf(w0[j], Y[b].y, r[j][1]);
+                if (a + b < PD) r[j][2] = b == 0 ? r[j][2] + w1[j] : fmaf(w1[j], Y[b].x, r[j][2]);
             }
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            o[j][0] = fmaf(r[j][0], X[a].x, o[j][0]);
-            o[j][1] = fmaf(r[j][0], X[a].y, o[j][1]);
-            o[j][2] = fmaf(r[j][1], X[a].x, o[j][2]);
-            o[j][3] = fmaf(r[j][2], X[a].x, o[j][3]);
+            o[j][0] = a == 0 ? o[j][0] + r[j][0] : fmaf(r[j][0], X[a].x, o[j][0]);
+            if (a >= 1) o[j][1] = a == 1 ? o[j][1] + r[j][0] : fmaf(r[j][0], X[a].y, o[j][1]);
+            if (a < PD) {
+                o[j][2] = a == 0 ? o[j][2] + r[j][1] : fmaf(r[j][1], X[a].x, o[j][2]);
+                o[j][3] = a == 0 ? o[j][3] + r[j][2] : fmaf(r[j][2], X[a].x, o[j][3]);
+            }
         }
     }
 }
@@ -209,14 +214,16 @@ __device__ __forceinline__ void test_sf(float* acc, const float2* X, const float
     constexpr Bidx<PD> BI{};
 #pragma unroll
     for (int a = 0; a <= PD; ++a) {
-        const float t0 = fmaf(X[a].y, gx, X[a].x * s), t1 = X[a].x * gy, t2 = X[a].x * gz;
+        // degree 0 is (1, 0): X, Y and Z start at degree 1
+        const float xa = a ? X[a - 1].x : 1.0f;
+        const float t0 = a ? fmaf(X[a - 1].y, gx, xa * s) : s, t1 = a ? xa * gy : gy, t2 = a ? xa * gz : gz;
 #pragma unroll
         for (int b = 0; b <= PD - a; ++b) {
-            const float q0 = fmaf(Y[b].x, t0, Y[b].y * t1), q1 = Y[b].x * t2;
+            const float q0 = b ? fmaf(Y[b - 1].x, t0, Y[b - 1].y * t1) : t0, q1 = b ? Y[b - 1].x * t2 : t2;
 #pragma unroll
             for (int c = 0; c <= PD - a - b; ++c) {
                 float& r = acc[BI.i[a][b][c]];
-                r = fmaf(Z[c].x, q0, fmaf(Z[c].y, q1, r));
+                r = c ? fmaf(Z[c - 1].x, q0, fmaf(Z[c - 1].y, q1, r)) : r + q0;
             }
         }
     }
@@ -458,12 +465,16 @@ __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, con
             }
             // P's values, written as 16-byte words (the padded row keeps the
             // stores of a quarter-warp on distinct banks)
-            constexpr int LW = (3 * L + 1) / 2;
+            constexpr int LW = S::LW;
             float2 LP[2 * LW];
-            legendre_f32<PD>(xp[0] * pP.ih[0], LP);
-            legendre_f32<PD>(xp[1] * pP.ih[1], LP + L);
-            legendre_f32<PD>(xp[2] * pP.ih[2], LP + 2 * L);
-            if (2 * LW > 3 * L) LP[2 * LW - 1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                float2 V[L];
+                legendre_f32<PD>(xp[d] * pP.ih[d], V);
+#pragma unroll
+                for (int n = 1; n < L; ++n) LP[d * PD + n - 1] = V[n];
+            }
+            if (2 * LW > 3 * PD) LP[2 * LW - 1] = make_float2(0.0f, 0.0f);
             float4* lw = reinterpret_cast<float4*>(s_w.loop.leg[tid]);
 #pragma unroll
             for (int k = 0; k < LW; ++k) lw[k] = make_float4(LP[2 * k].x, LP[2 * k].y, LP[2 * k + 1].x, LP[2 * k + 1].y);
@@ -472,16 +483,16 @@ __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, con
         // ---- test against P's basis: thread (slot, component) over the chunk's points ----
         if (tact) {
             for (int pt = slot; pt < nt * NQ2; pt += MF_SLOTS) {
-                float2 LG[2 * ((3 * L + 1) / 2)];
+                float2 LG[2 * S::LW];
                 const float4* lp = reinterpret_cast<const float4*>(s_w.loop.leg[pt]);
 #pragma unroll
-                for (int k = 0; k < (3 * L + 1) / 2; ++k) {
+                for (int k = 0; k < S::LW; ++k) {
                     const float4 q = lp[k];
                     LG[2 * k] = make_float2(q.x, q.y);
                     LG[2 * k + 1] = make_float2(q.z, q.w);
                 }
                 const float4 f = s_w.loop.flux[pt][ci];
-                test_sf<PD>(acc, LG, LG + L, LG + 2 * L, f.x, f.y, f.z, f.w);
+                test_sf<PD>(acc, LG, LG + PD, LG + 2 * PD, f.x, f.y, f.z, f.w);
             }
         }
     }
