@@ -14,10 +14,9 @@
 // every GEMM reads; activations and accumulation are FP32.  The forward GEMMs
 // run on the tcgen05 tensor cores (umma_gemm.cuh: the activations split into
 // TF32 hi and lo parts, the BF16 weights exact in TF32, FP32 accumulation in
-// tensor memory) whenever the shapes suit it, else on the FP32 SIMT kernel
-// k_gemm, which also runs the backward.  The concatenation [h a g] is never
-// formed: the tensor-core GEMM reads it as three K segments, the SIMT path as
-// three GEMMs on row slices of Wu accumulating into one output.  Aggregation
+// tensor memory) whenever the shapes suit it, else on the FP32 kernel of
+// gemm_jobs.cuh, which also runs the backward.  The concatenation [h a g] is never formed: both read it
+// as three segments.  Aggregation
 // is a CSR gather (fixed order); its adjoint uses the transposed CSR, so
 // training is deterministic.
 
@@ -31,6 +30,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gemm_jobs.cuh"
 #include "umma_gemm.cuh"
 #include "umma_ws.cuh"
 
@@ -40,92 +40,17 @@ const float* lymph_dev_blocks_f32(lymph_ctx* c);
 
 namespace {
 
-// ---------------------------------------------------------------------------
-// GEMM: C[M x N] (op) = op(A)[M x K] * op(B)[K x N] (+ bias), FP32 accumulate.
-// op(A)[m,k] = TA ? A[k*lda + m] : A[m*lda + k]; op(B)[k,n] = TB ? B[n*ldb + k]
-// : B[k*ldb + n].  64 x 64 tiles, 256 threads, 4 x 4 outputs per thread.
-// ---------------------------------------------------------------------------
-// EPI_STORE: C = v; EPI_ADD: C += v; EPI_RELU: Z = v, C = relu(v);
-// EPI_ADD_RELU: Z = v, C += relu(v); EPI_ACC_RELU_ADD: v += Z, Z = v, C += relu(v)
-// (v = the product plus the bias, Z the pre-activation buffer, same layout as C).
-enum { EPI_STORE = 0, EPI_ADD = 1, EPI_RELU = 2, EPI_ADD_RELU = 3, EPI_ACC_RELU_ADD = 4 };
-
-__device__ __forceinline__ float to_f(float v) { return v; }
-__device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-template <bool TA, bool TB, typename BT>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A, int lda,
-                                              const BT* __restrict__ B, int ldb, float* C, int ldc,
-                                              const float* __restrict__ bias, float* Zpre, int epi) {
-    constexpr int TM = 64, TN = 64, TK = 16;
-    __shared__ float As[TK][TM + 1];
-    __shared__ float Bs[TK][TN + 1];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int tr = tid / 16, tc = tid % 16;  // 16 x 16 threads, 4 x 4 each
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        for (int i = tid; i < TM * TK; i += 256) {
-            const int mm = i % TM, kk = i / TM;
-            const int m = m0 + mm, k = k0 + kk;
-            float v = 0.0f;
-            if (m < M && k < K) v = TA ? A[(int64_t)k * lda + m] : A[(int64_t)m * lda + k];
-            As[kk][mm] = v;
-        }
-        for (int i = tid; i < TN * TK; i += 256) {
-            const int nn = i % TN, kk = i / TN;
-            const int n = n0 + nn, k = k0 + kk;
-            float v = 0.0f;
-            if (n < N && k < K) v = to_f(TB ? B[(int64_t)n * ldb + k] : B[(int64_t)k * ldb + n]);
-            Bs[kk][nn] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[kk][tr + 16 * r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tc + 16 * c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] += a[r] * b[c];
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int m = m0 + tr + 16 * r;
-        if (m >= M) continue;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int n = n0 + tc + 16 * c;
-            if (n >= N) continue;
-            float v = acc[r][c] + (bias ? bias[n] : 0.0f);
-            float* dst = C + (int64_t)m * ldc + n;
-            if (epi == EPI_STORE) *dst = v;
-            else if (epi == EPI_ADD) *dst += v;
-            else {
-                if (epi == EPI_ACC_RELU_ADD) v += Zpre[(int64_t)m * ldc + n];
-                if (Zpre) Zpre[(int64_t)m * ldc + n] = v;
-                const float rv = v > 0.0f ? v : 0.0f;
-                if (epi == EPI_RELU) *dst = rv;
-                else *dst += rv;
-            }
-        }
-    }
-}
-
-// out[i, :] = sum_{k in row i} val[k] * in[idx[k], :]   (width columns)
+// out[i, :] = sum_{k in row i} val[k] * in[idx[k], :]   (width columns); with a
+// mask, zero where it is not positive (the ReLU's backward)
 __global__ void k_aggregate(int n, int width, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                            const float* __restrict__ val, const float* __restrict__ in, float* out) {
+                            const float* __restrict__ val, const float* __restrict__ in, const float* __restrict__ mask,
+                            float* out) {
     const int i = blockIdx.x;
     if (i >= n) return;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         float s = 0.0f;
         for (int k = ptr[i]; k < ptr[i + 1]; ++k) s += val[k] * in[(int64_t)idx[k] * width + c];
-        out[(int64_t)i * width + c] = s;
+        out[(int64_t)i * width + c] = mask && !(mask[(int64_t)i * width + c] > 0.0f) ? 0.0f : s;
     }
 }
 
@@ -134,7 +59,8 @@ __global__ void k_aggregate(int n, int width, const int32_t* __restrict__ ptr, c
 // neighbours runs in the CSR order, as in k_aggregate.
 __global__ void __launch_bounds__(256) k_aggregate_v4(int n, int width, const int32_t* __restrict__ ptr,
                                                       const int32_t* __restrict__ idx, const float* __restrict__ val,
-                                                      const float* __restrict__ in, float* out) {
+                                                      const float* __restrict__ in, const float* __restrict__ mask,
+                                                      float* out) {
     const int i = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (i >= n) return;
     const int k0 = ptr[i], k1 = ptr[i + 1];
@@ -145,23 +71,13 @@ __global__ void __launch_bounds__(256) k_aggregate_v4(int n, int width, const in
             const float4 v = *(const float4*)(in + (int64_t)idx[k] * width + c);
             s.x += w * v.x; s.y += w * v.y; s.z += w * v.z; s.w += w * v.w;
         }
+        if (mask) {
+            const float4 z = *(const float4*)(mask + (int64_t)i * width + c);
+            s.x = z.x > 0.0f ? s.x : 0.0f; s.y = z.y > 0.0f ? s.y : 0.0f;
+            s.z = z.z > 0.0f ? s.z : 0.0f; s.w = z.w > 0.0f ? s.w : 0.0f;
+        }
         *(float4*)(out + (int64_t)i * width + c) = s;
     }
-}
-
-// dz = dy * (z > 0)
-__global__ void k_relu_back(int64_t n, const float* __restrict__ dy, const float* __restrict__ z, float* dz) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dz[i] = z[i] > 0.0f ? dy[i] : 0.0f;
-}
-
-// column sums of dz [M x N] into db (bias gradient), one thread per column
-__global__ void k_colsum(int M, int N, const float* __restrict__ dz, float* db, int accumulate) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.0f;
-    for (int m = 0; m < M; ++m) s += dz[(int64_t)m * N + n];
-    db[n] = accumulate ? db[n] + s : s;
 }
 
 // loss = mean (y - t)^2 (partials per block, then host sum), dy = 2 (y - t) / n
@@ -282,6 +198,7 @@ struct lymph_mpnn {
     bool use_umma = true;         // LYMPH_MPNN_SIMT=1 selects the SIMT GEMMs for the forward too
     bool use_ws = true;           // LYMPH_UMMA_WS=0 selects the cp.async tensor-core kernel over the TMA one
     int* d_status = nullptr;      // bit 0: a tensor-core wait ran out
+    int sms = 1;                  // SMs of the device
 };
 
 namespace {
@@ -304,25 +221,47 @@ const __nv_bfloat16* B_(lymph_mpnn* n, const char* w, int l = 0) { return n->d_p
 
 int round16(int x) { return (x + 15) / 16 * 16; }
 
-// Bt[n][k] = W[k][n] for n < N, 0 for N <= n < Npad
-__global__ void k_transpose_w(int K, int N, int Npad, const __nv_bfloat16* __restrict__ W, float* Bt) {
-    const int64_t tot = (int64_t)Npad * K;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-        const int n = (int)(i / K), k = (int)(i % K);
-        Bt[i] = n < N ? __bfloat162float(W[(int64_t)k * N + n]) : 0.0f;
+// Bt[n][k] = W[k][n] for n < N, 0 for N <= n < Npad, of every weight matrix in
+// one launch (blockIdx.y: the matrix), 32 x 32 tiles through shared memory.
+constexpr int MAX_MATS = 2 + 2 * 8;   // W0, Wo and two per layer (L <= 8)
+struct TransposeArgs {
+    int K[MAX_MATS], N[MAX_MATS], Npad[MAX_MATS];
+    const __nv_bfloat16* W[MAX_MATS];
+    float* Bt[MAX_MATS];
+};
+__global__ void __launch_bounds__(256) k_transpose_w(const __grid_constant__ TransposeArgs A) {
+    __shared__ float t[32][33];
+    const int i = blockIdx.y, K = A.K[i], N = A.N[i], Npad = A.Npad[i];
+    const int tk = (K + 31) / 32, tiles = tk * ((Npad + 31) / 32), tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+    for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
+        const int k0 = b % tk * 32, n0 = b / tk * 32;
+        for (int j = ty; j < 32; j += 8)
+            t[j][tx] = k0 + j < K && n0 + tx < N ? __bfloat162float(A.W[i][(int64_t)(k0 + j) * N + n0 + tx]) : 0.0f;
+        __syncthreads();
+        for (int j = ty; j < 32; j += 8)
+            if (n0 + j < Npad && k0 + tx < K) A.Bt[i][(int64_t)(n0 + j) * K + k0 + tx] = t[tx][j];
+        __syncthreads();
     }
 }
 
 // Refreshes the transposed FP32 weight copies after the BF16 weights changed.
 void refresh_wt(lymph_mpnn* n) {
     if (!n->wt_dirty) return;
+    TransposeArgs A = {};
+    int nm = 0, most = 1;
     for (size_t i = 0; i < n->par.size(); ++i) {
         if (n->wt_off[i] < 0) continue;
         const auto& P = n->par[i];
-        const int K = (int)P.rows, N = (int)P.cols;
-        k_transpose_w<<<256, 256, 0, n->stream>>>(K, N, round16(N), n->d_pb + P.off, n->d_wt + n->wt_off[i]);
-        n->launches++;
+        A.K[nm] = (int)P.rows;
+        A.N[nm] = (int)P.cols;
+        A.Npad[nm] = round16((int)P.cols);
+        A.W[nm] = n->d_pb + P.off;
+        A.Bt[nm] = n->d_wt + n->wt_off[i];
+        most = std::max(most, ((A.K[nm] + 31) / 32) * ((A.Npad[nm] + 31) / 32));
+        ++nm;
     }
+    k_transpose_w<<<dim3((unsigned)most, (unsigned)nm), 256, 0, n->stream>>>(A);
+    n->launches++;
     n->wt_dirty = false;
 }
 
@@ -438,23 +377,77 @@ int read_status(lymph_mpnn* n, const char* who) {
     return LYMPH_OK;
 }
 
-template <bool TA, bool TB, typename BT>
-void gemm(lymph_mpnn* n, int M, int N, int K, const float* A, int lda, const BT* B, int ldb, float* C, int ldc,
-          const float* bias, float* Z, int epi) {
-    if (M <= 0 || N <= 0) return;
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    k_gemm<TA, TB, BT><<<grid, 256, 0, n->stream>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, Z, epi);
+// One launch of one or two independent FP32 GEMMs (gemm_jobs.cuh).
+void run_jobs(lymph_mpnn* n, jobs::Job a, const jobs::Job* b = nullptr) {
+    jobs::Args A;
+    A.n = b ? 2 : 1;
+    A.j[0] = a;
+    if (b) A.j[1] = *b;
+    unsigned grid = 0;
+    for (int i = 0; i < A.n; ++i) {
+        jobs::finish(A.j[i], n->sms);
+        grid += (unsigned)A.j[i].ctas();
+    }
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // the kernel waits for the one before it
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(jobs::THREADS);
+    cfg.stream = n->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, jobs::k_gemm_jobs, A);
     n->launches++;
 }
 
-void aggregate(lymph_mpnn* n, bool transposed, int width, const float* in, float* out) {
+// C = epi([segments] W + bias), W the BF16 parameter matrix `w`
+jobs::Job job_fwd(lymph_mpnn* n, const char* w, const char* bias, int l, std::initializer_list<jobs::Seg> segs, int N,
+                  float* C, float* z, const float* R, int epi) {
+    jobs::Job J = {};
+    J.kind = jobs::FWD; J.epi = epi;
+    J.M = n->n_nodes; J.N = N;
+    for (const jobs::Seg& s : segs) { J.a[J.na++] = s; J.K += s.w; }
+    J.W = B_(n, w, l); J.ldb = N;
+    J.C = C; J.ldc = N; J.bias = P_(n, bias, l); J.z = z; J.R = R;
+    return J;
+}
+
+// The gradient of a parameter matrix and of the bias that follows it:
+// [segments 1]^T dz
+jobs::Job job_dw(lymph_mpnn* n, const char* w, int l, std::initializer_list<jobs::Seg> segs, const float* dz, int N) {
+    jobs::Job J = {};
+    J.kind = jobs::DW; J.epi = jobs::STORE;
+    for (const jobs::Seg& s : segs) { J.a[J.na++] = s; J.M += s.w; }
+    J.M += 1;
+    J.N = N; J.K = n->n_nodes;
+    J.dz = dz; J.ldb = N;
+    J.C = G_(n, w, l); J.ldc = N;
+    return J;
+}
+
+// dh (+)= dz W[0:H]^T, with mask also dz_out = dh where mask > 0; rows H.. of W
+// (N > H): C2 = dz W[H:]^T
+jobs::Job job_dx(lymph_mpnn* n, const char* w, int l, const float* dz, int K, int N, bool add, const float* mask,
+                 float* dz_out, float* C2) {
+    jobs::Job J = {};
+    J.kind = jobs::DX; J.epi = jobs::GRAD;
+    J.M = n->n_nodes; J.N = N; J.K = K;
+    J.a[0] = {dz, K, K}; J.na = 1;
+    J.W = B_(n, w, l); J.ldb = K;
+    J.C = n->d_dh; J.ldc = n->H; J.n_add = n->H; J.add = add;
+    J.mask = mask; J.dz_out = dz_out; J.C2 = C2;
+    return J;
+}
+
+void aggregate(lymph_mpnn* n, bool transposed, int width, const float* in, float* out, const float* mask = nullptr) {
     const int32_t* p = transposed ? n->d_tp : n->d_wp;
     const int32_t* ix = transposed ? n->d_ti : n->d_wi;
     const float* v = transposed ? n->d_tv : n->d_wv;
     if (width % 4 == 0)  // rows of 16-byte multiples from cudaMalloc'd buffers: 16-byte aligned
-        k_aggregate_v4<<<(n->n_nodes + 7) / 8, 256, 0, n->stream>>>(n->n_nodes, width, p, ix, v, in, out);
+        k_aggregate_v4<<<(n->n_nodes + 7) / 8, 256, 0, n->stream>>>(n->n_nodes, width, p, ix, v, in, mask, out);
     else
-        k_aggregate<<<n->n_nodes, 128, 0, n->stream>>>(n->n_nodes, width, p, ix, v, in, out);
+        k_aggregate<<<n->n_nodes, 128, 0, n->stream>>>(n->n_nodes, width, p, ix, v, in, mask, out);
     n->launches++;
 }
 
@@ -517,27 +510,16 @@ void forward(lymph_mpnn* n, bool keep_z = true) {
         umma::Seg so[1] = {{n->d_h[n->L], H, H}};
         umma_gemm(n, (int)pidx(n, "Wo", 0), N, so, 1, P_(n, "bo"), n->d_y, O, nullptr, nullptr, umma::EPI_STORE);
     } else {
-        gemm<false, false, __nv_bfloat16>(n, N, H, F, n->d_x, F, B_(n, "W0"), H, n->d_h[0], H, P_(n, "b0"), n->d_z0,
-                                          EPI_RELU);
+        run_jobs(n, job_fwd(n, "W0", "b0", 0, {{n->d_x, F, F}}, H, n->d_h[0], keep_z ? n->d_z0 : nullptr, nullptr, jobs::RELU));
         for (int l = 0; l < n->L; ++l) {
             float* h = n->d_h[l];
-            float* h1 = n->d_h[l + 1];
-            cudaMemcpyAsync(h1, h, sizeof(float) * (size_t)N * H, cudaMemcpyDeviceToDevice, n->stream);
-            gemm<false, false, __nv_bfloat16>(n, N, H, H, h, H, B_(n, "Wm", l), H, n->d_m_[l], H, P_(n, "bm", l),
-                                              n->d_zm[l], EPI_RELU);
+            run_jobs(n, job_fwd(n, "Wm", "bm", l, {{h, H, H}}, H, n->d_m_[l], keep_z ? n->d_zm[l] : nullptr, nullptr,
+                                jobs::RELU));
             aggregate(n, false, H, n->d_m_[l], n->d_a[l]);
-            const __nv_bfloat16* Wu = B_(n, "Wu", l);
-            // zu = h Wu[0:H] + a Wu[H:2H] + g Wu[2H:] + bu ; h1 = h + relu(zu)
-            gemm<false, false, __nv_bfloat16>(n, N, H, H, h, H, Wu, H, n->d_zu[l], H, P_(n, "bu", l), nullptr,
-                                              EPI_STORE);
-            gemm<false, false, __nv_bfloat16>(n, N, H, H, n->d_a[l], H, Wu + (int64_t)H * H, H, n->d_zu[l], H,
-                                              nullptr, nullptr, EPI_ADD);
-            // last slice: finishes zu and adds relu(zu) into h1 in its epilogue
-            gemm<false, false, __nv_bfloat16>(n, N, H, G, n->d_gf, G, Wu + (int64_t)2 * H * H, H, h1, H, nullptr,
-                                              n->d_zu[l], EPI_ACC_RELU_ADD);
+            run_jobs(n, job_fwd(n, "Wu", "bu", l, {{h, H, H}, {n->d_a[l], H, H}, {n->d_gf, G, G}}, H, n->d_h[l + 1],
+                                keep_z ? n->d_zu[l] : nullptr, h, jobs::RES_RELU));
         }
-        gemm<false, false, __nv_bfloat16>(n, N, O, H, n->d_h[n->L], H, B_(n, "Wo"), O, n->d_y, O, P_(n, "bo"),
-                                          nullptr, EPI_STORE);
+        run_jobs(n, job_fwd(n, "Wo", "bo", 0, {{n->d_h[n->L], H, H}}, O, n->d_y, nullptr, nullptr, jobs::STORE));
     }
     if (n->gate_B) {
         const int64_t tot = (int64_t)N * 2 * n->gate_nd;
@@ -551,50 +533,28 @@ void forward(lymph_mpnn* n, bool keep_z = true) {
 const float* eff_out(const lymph_mpnn* n) { return n->gate_B ? n->d_yg : n->d_y; }
 int64_t eff_width(const lymph_mpnn* n) { return n->gate_B ? 2 * n->gate_nd : n->O; }
 
-// backward from d_dy; gradients into d_g
+// backward from d_dy; gradients into d_g.  Each launch pairs a weight
+// gradient with the input gradient that reads the same dz; an input
+// gradient's epilogue masks it for the ReLU below.
 void backward(lymph_mpnn* n) {
-    const int N = n->n_nodes, H = n->H, F = n->F, G = n->G, O = n->O;
-    // Wo, bo
-    gemm<true, false, float>(n, H, O, N, n->d_h[n->L], H, n->d_dy, O, G_(n, "Wo"), O, nullptr, nullptr, EPI_STORE);
-    k_colsum<<<(O + 127) / 128, 128, 0, n->stream>>>(N, O, n->d_dy, G_(n, "bo"), 0);
-    n->launches++;
-    // dh = dy Wo^T
-    gemm<false, true, __nv_bfloat16>(n, N, H, O, n->d_dy, O, B_(n, "Wo"), O, n->d_dh, H, nullptr, nullptr, EPI_STORE);
+    const int H = n->H, F = n->F, G = n->G, O = n->O;
+    auto below = [&](int l) { return l > 0 ? n->d_zu[l - 1] : n->d_z0; };   // pre-activation of h[l]
+    // Wo, bo; dh = dy Wo^T
+    jobs::Job x = job_dx(n, "Wo", 0, n->d_dy, O, H, false, below(n->L), n->d_dz, nullptr);
+    run_jobs(n, job_dw(n, "Wo", 0, {{n->d_h[n->L], H, H}}, n->d_dy, O), &x);
     for (int l = n->L - 1; l >= 0; --l) {
         float* h = n->d_h[l];
-        const __nv_bfloat16* Wu = B_(n, "Wu", l);
-        float* gWu = G_(n, "Wu", l);
-        // dzu = dh * (zu > 0)
-        k_relu_back<<<256, 256, 0, n->stream>>>((int64_t)N * H, n->d_dh, n->d_zu[l], n->d_dz);
-        n->launches++;
-        // dWu slices, dbu
-        gemm<true, false, float>(n, H, H, N, h, H, n->d_dz, H, gWu, H, nullptr, nullptr, EPI_STORE);
-        gemm<true, false, float>(n, H, H, N, n->d_a[l], H, n->d_dz, H, gWu + (int64_t)H * H, H, nullptr, nullptr,
-                                 EPI_STORE);
-        gemm<true, false, float>(n, G, H, N, n->d_gf, G, n->d_dz, H, gWu + (int64_t)2 * H * H, H, nullptr, nullptr,
-                                 EPI_STORE);
-        k_colsum<<<(H + 127) / 128, 128, 0, n->stream>>>(N, H, n->d_dz, G_(n, "bu", l), 0);
-        n->launches++;
-        // dh (residual path) += dzu Wu[0:H]^T ; da = dzu Wu[H:2H]^T
-        gemm<false, true, __nv_bfloat16>(n, N, H, H, n->d_dz, H, Wu, H, n->d_dh, H, nullptr, nullptr, EPI_ADD);
-        gemm<false, true, __nv_bfloat16>(n, N, H, H, n->d_dz, H, Wu + (int64_t)H * H, H, n->d_dtmp, H, nullptr,
-                                         nullptr, EPI_STORE);
-        // dm = W^T da ; dzm = dm * (zm > 0)
-        aggregate(n, true, H, n->d_dtmp, n->d_dm);
-        k_relu_back<<<256, 256, 0, n->stream>>>((int64_t)N * H, n->d_dm, n->d_zm[l], n->d_dz);
-        n->launches++;
-        gemm<true, false, float>(n, H, H, N, h, H, n->d_dz, H, G_(n, "Wm", l), H, nullptr, nullptr, EPI_STORE);
-        k_colsum<<<(H + 127) / 128, 128, 0, n->stream>>>(N, H, n->d_dz, G_(n, "bm", l), 0);
-        n->launches++;
-        gemm<false, true, __nv_bfloat16>(n, N, H, H, n->d_dz, H, B_(n, "Wm", l), H, n->d_dh, H, nullptr, nullptr,
-                                         EPI_ADD);
+        // dz = dzu: dWu, dbu; dh (residual path) += dzu Wu[0:H]^T, da = dzu Wu[H:2H]^T
+        x = job_dx(n, "Wu", l, n->d_dz, H, 2 * H, true, nullptr, nullptr, n->d_dtmp);
+        run_jobs(n, job_dw(n, "Wu", l, {{h, H, H}, {n->d_a[l], H, H}, {n->d_gf, G, G}}, n->d_dz, H), &x);
+        // dzm = (W^T da) * (zm > 0)
+        aggregate(n, true, H, n->d_dtmp, n->d_dm, n->d_zm[l]);
+        // dWm, dbm; dh += dzm Wm^T, dz of the layer below
+        x = job_dx(n, "Wm", l, n->d_dm, H, H, true, below(l), n->d_dz, nullptr);
+        run_jobs(n, job_dw(n, "Wm", l, {{h, H, H}}, n->d_dm, H), &x);
     }
-    // dz0 = dh * (z0 > 0); dW0 = x^T dz0; db0
-    k_relu_back<<<256, 256, 0, n->stream>>>((int64_t)N * H, n->d_dh, n->d_z0, n->d_dz);
-    n->launches++;
-    gemm<true, false, float>(n, F, H, N, n->d_x, F, n->d_dz, H, G_(n, "W0"), H, nullptr, nullptr, EPI_STORE);
-    k_colsum<<<(H + 127) / 128, 128, 0, n->stream>>>(N, H, n->d_dz, G_(n, "b0"), 0);
-    n->launches++;
+    // dW0 = x^T dz0, db0
+    run_jobs(n, job_dw(n, "W0", 0, {{n->d_x, F, F}}, n->d_dz, H));
 }
 
 int set_graph(lymph_mpnn* n, int n_nodes, const int32_t* wp, const int32_t* wi, const float* wv, const float* gfeat) {
@@ -904,6 +864,8 @@ int lymph_mpnn_create(int32_t F, int32_t H, int32_t O, int32_t L, int32_t G, lym
     const char* ws = std::getenv("LYMPH_UMMA_WS");
     n->use_ws = !(ws && ws[0] == '0');
     if (cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess) { delete n; lymph_set_error("lymph_mpnn_create: stream"); return LYMPH_ERR_CUDA; }
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, dev);
     size_t b = sizeof(float) * (size_t)n->n_par;
     if (cudaMalloc(&n->d_p, b) != cudaSuccess || cudaMalloc(&n->d_g, b) != cudaSuccess || cudaMalloc(&n->d_m, b) != cudaSuccess ||
         cudaMalloc(&n->d_v, b) != cudaSuccess || cudaMalloc(&n->d_pb, sizeof(__nv_bfloat16) * (size_t)n->n_par) != cudaSuccess ||
@@ -1010,13 +972,13 @@ int lymph_mpnn_loss_grad(lymph_mpnn* n, const float* x, const float* target, dou
     LYMPH_CUDA_TRY(cudaGetLastError());
     double part[nb];
     LYMPH_CUDA_TRY(cudaMemcpyAsync(part, n->d_partial, sizeof(double) * nb, cudaMemcpyDeviceToHost, n->stream));
-    LYMPH_CUDA_TRY(cudaStreamSynchronize(n->stream));
-    if (loss) {
+    const int rc = read_status(n, "lymph_mpnn_loss_grad");   // synchronises
+    if (loss && rc != LYMPH_ERR_CUDA) {
         double s = 0.0;
         for (int i = 0; i < nb; ++i) s += part[i];
         *loss = s / (double)ny;
     }
-    return read_status(n, "lymph_mpnn_loss_grad");
+    return rc;
 }
 
 // Switches the output head to the gated form over the first B feature blocks
