@@ -185,8 +185,14 @@ template <int PD> __device__ __forceinline__ void load_der(DerTab<PD>* dst) {
     for (int i = threadIdx.x; i < (int)(sizeof(DerTab<PD>) / sizeof(short)); i += blockDim.x)
         reinterpret_cast<short*>(dst)[i] = src[i];
 }
-__device__ __forceinline__ double der_weight(int n, int t) {  // (2m + 1) for m = n - 1 - 2t
-    return n - 1 - 2 * t >= 0 ? (double)(2 * (n - 1 - 2 * t) + 1) : 0.0;
+// The weights of a box: w[f][k][t] = scale (2m + 1) / h_k for term t of d_k phi_f,
+// m = n_k - 1 - 2t (0: no such term), formed once per CTA: a division per term
+// and pair cost more than the expansion itself.
+template <int PD> __device__ __forceinline__ void load_weights(const DerTab<PD>& der, const double* hb, double scale, double* w) {
+    for (int i = threadIdx.x; i < Deg<PD>::NP * 6; i += blockDim.x) {
+        const int f = i / 6, k = i % 6 / 2, m = der.deg[f][k] - 1 - 2 * (i % 2);
+        w[i] = m >= 0 ? scale * (double)(2 * m + 1) / hb[k] : 0.0;
+    }
 }
 
 struct AsmArgs {
@@ -217,12 +223,14 @@ struct AsmArgs {
 
 // Interval constants of a bounding box per coordinate, as legendre_1d forms them.
 struct BoxC {
-    double mb[3], hb[3], sh[3];
+    double mb[3], hb[3], sh[3], ih[3], is[3];   // is: 1 / sqrt(hb)
 };
 __device__ __forceinline__ void box_consts(const double* bb, BoxC* B, int d) {
     B->hb[d] = (bb[2 * d + 1] - bb[2 * d]) / 2.0;
     B->mb[d] = (bb[2 * d + 1] + bb[2 * d]) / 2.0;
     B->sh[d] = sqrt(B->hb[d]);
+    B->ih[d] = 1.0 / B->hb[d];
+    B->is[d] = 1.0 / B->sh[d];
 }
 // The scaled Legendre values of degrees 0..PD at coordinate x of direction d:
 // legendre_1d's values, with the interval's constants and the normalised
@@ -232,6 +240,24 @@ __device__ __forceinline__ void legendre_vals(const BoxC* B, int d, double x, do
     const double xp = (x - B->mb[d]) / B->hb[d], sh = B->sh[d];
 #pragma unroll
     for (int n = 0; n <= PD; ++n) v[n] = lp_nonnorm(xp, n) / sh;
+}
+
+// The same to rounding, for the operator blocks: the three-term recurrence and
+// products with the interval's reciprocals instead of a division per degree
+// (ih = 1 / hb, is = 1 / sqrt(hb)).
+template <int PD>
+__device__ __forceinline__ void legendre_rec(double mb, double ih, double is, double x, double* v) {
+    const double xp = (x - mb) * ih;
+    double l0 = is, l1 = xp * is;
+    v[0] = l0;
+    v[1] = l1;
+#pragma unroll
+    for (int n = 1; n < PD; ++n) {
+        const double l2 = fma((2.0 * n + 1.0) / (n + 1.0) * xp, l1, -(n / (n + 1.0)) * l0);
+        v[n + 1] = l2;
+        l0 = l1;
+        l1 = l2;
+    }
 }
 
 // Coordinate j of the affine map of face f of a tetrahedron: cm[l] =
@@ -410,7 +436,7 @@ __global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
                 const double* nt = &A.ref->nodtria2[q * 4];
                 double x = 0.0;
                 for (int l = 0; l < 4; ++l) x = x + cm[l] * nt[l];
-                legendre_vals<PD>(&box, d, x, tleg + it * L1);
+                legendre_rec<PD>(box.mb[d], box.ih[d], box.is[d], x, tleg + it * L1);
                 if (d == 0) tw[qq] = A.ref->weitria2[q] * A.area[A.bf[eb + fi]];
             }
             __syncthreads();
@@ -437,6 +463,9 @@ __global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
 #pragma unroll
                 for (int j = (WHICH == ASM_ADG ? 6 : 0); j < FACE_F; ++j) mats[(2 + j) * NS + e] = acc[u][j];
         }
+        __syncthreads();                     // the last faces' tables are read
+        double* wder = tphi;                 // [NP][3][2], over them
+        load_weights<PD>(der, box.hb, 1.0, wder);
         __syncthreads();
         // ---- the block from the moments, written column-major ----
         const double* ML = mats;
@@ -456,8 +485,8 @@ __global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
                 for (int t = 0; t < 2; ++t) {
                     ia[d][t] = der.idx[a][d][t];
                     ib[d][t] = der.idx[b][d][t];
-                    wa[d][t] = der_weight(der.deg[a][d], t) / box.hb[d];
-                    wb[d][t] = der_weight(der.deg[b][d], t) / box.hb[d];
+                    wa[d][t] = wder[a * 6 + d * 2 + t];
+                    wb[d][t] = wder[b * 6 + d * 2 + t];
                 }
             double V[3][3], tr = 0.0;        // lambda D_i M D_j^T + mu D_j M D_i^T
             double Gm[3][3];
@@ -587,7 +616,7 @@ __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_
             const double* nt = &A.ref->nodtria2[q * 4];
             double x = 0.0;
             for (int l = 0; l < 4; ++l) x = x + cm[l] * nt[l];
-            legendre_vals<PD>(&box[s], d, x, tleg + it * L1);
+            legendre_rec<PD>(box[s].mb[d], box[s].ih[d], box[s].is[d], x, tleg + it * L1);
         }
         __syncthreads();
         const double ar = A.area[code];
@@ -628,9 +657,15 @@ __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_
             for (int j = 0; j < 6; ++j) SP[u][j] = fma(ffac[6 + j], p[u], SP[u][j]);
         }
     }
+    double* wder = fphi;                                 // [2][NP][3][2], over the tables
+    static_assert(2 * NP * 6 <= 2 * NQ2 * NP + 2 * NQ2 * 3 * L1, "the weights fit the tables");
+    __syncthreads();   // the last triangle's tables are read
+    if (WHICH == ASM_K) {
+        load_weights<PD>(der, box[0].hb, -0.5 * A.theta, wder);
+        load_weights<PD>(der, box[1].hb, -0.5, wder + NP * 6);
+    }
     __syncthreads();
     double* o = A.out + k * ND * ND;
-    const double mth = -0.5 * A.theta;
 #pragma unroll
     for (int u = 0; u < PPT; ++u) {
         const int pr = tid + u * T;
@@ -647,9 +682,8 @@ __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
-                    const double w = der_weight(der.deg[a][i], t);
-                    if (w != 0.0) {
-                        const double wl = mth * (w / box[0].hb[i]);
+                    const double wl = wder[a * 6 + i * 2 + t];
+                    if (wl != 0.0) {
                         const int x = b * NP + der.idx[a][i][t];
 #pragma unroll
                         for (int j = 0; j < 3; ++j) {
@@ -658,9 +692,8 @@ __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_
                         }
                         tr = fma(wl, PM[i * NPAIR + x], tr);
                     }
-                    const double w2 = der_weight(der.deg[b][i], t);
-                    if (w2 != 0.0) {
-                        const double wr = -0.5 * (w2 / box[1].hb[i]);
+                    const double wr = wder[(NP + b) * 6 + i * 2 + t];
+                    if (wr != 0.0) {
                         const int x = der.idx[b][i][t] * NP + a;
 #pragma unroll
                         for (int j = 0; j < 3; ++j) {
@@ -962,8 +995,7 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
                     double x = 0.0;
                     for (int l = 0; l < 4; ++l) x = x + fk[d * 4 + l] * nt[l];
                     legendre_vals<PD>(&box, d, x, s_leg + it * L1);
-                    s_sc[it] = sin(DATA_PI * x);
-                    s_sc[R * 3 + it] = cos(DATA_PI * x);
+                    sincos(DATA_PI * x, &s_sc[it], &s_sc[R * 3 + it]);
                 }
                 __syncthreads();
                 for (int qq = tid; qq < nq; qq += T) {
@@ -1017,8 +1049,7 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
                 double y = 0.0;
                 for (int kk = 0; kk < 4; ++kk)
                     for (int tt = 0; tt < 4; ++tt) y = y + fk[j * 4 + kk] * nm[kk * 4 + tt] * nt[tt];
-                s_sc[it] = sin(DATA_PI * y);
-                s_sc[R * 3 + it] = cos(DATA_PI * y);
+                sincos(DATA_PI * y, &s_sc[it], &s_sc[R * 3 + it]);
             }
             __syncthreads();
             for (int q = tid; q < NQ2; q += T) {
