@@ -887,6 +887,8 @@ __device__ inline void dev_analytic(int id, const double* sn, const double* cs, 
     }
 }
 
+enum { VEC_RHS = 0, VEC_PROJECT = 1 };   // MAKE_RHS_FREE, L2 projection
+
 struct VecArgs {
     const int32_t* poly_ptr;
     const int32_t* poly_tets;
@@ -902,7 +904,6 @@ struct VecArgs {
     const double* hk;
     const RefTables* ref;
     double alpha, theta;
-    int mode;            // 0 = RHS (MAKE_RHS_FREE), 1 = L2 projection
     int fid, did, nid;   // data function ids
     const double* R;     // modal factor (projection only)
     double scale;
@@ -950,8 +951,8 @@ __device__ inline void lane_solve_rtr(int NP, const double* __restrict__ R, doub
 // ic_displacement, uex_stat) do no quadrature.  Values and sums keep
 // legendre_1d's and the reference's order: the projection's solve amplifies a
 // change of rounding by the condition number of the mass matrix.
-template <int PD>
-__global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
+template <int PD, int MODE>
+__global__ void __launch_bounds__(VecShape<PD>::T, PD < 3 ? 1 : (MODE == VEC_PROJECT ? 7 : 5)) k_vector(VecArgs A) {
     using D = Deg<PD>;
     constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = D::NQ2, T = VecShape<PD>::T, R = VecShape<PD>::R, L1 = PD + 1;
     extern __shared__ double vsm[];
@@ -968,9 +969,9 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
     load_der<PD>(&der);
     if (tid < 3) box_consts(&A.bbox[P * 6], &box, tid);
     for (int i = tid; i < ND; i += T) s_acc[i] = 0.0;
-    const bool vol = A.mode == 0 ? A.fid != LYMPH_F_NULL
+    const bool vol = MODE == VEC_RHS ? A.fid != LYMPH_F_NULL
                                  : (A.fid == LYMPH_FUN_IC_VELOCITY || A.fid == LYMPH_FUN_UEX);
-    const bool bnd = A.mode == 0 && (A.did != LYMPH_GD_NULL || A.nid == LYMPH_GN);
+    const bool bnd = MODE == VEC_RHS && (A.did != LYMPH_GD_NULL || A.nid == LYMPH_GN);
     const int k1 = vol || bnd ? A.poly_ptr[P + 1] : A.poly_ptr[P];
     for (int kt = A.poly_ptr[P]; kt < k1; ++kt) {
         const int t = A.poly_tets[kt];
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
         double s = 0.0;   // this thread's row (T >= ND)
         static_assert(T >= ND, "one thread per row");
         if (vol) {
-            if (A.mode != 0 && tid < ND) s = s_acc[tid];
+            if (MODE != VEC_RHS && tid < ND) s = s_acc[tid];
             for (int q0 = 0; q0 < NQ3; q0 += R) {
                 const int nq = (NQ3 - q0) < R ? (NQ3 - q0) : R;
                 __syncthreads();
@@ -1001,7 +1002,7 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
                 for (int qq = tid; qq < nq; qq += T) {
                     double r[3];
                     const double *sn = &s_sc[qq * 3], *cs = &s_sc[R * 3 + qq * 3];
-                    if (A.mode == 0) dev_forcing(A.fid, lam, mu, rho, sn, cs, r);
+                    if (MODE == VEC_RHS) dev_forcing(A.fid, lam, mu, rho, sn, cs, r);
                     else dev_analytic(A.fid, sn, cs, r);
                     const double w = aj * A.ref->weitet3[q0 + qq];
                     s_wd[qq * 3 + 0] = w * r[0]; s_wd[qq * 3 + 1] = w * r[1]; s_wd[qq * 3 + 2] = w * r[2];
@@ -1019,13 +1020,13 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
                 }
             }
             if (tid < ND) {
-                if (A.mode == 0) s_acc[tid] += s;
+                if (MODE == VEC_RHS) s_acc[tid] += s;
                 else s_acc[tid] = s;
             }
         }
-        if (!bnd) continue;
         // boundary faces of this tetrahedron (only boundary faces are added, :809-819)
-        for (int f = 0; f < 4; ++f) {
+        if constexpr (MODE == VEC_RHS)
+        for (int f = 0; bnd && f < 4; ++f) {
             const int E2 = A.neigh[t * 4 + f];
             if (E2 != LYMPH_BC_DIRI && E2 != LYMPH_BC_NEUM) continue;
             if (E2 == LYMPH_BC_DIRI ? A.did == LYMPH_GD_NULL : A.nid != LYMPH_GN) continue;   // zero data
@@ -1107,7 +1108,7 @@ __global__ void __launch_bounds__(VecShape<PD>::T) k_vector(VecArgs A) {
         }
     }
     __syncthreads();
-    if (A.mode == 0) {
+    if (MODE == VEC_RHS) {
         for (int r = tid; r < ND; r += T) A.out[(int64_t)P * ND + r] = s_acc[r];
         return;
     }
@@ -1273,19 +1274,19 @@ int assemble_degree(lymph_ctx* c, double* out, bool write_mass) {
     }
 }
 
-template <int PD>
-int launch_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scale, double* out) {
+template <int PD, int MODE>
+int launch_vector(lymph_ctx* c, int fid, int did, int nid, double scale, double* out) {
     VecArgs A;
     A.poly_ptr = c->d_poly_ptr; A.poly_tets = c->d_poly_tets; A.tet_mat = c->d_tet_mat; A.neigh = c->d_neigh;
     A.fun_tag = c->d_fun_tag; A.mat = c->d_mat; A.fk = c->d_fk; A.jdet = c->d_jdet; A.nrm = c->d_normal;
     A.area = c->d_area; A.bbox = c->d_bbox; A.hk = c->d_hk; A.ref = c->d_ref; A.alpha = c->alpha; A.theta = c->theta;
-    A.mode = mode; A.fid = fid; A.did = did; A.nid = nid; A.R = c->d_Rm; A.scale = scale; A.out = out;
+    A.fid = fid; A.did = did; A.nid = nid; A.R = c->d_Rm; A.scale = scale; A.out = out;
     using D = Deg<PD>;
     using V = VecShape<PD>;
     const size_t face = (size_t)D::NQ2 * 3 * (D::NP + PD + 1);   // gradient tables of a boundary face (RHS only)
-    const size_t smem = sizeof(double) * ((size_t)D::ND + (size_t)V::R * (D::NP + 3 * (PD + 1) + 9) + (mode == 0 ? face : 0));
-    LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_vector<PD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_vector<PD><<<c->n_poly, V::T, smem, c->stream>>>(A);
+    const size_t smem = sizeof(double) * ((size_t)D::ND + (size_t)V::R * (D::NP + 3 * (PD + 1) + 9) + (MODE == VEC_RHS ? face : 0));
+    LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_vector<PD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_vector<PD, MODE><<<c->n_poly, V::T, smem, c->stream>>>(A);
     c->launches++;
     LYMPH_CUDA_TRY(cudaGetLastError());
     return LYMPH_OK;
@@ -1400,10 +1401,14 @@ int lymph_dev_double_couple(lymph_ctx* c, int t, int P, const double moment[9], 
 
 int lymph_dev_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scale, double* out) {
     switch (c->p) {
-        case 1: return launch_vector<1>(c, mode, fid, did, nid, scale, out);
-        case 2: return launch_vector<2>(c, mode, fid, did, nid, scale, out);
-        case 3: return launch_vector<3>(c, mode, fid, did, nid, scale, out);
-        case 4: return launch_vector<4>(c, mode, fid, did, nid, scale, out);
+        case 1: return mode == VEC_RHS ? launch_vector<1, VEC_RHS>(c, fid, did, nid, scale, out)
+                                       : launch_vector<1, VEC_PROJECT>(c, fid, did, nid, scale, out);
+        case 2: return mode == VEC_RHS ? launch_vector<2, VEC_RHS>(c, fid, did, nid, scale, out)
+                                       : launch_vector<2, VEC_PROJECT>(c, fid, did, nid, scale, out);
+        case 3: return mode == VEC_RHS ? launch_vector<3, VEC_RHS>(c, fid, did, nid, scale, out)
+                                       : launch_vector<3, VEC_PROJECT>(c, fid, did, nid, scale, out);
+        case 4: return mode == VEC_RHS ? launch_vector<4, VEC_RHS>(c, fid, did, nid, scale, out)
+                                       : launch_vector<4, VEC_PROJECT>(c, fid, did, nid, scale, out);
         default: lymph_set_error("degree not supported on the device"); return LYMPH_ERR_INVALID;
     }
 }
