@@ -28,6 +28,7 @@ int lymph_dev_mass(lymph_ctx* c);
 int lymph_dev_self_tc(lymph_ctx* c, float* out, bool block_csr);
 int lymph_dev_nb_tc(lymph_ctx* c, float* out, const int64_t* list, int64_t n_list);
 int lymph_dev_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scale, double* out);
+int lymph_dev_block_exponents(lymph_ctx* c);
 int lymph_dev_step(lymph_ctx* c, int off, double g, bool fresh);
 int lymph_dev_run_start(lymph_ctx* c);
 int lymph_dev_first_step(lymph_ctx* c, double g);
@@ -597,10 +598,18 @@ int lymph_make_matrices(lymph_ctx* c) {
         c->device_bytes += (int64_t)(nK * es);
     }
     if (!c->d_M) LYMPH_TRY(alloc_mass(c));
+    if (c->precision == LYMPH_FP64 && c->p >= 3 && !c->d_Kex) {
+        Arena ar;
+        ar.raw(&c->d_Kex, (size_t)c->n_blocks);
+        LYMPH_TRY(ar.make(c));
+    }
     c->k32_valid = false;  // an FP32 copy made from earlier blocks is stale
     c->rhs_version++;      // and so is any cached M^-1 F
     if (c->precision == LYMPH_MIXED) LYMPH_TRY(make_mixed_blocks(c));
-    else LYMPH_TRY(lymph_dev_assemble(c, LYMPH_BLOCKS_K, (double*)c->d_K, true));
+    else {
+        LYMPH_TRY(lymph_dev_assemble(c, LYMPH_BLOCKS_K, (double*)c->d_K, true));
+        LYMPH_TRY(lymph_dev_block_exponents(c));
+    }
     LYMPH_TRY(lymph_dev_cholesky(c));
     LYMPH_TRY(lymph_dev_damping(c, true));
     LYMPH_TRY(lymph_sync_status(c, "lymph_make_matrices"));

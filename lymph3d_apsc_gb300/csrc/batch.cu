@@ -218,6 +218,7 @@ int refresh_problems(lymph_batch* b) {
         P.a.row_ptr = c->d_row_ptr;
         P.a.col = c->d_col;
         P.a.K = c->d_K;
+        P.a.Kex = c->d_Kex;
         P.a.Minv = c->d_Minv;
         P.a.rhs_stat = c->d_rhs_stat;
         P.a.rhs_dyn = c->d_rhs_dyn;

@@ -819,6 +819,7 @@ void lymph_mf_batch_problem(const lymph_ctx* c, int* status, void* out) {
     s.row_ptr = c->d_row_ptr;
     s.col = c->d_col;
     s.K = c->d_K;
+    s.Kex = nullptr;
     s.Minv = c->d_Minv;
     s.rhs_stat = c->d_rhs_stat;
     s.rhs_dyn = c->d_rhs_dyn;

@@ -318,7 +318,8 @@ int launch_ctx(lymph_ctx* c, const StepArgs& A, bool fresh = false) {
 
 StepArgs base_args(lymph_ctx* c) {
     StepArgs A;
-    A.row_ptr = c->d_row_ptr; A.col = c->d_col; A.K = c->d_K; A.Minv = c->d_Minv;
+    A.row_ptr = c->d_row_ptr; A.col = c->d_col; A.K = c->d_K; A.Kex = c->d_Kex;
+    A.Minv = c->d_Minv;
     A.rhs_stat = c->d_rhs_stat; A.rhs_dyn = c->d_rhs_dyn; A.gvals = nullptr; A.step_idx = nullptr;
     A.step_off = 0; A.g = 0.0; A.u32_out = nullptr;
     A.u0 = nullptr; A.un = nullptr; A.out = nullptr; A.partial = c->d_partial; A.dt = c->dt; A.status = c->d_status;
@@ -387,6 +388,23 @@ int lymph_dev_apply_fp32(lymph_ctx* c, const float* K32, const double* u, double
     A.u0 = u;
     A.out = out;
     return launch_step_p<float, MODE_APPLY>(c, A);
+}
+
+// The largest biased exponent of each FP64 block's entries (at least 200, so that
+// an entry of exponent 0 is shifted out of the integer accumulator; far above
+// any where the block holds infinities or NaN), a CTA per block.
+__global__ void __launch_bounds__(256) k_block_exponents(const double* __restrict__ K, int nd2, int64_t block0, int32_t* ex) {
+    __shared__ int s_e[8];
+    const int64_t k = block0 + blockIdx.x;
+    int e = 200;
+    for (int i = threadIdx.x; i < nd2; i += 256) e = max(e, __double2hiint(K[k * nd2 + i]) >> 20 & 0x7ff);
+    e = __reduce_max_sync(0xffffffffu, e);
+    if ((threadIdx.x & 31) == 0) s_e[threadIdx.x >> 5] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) e = max(e, s_e[w]);
+        ex[k] = e == 0x7ff ? EXP_NONFINITE : e;
+    }
 }
 
 // dst[i] = (float)src[i]
@@ -487,6 +505,20 @@ int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double
     k_l2_partial<<<c->n_poly, L2_THREADS, 0, c->stream>>>(c->Np, c->d_Mm, uh, uex, c->d_partial);
     k_sum<<<1, 1024, 0, c->stream>>>(c->n_poly, c->d_partial, d_out);
     c->launches += 2;
+    LYMPH_CUDA_TRY(cudaGetLastError());
+    return LYMPH_OK;
+}
+
+// The exponents of the assembled FP64 blocks that the integer columns of the step
+// kernel need (p = 3, 4).
+int lymph_dev_block_exponents(lymph_ctx* c) {
+    if (!c->d_Kex) return LYMPH_OK;
+    const int64_t chunk = 1 << 20;
+    for (int64_t b0 = 0; b0 < c->n_blocks; b0 += chunk) {
+        const unsigned nb = (unsigned)(c->n_blocks - b0 < chunk ? c->n_blocks - b0 : chunk);
+        k_block_exponents<<<nb, 256, 0, c->stream>>>((const double*)c->d_K, c->nd * c->nd, b0, c->d_Kex);
+        c->launches++;
+    }
     LYMPH_CUDA_TRY(cudaGetLastError());
     return LYMPH_OK;
 }

@@ -3,9 +3,83 @@
 // (batch.cu).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace stepk {
+
+// ---- FP64 products on the integer pipe ----
+//
+// The GB300 retires 2 FP64 multiply-adds per clock and SM, which holds a product
+// with FP64 blocks at two thirds of the copy bandwidth, while its integer pipe idles.
+// At p = 3 and 4, 60 % of each row's columns (the last ones, c >= C0) are therefore
+// multiplied there: a block entry and a coefficient are doubles as before, their
+// mantissas multiply to the product's top 64 bits (relative error below 2^-61; an
+// FP64 product rounds to 2^-53), and the product, shifted by the exponents, adds up
+// exactly in a 128-bit accumulator whose top stands at the largest product any
+// block of the row could have.  A term loses bits only below 2^-117 of that.  The
+// sum is rounded to FP64 once per 16 blocks, so the row's error falls (K u of
+// random, graded and near-constant states: by 40 % in the mean).
+// 16 steps of 46,767 polyhedra at p = 3: 56.0 -> 38.0 ms (61 -> 90 % of the copy
+// bandwidth); 24 steps of a mesh of 17^3 cubes at p = 4: 18.8 -> 13.2 ms.
+constexpr bool int_columns(int p, size_t elem) { return p >= 3 && elem == 8; }
+constexpr int INT_HEAD = 10;         // bits of headroom: at most 2^9 terms of a thread
+constexpr int EXP_NONE = -(1 << 20);
+constexpr int EXP_NONFINITE = 1 << 20;
+
+// |x| = m 2^(e - 1086), m with its top bit set (m = 0, e = EXP_NONE for zero).
+__device__ __forceinline__ unsigned long long split_mantissa(double x, int* e) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+    const int ef = (int)(b >> 52);
+    if (ef == 0x7ff) { *e = EXP_NONFINITE; return 0; }
+    if (ef > 0) { *e = ef; return 1ull << 63 | b << 11; }
+    if (b == 0) { *e = EXP_NONE; return 0; }
+    const int lz = __clzll((long long)b);
+    *e = 12 - lz;
+    return b << lz;
+}
+
+struct Acc128 {
+    unsigned long long lo;
+    long long hi;
+};
+// acc += K u; u: the mantissa's words, the shift before K's exponent, the sign in bit 31.
+__device__ __forceinline__ void int_fma(Acc128& acc, double K, const uint4 u) {
+    const unsigned kh = (unsigned)__double2hiint(K), kl = (unsigned)__double2loint(K);
+    // K's mantissa with its top bit set; a zero or denormal entry's exponent 0
+    // shifts it out of the accumulator
+    const unsigned mh = __funnelshift_l(kl, kh, 11) | 0x80000000u, ml = kl << 11;
+    const unsigned long long p =
+        (unsigned long long)mh * u.x + __umulhi(mh, u.y) + (unsigned long long)__umulhi(ml, u.x);
+    const unsigned s = u.z - (kh >> 20 & 0x7ff);
+    unsigned long long vh, v1, v2;   // (p 2^64) >> s in two words; PTX shifts by 64 and more give 0
+    asm("shr.u64 %0, %1, %2;" : "=l"(vh) : "l"(p), "r"(s));
+    asm("shl.b64 %0, %1, %2;" : "=l"(v1) : "l"(p), "r"(64u - s));
+    asm("shr.u64 %0, %1, %2;" : "=l"(v2) : "l"(p), "r"(s - 64u));
+    const unsigned m32 = (unsigned)((int)(kh ^ u.w) >> 31);   // all ones: a negative product
+    const unsigned long long m = (unsigned long long)m32 << 32 | m32;
+    const unsigned long long a = (v1 | v2) ^ m, b = vh ^ m;
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %2, 1;\n\t"     // carry: + 1 for a negated term
+        "addc.cc.u64 %0, %0, %3;\n\t"
+        "addc.u64 %1, %1, %4;\n\t}"
+        : "+l"(acc.lo), "+l"(acc.hi)
+        : "r"(m32), "l"(a), "l"(b));
+}
+// The accumulator's value: acc 2^(R - 2162), R the exponent its top stands at.
+__device__ __forceinline__ double acc_value(Acc128 acc, int R) {
+    if (R == EXP_NONE) return 0.0;
+    if (R >= EXP_NONFINITE / 2) return __longlong_as_double(0x7ff8000000000000ll);
+    const bool neg = acc.hi < 0;
+    if (neg) {
+        acc.lo = ~acc.lo + 1;
+        acc.hi = ~acc.hi + (acc.lo == 0);
+    }
+    const double d = fma((double)acc.lo, 5.42101086242752217e-20 /* 2^-64 */, (double)(unsigned long long)acc.hi);
+    const double v = ldexp(d, R - 2098);
+    return neg ? -v : v;
+}
 
 template <int P> struct Deg {
     static constexpr int NP = (P + 1) * (P + 2) * (P + 3) / 6;
@@ -18,7 +92,7 @@ template <int P> struct Shape {
     static constexpr int ND = Deg<P>::ND;
     static constexpr int S = P == 1 ? 8 : (P == 2 ? 8 : (P == 3 ? 4 : 3));
     static constexpr int T = ((ND * S + 31) / 32) * 32;       // 96, 256, 256, 320
-    static constexpr int MINB = P == 1 ? 16 : (P == 4 ? 4 : 6);
+    static constexpr int MINB = P == 1 ? 16 : (P == 4 ? 3 : 6);
 };
 
 constexpr int64_t STEP_PREFETCH = 32 * 1024;   // bytes of a row's blocks prefetched before its state is ready
@@ -39,6 +113,7 @@ struct StepArgs {
     const int32_t* row_ptr;
     const int32_t* col;
     const void* K;             // [n_blocks][ND][ND] column-major (double or float)
+    const int32_t* Kex;        // FP64 at p = 3, 4: largest biased exponent of each block's entries
     const double* Minv;        // [n_poly][NP][NP] column-major inverse of M_loc
     const double* rhs_stat;
     const double* rhs_dyn;
@@ -100,7 +175,16 @@ __device__ __forceinline__ float ld_stream(const float* p) { return __ldcs(p); }
 template <int PD, typename KT, int S_ = Shape<PD>::S> struct SmemSize {
     static constexpr int ND = Deg<PD>::ND, S = S_;
     static constexpr size_t b_offset = ((sizeof(KT) * (size_t)(NBB * ND + S * ND)) + 15) & ~(size_t)15;
-    static constexpr size_t bytes = b_offset + sizeof(double) * (ND + finish_scratch(ND, MAX_STEP_THREADS));
+    // the columns of the integer pipe: a thread's last NI of CPT, c >= C0 (12 of 35:
+    // 14.1 and 44.0 ms for the runs above, 16 of 35: 13.5 and 41.0, 19 of 35: 13.4 and
+    // 38.1, 24 of 35: 13.2 and 38.9)
+    static constexpr int CPT = (ND + S - 1) / S, NI = int_columns(PD, sizeof(KT)) ? CPT * 21 / 35 : 0;
+    static constexpr int C0 = (CPT - NI) * S < ND ? (CPT - NI) * S : ND, NC = ND - C0;
+    static_assert(NI * NBB < 1 << (INT_HEAD - 1), "the accumulator's headroom");
+    static constexpr size_t m_offset =
+        (b_offset + sizeof(double) * (ND + finish_scratch(ND, MAX_STEP_THREADS)) + 15) & ~(size_t)15;
+    static constexpr size_t r_offset = m_offset + sizeof(uint4) * NBB * NC;
+    static constexpr size_t bytes = r_offset + (NI ? sizeof(int) : 0);
 };
 
 // y_r = sum_c A(r, c) w_c for rows r < ND of a column-major ND x ND matrix in
@@ -252,14 +336,45 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
         pdl_wait();
     }
 
+    using SZ = SmemSize<PD, KT, S>;
+    constexpr int NI = SZ::NI, C0 = SZ::C0, NC = SZ::NC, JF = CPT - NI;
+    uint4* s_m = (uint4*)(smem + SZ::m_offset);   // the integer columns' coefficients
+    int* s_R = (int*)(smem + SZ::r_offset);       // the accumulators' exponent
+
     AT acc0 = 0, acc1 = 0;
     for (int b0 = rb; b0 < re; b0 += NBB) {
         const int nb = (re - b0) < NBB ? (re - b0) : NBB;
+        if (NI && tid == 0) *s_R = EXP_NONE;
         __syncthreads();
         for (int i = tid; i < nb * ND; i += nthr) {
             const int bb = i / ND, c = i % ND;
             const int64_t q = (int64_t)A.col[b0 + bb] * ND + c;
             s_u[i] = (AT)((MODE == MODE_FIRST || MODE == MODE_BILIN) ? A.u0[q] : A.un[q]);
+        }
+        Acc128 iacc = {0, 0};
+        int R = EXP_NONE;
+        if constexpr (NI > 0) {
+            __syncthreads();
+            // mantissas and exponents of the integer columns, then the largest
+            // exponent a product of the row can have
+            int mx = EXP_NONE;
+            for (int i = tid; i < nb * NC; i += nthr) {
+                const int bb = i / NC, kx = A.Kex[b0 + bb];
+                const double u = s_u[bb * ND + C0 + i - bb * NC];
+                int e;
+                const unsigned long long m = split_mantissa(u, &e);
+                s_m[i] = make_uint4((unsigned)(m >> 32), (unsigned)m, (unsigned)e, u < 0.0 ? 0x80000000u : 0u);
+                if (e > EXP_NONE) mx = max(mx, e + kx);
+                else if (kx == EXP_NONFINITE) mx = kx;
+            }
+            mx = __reduce_max_sync(0xffffffffu, mx);
+            if ((tid & 31) == 0 && mx > EXP_NONE) atomicMax(s_R, mx);
+            __syncthreads();
+            R = *s_R;
+            for (int i = tid; i < nb * NC; i += nthr) {   // each thread's own entries
+                const int e = (int)s_m[i].z;
+                s_m[i].z = e > EXP_NONE && R < EXP_NONFINITE / 2 ? (unsigned)(INT_HEAD + R - e) : 1u << 16;
+            }
         }
         __syncthreads();
         if (act) {
@@ -276,11 +391,18 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
                 for (int j = 0; j < CPT; ++j) {
                     const int c = s + j * S;
                     if (c < ND) {
+                        if constexpr (NI > 0) {
+                            if (j >= JF) {
+                                int_fma(iacc, kv[j], s_m[bb * NC + c - C0]);
+                                continue;
+                            }
+                        }
                         if (j & 1) acc1 += (AT)kv[j] * ub[c];
                         else acc0 += (AT)kv[j] * ub[c];
                     }
                 }
             }
+            if constexpr (NI > 0) acc1 += acc_value(iacc, R);
         }
     }
     if (act) s_red[s * ND + r] = acc0 + acc1;
