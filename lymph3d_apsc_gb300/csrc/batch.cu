@@ -229,6 +229,7 @@ int refresh_problems(lymph_batch* b) {
         P.a.dt = c->dt;
         P.a.status = b->d_status;
         P.a.n_poly = c->n_poly;
+        P.a.prefetch = 1;
         P.buf[0] = c->d_buf[0];
         P.buf[1] = c->d_buf[1];
         P.cur0 = c->cur;

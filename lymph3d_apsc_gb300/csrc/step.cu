@@ -274,7 +274,10 @@ __global__ void k_normalize(int64_t n, const double* __restrict__ y, const doubl
 
 template <int PD, typename KT, int MODE>
 int launch_step_t(lymph_ctx* c, const StepArgs& A) {
-    if (MODE == MODE_STEP) {
+    // p = 1 in one wave of 8 to 16 CTAs per SM: an early launch unbalances the SMs and a
+    // late one comes too late (48 steps of 1,728 polyhedra: 475 us in FP32, plain 390 us)
+    const bool plain = PD == 1 && c->n_poly > 8 * 152 && c->n_poly <= 16 * 152;
+    if (MODE == MODE_STEP && !plain) {
         LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
     } else {
         k_step<PD, KT, MODE><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
@@ -324,6 +327,7 @@ StepArgs base_args(lymph_ctx* c) {
     A.step_off = 0; A.g = 0.0; A.u32_out = nullptr;
     A.u0 = nullptr; A.un = nullptr; A.out = nullptr; A.partial = c->d_partial; A.dt = c->dt; A.status = c->d_status;
     A.n_poly = c->n_poly;
+    A.prefetch = c->n_blocks * c->nd * c->nd * (c->precision == LYMPH_FP64 ? 8 : 4) <= STEP_PREFETCH_MAX;
     A.abs_idx = c->n_abs > 0 ? c->d_abs_idx : nullptr;
     A.Dabs = c->d_Dabs;
     A.Winv = c->d_Winv;

@@ -95,7 +95,13 @@ template <int P> struct Shape {
     static constexpr int MINB = P == 1 ? 16 : (P == 4 ? 3 : 6);
 };
 
-constexpr int64_t STEP_PREFETCH = 32 * 1024;   // bytes of a row's blocks prefetched before its state is ready
+// Bytes of a row's blocks prefetched before its state is ready, while a step's
+// blocks have at most 512 MB: then the prefetch is worth 1 to 10 % (48 FP32 steps
+// of 2,744 polyhedra at p = 3: 2.00 against 2.21 ms), with more it displaces what the
+// 129 MB L2 keeps from step to step (4,096 at p = 4: 9.62 against 8.92 ms; of 10,648
+// at p = 3: 8.37 against 7.66 ms).
+constexpr int STEP_PREFETCH = 32 * 1024;
+constexpr int64_t STEP_PREFETCH_MAX = 512ll << 20;
 
 constexpr int NBB = 16;   // neighbour blocks staged in shared memory at once
 
@@ -134,15 +140,22 @@ struct StepArgs {
     double dt;
     int* status;
     int n_poly;
+    int prefetch;              // whether a step prefetches its rows' heads
 };
 
 // Programmatic dependent launch: a step kernel starts while the one before it
 // finishes, reads what no step writes, and waits for that kernel and its writes
-// before it touches a state.  A no-op on a plain launch.
-__device__ __forceinline__ void pdl_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// before it touches a state.  No-ops on a plain launch.  The next step's CTAs may
+// be placed once every CTA of this one has triggered or ended.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// With stored blocks a grid of at most one CTA per SM (8 at p = 1) triggers as soon
+// as it may touch the state, a larger one when a CTA has summed its row: CTAs that
+// are placed early fill the slots of the SMs that are done first and leave the
+// others idle (48 steps of 512 polyhedra in FP64: p = 3 1.70 against 1.26 ms, p = 4
+// 6.0 against 4.3 ms with FP64 products alone; of 125 polyhedra at p = 4: 1.17
+// against 1.34 ms, of 1,000 at p = 1 374 against 433 us).
+__device__ __forceinline__ bool trigger_early(int p) { return gridDim.x <= (p == 1 ? 8u : 1u) * 152u; }
 
 // Launches a step kernel that may start before the stream's previous kernel ends.
 template <typename K, typename A>
@@ -328,12 +341,13 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
     const int rb = A.row_ptr[P], re = A.row_ptr[P + 1];
     const KT* Kbase = (const KT*)A.K;
     if (MODE == MODE_STEP) {
-        if (tid == 0) {   // the head of the row's blocks and M^-1, while the previous step ends
+        if (A.prefetch && tid == 0) {   // the head of the row's blocks and M^-1, while the previous step ends
             const int64_t row = (int64_t)(re - rb) * ND * ND * (int64_t)sizeof(KT);
             prefetch_inside(Kbase + (int64_t)rb * ND * ND, row < STEP_PREFETCH ? row : STEP_PREFETCH);
             prefetch_inside(A.Minv + (int64_t)P * Deg<PD>::NP * Deg<PD>::NP, (int64_t)Deg<PD>::NP * Deg<PD>::NP * 8);
         }
         pdl_wait();
+        if (trigger_early(PD)) pdl_trigger();
     }
 
     using SZ = SmemSize<PD, KT, S>;
@@ -405,6 +419,7 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
             if constexpr (NI > 0) acc1 += acc_value(iacc, R);
         }
     }
+    if (MODE == MODE_STEP) pdl_trigger();
     if (act) s_red[s * ND + r] = acc0 + acc1;
     __syncthreads();
     double y = 0.0;
