@@ -53,10 +53,11 @@ static_assert(WS_SPLIT_WARPS % 4 == 0, "whole groups of 4 warps (one per TMEM la
 
 struct alignas(64) WsArgs {
     CUtensorMap mapA[3];  // per K segment: [M][K_s] FP32, box 32 x 128, 128-byte swizzle
-    CUtensorMap mapB;     // [Npad][Ktot] FP32, box 32 x min(Npad, 256), 128-byte swizzle
+    CUtensorMap mapB;     // [Npad][Ktot] FP32, box 32 x min(Npad, bn), 128-byte swizzle
     int segK[3];
     int nseg;
     int M, N, Npad, Ktot;
+    int bn;               // columns per CTA (32 to WS_BN)
     const float* bias;
     float* C;
     int ldc;
@@ -105,8 +106,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_umma_gemm_ws(const __grid_con
     __shared__ int s_abort;
     __shared__ int s_issued[WS_STAGES];  // per stage the last k-step whose TMA loads were issued (-1: none)
     const int t = threadIdx.x, warp = t / 32, lane = t % 32;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * WS_BN;
-    const int nb = (a.Npad - n0) < WS_BN ? (a.Npad - n0) : WS_BN;  // this CTA's columns (multiple of 16)
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * a.bn;
+    const int nb = (a.Npad - n0) < a.bn ? (a.Npad - n0) : a.bn;  // this CTA's columns (multiple of 16)
     uint32_t ncols = 32;
     while ((int)ncols < nb) ncols <<= 1;
     int T = 0;
@@ -138,7 +139,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_umma_gemm_ws(const __grid_con
     if (warp == 0) {
         // ---- producer ----
         if (lane == 0) {
-            const uint32_t bytes = (uint32_t)(BM * BK * 4 + nb * BK * 4);
+            // whole boxes: what lies outside the tensor is zero-filled and counted
+            const uint32_t bytes = (uint32_t)(BM * BK * 4 + (a.Npad < a.bn ? a.Npad : a.bn) * BK * 4);
             int kt = 0, koff = 0;
             for (int sg = 0; sg < a.nseg && !*abort; ++sg) {
                 for (int k0 = 0; k0 < a.segK[sg]; k0 += BK, ++kt) {
