@@ -28,6 +28,7 @@ int lymph_dev_mass(lymph_ctx* c);
 int lymph_dev_self_tc(lymph_ctx* c, float* out, bool block_csr);
 int lymph_dev_nb_tc(lymph_ctx* c, float* out, const int64_t* list, int64_t n_list);
 int lymph_dev_vector(lymph_ctx* c, int mode, int fid, int did, int nid, double scale, double* out);
+bool lymph_dev_int_columns(const lymph_ctx* c);
 int lymph_dev_block_exponents(lymph_ctx* c);
 int lymph_dev_step(lymph_ctx* c, int off, double g, bool fresh);
 int lymph_dev_run_start(lymph_ctx* c);
@@ -598,7 +599,7 @@ int lymph_make_matrices(lymph_ctx* c) {
         c->device_bytes += (int64_t)(nK * es);
     }
     if (!c->d_M) LYMPH_TRY(alloc_mass(c));
-    if (c->precision == LYMPH_FP64 && c->p >= 3 && !c->d_Kex) {
+    if (lymph_dev_int_columns(c) && !c->d_Kex) {
         Arena ar;
         ar.raw(&c->d_Kex, (size_t)c->n_blocks);
         LYMPH_TRY(ar.make(c));

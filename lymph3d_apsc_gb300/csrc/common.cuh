@@ -91,7 +91,7 @@ struct lymph_ctx {
     int32_t* d_bf = nullptr;
     // operator
     void* d_K = nullptr;            // [n_blocks][nd][nd] column-major per block (FP64 or FP32)
-    int32_t* d_Kex = nullptr;       // FP64, p = 3, 4: largest exponent of each block (step_body.cuh)
+    int32_t* d_Kex = nullptr;       // FP64 with integer columns: largest exponent of each block (step_body.cuh)
     float* d_K32 = nullptr;         // FP32 copy of FP64 blocks for the surrogate's operator apply (on demand)
     bool k32_valid = false;
     bool surrogate_apply_fp32 = false;  // lymph_surrogate_apply_fp32

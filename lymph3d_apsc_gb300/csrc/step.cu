@@ -23,10 +23,10 @@ namespace {
 using namespace stepk;
 
 // One CTA per polyhedron.
-template <int PD, typename KT, int MODE>
+template <int PD, typename KT, int MODE, bool INT = int_columns(PD, sizeof(KT))>
 __global__ void __launch_bounds__(Shape<PD>::T, Shape<PD>::MINB) k_step(StepArgs A) {
-    __shared__ __align__(16) char smem[SmemSize<PD, KT>::bytes];
-    step_poly<PD, KT, MODE>(A, blockIdx.x, smem);
+    __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
+    step_poly<PD, KT, MODE, Shape<PD>::S, INT>(A, blockIdx.x, smem);
 }
 
 __global__ void k_bump(int64_t* idx, int n) { *idx += n; }
@@ -272,18 +272,26 @@ __global__ void k_normalize(int64_t n, const double* __restrict__ y, const doubl
         x[i] = y[i] * inv;
 }
 
-template <int PD, typename KT, int MODE>
-int launch_step_t(lymph_ctx* c, const StepArgs& A) {
+template <int PD, typename KT, int MODE, bool INT>
+int launch_step_i(lymph_ctx* c, const StepArgs& A) {
     // p = 1 in one wave of 8 to 16 CTAs per SM: an early launch unbalances the SMs and a
     // late one comes too late (48 steps of 1,728 polyhedra: 475 us in FP32, plain 390 us)
     const bool plain = PD == 1 && c->n_poly > 8 * 152 && c->n_poly <= 16 * 152;
     if (MODE == MODE_STEP && !plain) {
-        LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
+        LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE, INT>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
     } else {
-        k_step<PD, KT, MODE><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
+        k_step<PD, KT, MODE, INT><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
     }
     c->launches++;
     return LYMPH_OK;
+}
+
+template <int PD, typename KT, int MODE>
+int launch_step_t(lymph_ctx* c, const StepArgs& A) {
+    if constexpr (PD == 2 && sizeof(KT) == 8) {
+        if (A.Kex) return launch_step_i<PD, KT, MODE, true>(c, A);
+    }
+    return launch_step_i<PD, KT, MODE, int_columns(PD, sizeof(KT))>(c, A);
 }
 
 template <typename KT, int MODE>
@@ -513,8 +521,18 @@ int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double
     return LYMPH_OK;
 }
 
-// The exponents of the assembled FP64 blocks that the integer columns of the step
-// kernel need (p = 3, 4).
+// Whether the context's step kernel multiplies columns on the integer pipe: FP64
+// blocks at p = 3 and 4, and at p = 2 on long rows (8 blocks or more on average)
+// from 4 CTAs per SM on: 46,767 polyhedra 16.2 -> 14.5 ms for 16 steps, 737 442 ->
+// 388 us.  The preparation of the coefficients costs a short row what it gains
+// (hexahedra, 7 blocks: 8,000 5.64 -> 5.66 ms for 48 steps), a small grid more (125:
+// 345 -> 405 us), and p = 1 at any size (46,767: 4.06 -> 4.25 ms).
+bool lymph_dev_int_columns(const lymph_ctx* c) {
+    if (c->precision != LYMPH_FP64) return false;
+    return c->p >= 3 || (c->p == 2 && c->n_poly >= 4 * 152 && c->n_blocks >= 8 * (int64_t)c->n_poly);
+}
+
+// The exponents of the assembled FP64 blocks that the integer columns need.
 int lymph_dev_block_exponents(lymph_ctx* c) {
     if (!c->d_Kex) return LYMPH_OK;
     const int64_t chunk = 1 << 20;

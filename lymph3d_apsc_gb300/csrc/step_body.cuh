@@ -13,7 +13,7 @@ namespace stepk {
 //
 // The GB300 retires 2 FP64 multiply-adds per clock and SM, which holds a product
 // with FP64 blocks at two thirds of the copy bandwidth, while its integer pipe idles.
-// At p = 3 and 4, 60 % of each row's columns (the last ones, c >= C0) are therefore
+// At p = 3 and 4, and at p = 2 where it pays (lymph_dev_int_columns), 60 % of each row's columns (the last ones, c >= C0) are therefore
 // multiplied there: a block entry and a coefficient are doubles as before, their
 // mantissas multiply to the product's top 64 bits (relative error below 2^-61; an
 // FP64 product rounds to 2^-53), and the product, shifted by the exponents, adds up
@@ -119,7 +119,7 @@ struct StepArgs {
     const int32_t* row_ptr;
     const int32_t* col;
     const void* K;             // [n_blocks][ND][ND] column-major (double or float)
-    const int32_t* Kex;        // FP64 at p = 3, 4: largest biased exponent of each block's entries
+    const int32_t* Kex;        // with integer columns: largest biased exponent of each block's entries
     const double* Minv;        // [n_poly][NP][NP] column-major inverse of M_loc
     const double* rhs_stat;
     const double* rhs_dyn;
@@ -185,13 +185,13 @@ __device__ __forceinline__ float ld_stream(const float* p) { return __ldcs(p); }
 // and the row partial sums in the accumulation type, then the FP64 right-hand
 // side at an offset rounded up to 16 bytes (with FP32 blocks and odd ND the
 // raw offset is not 8-byte aligned).
-template <int PD, typename KT, int S_ = Shape<PD>::S> struct SmemSize {
+template <int PD, typename KT, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT))> struct SmemSize {
     static constexpr int ND = Deg<PD>::ND, S = S_;
     static constexpr size_t b_offset = ((sizeof(KT) * (size_t)(NBB * ND + S * ND)) + 15) & ~(size_t)15;
     // the columns of the integer pipe: a thread's last NI of CPT, c >= C0 (12 of 35:
     // 14.1 and 44.0 ms for the runs above, 16 of 35: 13.5 and 41.0, 19 of 35: 13.4 and
     // 38.1, 24 of 35: 13.2 and 38.9)
-    static constexpr int CPT = (ND + S - 1) / S, NI = int_columns(PD, sizeof(KT)) ? CPT * 21 / 35 : 0;
+    static constexpr int CPT = (ND + S - 1) / S, NI = INT ? CPT * 21 / 35 : 0;
     static constexpr int C0 = (CPT - NI) * S < ND ? (CPT - NI) * S : ND, NC = ND - C0;
     static_assert(NI * NBB < 1 << (INT_HEAD - 1), "the accumulator's headroom");
     static constexpr size_t m_offset =
@@ -325,15 +325,16 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
 // the number of column slices (the tile shape; the CTA needs ND * S_ threads).
 // Every thread of the CTA must call this (it synchronises); threads beyond the
 // degree's shape only help with the gather.
-template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S>
+template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT))>
 __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) {
     constexpr int ND = Deg<PD>::ND, S = S_;
     constexpr int CPT = (ND + S - 1) / S;
     using AT = KT;  // FP64 blocks accumulate in FP64, FP32 blocks in FP32
     AT* s_u = (AT*)smem;
     AT* s_red = s_u + NBB * ND;
-    double* s_b = (double*)(smem + SmemSize<PD, KT, S>::b_offset);
-    static_assert(SmemSize<PD, KT, S>::b_offset % 16 == 0, "FP64 rhs must be 16-byte aligned");
+    using SZ = SmemSize<PD, KT, S, INT>;
+    double* s_b = (double*)(smem + SZ::b_offset);
+    static_assert(SZ::b_offset % 16 == 0, "FP64 rhs must be 16-byte aligned");
     const int nthr = blockDim.x;
     const int tid = threadIdx.x;
     const int r = tid % ND, s = tid / ND;
@@ -350,7 +351,6 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
         if (trigger_early(PD)) pdl_trigger();
     }
 
-    using SZ = SmemSize<PD, KT, S>;
     constexpr int NI = SZ::NI, C0 = SZ::C0, NC = SZ::NC, JF = CPT - NI;
     uint4* s_m = (uint4*)(smem + SZ::m_offset);   // the integer columns' coefficients
     int* s_R = (int*)(smem + SZ::r_offset);       // the accumulators' exponent

@@ -1,4 +1,4 @@
-"""FP64 blocks of p = 3 and 4 multiply most of each row's columns on the
+"""FP64 blocks of p = 3 and 4 (p = 2 on larger meshes) multiply most of each row's columns on the
 integer pipe (step_body.cuh): exact products of the doubles' mantissas to 64
 bits, summed in 128.
 
@@ -25,7 +25,8 @@ def _solver(p, kind="bfs"):
     if kind == "tet":
         m = M.cube(2, bc="reference", agglomeration="tet", jitter=0.2)
     else:
-        m = M.cube(3, bc="reference", agglomeration="bfs", seed=1, group=(4, 12), jitter=0.15)
+        # p = 2 takes this path from 608 polyhedra of long rows on
+        m = M.cube(10 if p == 2 else 3, bc="reference", agglomeration="bfs", seed=1, group=(4, 12), jitter=0.15)
         m.mat, m.tet_mat = M.lognormal_materials(m.n_poly, seed=1), m.tet_poly.copy()
     g = MatrixFree(m, p, 1e-4)
     g.MAKE_MATRICES_FREE()
@@ -45,8 +46,7 @@ def _states(g, rng):
             "denormal": u * 1e-310, "holes": holes, "graded up": u * 10.0 ** (3.0 * deg)}
 
 
-@pytest.mark.parametrize("kind", ["tet", "bfs"])
-@pytest.mark.parametrize("p", [3, 4])
+@pytest.mark.parametrize("p,kind", [(2, "bfs"), (3, "tet"), (3, "bfs"), (4, "tet"), (4, "bfs")])
 def test_operator_error_is_that_of_fp64(require_gpu, kind, p):
     g = _solver(p, kind)
     K, (rp, col) = g.blocks(), g.pattern()
@@ -80,7 +80,7 @@ def test_operator_error_is_that_of_fp64(require_gpu, kind, p):
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
 @pytest.mark.parametrize("column", [0, -1])
-@pytest.mark.parametrize("p", [3, 4])
+@pytest.mark.parametrize("p", [2, 3, 4])
 def test_non_finite_states_are_reported(require_gpu, p, column, bad):
     g = _solver(p)
     u = np.random.default_rng(0).standard_normal((g.n_poly, g.nd))
