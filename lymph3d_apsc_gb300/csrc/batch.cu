@@ -67,7 +67,7 @@ constexpr int kBatchShapes[BATCH_SHAPES][5] = {{0, 8, 8, 4, 3}, {0, 16, 10, 5, 3
 constexpr size_t zmax(size_t a, size_t b) { return a > b ? a : b; }
 template <typename KT, int V> struct ShapeSmem {
     static constexpr size_t bytes =
-        zmax(zmax(SmemSize<1, KT, kBatchShapes[V][1]>::bytes, SmemSize<2, KT, kBatchShapes[V][2]>::bytes),
+        zmax(zmax(SmemSize<1, KT, kBatchShapes[V][1]>::bytes, SmemSize<2, KT, kBatchShapes[V][2], sizeof(KT) == 8>::bytes),
              zmax(SmemSize<3, KT, kBatchShapes[V][3]>::bytes, SmemSize<4, KT, kBatchShapes[V][4]>::bytes));
 };
 template <typename KT> struct BatchSmem {
@@ -101,7 +101,15 @@ k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ it
         A.step_off = off;
         switch (probs[w.x].p) {
             case 1: step_poly<1, KT, MODE_STEP, kBatchShapes[V][1]>(A, w.y, smem); break;
-            case 2: step_poly<2, KT, MODE_STEP, kBatchShapes[V][2]>(A, w.y, smem); break;
+            case 2:
+                if constexpr (sizeof(KT) == 8) {
+                    if (A.Kex) {   // integer columns, as the problem alone
+                        step_poly<2, KT, MODE_STEP, kBatchShapes[V][2], true>(A, w.y, smem);
+                        break;
+                    }
+                }
+                step_poly<2, KT, MODE_STEP, kBatchShapes[V][2]>(A, w.y, smem);
+                break;
             case 3: step_poly<3, KT, MODE_STEP, kBatchShapes[V][3]>(A, w.y, smem); break;
             default: step_poly<4, KT, MODE_STEP, kBatchShapes[V][4]>(A, w.y, smem); break;
         }
