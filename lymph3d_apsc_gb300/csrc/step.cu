@@ -29,6 +29,14 @@ __global__ void __launch_bounds__(Shape<PD>::T, Shape<PD>::MINB) k_step(StepArgs
     step_poly<PD, KT, MODE, Shape<PD>::S, INT>(A, blockIdx.x, smem);
 }
 
+// The same for at most SMALL_POLY polyhedra without absorbing faces, p <= 3.
+template <int PD, typename KT, bool INT = int_columns(PD, sizeof(KT))>
+__global__ void __launch_bounds__(Shape<PD>::T, 2) k_step_small(StepArgs A) {
+    __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
+    extern __shared__ __align__(16) char dyn[];
+    step_poly<PD, KT, MODE_STEP, Shape<PD>::S, INT, true>(A, blockIdx.x, smem, dyn);
+}
+
 __global__ void k_bump(int64_t* idx, int n) { *idx += n; }
 
 // COMPUTE_ERROR_L2_MATRIX_FREE body per polyhedron: sum_i du_i^T M du_i.
@@ -277,6 +285,17 @@ int launch_step_i(lymph_ctx* c, const StepArgs& A) {
     // p = 1 in one wave of 8 to 16 CTAs per SM: an early launch unbalances the SMs and a
     // late one comes too late (48 steps of 1,728 polyhedra: 475 us in FP32, plain 390 us)
     const bool plain = PD == 1 && c->n_poly > 8 * 152 && c->n_poly <= 16 * 152;
+    if constexpr (MODE == MODE_STEP && PD <= 3) {
+        if (c->n_poly <= SMALL_POLY && !A.abs_idx) {
+            constexpr size_t bytes = SmallSmem<PD, KT>::bytes;
+            static const cudaError_t e = cudaFuncSetAttribute(k_step_small<PD, KT, INT>,
+                                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            LYMPH_CUDA_TRY(e);
+            LYMPH_CUDA_TRY(launch_pdl(k_step_small<PD, KT, INT>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A, bytes));
+            c->launches++;
+            return LYMPH_OK;
+        }
+    }
     if (MODE == MODE_STEP && !plain) {
         LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE, INT>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
     } else {

@@ -159,7 +159,7 @@ __device__ __forceinline__ bool trigger_early(int p) { return gridDim.x <= (p ==
 
 // Launches a step kernel that may start before the stream's previous kernel ends.
 template <typename K, typename A>
-inline cudaError_t launch_pdl(K kernel, unsigned grid, unsigned block, cudaStream_t st, const A& arg) {
+inline cudaError_t launch_pdl(K kernel, unsigned grid, unsigned block, cudaStream_t st, const A& arg, size_t smem = 0) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -167,6 +167,7 @@ inline cudaError_t launch_pdl(K kernel, unsigned grid, unsigned block, cudaStrea
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.stream = st;
+    cfg.dynamicSmemBytes = smem;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, arg);
@@ -319,14 +320,64 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
     }
 }
 
+// ---- meshes of at most one polyhedron per SM ----
+//
+// A step is then a chain of latencies, and the next step's CTA already sits beside
+// this one's while it runs: it copies the head of its block row, M^-1, the column
+// indices and the blocks' exponents into its shared memory before it waits for the
+// state, and reads right-hand side and own coefficients with the gather instead of
+// one after another at the end.  Two CTAs share an SM's 227 KB.
+// 48 steps of 125 hexahedra: p = 1 in FP64 267 -> 240 us, p = 2 346 -> 335 (FP64-pipe
+// bound), p = 3 627 -> 591, in FP32 263 -> 239, 285 -> 265, 371 -> 337; 100 FP64 steps
+// of 90 polyhedra (10 blocks a row): 605 -> 503, 852 -> 803, 1,856 -> 1,615 us.
+constexpr int SMALL_POLY = 152;
+constexpr int SMALL_STAGE = 88 * 1024;   // bytes of staged blocks per CTA
+template <int PD, typename KT> struct SmallSmem {
+    static constexpr int ND = Deg<PD>::ND, NP = Deg<PD>::NP;
+    static constexpr int FIT = SMALL_STAGE / (ND * ND * (int)sizeof(KT)), STAGE = FIT < NBB ? FIT : NBB;
+    static constexpr size_t minv_offset = (size_t)STAGE * ND * ND * sizeof(KT);   // 16-byte multiples for p <= 3
+    static constexpr size_t col_offset = minv_offset + sizeof(double) * NP * NP;
+    static constexpr size_t bytes = col_offset + 2 * sizeof(int) * NBB;
+};
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// What finish_poly reads of polyhedron P's own, row tid.
+struct Own { double rs, rd, g, un, u0; };
+
+// finish_poly for MODE_STEP without absorbing faces, its inputs already read.
+template <int PD>
+__device__ __forceinline__ void finish_small(const StepArgs& A, int P, double y, double* s_b, const Own& o, const double* s_Mi) {
+    constexpr int NP = Deg<PD>::NP, ND = Deg<PD>::ND;
+    const int tid = threadIdx.x;
+    if (tid < ND) s_b[tid] = -y + o.rs + o.rd * o.g;
+    __syncthreads();
+    if (tid < ND) {
+        const int i = tid / NP, m = tid % NP;
+        const double* Mi = s_Mi + m;
+        const double* bi = s_b + i * NP;
+        double x0 = 0.0, x1 = 0.0;
+#pragma unroll
+        for (int c = 0; c < NP; c += 2) {
+            x0 += Mi[c * NP] * bi[c];
+            if (c + 1 < NP) x1 += Mi[(c + 1) * NP] * bi[c + 1];
+        }
+        const double x = x0 + x1, dt2 = A.dt * A.dt;
+        const double v = dt2 * x + 2.0 * o.un - o.u0;
+        if (!isfinite(v)) atomicOr(A.status, ST_NONFINITE);
+        A.out[(int64_t)P * ND + tid] = v;
+    }
+}
+
 // The block row of polyhedron P is one contiguous column-major
 // [ND x nb*ND] matrix (its blocks are adjacent in memory), multiplied by the
 // gathered coefficients of the column polyhedra, then finish_poly.  S_ is
 // the number of column slices (the tile shape; the CTA needs ND * S_ threads).
 // Every thread of the CTA must call this (it synchronises); threads beyond the
 // degree's shape only help with the gather.
-template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT))>
-__device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) {
+// SMALL: dyn is the shared memory of SmallSmem.
+template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT)), bool SMALL = false>
+__device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, char* dyn = nullptr) {
     constexpr int ND = Deg<PD>::ND, S = S_;
     constexpr int CPT = (ND + S - 1) / S;
     using AT = KT;  // FP64 blocks accumulate in FP64, FP32 blocks in FP32
@@ -341,7 +392,31 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
     const bool act = tid < ND * S;
     const int rb = A.row_ptr[P], re = A.row_ptr[P + 1];
     const KT* Kbase = (const KT*)A.K;
-    if (MODE == MODE_STEP) {
+    using SS = SmallSmem<PD, KT>;
+    int* s_col = (int*)(dyn + SS::col_offset);
+    Own own = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const int nst = SMALL ? (re - rb < SS::STAGE ? re - rb : SS::STAGE) : 0;
+    if constexpr (SMALL) {
+        const int n16 = nst * (int)(ND * ND * sizeof(KT) / 16), m16 = Deg<PD>::NP * Deg<PD>::NP / 2;
+        const char* src = (const char*)(Kbase + (int64_t)rb * ND * ND);
+        for (int i = tid; i < n16; i += nthr) cp16(dyn + 16 * i, src + 16 * i);
+        const char* mi = (const char*)(A.Minv + (int64_t)P * Deg<PD>::NP * Deg<PD>::NP);
+        for (int i = tid; i < m16; i += nthr) cp16(dyn + SS::minv_offset + 16 * i, mi + 16 * i);
+        if (tid < NBB && tid < re - rb) {
+            s_col[tid] = A.col[rb + tid];
+            if (INT) s_col[NBB + tid] = A.Kex[rb + tid];
+        }
+        pdl_wait();
+        pdl_trigger();
+        if (tid < ND) {
+            const int64_t q = (int64_t)P * ND + tid;
+            own.g = A.gvals ? A.gvals[*A.step_idx + A.step_off] : A.g;
+            own.rs = A.rhs_stat[q];
+            own.rd = A.rhs_dyn[q];
+            own.un = A.un[q];
+            own.u0 = A.u0[q];
+        }
+    } else if (MODE == MODE_STEP) {
         if (A.prefetch && tid == 0) {   // the head of the row's blocks and M^-1, while the previous step ends
             const int64_t row = (int64_t)(re - rb) * ND * ND * (int64_t)sizeof(KT);
             prefetch_inside(Kbase + (int64_t)rb * ND * ND, row < STEP_PREFETCH ? row : STEP_PREFETCH);
@@ -360,9 +435,10 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
         const int nb = (re - b0) < NBB ? (re - b0) : NBB;
         if (NI && tid == 0) *s_R = EXP_NONE;
         __syncthreads();
+        const bool staged = SMALL && b0 == rb;
         for (int i = tid; i < nb * ND; i += nthr) {
             const int bb = i / ND, c = i % ND;
-            const int64_t q = (int64_t)A.col[b0 + bb] * ND + c;
+            const int64_t q = (int64_t)(staged ? s_col[bb] : A.col[b0 + bb]) * ND + c;
             s_u[i] = (AT)((MODE == MODE_FIRST || MODE == MODE_BILIN) ? A.u0[q] : A.un[q]);
         }
         Acc128 iacc = {0, 0};
@@ -373,7 +449,7 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
             // exponent a product of the row can have
             int mx = EXP_NONE;
             for (int i = tid; i < nb * NC; i += nthr) {
-                const int bb = i / NC, kx = A.Kex[b0 + bb];
+                const int bb = i / NC, kx = staged ? s_col[NBB + bb] : A.Kex[b0 + bb];
                 const double u = s_u[bb * ND + C0 + i - bb * NC];
                 int e;
                 const unsigned long long m = split_mantissa(u, &e);
@@ -390,16 +466,16 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
                 s_m[i].z = e > EXP_NONE && R < EXP_NONFINITE / 2 ? (unsigned)(INT_HEAD + R - e) : 1u << 16;
             }
         }
+        if (SMALL && b0 == rb) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         if (act) {
-            for (int bb = 0; bb < nb; ++bb) {
-                const KT* Kb = Kbase + (int64_t)(b0 + bb) * ND * ND + r;
+            const auto block = [&](int bb, auto load) {
                 const AT* ub = s_u + bb * ND;
                 KT kv[CPT];
 #pragma unroll
                 for (int j = 0; j < CPT; ++j) {
                     const int c = s + j * S;
-                    kv[j] = (c < ND) ? ld_stream(Kb + (int64_t)c * ND) : (KT)0;
+                    kv[j] = (c < ND) ? load(c * ND + r) : (KT)0;
                 }
 #pragma unroll
                 for (int j = 0; j < CPT; ++j) {
@@ -415,17 +491,32 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem) 
                         else acc0 += (AT)kv[j] * ub[c];
                     }
                 }
+            };
+            int bb = 0;
+            if constexpr (SMALL) {
+                if (b0 == rb) {
+#pragma unroll 2
+                    for (; bb < nst; ++bb) {
+                        const KT* Kb = (const KT*)dyn + bb * ND * ND;
+                        block(bb, [&](int e) { return Kb[e]; });
+                    }
+                }
+            }
+            for (; bb < nb; ++bb) {
+                const KT* Kb = Kbase + (int64_t)(b0 + bb) * ND * ND;
+                block(bb, [&](int e) { return ld_stream(Kb + e); });
             }
             if constexpr (NI > 0) acc1 += acc_value(iacc, R);
         }
     }
-    if (MODE == MODE_STEP) pdl_trigger();
+    if (MODE == MODE_STEP && !SMALL) pdl_trigger();
     if (act) s_red[s * ND + r] = acc0 + acc1;
     __syncthreads();
     double y = 0.0;
     if (tid < ND)
         for (int ss = 0; ss < S; ++ss) y += (double)s_red[ss * ND + tid];
-    finish_poly<PD, MODE>(A, P, y, s_b);
+    if constexpr (SMALL) finish_small<PD>(A, P, y, s_b, own, (const double*)(dyn + SS::minv_offset));
+    else finish_poly<PD, MODE>(A, P, y, s_b);
 }
 
 }  // namespace stepk
