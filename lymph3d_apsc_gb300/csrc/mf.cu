@@ -158,52 +158,95 @@ template <int PD> struct Bidx {
 //   r0_a = sum_b w0_ab Y_b,  r1_a = sum_b w0_ab Y'_b,  r2_a = sum_b w1_ab Y_b,
 //   v = sum_a r0_a X_a, d_x = sum_a r0_a X'_a, d_y = sum_a r1_a X_a, d_z = sum_a r2_a X_a
 // (unscaled: the caller applies the bounding-box factors).  uc[i] holds
-// (u_0, u_1, u_2, 0) of basis function i.  Each w sum runs over c = p-a-b
+// (u_0, u_1, u_2, u_2) of basis function i.  Each w sum runs over c = p-a-b
 // down to 0 (the basis order), each r sum over b = 0.., each output over
 // a = 0..; one (a, b) group is live at a time, so the three components cost
 // no more registers than one did with every w_ab held.  L_0 = 1, L'_0 = 0 and
 // L'_1 = 1 are left out of the products (63 of 405 multiply-adds at p = 4).
+//
+// The sums of components 0 and 1 are the halves of packed FP32 pairs, and of
+// component 2 w0 and w1, then r0 and r2, then v and d_z: one instruction for two
+// multiply-adds, each rounded as before (the kernel issues in every second slot at
+// most, FP64 taking half of what is left: 65 steps of 46,767 polyhedra at p = 4 58.1
+// -> 56.7 ms, of 10,648 9.43 -> 9.03 ms for 49).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 template <int PD>
 __device__ __forceinline__ void eval_sf3(const float4* uc, const float2* X, const float2* Y, const float2* Z,
                                          float (&o)[3][4]) {
     constexpr Bidx<PD> BI{};
-#pragma unroll
-    for (int j = 0; j < 3; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+    f32x2 op[4] = {0, 0, 0, 0}, oc = 0;     // components 0, 1; component 2: (v, d_z),
+    float oc1 = 0.0f, oc2 = 0.0f;           // d_x, d_y
 #pragma unroll
     for (int a = 0; a <= PD; ++a) {
-        float r[3][3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) r[j][0] = r[j][1] = r[j][2] = 0.0f;
+        f32x2 rp0 = 0, rp1 = 0, rp2 = 0, rc = 0;   // rc: (r0, r2) of component 2
+        float rc1 = 0.0f;
 #pragma unroll
         for (int b = 0; b <= PD - a; ++b) {
-            float w0[3] = {0.0f, 0.0f, 0.0f}, w1[3] = {0.0f, 0.0f, 0.0f};
+            f32x2 w0 = 0, w1 = 0, wc = 0;           // wc: (w0, w1) of component 2
 #pragma unroll
             for (int c = PD - a - b; c >= 0; --c) {
-                const float4 uu = uc[BI.i[a][b][c]];
-                const float u3[3] = {uu.x, uu.y, uu.z};
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    w0[j] = c == 0 ? w0[j] + u3[j] : fmaf(u3[j], Z[c].x, w0[j]);
-                    if (c >= 1) w1[j] = c == 1 ? w1[j] + u3[j] : fmaf(u3[j], Z[c].y, w1[j]);
+                const ulonglong2 uu = *reinterpret_cast<const ulonglong2*>(uc + BI.i[a][b][c]);   // (u0, u1), (u2, u2)
+                if (c == 0) {
+                    w0 = add2(w0, uu.x);
+                    wc = pack2(lo2(wc) + lo2(uu.y), hi2(wc));
+                } else {
+                    w0 = fma2(uu.x, pack2(Z[c].x, Z[c].x), w0);
+                    w1 = c == 1 ? add2(w1, uu.x) : fma2(uu.x, pack2(Z[c].y, Z[c].y), w1);
+                    wc = fma2(uu.y, pack2(Z[c].x, c == 1 ? 1.0f : Z[c].y), wc);
                 }
             }
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                r[j][0] = b == 0 ? r[j][0] + w0[j] : fmaf(w0[j], Y[b].x, r[j][0]);
-                if (b >= 1) r[j][1] = b == 1 ? r[j][1] + w0[j] : fmaf(w0[j], Y[b].y, r[j][1]);
-                if (a + b < PD) r[j][2] = b == 0 ? r[j][2] + w1[j] : fmaf(w1[j], Y[b].x, r[j][2]);
+            const f32x2 yx = pack2(Y[b].x, Y[b].x);
+            rp0 = b == 0 ? add2(rp0, w0) : fma2(w0, yx, rp0);
+            if (b >= 1) rp1 = b == 1 ? add2(rp1, w0) : fma2(w0, pack2(Y[b].y, Y[b].y), rp1);
+            if (b >= 1) rc1 = b == 1 ? rc1 + lo2(wc) : fmaf(lo2(wc), Y[b].y, rc1);
+            if (a + b < PD) {
+                rp2 = b == 0 ? add2(rp2, w1) : fma2(w1, yx, rp2);
+                rc = b == 0 ? add2(rc, wc) : fma2(wc, yx, rc);
+            } else {
+                rc = pack2(b == 0 ? lo2(rc) + lo2(wc) : fmaf(lo2(wc), Y[b].x, lo2(rc)), hi2(rc));
             }
         }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            o[j][0] = a == 0 ? o[j][0] + r[j][0] : fmaf(r[j][0], X[a].x, o[j][0]);
-            if (a >= 1) o[j][1] = a == 1 ? o[j][1] + r[j][0] : fmaf(r[j][0], X[a].y, o[j][1]);
-            if (a < PD) {
-                o[j][2] = a == 0 ? o[j][2] + r[j][1] : fmaf(r[j][1], X[a].x, o[j][2]);
-                o[j][3] = a == 0 ? o[j][3] + r[j][2] : fmaf(r[j][2], X[a].x, o[j][3]);
-            }
+        const f32x2 xx = pack2(X[a].x, X[a].x);
+        op[0] = a == 0 ? add2(op[0], rp0) : fma2(rp0, xx, op[0]);
+        if (a >= 1) {
+            op[1] = a == 1 ? add2(op[1], rp0) : fma2(rp0, pack2(X[a].y, X[a].y), op[1]);
+            oc1 = a == 1 ? oc1 + lo2(rc) : fmaf(lo2(rc), X[a].y, oc1);
+        }
+        if (a < PD) {
+            op[2] = a == 0 ? add2(op[2], rp1) : fma2(rp1, xx, op[2]);
+            op[3] = a == 0 ? add2(op[3], rp2) : fma2(rp2, xx, op[3]);
+            oc2 = a == 0 ? oc2 + rc1 : fmaf(rc1, X[a].x, oc2);
+            oc = a == 0 ? add2(oc, rc) : fma2(rc, xx, oc);
+        } else {
+            oc = pack2(fmaf(lo2(rc), X[a].x, lo2(oc)), hi2(oc));
         }
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        o[0][k] = lo2(op[k]);
+        o[1][k] = hi2(op[k]);
+    }
+    o[2][0] = lo2(oc);
+    o[2][1] = oc1;
+    o[2][2] = oc2;
+    o[2][3] = hi2(oc);
 }
 
 // The transpose: acc_abc += X'_a Y_b Z_c gx + X_a Y'_b Z_c gy + X_a Y_b Z'_c gz
@@ -288,7 +331,7 @@ template <int PD> struct MfSmem {
         Fin fin;
     };
     Work w;
-    float4 uQ[2][S::CT][S::NP];        // (u_0, u_1, u_2, 0) per basis function
+    float4 uQ[2][S::CT][S::NP];        // (u_0, u_1, u_2, u_2) per basis function
     alignas(16) MfTri tri[2][S::CT];
     alignas(16) MfPoly polyQ[2][S::CT];
     float quad[3 * S::NQ2];
@@ -310,7 +353,7 @@ static_assert(mf_smem_aligned<1>() && mf_smem_aligned<2>() && mf_smem_aligned<3>
 // The pass of polyhedron P (every thread of the CTA calls it; it
 // synchronises): the per-problem tables come from A, the state, right-hand
 // sides and M^-1 from sa, the operator input in FP32, [n_poly][Np]
-// (u_0, u_1, u_2, 0), from u32.
+// (u_0, u_1, u_2, u_2), from u32.
 template <int PD, int MODE>
 __device__ __forceinline__ void mf_poly(const MfArgs& A, const StepArgs& sa, const float4* u32, int P, char* smem) {
     using S = MfShape<PD>;
@@ -583,17 +626,17 @@ __global__ void k_mf_u32_batch(const MfBatchProblem* __restrict__ probs, const i
     const int NP = (pb.p + 1) * (pb.p + 2) * (pb.p + 3) / 6;
     const double* u = pb.buf[pb.cur0 ^ (int)(k & 1)] + (int64_t)w.y * 3 * NP;
     float4* o = const_cast<float4*>(pb.a.u32) + (int64_t)w.y * NP;
-    for (int m = lane; m < NP; m += 32) o[m] = make_float4((float)u[m], (float)u[NP + m], (float)u[2 * NP + m], 0.0f);
+    for (int m = lane; m < NP; m += 32) o[m] = make_float4((float)u[m], (float)u[NP + m], (float)u[2 * NP + m], (float)u[2 * NP + m]);
 }
 
-// u32[P][m] = (u[P][0][m], u[P][1][m], u[P][2][m], 0): the operator input in
+// u32[P][m] = (u[P][0][m], u[P][1][m], u[P][2][m] twice): the operator input in
 // FP32, converted once instead of once per triangle that reads it (before a
 // single pass and the first of a run; each step leaves the next one's copy).
 __global__ void k_mf_u32(int64_t n, int NP, const double* __restrict__ u, float4* __restrict__ u32) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t P = i / NP, m = i - P * NP;
         const double* up = u + P * 3 * NP + m;
-        u32[i] = make_float4((float)up[0], (float)up[NP], (float)up[2 * NP], 0.0f);
+        u32[i] = make_float4((float)up[0], (float)up[NP], (float)up[2 * NP], (float)up[2 * NP]);
     }
 }
 
@@ -760,7 +803,6 @@ int lymph_mf_setup(lymph_ctx* c, const RefTables& R) {
             LYMPH_CUDA_TRY(cudaMalloc(&p, bytes));
             c->d_mf_u32[b] = p;
             c->device_bytes += (int64_t)bytes;
-            // a step writes three of a record's four floats
             LYMPH_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, c->stream));
         }
         LYMPH_CUDA_TRY(cudaMalloc(&p, sizeof(int32_t) * MF_REC * (size_t)c->n_poly));

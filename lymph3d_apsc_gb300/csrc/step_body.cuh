@@ -201,6 +201,12 @@ template <int PD, typename KT, int S_ = Shape<PD>::S, bool INT = int_columns(PD,
     static constexpr size_t bytes = r_offset + (NI ? sizeof(int) : 0);
 };
 
+// Component i of the FP32 record (u_0, u_1, u_2, u_2) of basis function q.
+__device__ __forceinline__ void store_u32(float* u32, int64_t q, int i, double v) {
+    u32[q * 4 + i] = (float)v;
+    if (i == 2) u32[q * 4 + 3] = (float)v;
+}
+
 // y_r = sum_c A(r, c) w_c for rows r < ND of a column-major ND x ND matrix in
 // device memory, w in shared memory, by every thread of the CTA: the columns in
 // blockDim / ND slices (several loads of a row in flight at once; one thread
@@ -286,7 +292,7 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
                 const double v = x + 2.0 * A.un[q] - A.u0[q];
                 if (!isfinite(v)) atomicOr(A.status, ST_NONFINITE);
                 A.out[q] = v;
-                if (U32 && A.u32_out) A.u32_out[((int64_t)P * NP + tid % NP) * 4 + tid / NP] = (float)v;
+                if (U32 && A.u32_out) store_u32(A.u32_out, (int64_t)P * NP + tid % NP, tid / NP, v);
             }
             return;
         }
@@ -316,7 +322,7 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
         }
         if (!isfinite(v)) atomicOr(A.status, ST_NONFINITE);
         A.out[q] = v;
-        if (U32 && MODE == MODE_STEP && A.u32_out) A.u32_out[((int64_t)P * NP + m) * 4 + i] = (float)v;
+        if (U32 && MODE == MODE_STEP && A.u32_out) store_u32(A.u32_out, (int64_t)P * NP + m, i, v);
     }
 }
 
