@@ -235,6 +235,7 @@ int refresh_problems(lymph_batch* b) {
         P.a.Dabs = c->d_Dabs;
         P.a.Winv = c->d_Winv;
         P.a.dt = c->dt;
+        P.a.dt2 = c->dt * c->dt;
         P.a.status = b->d_status;
         P.a.n_poly = c->n_poly;
         P.a.prefetch = 1;

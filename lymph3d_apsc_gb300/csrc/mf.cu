@@ -880,6 +880,7 @@ void lymph_mf_batch_problem(const lymph_ctx* c, int* status, void* out) {
     s.Dabs = c->d_Dabs;
     s.Winv = c->d_Winv;
     s.dt = c->dt;
+    s.dt2 = c->dt * c->dt;
     s.status = status;
     s.n_poly = c->n_poly;
     s.prefetch = 0;

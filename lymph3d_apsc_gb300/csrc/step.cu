@@ -352,7 +352,7 @@ StepArgs base_args(lymph_ctx* c) {
     A.Minv = c->d_Minv;
     A.rhs_stat = c->d_rhs_stat; A.rhs_dyn = c->d_rhs_dyn; A.gvals = nullptr; A.step_idx = nullptr;
     A.step_off = 0; A.g = 0.0; A.u32_out = nullptr;
-    A.u0 = nullptr; A.un = nullptr; A.out = nullptr; A.partial = c->d_partial; A.dt = c->dt; A.status = c->d_status;
+    A.u0 = nullptr; A.un = nullptr; A.out = nullptr; A.partial = c->d_partial; A.dt = c->dt; A.dt2 = c->dt * c->dt; A.status = c->d_status;
     A.n_poly = c->n_poly;
     A.prefetch = c->n_blocks * c->nd * c->nd * (c->precision == LYMPH_FP64 ? 8 : 4) <= STEP_PREFETCH_MAX;
     A.abs_idx = c->n_abs > 0 ? c->d_abs_idx : nullptr;
