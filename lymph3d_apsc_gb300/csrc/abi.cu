@@ -109,6 +109,15 @@ bool build_ref_tables(int p, RefTables& R) {
             R.weitria2[c] = std::fabs(0.125 * (1 - s)) * (w[i] * w[j]);
             ++c;
         }
+    int32_t nf = 0;
+    double xyw[3 * MAX_FACE_NQ];
+    if (lymph_mf_face_rule(p, &nf, xyw) != LYMPH_OK || nf != face_rule_points(p)) return false;
+    for (int q = 0; q < nf; ++q) {
+        R.facenod[q * 4 + 0] = xyw[3 * q];
+        R.facenod[q * 4 + 1] = xyw[3 * q + 1];
+        R.facenod[q * 4 + 2] = R.facenod[q * 4 + 3] = 1.0;
+        R.facewei[q] = xyw[3 * q + 2];
+    }
     // node_maps[f][row][col]
     auto nm = [&](int f, int r, int cc) -> double& { return R.node_maps[f * 16 + r * 4 + cc]; };
     nm(0, 0, 1) = 1; nm(0, 1, 0) = 1; nm(0, 3, 3) = 1;

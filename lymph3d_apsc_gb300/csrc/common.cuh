@@ -44,6 +44,8 @@ constexpr int MAX_DEGREE = 4;     // device path supports p = 1..4 (Np <= 35)
 constexpr int MAX_NP = 35;
 constexpr int MAX_NQ3 = 125;
 constexpr int MAX_NQ2 = 25;
+constexpr int MAX_FACE_NQ = 16;
+constexpr int face_rule_points(int p) { return p == 1 ? 3 : (p == 2 ? 6 : (p == 3 ? 12 : 16)); }
 
 // ---------------------------------------------------------------------------
 // reference tables in device memory (one copy per context, degree-specific)
@@ -53,6 +55,8 @@ struct RefTables {
     double weitet3[MAX_NQ3];
     double nodtria2[MAX_NQ2 * 4];  // [q][4]  (s, t, 1, 1)
     double weitria2[MAX_NQ2];
+    double facenod[MAX_FACE_NQ * 4];  // the operator's triangle rule (mf.cu): (xi, eta, 1, 1)
+    double facewei[MAX_FACE_NQ];
     double node_maps[4 * 16];      // [face][row][col]
     int blist[MAX_NP * 3];         // [f][3]
 };

@@ -78,7 +78,10 @@ static_assert(sizeof(MfPoly) == 16, "MfPoly is one 16-byte copy");
 // (derive_face_rules.py beside this file solves them to 40 digits;
 // tests/test_abi_cpu.py checks every moment of the values below).
 constexpr int MF_FACE_NQ[5] = {0, 3, 6, 12, 16};
-constexpr int MF_FACE_NQ_MAX = 16;
+constexpr int MF_FACE_NQ_MAX = MAX_FACE_NQ;
+static_assert(MF_FACE_NQ[1] == face_rule_points(1) && MF_FACE_NQ[2] == face_rule_points(2) &&
+                  MF_FACE_NQ[3] == face_rule_points(3) && MF_FACE_NQ[4] == face_rule_points(4),
+              "the assembly kernels' face points");
 // (xi, eta, w) per node, degrees 1..4 one after another
 constexpr double kFaceRule[3 * (3 + 6 + 12 + 16)] = {
     // p = 1, exact to degree 2

@@ -139,7 +139,10 @@ __device__ inline void face_point(const double* fk, const RefTables* ref, int f,
 // pair (a, b) at b (b + 1) / 2 + a); a neighbour block owns all Np^2 pairs.
 // The thread counts fill whole rounds of pairs with FP64 lanes (the pipe
 // retires 2 lanes per clock and SM whether they are used or not): p = 4,
-// 630 of 640 and 1225 of 1280 lanes; p = 3, 210 of 224 and 400 of 416.
+// 630 of 640 and 1225 of 1280 lanes; p = 3, 210 of 224 and 400 of 416.  The face
+// integrands are polynomials of degree 2 p, so the triangle rule of the matrix-free
+// terms (mf.cu) gives the reference's integrals from 3 / 6 / 12 / 16 points instead
+// of 4 / 9 / 16 / 25 (970 polyhedra, p = 4: 3.44 -> 3.03 ms, self blocks 5.24 -> 4.90).
 template <int PD> struct AsmShape {
     using D = Deg<PD>;
     static constexpr int NP = D::NP, L1 = PD + 1;
@@ -147,7 +150,8 @@ template <int PD> struct AsmShape {
     static constexpr int T = PD == 4 ? 320 : (PD == 3 ? 224 : (PD == 2 ? 64 : 32));       // self blocks
     static constexpr int PPT = (NS + T - 1) / T;
     static constexpr int R = PD == 4 ? 50 : (PD == 3 ? 64 : (PD == 2 ? 27 : 8));          // tabulated points at once
-    static constexpr int FB = R / D::NQ2;                                                 // faces at once
+    static constexpr int FQ = face_rule_points(PD);                                       // points of a face
+    static constexpr int FB = R / FQ;                                                     // faces at once
     static constexpr int TN = PD == 4 ? 320 : (PD == 3 ? 416 : (PD == 2 ? 64 : 32));      // neighbour blocks
     static constexpr int PPTN = (D::NPAIR + TN - 1) / TN;
     static_assert(FB >= 1, "one face per table at least");
@@ -329,7 +333,7 @@ template <int PD, int WHICH>
 __global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
     using D = Deg<PD>;
     using S = AsmShape<PD>;
-    constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = D::NQ2, NS = S::NS, T = S::T, PPT = S::PPT, R = S::R,
+    constexpr int NP = D::NP, ND = D::ND, NQ3 = D::NQ3, NQ2 = S::FQ, NS = S::NS, T = S::T, PPT = S::PPT, R = S::R,
                   L1 = S::L1, FB = S::FB;
     constexpr int NMAT = WHICH == ASM_MASS ? 0 : 14;   // lambda M, mu M, c lambda n_j P (3), c mu n_j P (3), sigma T P (6)
     extern __shared__ double sm[];
@@ -446,11 +450,11 @@ __global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
             for (int it = tid; it < nf * NQ2 * 3; it += T) {
                 const int qq = it / 3, d = it - qq * 3, fi = qq / NQ2, q = qq - fi * NQ2;
                 const double* cm = fmap + fi * 12 + d * 4;
-                const double* nt = &A.ref->nodtria2[q * 4];
+                const double* nt = &A.ref->facenod[q * 4];
                 double x = 0.0;
                 for (int l = 0; l < 4; ++l) x = x + cm[l] * nt[l];
                 legendre_rec<PD>(box.mb[d], box.ih[d], box.is[d], x, tleg + it * L1);
-                if (d == 0) tw[qq] = A.ref->weitria2[q] * A.area[A.bf[eb + fi]];
+                if (d == 0) tw[qq] = A.ref->facewei[q] * A.area[A.bf[eb + fi]];
             }
             __syncthreads();
             products(nf * NQ2);
@@ -583,8 +587,8 @@ __global__ void __launch_bounds__(AsmShape<PD>::T) k_assemble_self(AsmArgs A) {
 
 // One neighbour block K_PQ = -theta/2 I - S - IT/2 per CTA (or the DG norm's
 // -S), from the moments P(a, b) = sum_q W phi^P_a phi^Q_b of the triangles P
-// shares with Q, as in k_assemble_self: 25 multiply-adds per triangle and
-// pair for the moment (p = 4), 12 for its weighted sums, and the derivative
+// shares with Q, as in k_assemble_self: 16 multiply-adds per triangle and
+// pair for the moment (p = 4; 25 with the reference's rule), 12 for its weighted sums, and the derivative
 // expansion once per block,
 //     I(i,j)  = D_i PL_j + D_j PM_i + delta_ij sum_k D_k PM_k,
 //     IT(i,j) = PL_j D_i^T + PM_i D_j^T + delta_ij sum_k PM_k D_k^T
@@ -595,7 +599,7 @@ template <int PD, int WHICH>
 __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_nb(AsmArgs A) {
     using D = Deg<PD>;
     using S = AsmShape<PD>;
-    constexpr int NP = D::NP, ND = D::ND, NQ2 = D::NQ2, NPAIR = D::NPAIR, T = S::TN, PPT = S::PPTN, L1 = S::L1;
+    constexpr int NP = D::NP, ND = D::ND, NQ2 = S::FQ, NPAIR = D::NPAIR, T = S::TN, PPT = S::PPTN, L1 = S::L1;
     extern __shared__ double sm[];
     double* PL = sm;                                     // [3][NPAIR], pair (a, b) at b NP + a
     double* PM = PL + (WHICH == ASM_K ? 3 * NPAIR : 0);  // [3][NPAIR]
@@ -626,7 +630,7 @@ __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_
         for (int it = tid; it < 2 * NQ2 * 3; it += T) {
             const int s = it / (NQ2 * 3), r = it - s * NQ2 * 3, q = r / 3, d = r - q * 3;
             const double* cm = fmap + d * 4;
-            const double* nt = &A.ref->nodtria2[q * 4];
+            const double* nt = &A.ref->facenod[q * 4];
             double x = 0.0;
             for (int l = 0; l < 4; ++l) x = x + cm[l] * nt[l];
             legendre_rec<PD>(box[s].mb[d], box[s].ih[d], box[s].is[d], x, tleg + it * L1);
@@ -637,7 +641,7 @@ __global__ void __launch_bounds__(AsmShape<PD>::TN, PD == 4 ? 2 : 1) k_assemble_
             const int s = it / (NQ2 * NP), r = it - s * NQ2 * NP, q = r / NP, f = r - q * NP;
             const double* tq = tleg + (s * NQ2 + q) * 3 * L1;
             double ph = tq[der.deg[f][0]] * tq[L1 + der.deg[f][1]] * tq[2 * L1 + der.deg[f][2]];
-            if (s == 1) ph *= A.ref->weitria2[q] * ar;
+            if (s == 1) ph *= A.ref->facewei[q] * ar;
             fphi[it] = ph;
         }
         __syncthreads();
@@ -733,7 +737,7 @@ template <int PD, int WHICH> size_t asm_self_smem() {
 }
 template <int PD, int WHICH> size_t asm_nb_smem() {
     using S = AsmShape<PD>;
-    constexpr int NQ2 = Deg<PD>::NQ2;
+    constexpr int NQ2 = S::FQ;
     return sizeof(double) * ((WHICH == ASM_K ? 6 * (size_t)Deg<PD>::NPAIR : 0) + 2 * (size_t)NQ2 * S::NP +
                              2 * (size_t)NQ2 * 3 * S::L1 + FACE_F + 12);
 }
