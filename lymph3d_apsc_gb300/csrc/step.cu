@@ -288,9 +288,8 @@ int launch_step_i(lymph_ctx* c, const StepArgs& A) {
     if constexpr (MODE == MODE_STEP && PD <= 3) {
         if (c->n_poly <= SMALL_POLY && !A.abs_idx) {
             constexpr size_t bytes = SmallSmem<PD, KT>::bytes;
-            static const cudaError_t e = cudaFuncSetAttribute(k_step_small<PD, KT, INT>,
-                                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            LYMPH_CUDA_TRY(e);
+            LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_step_small<PD, KT, INT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)bytes));
             LYMPH_CUDA_TRY(launch_pdl(k_step_small<PD, KT, INT>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A, bytes));
             c->launches++;
             return LYMPH_OK;

@@ -3,8 +3,8 @@
 // MMAs of the activations' hi and lo parts against BF16-exact weights, FP32
 // accumulation in tensor memory, bias / ReLU / residual epilogue).
 //
-// One CTA computes a 128-row x min(N, 256)-column tile with 2 + WS_SPLIT_WARPS
-// warps:
+// One CTA computes a 128-row x min(N, bn)-column tile (bn: 32 to 256, by the number
+// of row tiles) with 2 + WS_SPLIT_WARPS warps:
 //   warp 0      producer: one thread issues the TMA loads
 //               (cp.async.bulk.tensor.2d, 128-byte swizzle) of the A and B
 //               tiles of each 32-wide k-step into a 3-stage ring, arming the
