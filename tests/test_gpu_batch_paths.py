@@ -1,7 +1,7 @@
 """A batch equals its problems stepped alone, bit for bit, where a lone problem
 takes a step kernel of its own: FP64 at p = 2 with integer columns (608 polyhedra
-of long rows), and at most one polyhedron per SM (rows of 4 to over 16 blocks,
-125 polyhedra, and 216 beyond the rule)."""
+of long rows), and at most one polyhedron per SM (rows of 4 to 18 blocks,
+52 to 125 polyhedra, and 216 beyond the rule)."""
 import numpy as np
 import pytest
 
@@ -12,6 +12,7 @@ from test_gpu_batch import _gvals, _prepared
 pytestmark = pytest.mark.gpu
 
 BFS = dict(agglomeration="bfs", jitter=0.15, seed=2)
+WIDE = dict(n=8, bc="reference", agglomeration="bfs", group=(8, 100), jitter=0.15, seed=1)   # a row of 18 blocks
 
 
 @pytest.mark.parametrize("precision,specs", [
@@ -20,6 +21,8 @@ BFS = dict(agglomeration="bfs", jitter=0.15, seed=2)
     (_lib.MIXED, [(dict(n=5, agglomeration="hex"), p, 1e-4) for p in (1, 2, 3)]),
     (_lib.FP64, [(dict(n=5, group=(4, 12), **BFS), p, 1e-4) for p in (1, 2, 3)]),
     (_lib.MIXED, [(dict(n=5, group=(4, 12), **BFS), p, 1e-4) for p in (1, 2, 3)]),
+    (_lib.FP64, [(WIDE, p, 1e-4) for p in (1, 2, 3, 4)]),
+    (_lib.MIXED, [(WIDE, p, 1e-4) for p in (1, 2, 3)]),
     (_lib.MIXED, [(dict(n=6, agglomeration="hex"), p, 1e-4) for p in (1, 3)]),
 ])
 def test_batch_equals_problems_alone(require_gpu, precision, specs):

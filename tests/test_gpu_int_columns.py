@@ -24,6 +24,8 @@ pytestmark = pytest.mark.gpu
 def _solver(p, kind="bfs"):
     if kind == "tet":
         m = M.cube(2, bc="reference", agglomeration="tet", jitter=0.2)
+    elif kind == "wide":   # a row of 17 blocks: a second batch of the gather
+        m = M.cube(7, bc="reference", agglomeration="bfs", seed=1, group=(8, 100), jitter=0.15)
     else:
         # p = 2 takes this path from 608 polyhedra of long rows on
         m = M.cube(10 if p == 2 else 3, bc="reference", agglomeration="bfs", seed=1, group=(4, 12), jitter=0.15)
@@ -46,7 +48,7 @@ def _states(g, rng):
             "denormal": u * 1e-310, "holes": holes, "graded up": u * 10.0 ** (3.0 * deg)}
 
 
-@pytest.mark.parametrize("p,kind", [(2, "bfs"), (3, "tet"), (3, "bfs"), (4, "tet"), (4, "bfs")])
+@pytest.mark.parametrize("p,kind", [(2, "bfs"), (3, "tet"), (3, "bfs"), (3, "wide"), (4, "tet"), (4, "bfs"), (4, "wide")])
 def test_operator_error_is_that_of_fp64(require_gpu, kind, p):
     g = _solver(p, kind)
     K, (rp, col) = g.blocks(), g.pattern()
