@@ -211,26 +211,18 @@ __device__ __forceinline__ void store_u32(float* u32, int64_t q, int i, double v
     if (i == 2) u32[q * 4 + 3] = (float)v;
 }
 
-// y_r = sum_c A(r, c) w_c for rows r < ND of a column-major ND x ND matrix in
-// device memory, w in shared memory, by every thread of the CTA: the columns in
-// blockDim / ND slices (several loads of a row in flight at once; one thread
-// per row ran a chain of ND dependent loads: 1.96 -> 1.55 ms for 81 matrix-free
-// steps of 1,300 polyhedra at p = 2), the slices' sums added in order.
-// s_p holds blockDim doubles.  Returns y_tid for tid < ND; synchronises.
+// Columns c0, c0 + step, ... of row r of a column-major ND x ND matrix in device
+// memory times w in shared memory, one chain in increasing c (the FP32 operators'
+// steps carry a change of rounding here back through their inputs: on tetrahedra at
+// p = 4 sums in slices ended 4e-5 apart after 74 steps).  Sixteen loads are in flight
+// at once (80 matrix-free steps of 1,273 polyhedra at p = 2: 1.24 ms, 1.92 with rolled
+// chains and without the overlapping launches, 1.18 with sums in slices).
 template <int ND>
-__device__ __forceinline__ double cta_matvec(const double* __restrict__ A, const double* s_w, double* s_p) {
-    const int tid = threadIdx.x, S = blockDim.x / ND, r = tid % ND, s = tid / ND;
+__device__ __forceinline__ double row_chain(const double* __restrict__ A, const double* w, int r, int c0, int step) {
     double a = 0.0;
-    if (s < S) {
-#pragma unroll 8
-        for (int c = s; c < ND; c += S) a = fma(__ldg(A + c * ND + r), s_w[c], a);
-        s_p[s * ND + r] = a;
-    }
-    __syncthreads();
-    double y = 0.0;
-    if (tid < ND)
-        for (int k = 0; k < S; ++k) y += s_p[k * ND + tid];
-    return y;
+#pragma unroll 16
+    for (int c = c0; c < ND; c += step) a = fma(__ldg(A + c * ND + r), w[c], a);
+    return a;
 }
 
 // The end of one polyhedron's step once thread tid < ND holds y = (K u)_tid
@@ -285,12 +277,21 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
         // MODE_STEP: D (u^n - u^{n-1}); MODE_FIRST: D v^0 (v^0 is in un)
         if (tid < ND) s_w[tid] = (MODE == MODE_STEP) ? A.un[base + tid] - A.u0[base + tid] : A.un[base + tid];
         __syncthreads();
-        const double dv = cta_matvec<ND>(A.Dabs + (int64_t)ai * ND * ND, s_w, s_p);
+        const double dv = tid < ND ? row_chain<ND>(A.Dabs + (int64_t)ai * ND * ND, s_w, tid, 0, 1) : 0.0;
         if (tid < ND) s_b[tid] = (MODE == MODE_STEP) ? A.dt * A.dt * s_b[tid] - A.dt * dv : s_b[tid] - dv;
         __syncthreads();
         if (MODE == MODE_STEP) {
             // u^{n+1} = 2 u^n - u^{n-1} + W^-1 (dt^2 (F - K u^n) - dt D (u^n - u^{n-1}))
-            const double x = cta_matvec<ND>(A.Winv + (int64_t)ai * ND * ND, s_b, s_p);
+            // the even and the odd columns, side by side where the CTA has the threads
+            const double* W = A.Winv + (int64_t)ai * ND * ND;
+            double x = 0.0;
+            if (blockDim.x >= 2 * ND) {
+                if (tid < 2 * ND) s_p[tid] = row_chain<ND>(W, s_b, tid % ND, tid / ND, 2);
+                __syncthreads();
+                if (tid < ND) x = s_p[tid] + s_p[ND + tid];
+            } else if (tid < ND) {
+                x = row_chain<ND>(W, s_b, tid, 0, 2) + row_chain<ND>(W, s_b, tid, 1, 2);
+            }
             if (tid < ND) {
                 const int64_t q = base + tid;
                 const double v = x + 2.0 * A.un[q] - A.u0[q];

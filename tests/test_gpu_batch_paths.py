@@ -24,6 +24,10 @@ WIDE = dict(n=8, bc="reference", agglomeration="bfs", group=(8, 100), jitter=0.1
     (_lib.FP64, [(WIDE, p, 1e-4) for p in (1, 2, 3, 4)]),
     (_lib.MIXED, [(WIDE, p, 1e-4) for p in (1, 2, 3)]),
     (_lib.MIXED, [(dict(n=6, agglomeration="hex"), p, 1e-4) for p in (1, 3)]),
+    # absorbing sides: the damping products keep one order whatever the CTA's size
+    (_lib.FP64, [(dict(n=3, bc="absorbing", **BFS), p, 1e-4) for p in (1, 2, 3, 4)]),
+    (_lib.MIXED, [(dict(n=3, bc="absorbing", **BFS), p, 1e-4) for p in (1, 2, 3, 4)]),
+    (_lib.MIXED_MF, [(dict(n=3, bc="absorbing", **BFS), p, 1e-4) for p in (1, 2, 3, 4)]),
 ])
 def test_batch_equals_problems_alone(require_gpu, precision, specs):
     batch_solvers = [_prepared(s, precision) for s in specs]
