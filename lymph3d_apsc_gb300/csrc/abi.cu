@@ -13,6 +13,7 @@
 #include <cstring>
 #include <atomic>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -214,33 +215,46 @@ struct Fnv64 {
     template <typename T> void add_value(T v) { add(&v, sizeof(v)); }
 };
 
-// The hash of the mesh descriptor's arrays, from the device's copies, when a
-// checkpoint first needs it (byte by byte, it takes longer than the rest of the
-// host's part of lymph_create).
-int mesh_hash(lymph_ctx* c, uint64_t* out) {
-    if (!c->have_mesh_hash) {
-        const size_t nt = (size_t)c->n_tet;
-        struct { const void* d; size_t bytes; bool in; } part[] = {
-            {c->d_coords, sizeof(double) * 3 * (size_t)c->n_node, true}, {c->d_tet_vert, sizeof(int32_t) * 4 * nt, true},
-            {c->d_tet_poly, sizeof(int32_t) * nt, true}, {c->d_tet_mat, sizeof(int32_t) * nt, true},
-            {c->d_neigh, sizeof(int32_t) * 4 * nt, true}, {c->d_fun_tag, sizeof(int32_t) * 4 * nt, c->given_fun_tag},
-            {c->d_mat, sizeof(double) * 3 * (size_t)c->n_mat, true}};
-        Fnv64 f;
-        f.add_value((int32_t)c->n_node); f.add_value((int32_t)c->n_tet); f.add_value((int32_t)c->n_poly); f.add_value((int32_t)c->n_mat);
-        std::vector<char> h;
-        for (const auto& q : part) {
-            if (!q.in) continue;
-            h.resize(q.bytes);
-            LYMPH_CUDA_TRY(cudaMemcpyAsync(h.data(), q.d, q.bytes, cudaMemcpyDeviceToHost, c->stream));
-            LYMPH_CUDA_TRY(cudaStreamSynchronize(c->stream));
-            f.add(h.data(), q.bytes);
+// The hash of the mesh descriptor's arrays, formed beside the rest of lymph_create
+// by a thread that has ended when the call returns: byte by byte it takes about as long
+// as all of it (384,000 tetrahedra: 20 ms; lymph_create 26.6 ms without it, 27.3 with).
+// Without a thread to be had it is formed in place.
+class MeshHash {
+  public:
+    explicit MeshHash(const lymph_mesh_desc* m) : mesh_(m) {
+        try {
+            thread_ = std::thread([this] { form(); });
+        } catch (...) {
+            form();
         }
-        c->mesh_hash = f.h;
-        c->have_mesh_hash = true;
     }
-    *out = c->mesh_hash;
-    return LYMPH_OK;
-}
+    ~MeshHash() { wait(); }
+    uint64_t get() {
+        wait();
+        return hash_;
+    }
+
+  private:
+    const lymph_mesh_desc* mesh_;
+    uint64_t hash_ = 0;
+    std::thread thread_;
+    void wait() {
+        if (thread_.joinable()) thread_.join();
+    }
+    void form() {
+        const lymph_mesh_desc* m = mesh_;
+        Fnv64 f;
+        f.add_value(m->n_node); f.add_value(m->n_tet); f.add_value(m->n_poly); f.add_value(m->n_mat);
+        f.add(m->coords, sizeof(double) * 3 * (size_t)m->n_node);
+        f.add(m->tet_vert, sizeof(int32_t) * 4 * (size_t)m->n_tet);
+        f.add(m->tet_poly, sizeof(int32_t) * (size_t)m->n_tet);
+        f.add(m->tet_mat, sizeof(int32_t) * (size_t)m->n_tet);
+        f.add(m->neigh, sizeof(int32_t) * 4 * (size_t)m->n_tet);
+        if (m->fun_tag) f.add(m->fun_tag, sizeof(int32_t) * 4 * (size_t)m->n_tet);
+        f.add(m->mat, sizeof(double) * 3 * (size_t)m->n_mat);
+        hash_ = f.h;
+    }
+};
 
 // The checkpoint file: this header, then u^{n-1} and u^n as [n_poly][3Np]
 // doubles (the device layout), all in the host's byte order.
@@ -403,6 +417,7 @@ int lymph_create(const lymph_mesh_desc* m, const lymph_params* prm, lymph_ctx** 
         static std::atomic<uint64_t> next_uid{1};
         c->uid = next_uid++;
     }
+    MeshHash hash(m);
     int rc = LYMPH_OK;
     auto fail = [&](int code) { lymph_destroy(c); return code; };
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -473,7 +488,6 @@ int lymph_create(const lymph_mesh_desc* m, const lymph_params* prm, lymph_ctx** 
     if (!build_ref_tables(c->p, ref)) { lymph_set_error("lymph_create: no quadrature table"); return fail(LYMPH_ERR_INVALID); }
     std::vector<int32_t> ftag(4 * (size_t)nt, 1);
     if (m->fun_tag) std::memcpy(ftag.data(), m->fun_tag, sizeof(int32_t) * 4 * (size_t)nt);
-    c->given_fun_tag = m->fun_tag != nullptr;
     // ---- device arrays ----
     Arena ar;
     ar.copy(&c->d_coords, m->coords, 3 * (size_t)m->n_node);
@@ -516,6 +530,7 @@ int lymph_create(const lymph_mesh_desc* m, const lymph_params* prm, lymph_ctx** 
     c->gvals_cap = 4096;
     if ((rc = dalloc(c, &c->d_gvals, (size_t)c->gvals_cap))) return fail(rc);
     if ((rc = lymph_dev_geometry(c))) return fail(rc);
+    c->mesh_hash = hash.get();
     if ((rc = lymph_sync_status(c, "lymph_create"))) return fail(rc);
     *out = c;
     return LYMPH_OK;
@@ -869,7 +884,7 @@ int lymph_checkpoint_save(lymph_ctx* c, const char* path, double t, int64_t step
     h.version = 1;
     h.precision = c->precision;
     h.degree = c->p;
-    LYMPH_TRY(mesh_hash(c, &h.mesh_hash));
+    h.mesh_hash = c->mesh_hash;
     h.n_poly = c->n_poly;
     h.nd = c->nd;
     h.dt = c->dt; h.alpha = c->alpha; h.theta = c->theta;
@@ -907,13 +922,7 @@ int lymph_checkpoint_load(lymph_ctx* c, const char* path, double* t, int64_t* st
     };
     if (std::fread(&h, sizeof(h), 1, f) != 1 || std::memcmp(h.magic, "LYMPHCK1", 8) != 0 || h.version != 1)
         return bad("not a checkpoint of this library");
-    uint64_t own = 0;
-    const int rc_hash = mesh_hash(c, &own);
-    if (rc_hash) {
-        std::fclose(f);
-        return rc_hash;
-    }
-    if (h.mesh_hash != own || h.n_poly != c->n_poly) return bad("written for another mesh");
+    if (h.mesh_hash != c->mesh_hash || h.n_poly != c->n_poly) return bad("written for another mesh");
     if (h.degree != c->p || h.nd != c->nd) return bad("written for another degree");
     if (h.precision != c->precision) return bad("written for another precision mode");
     if (h.dt != c->dt || h.alpha != c->alpha || h.theta != c->theta) return bad("written with another dt, alpha or theta");

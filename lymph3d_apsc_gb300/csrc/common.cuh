@@ -70,8 +70,7 @@ struct lymph_ctx {
     double alpha = 10.0, theta = -1.0, dt = 1e-3;
     // sizes
     int n_node = 0, n_tet = 0, n_poly = 0, n_mat = 0;
-    uint64_t mesh_hash = 0;         // FNV-1a of the mesh descriptor's arrays (checkpoints carry it), when first needed
-    bool have_mesh_hash = false, given_fun_tag = false;
+    uint64_t mesh_hash = 0;         // FNV-1a of the mesh descriptor's arrays (checkpoints carry it)
     std::vector<void*> arenas;      // device allocations that hold the arrays below but for the few noted in lymph_destroy
     uint64_t uid = 0;               // unique per context in the process (caches keyed by context)
     int64_t rhs_version = 0;        // bumped whenever rhs_dyn or M^-1 change (caches of M^-1 F)

@@ -1,0 +1,37 @@
+"""The library's host side on a fake CUDA runtime (fake_cudart.c): which calls it
+makes, and what it does when one fails.  No GPU."""
+import struct
+
+from lymph3d_apsc_gb300 import mesh as M
+from fake_runtime import run
+
+SOLVER = """
+m = M.cube(3, bc="reference", agglomeration="bfs", seed=1, group=(4, 12))
+s = MatrixFree(m, 3, 1e-4, precision=_lib.{precision})
+s.MAKE_MATRICES_FREE()
+"""
+
+
+def _fnv(*parts):
+    h = 1469598103934665603
+    for p in parts:
+        for b in p:
+            h = (h ^ b) * 1099511628211 % 2**64
+    return h
+
+
+def test_the_mesh_hash_is_formed_with_the_context(tmp_path):
+    """A checkpoint's save and load copy the two states and nothing else; the hash in
+    the file is that of the mesh descriptor's arrays."""
+    path = tmp_path / "c.ckpt"
+    save, load = run(SOLVER.format(precision="FP64") + f"""
+fake.fake_clear(); s.save_checkpoint({str(path)!r}, 0.5, 3); out(calls())
+fake.fake_clear(); s.load_checkpoint({str(path)!r}); out(calls())
+""", tmp_path)
+    assert save.count("d") == 2 and save.count("u") == 0
+    assert load.count("u") == 2 and load.count("d") == 0
+    m = M.cube(3, bc="reference", agglomeration="bfs", seed=1, group=(4, 12))
+    parts = [struct.pack("<4i", m.n_node, m.n_tet, m.n_poly, len(m.mat))]
+    parts += [a.tobytes() for a in (m.coords, m.tet_vert, m.tet_poly, m.tet_mat, m.neigh, m.fun_tag, m.mat)]
+    raw = path.read_bytes()
+    assert struct.pack("<Q", _fnv(*parts)) in raw[:128]
