@@ -768,6 +768,11 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
     LYMPH_CUDA_TRY(cudaEventCreate(&e0));
     LYMPH_CUDA_TRY(cudaEventCreate(&e1));
     int rc = lymph_dev_run_start(c);
+    const auto done = [&] {
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        return rc;
+    };
     if (ms_kernel) {
         // per-launch events around every step kernel (no graph)
         std::vector<cudaEvent_t> ev(2 * n);
@@ -777,13 +782,15 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
             cudaEventRecord(ev[2 * i], c->stream);
             rc = lymph_dev_step(c, 0, 0.0, true);
             cudaEventRecord(ev[2 * i + 1], c->stream);
-            if (rc == LYMPH_OK) rc = lymph_dev_bump(c, 1);
-            c->cur ^= 1;
+            if (rc == LYMPH_OK) {
+                c->cur ^= 1;
+                rc = lymph_dev_bump(c, 1);
+            }
         }
         cudaEventRecord(e1, c->stream);
         cudaEventSynchronize(e1);
         float sum = 0.0f;
-        for (int64_t i = 0; i < n; ++i) {
+        for (int64_t i = 0; i < n && rc == LYMPH_OK; ++i) {
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, ev[2 * i], ev[2 * i + 1]);
             sum += ms;
@@ -804,15 +811,19 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
                 int cur0 = c->cur;
                 LYMPH_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
                 int64_t l0 = c->launches;
-                for (int j = 0; j < R; ++j) {
-                    lymph_dev_step(c, j, 0.0, true);
+                for (int j = 0; j < R && rc == LYMPH_OK; ++j) {
+                    rc = lymph_dev_step(c, j, 0.0, true);
                     c->cur ^= 1;
                 }
-                lymph_dev_bump(c, R);
+                if (rc == LYMPH_OK) rc = lymph_dev_bump(c, R);
                 c->graph_launches = c->launches - l0;
                 c->launches = l0;
                 cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
                 c->cur = cur0;
+                if (rc) {   // a graph without one of its launches would leave steps out
+                    if (ce == cudaSuccess) cudaGraphDestroy(graph);
+                    return done();
+                }
                 if (ce != cudaSuccess) { lymph_set_error(std::string("graph capture: ") + cudaGetErrorString(ce)); return LYMPH_ERR_CUDA; }
                 ce = cudaGraphInstantiate(&c->graph_exec, graph, 0);
                 cudaGraphDestroy(graph);
@@ -828,20 +839,19 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
                 c->launches += c->graph_launches;
             }
         }
-        for (int off = 0; i < n; ++i, ++off) {  // the rest: step_idx stands at a multiple of R
-            LYMPH_TRY(lymph_dev_step(c, off, 0.0, true));
-            c->cur ^= 1;
+        for (int off = 0; i < n && rc == LYMPH_OK; ++i, ++off) {  // the rest: step_idx stands at a multiple of R
+            rc = lymph_dev_step(c, off, 0.0, true);
+            if (rc == LYMPH_OK) c->cur ^= 1;
         }
         cudaEventRecord(e1, c->stream);
     }
+    if (rc) return done();
     cudaEventSynchronize(e1);
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, e0, e1);
     if (ms_total) *ms_total = ms;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     *t_inout = t;
-    LYMPH_TRY(rc);
+    LYMPH_TRY(done());
     return lymph_sync_status(c, "lymph_run_steps");
 }
 

@@ -332,9 +332,14 @@ int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, bool use_graph) {
             cudaGraph_t g;
             LYMPH_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
             int64_t l0 = b->launches;
-            for (int j = 0; j < R; ++j) launch_step(b, g_stride, j, j == R - 1 ? R : 0);
+            int rc = LYMPH_OK;
+            for (int j = 0; j < R && rc == LYMPH_OK; ++j) rc = launch_step(b, g_stride, j, j == R - 1 ? R : 0);
             b->launches = l0;
             cudaError_t e = cudaStreamEndCapture(b->stream, &g);
+            if (rc) {   // a graph without one of its launches would leave work out
+                if (e == cudaSuccess) cudaGraphDestroy(g);
+                return rc;
+            }
             if (e != cudaSuccess) { lymph_set_error(std::string("batch graph capture: ") + cudaGetErrorString(e)); return LYMPH_ERR_CUDA; }
             e = cudaGraphInstantiate(&b->graph, g, 0);
             cudaGraphDestroy(g);

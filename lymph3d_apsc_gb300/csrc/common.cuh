@@ -21,6 +21,7 @@ void lymph_set_error(const std::string& msg);
         cudaError_t _e = (expr);                                                         \
         if (_e != cudaSuccess) {                                                         \
             lymph_set_error(std::string(#expr) + ": " + cudaGetErrorString(_e));         \
+            (void)cudaGetLastError(); /* reported here, not by the next call's check */  \
             return (_e == cudaErrorMemoryAllocation) ? LYMPH_ERR_OOM : LYMPH_ERR_CUDA;   \
         }                                                                                \
     } while (0)

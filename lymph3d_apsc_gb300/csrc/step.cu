@@ -299,6 +299,7 @@ int launch_step_i(lymph_ctx* c, const StepArgs& A) {
         LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE, INT>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
     } else {
         k_step<PD, KT, MODE, INT><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
+        LYMPH_CUDA_TRY(cudaGetLastError());
     }
     c->launches++;
     return LYMPH_OK;
@@ -383,6 +384,7 @@ int lymph_dev_step(lymph_ctx* c, int off, double g, bool fresh) {
 // step_idx += n
 int lymph_dev_bump(lymph_ctx* c, int n) {
     k_bump<<<1, 1, 0, c->stream>>>(c->d_step_idx, n);
+    LYMPH_CUDA_TRY(cudaGetLastError());
     c->launches++;
     return LYMPH_OK;
 }

@@ -1,7 +1,7 @@
 /* A stand-in for the CUDA runtime's entry points that the library calls, preloaded by
  * tests of its host side: device memory is host memory, kernels do nothing, and each
- * call is noted as one letter.  fake_fail_launch(n) makes the n-th launch from then
- * on with attributes (cudaLaunchKernelEx) fail as a launch can. */
+ * call is noted as one letter.  fake_fail_launch(n) makes the n-th kernel launch from
+ * then on fail as a launch can. */
 #include <stdlib.h>
 #include <string.h>
 
@@ -54,17 +54,19 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f
 int __cudaGetKernel(void** k, const void* f) { *k = (void*)f; return 0; }
 unsigned __cudaPushCallConfiguration(dim3_ g, dim3_ b, size_t s, void* st) { g_ = g; b_ = b; s_ = s; st_ = st; return 0; }
 int __cudaPopCallConfiguration(dim3_* g, dim3_* b, size_t* s, void* st) { *g = g_; *b = b_; *s = s_; *(void**)st = st_; return 0; }
-int __cudaLaunchKernel(void* k, dim3_ g, dim3_ b, void** a, size_t s, void* st) {
-    (void)k; (void)g; (void)b; (void)a; (void)s; (void)st;
-    note('K');
-    return 0;
-}
-int cudaLaunchKernelExC(const void* cfg, const void* f, void** a) {
-    (void)cfg; (void)f; (void)a;
+static int launch(char c) {
     if (fail_ > 0 && --fail_ == 0) {
         note('!');
         return err_ = 701;   /* cudaErrorLaunchOutOfResources */
     }
-    note('X');
+    note(c);
     return 0;
+}
+int __cudaLaunchKernel(void* k, dim3_ g, dim3_ b, void** a, size_t s, void* st) {
+    (void)k; (void)g; (void)b; (void)a; (void)s; (void)st;
+    return launch('K');
+}
+int cudaLaunchKernelExC(const void* cfg, const void* f, void** a) {
+    (void)cfg; (void)f; (void)a;
+    return launch('X');
 }

@@ -2,6 +2,8 @@
 makes, and what it does when one fails.  No GPU."""
 import struct
 
+import pytest
+
 from lymph3d_apsc_gb300 import mesh as M
 from fake_runtime import run
 
@@ -35,3 +37,39 @@ fake.fake_clear(); s.load_checkpoint({str(path)!r}); out(calls())
     parts += [a.tobytes() for a in (m.coords, m.tet_vert, m.tet_poly, m.tet_mat, m.neigh, m.fun_tag, m.mat)]
     raw = path.read_bytes()
     assert struct.pack("<Q", _fnv(*parts)) in raw[:128]
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED", "MIXED_MF"])
+@pytest.mark.parametrize("nth", [1, 7, 17, 20])
+def test_a_failed_launch_of_a_run_is_reported(tmp_path, precision, nth):
+    """The nth launch of 40 steps fails (the 17th: the counter at the end of the graph of 16
+    steps; the matrix-free run's first converts the state): an error, not a graph that
+    leaves a step out; the next run is whole."""
+    failed, log, again, log2 = run(SOLVER.format(precision=precision) + f"""
+fake.fake_clear(); fake.fake_fail_launch({nth})
+try:
+    s.run_steps(s.dt, 1.0, max_steps=40); out(False)
+except LymphError:
+    out(True)
+out(calls()); fake.fake_clear()
+s.run_steps(s.dt, 1.0, max_steps=40); out(True); out(calls())
+""", tmp_path)
+    assert "!" in log and failed
+    if "[" in log2:   # else the graph was whole before the failure
+        assert log2[log2.index("["):log2.index("]")].count("X") == 16
+    assert log2.count("G") == 2 and log2[log2.rindex("G"):].count("X") == 8
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED", "MIXED_MF"])
+@pytest.mark.parametrize("nth", [1, 2, 9, 31])
+def test_a_failed_launch_of_a_batch_is_reported(tmp_path, precision, nth):
+    failed, log = run(SOLVER.format(precision=precision) + f"""
+b = E.Batch([s])
+fake.fake_clear(); fake.fake_fail_launch({nth})
+try:
+    b.run(np.zeros((1, 32))); out(False)
+except LymphError:
+    out(True)
+out(calls())
+""", tmp_path)
+    assert "!" in log and failed
