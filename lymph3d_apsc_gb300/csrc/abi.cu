@@ -767,6 +767,7 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
     cudaEvent_t e0, e1;
     LYMPH_CUDA_TRY(cudaEventCreate(&e0));
     LYMPH_CUDA_TRY(cudaEventCreate(&e1));
+    cudaEventRecord(e0, c->stream);   // the conversion of the first state is part of the time that is reported
     int rc = lymph_dev_run_start(c);
     const auto done = [&] {
         cudaEventDestroy(e0);
@@ -777,7 +778,6 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
         // per-launch events around every step kernel (no graph)
         std::vector<cudaEvent_t> ev(2 * n);
         for (auto& e : ev) cudaEventCreate(&e);
-        cudaEventRecord(e0, c->stream);
         for (int64_t i = 0; i < n && rc == LYMPH_OK; ++i) {
             cudaEventRecord(ev[2 * i], c->stream);
             rc = lymph_dev_step(c, 0, 0.0, true);
@@ -804,7 +804,6 @@ int lymph_run_steps(lymph_ctx* c, double stop_time, int64_t max_steps, double* t
             c->graph_exec = nullptr;
         }
         int64_t i = 0;
-        cudaEventRecord(e0, c->stream);
         if (n >= R) {
             if (!c->graph_exec) {
                 cudaGraph_t graph;

@@ -73,3 +73,14 @@ except LymphError:
 out(calls())
 """, tmp_path)
     assert "!" in log and failed
+
+
+@pytest.mark.parametrize("timed", [False, True])
+def test_the_reported_time_holds_every_kernel_of_a_run(tmp_path, timed):
+    """run_steps' first event comes before the first kernel (matrix-free: the conversion
+    of the first state), its last after the last."""
+    log, = run(SOLVER.format(precision="MIXED_MF") + f"""
+fake.fake_clear(); s.run_steps(s.dt, 1.0, max_steps=21, kernel_timing={timed}); out(calls())
+""", tmp_path)
+    log = "".join(c for c in log if c in "EKXG")
+    assert log[0] == "E" and log[-1] == "E" and "K" in log
