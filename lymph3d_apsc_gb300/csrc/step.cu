@@ -22,11 +22,15 @@ namespace {
 
 using namespace stepk;
 
-// One CTA per polyhedron.
-template <int PD, typename KT, int MODE, bool INT = int_columns(PD, sizeof(KT))>
-__global__ void __launch_bounds__(Shape<PD>::T, Shape<PD>::MINB) k_step(StepArgs A) {
+// One CTA per polyhedron.  Without the code of absorbing faces (ABS) p = 1 takes 32 registers
+// instead of 38 with FP32 blocks, so 21 CTAs fit an SM instead of 17: 48 steps of 46,861
+// polyhedra 5.08 -> 4.42 ms, of 3,013 466 -> 430 us.  The integer columns of p = 2 keep few values
+// per thread and wait for their loads: 8 CTAs per SM (32 registers) instead of 6 take
+// 46,861 polyhedra from 46.2 to 37.8 ms, 737 from 0.89 to 0.87 (45.7 and 1.02 with FP64 products).
+template <int PD, typename KT, int MODE, bool INT, bool ABS>
+__global__ void __launch_bounds__(Shape<PD>::T, PD == 2 && INT ? 8 : Shape<PD>::MINB) k_step(StepArgs A) {
     __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
-    step_poly<PD, KT, MODE, Shape<PD>::S, INT>(A, blockIdx.x, smem);
+    step_poly<PD, KT, MODE, Shape<PD>::S, INT, false, ABS, PD == 3 ? 8 : 16>(A, blockIdx.x, smem);
 }
 
 // The same for at most SMALL_POLY polyhedra without absorbing faces, p <= 3.
@@ -295,14 +299,20 @@ int launch_step_i(lymph_ctx* c, const StepArgs& A) {
             return LYMPH_OK;
         }
     }
-    if (MODE == MODE_STEP && !plain) {
-        LYMPH_CUDA_TRY(launch_pdl(k_step<PD, KT, MODE, INT>, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
-    } else {
-        k_step<PD, KT, MODE, INT><<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
-        LYMPH_CUDA_TRY(cudaGetLastError());
+    const auto go = [&](auto kernel) -> int {
+        if (MODE == MODE_STEP && !plain) {
+            LYMPH_CUDA_TRY(launch_pdl(kernel, (unsigned)c->n_poly, Shape<PD>::T, c->stream, A));
+        } else {
+            kernel<<<c->n_poly, Shape<PD>::T, 0, c->stream>>>(A);
+            LYMPH_CUDA_TRY(cudaGetLastError());
+        }
+        c->launches++;
+        return LYMPH_OK;
+    };
+    if constexpr (MODE == MODE_STEP || MODE == MODE_FIRST) {
+        if (A.abs_idx) return go(k_step<PD, KT, MODE, INT, true>);
     }
-    c->launches++;
-    return LYMPH_OK;
+    return go(k_step<PD, KT, MODE, INT, false>);
 }
 
 template <int PD, typename KT, int MODE>
@@ -542,11 +552,14 @@ int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double
 }
 
 // Whether the context's step kernel multiplies columns on the integer pipe: FP64
-// blocks at p = 3 and 4, and at p = 2 on long rows (8 blocks or more on average)
-// from 4 CTAs per SM on: 46,767 polyhedra 16.2 -> 14.5 ms for 16 steps, 737 442 ->
-// 388 us.  The preparation of the coefficients costs a short row what it gains
-// (hexahedra, 7 blocks: 8,000 5.64 -> 5.66 ms for 48 steps), a small grid more (125:
-// 345 -> 405 us), and p = 1 at any size (46,767: 4.06 -> 4.25 ms).
+// blocks at p = 3 and 4 (48 steps, FP64 products alone -> integer columns: tetrahedra, 4
+// to 5 blocks a row, p = 3, 48 / 384 / 6,000 polyhedra 0.43 / 0.93 / 10.1 -> 0.41 / 0.76 /
+// 7.5 ms, p = 4 0.91 / 2.50 / 28.6 -> 0.81 / 1.76 / 20.8; 125 hexahedra 0.53 -> 0.52 and 1.22
+// -> 1.08; no mesh of 21 polyhedra or more was slower), and at p = 2 on long rows (8
+// blocks or more on average) from 4 CTAs per SM on: 46,861 polyhedra 45.7 -> 37.8 ms for
+// 48 steps, 737 1.02 -> 0.87.  There the preparation of the coefficients cost a short row
+// what it gained (hexahedra, 7 blocks: 8,000 5.64 -> 5.66 ms), a small grid more (125:
+// 345 -> 405 us), and p = 1 at any size (46,767, 16 steps: 4.06 -> 4.25 ms).
 bool lymph_dev_int_columns(const lymph_ctx* c) {
     if (c->precision != LYMPH_FP64) return false;
     return c->p >= 3 || (c->p == 2 && c->n_poly >= 4 * 152 && c->n_blocks >= 8 * (int64_t)c->n_poly);

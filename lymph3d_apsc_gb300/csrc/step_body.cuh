@@ -106,9 +106,10 @@ constexpr int64_t STEP_PREFETCH_MAX = 512ll << 20;
 constexpr int NBB = 16;   // neighbour blocks staged in shared memory at once
 
 // Doubles of scratch finish_poly needs behind the right-hand side for polyhedra
-// with absorbing faces: a vector of ND and a partial sum per thread.
+// with absorbing faces: a vector of ND, and two partial sums per row where the CTA
+// has the threads to form them side by side.
 constexpr int MAX_STEP_THREADS = 320;
-constexpr int finish_scratch(int nd, int threads) { return nd + threads; }
+constexpr int finish_scratch(int nd, int threads) { return nd + (threads >= 2 * nd ? 2 * nd : 0); }
 
 // MODE_APPLY: out = M^-1 K u (power iteration for the CFL bound)
 // MODE_BILIN: partial[P] = un_P . (K u0)_P (the bilinear form of the leapfrog energy)
@@ -217,10 +218,10 @@ __device__ __forceinline__ void store_u32(float* u32, int64_t q, int i, double v
 // p = 4 sums in slices ended 4e-5 apart after 74 steps).  Sixteen loads are in flight
 // at once (80 matrix-free steps of 1,273 polyhedra at p = 2: 1.24 ms, 1.92 with rolled
 // chains and without the overlapping launches, 1.18 with sums in slices).
-template <int ND>
+template <int ND, int UNROLL>
 __device__ __forceinline__ double row_chain(const double* __restrict__ A, const double* w, int r, int c0, int step) {
     double a = 0.0;
-#pragma unroll 16
+#pragma unroll UNROLL
     for (int c = c0; c < ND; c += step) a = fma(__ldg(A + c * ND + r), w[c], a);
     return a;
 }
@@ -235,7 +236,9 @@ __device__ __forceinline__ double row_chain(const double* __restrict__ A, const 
 // thread of the CTA must call this (it synchronises).
 // U32: also leave the FP32 copy of u^{n+1} (A.u32_out) for the next
 // matrix-free step.
-template <int PD, int MODE, bool U32 = false>
+// ABS: with the code of polyhedra with absorbing faces; CHAIN: the loads of a damping
+// chain in flight.
+template <int PD, int MODE, bool U32 = false, bool ABS = true, int CHAIN = 16>
 __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, double* s_b) {
     constexpr int NP = Deg<PD>::NP, ND = Deg<PD>::ND;
     const int tid = threadIdx.x;
@@ -270,14 +273,14 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
     }
     __syncthreads();
     // polyhedra with absorbing faces (the index is the same for the whole CTA)
-    const int ai = (MODE == MODE_STEP || MODE == MODE_FIRST) && A.abs_idx ? A.abs_idx[P] : -1;
+    const int ai = ABS && (MODE == MODE_STEP || MODE == MODE_FIRST) && A.abs_idx ? A.abs_idx[P] : -1;
     if (ai >= 0) {
         const int64_t base = (int64_t)P * ND;
         double *s_w = s_b + ND, *s_p = s_w + ND;
         // MODE_STEP: D (u^n - u^{n-1}); MODE_FIRST: D v^0 (v^0 is in un)
         if (tid < ND) s_w[tid] = (MODE == MODE_STEP) ? A.un[base + tid] - A.u0[base + tid] : A.un[base + tid];
         __syncthreads();
-        const double dv = tid < ND ? row_chain<ND>(A.Dabs + (int64_t)ai * ND * ND, s_w, tid, 0, 1) : 0.0;
+        const double dv = tid < ND ? row_chain<ND, CHAIN>(A.Dabs + (int64_t)ai * ND * ND, s_w, tid, 0, 1) : 0.0;
         if (tid < ND) s_b[tid] = (MODE == MODE_STEP) ? A.dt * A.dt * s_b[tid] - A.dt * dv : s_b[tid] - dv;
         __syncthreads();
         if (MODE == MODE_STEP) {
@@ -286,11 +289,11 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
             const double* W = A.Winv + (int64_t)ai * ND * ND;
             double x = 0.0;
             if (blockDim.x >= 2 * ND) {
-                if (tid < 2 * ND) s_p[tid] = row_chain<ND>(W, s_b, tid % ND, tid / ND, 2);
+                if (tid < 2 * ND) s_p[tid] = row_chain<ND, CHAIN>(W, s_b, tid % ND, tid / ND, 2);
                 __syncthreads();
                 if (tid < ND) x = s_p[tid] + s_p[ND + tid];
             } else if (tid < ND) {
-                x = row_chain<ND>(W, s_b, tid, 0, 2) + row_chain<ND>(W, s_b, tid, 1, 2);
+                x = row_chain<ND, CHAIN>(W, s_b, tid, 0, 2) + row_chain<ND, CHAIN>(W, s_b, tid, 1, 2);
             }
             if (tid < ND) {
                 const int64_t q = base + tid;
@@ -387,7 +390,8 @@ __device__ __forceinline__ void finish_small(const StepArgs& A, int P, double y,
 // Every thread of the CTA must call this (it synchronises); threads beyond the
 // degree's shape only help with the gather.
 // SMALL: dyn is the shared memory of SmallSmem.
-template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT)), bool SMALL = false>
+template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT)), bool SMALL = false,
+          bool ABS = true, int CHAIN = 16>
 __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, char* dyn = nullptr) {
     constexpr int ND = Deg<PD>::ND, S = S_;
     constexpr int CPT = (ND + S - 1) / S;
@@ -480,14 +484,8 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, 
         if (SMALL && b0 == rb) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         if (act) {
-            const auto block = [&](int bb, auto load) {
+            const auto products = [&](int bb, const KT(&kv)[CPT]) {
                 const AT* ub = s_u + bb * ND;
-                KT kv[CPT];
-#pragma unroll
-                for (int j = 0; j < CPT; ++j) {
-                    const int c = s + j * S;
-                    kv[j] = (c < ND) ? load(c * ND + r) : (KT)0;
-                }
 #pragma unroll
                 for (int j = 0; j < CPT; ++j) {
                     const int c = s + j * S;
@@ -508,14 +506,23 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, 
                 if (b0 == rb) {
 #pragma unroll 2
                     for (; bb < nst; ++bb) {
-                        const KT* Kb = (const KT*)dyn + bb * ND * ND;
-                        block(bb, [&](int e) { return Kb[e]; });
+                        const KT* Kb = (const KT*)dyn + bb * ND * ND + r;
+                        KT kv[CPT];
+#pragma unroll
+                        for (int j = 0; j < CPT; ++j) kv[j] = s + j * S < ND ? Kb[(s + j * S) * ND] : (KT)0;
+                        products(bb, kv);
                     }
                 }
             }
             for (; bb < nb; ++bb) {
-                const KT* Kb = Kbase + (int64_t)(b0 + bb) * ND * ND;
-                block(bb, [&](int e) { return ld_stream(Kb + e); });
+                const KT* Kb = Kbase + (int64_t)(b0 + bb) * ND * ND + r;
+                KT kv[CPT];
+#pragma unroll
+                for (int j = 0; j < CPT; ++j) {
+                    const int c = s + j * S;
+                    kv[j] = (c < ND) ? ld_stream(Kb + (int64_t)c * ND) : (KT)0;
+                }
+                products(bb, kv);
             }
             if constexpr (NI > 0) acc1 += acc_value(iacc, R);
         }
@@ -527,7 +534,7 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, 
     if (tid < ND)
         for (int ss = 0; ss < S; ++ss) y += (double)s_red[ss * ND + tid];
     if constexpr (SMALL) finish_small<PD>(A, P, y, s_b, own, (const double*)(dyn + SS::minv_offset));
-    else finish_poly<PD, MODE>(A, P, y, s_b);
+    else finish_poly<PD, MODE, false, ABS, CHAIN>(A, P, y, s_b);
 }
 
 }  // namespace stepk
