@@ -27,10 +27,12 @@ using namespace stepk;
 // polyhedra 5.08 -> 4.42 ms, of 3,013 466 -> 430 us.  The integer columns of p = 2 keep few values
 // per thread and wait for their loads: 8 CTAs per SM (32 registers) instead of 6 take
 // 46,861 polyhedra from 46.2 to 37.8 ms, 737 from 0.89 to 0.87 (45.7 and 1.02 with FP64 products).
+// The FP64 products of p = 2 load two blocks at once (8,000 hexahedra 5.47 -> 5.42 ms, 2,197
+// 1.65 -> 1.62): left to itself the compiler loads one once the damping's code is gone.
 template <int PD, typename KT, int MODE, bool INT, bool ABS>
 __global__ void __launch_bounds__(Shape<PD>::T, PD == 2 && INT ? 8 : Shape<PD>::MINB) k_step(StepArgs A) {
     __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
-    step_poly<PD, KT, MODE, Shape<PD>::S, INT, false, ABS, PD == 3 ? 8 : 16>(A, blockIdx.x, smem);
+    step_poly<PD, KT, MODE, Shape<PD>::S, INT, false, ABS, PD == 3 ? 8 : 16, PD == 2 && sizeof(KT) == 8 && !INT ? 2 : 0>(A, blockIdx.x, smem);
 }
 
 // The same for at most SMALL_POLY polyhedra without absorbing faces, p <= 3.

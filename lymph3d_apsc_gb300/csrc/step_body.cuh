@@ -389,9 +389,9 @@ __device__ __forceinline__ void finish_small(const StepArgs& A, int P, double y,
 // the number of column slices (the tile shape; the CTA needs ND * S_ threads).
 // Every thread of the CTA must call this (it synchronises); threads beyond the
 // degree's shape only help with the gather.
-// SMALL: dyn is the shared memory of SmallSmem.
+// SMALL: dyn is the shared memory of SmallSmem.  BLOCKS: blocks loaded at once, 0: the compiler's choice.
 template <int PD, typename KT, int MODE, int S_ = Shape<PD>::S, bool INT = int_columns(PD, sizeof(KT)), bool SMALL = false,
-          bool ABS = true, int CHAIN = 16>
+          bool ABS = true, int CHAIN = 16, int BLOCKS = 0>
 __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, char* dyn = nullptr) {
     constexpr int ND = Deg<PD>::ND, S = S_;
     constexpr int CPT = (ND + S - 1) / S;
@@ -514,15 +514,21 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, 
                     }
                 }
             }
-            for (; bb < nb; ++bb) {
-                const KT* Kb = Kbase + (int64_t)(b0 + bb) * ND * ND + r;
+            const auto block = [&](int k) {
+                const KT* Kb = Kbase + (int64_t)(b0 + k) * ND * ND + r;
                 KT kv[CPT];
 #pragma unroll
                 for (int j = 0; j < CPT; ++j) {
                     const int c = s + j * S;
                     kv[j] = (c < ND) ? ld_stream(Kb + (int64_t)c * ND) : (KT)0;
                 }
-                products(bb, kv);
+                products(k, kv);
+            };
+            if constexpr (BLOCKS > 0) {
+#pragma unroll BLOCKS
+                for (; bb < nb; ++bb) block(bb);
+            } else {
+                for (; bb < nb; ++bb) block(bb);
             }
             if constexpr (NI > 0) acc1 += acc_value(iacc, R);
         }
