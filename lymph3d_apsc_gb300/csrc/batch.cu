@@ -50,6 +50,12 @@ namespace {
 
 constexpr int BATCH_THREADS = 320;   // the p = 4 shape; lower degrees leave lanes idle
 constexpr int BATCH_MINB = 4;
+// A row's head is prefetched before its coefficients are gathered where that pays: in
+// batches of p = 1 and 2 alone, and from 3.4 GB of blocks per step on but for FP32 at p = 4
+// (profitable side first, 48 steps; problems of 3^3..8^3 x 6: p = 2 in FP32 3.17 against 3.77 ms,
+// p = 1 in FP64 2.42 against 2.63, degrees 1 to 4 in FP32 without 13.5 against 14.0; of
+// 14^3..26^3, degrees 1 to 4 in FP32, 148.4 against 153.7).
+constexpr int64_t BATCH_PREFETCH_MIN = 3400000000ll;
 constexpr int BATCH_QUEUES = 4;      // item counters: one per degree on the matrix-free path
 
 struct BatchProblem {
@@ -65,24 +71,39 @@ constexpr int BATCH_SHAPES = 3;
 constexpr int kBatchShapes[BATCH_SHAPES][5] = {{0, 8, 8, 4, 3}, {0, 16, 10, 5, 3}, {0, 24, 10, 5, 2}};
 
 constexpr size_t zmax(size_t a, size_t b) { return a > b ? a : b; }
-template <typename KT, int V> struct ShapeSmem {
+// FP64 problems of p = 2 have their integer columns in shape 0 alone (the others group a
+// row's sums in another way than a lone problem anyway, and are faster without).
+constexpr bool batch_int2(size_t elem, int shape) { return elem == 8 && shape == 0; }
+template <typename KT, int V, bool HIGH> struct BatchSmem {
+    static constexpr size_t low =
+        zmax(SmemSize<1, KT, kBatchShapes[V][1]>::bytes, SmemSize<2, KT, kBatchShapes[V][2], batch_int2(sizeof(KT), V)>::bytes);
     static constexpr size_t bytes =
-        zmax(zmax(SmemSize<1, KT, kBatchShapes[V][1]>::bytes, SmemSize<2, KT, kBatchShapes[V][2], sizeof(KT) == 8>::bytes),
-             zmax(SmemSize<3, KT, kBatchShapes[V][3]>::bytes, SmemSize<4, KT, kBatchShapes[V][4]>::bytes));
-};
-template <typename KT> struct BatchSmem {
-    static constexpr size_t bytes = zmax(ShapeSmem<KT, 0>::bytes, zmax(ShapeSmem<KT, 1>::bytes, ShapeSmem<KT, 2>::bytes));
+        HIGH ? zmax(low, zmax(SmemSize<3, KT, kBatchShapes[V][3]>::bytes, SmemSize<4, KT, kBatchShapes[V][4]>::bytes)) : low;
 };
 static_assert(Deg<1>::ND * kBatchShapes[2][1] <= BATCH_THREADS && Deg<2>::ND * kBatchShapes[1][2] <= BATCH_THREADS &&
                   Deg<3>::ND * kBatchShapes[1][3] <= BATCH_THREADS && Deg<4>::ND * kBatchShapes[0][4] <= BATCH_THREADS,
               "every tile shape fits the CTA");
 
-template <typename KT, int V>
-__global__ void __launch_bounds__(BATCH_THREADS, BATCH_MINB)
+// MINB: CTAs per SM that the registers are bounded for.  HIGH: with the code of p = 3 and
+// 4.  ABS: with the code of absorbing faces.  48 registers (MINB = 4) hold the loads of an
+// FP32 row in flight only if the item's arguments stay out of them, in shared memory, and
+// so does the damping's code: with both in them 48 steps of 64 problems of 3^3..8^3 x 6 took
+// 14.95 ms instead of 13.6, of 5 of 20^3..26^3 at p = 3 60.4 instead of 50.2.  The FP64
+// kernels are faster with the arguments in registers (64 registers: 19.3 against 20.3 ms).
+// FP64 with a grid of at most three CTAs per SM, which the tuner takes where the items are
+// few, has 64 registers (24 problems of 2^3..4^3 x 6: 2.81 -> 2.33 ms), and in the shapes
+// without integer columns at p = 2 a kernel of p = 1 and 2 alone (5 problems of 20^3..26^3
+// at p = 1, tuned: 18.7 -> 18.0 ms, at p = 2 42.9 -> 40.0).
+template <typename KT, int V, int MINB, bool HIGH, bool ABS>
+__global__ void __launch_bounds__(BATCH_THREADS, MINB)
 k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ items, int n_items, int* queue,
              const int64_t* step_idx, int off, const double* gvals, int64_t g_stride) {
-    __shared__ __align__(16) char smem[BatchSmem<KT>::bytes];
+    constexpr bool SHARED = sizeof(KT) == 4;
+    constexpr int CHAIN = 4;
+    __shared__ __align__(16) char smem[BatchSmem<KT, V, HIGH>::bytes];
     __shared__ int s_item;
+    __shared__ __align__(8) char s_args[SHARED ? sizeof(StepArgs) : 8];
+    static_assert(sizeof(StepArgs) % 8 == 0, "copied as 8-byte words");
     const int64_t k = *step_idx + off;   // off: the step's place in the graph
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
@@ -91,27 +112,40 @@ k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ it
         __syncthreads();
         if (it >= n_items) break;
         const int2 w = items[it];
-        StepArgs A = probs[w.x].a;
-        const int cur = probs[w.x].cur0 ^ (int)(k & 1);
-        A.un = probs[w.x].buf[cur];
-        A.u0 = probs[w.x].buf[cur ^ 1];
-        A.out = probs[w.x].buf[cur ^ 1];
-        A.gvals = gvals + (int64_t)w.x * g_stride;
-        A.step_idx = step_idx;
-        A.step_off = off;
-        switch (probs[w.x].p) {
-            case 1: step_poly<1, KT, MODE_STEP, kBatchShapes[V][1]>(A, w.y, smem); break;
-            case 2:
-                if constexpr (sizeof(KT) == 8) {
-                    if (A.Kex) {   // integer columns, as the problem alone
-                        step_poly<2, KT, MODE_STEP, kBatchShapes[V][2], true>(A, w.y, smem);
-                        break;
-                    }
-                }
-                step_poly<2, KT, MODE_STEP, kBatchShapes[V][2]>(A, w.y, smem);
-                break;
-            case 3: step_poly<3, KT, MODE_STEP, kBatchShapes[V][3]>(A, w.y, smem); break;
-            default: step_poly<4, KT, MODE_STEP, kBatchShapes[V][4]>(A, w.y, smem); break;
+        const BatchProblem& pb = probs[w.x];
+        const auto at_step = [&](StepArgs& A) {
+            const int cur = pb.cur0 ^ (int)(k & 1);
+            A.un = pb.buf[cur];
+            A.u0 = pb.buf[cur ^ 1];
+            A.out = pb.buf[cur ^ 1];
+            A.gvals = gvals + (int64_t)w.x * g_stride;
+            A.step_idx = step_idx;
+            A.step_off = off;
+        };
+        const auto go = [&](const StepArgs& A) {
+            if constexpr (HIGH) {
+                if (pb.p == 3) return step_poly<3, KT, MODE_STEP, kBatchShapes[V][3], int_columns(3, sizeof(KT)), false, ABS, CHAIN>(A, w.y, smem);
+                if (pb.p == 4) return step_poly<4, KT, MODE_STEP, kBatchShapes[V][4], int_columns(4, sizeof(KT)), false, ABS, CHAIN>(A, w.y, smem);
+            }
+            if (pb.p == 1) return step_poly<1, KT, MODE_STEP, kBatchShapes[V][1], false, false, ABS, CHAIN>(A, w.y, smem);
+            if constexpr (batch_int2(sizeof(KT), V)) {
+                if (A.Kex)   // integer columns, as the problem alone
+                    return step_poly<2, KT, MODE_STEP, kBatchShapes[V][2], true, false, ABS, CHAIN>(A, w.y, smem);
+            }
+            step_poly<2, KT, MODE_STEP, kBatchShapes[V][2], false, false, ABS, CHAIN>(A, w.y, smem);
+        };
+        if constexpr (SHARED) {
+            // the reads of the previous item's are over: a barrier parts them from here
+            for (int i = threadIdx.x; i < (int)(sizeof(StepArgs) / 8); i += blockDim.x)
+                ((int64_t*)s_args)[i] = ((const int64_t*)&pb.a)[i];
+            __syncthreads();
+            if (threadIdx.x == 0) at_step(*(StepArgs*)s_args);
+            __syncthreads();
+            go(*(const StepArgs*)s_args);
+        } else {
+            StepArgs A = pb.a;
+            at_step(A);
+            go(A);
         }
     }
 }
@@ -185,6 +219,8 @@ struct lymph_batch {
     int64_t launches = 0;
     int step_nl = 2;     // kernels one batched step launches
     int sms = 0;
+    bool high = false;        // a problem of p = 3 or 4
+    bool absorbing = false;   // a problem with absorbing faces
     std::string key;
 };
 
@@ -218,6 +254,8 @@ int refresh_problems(lymph_batch* b) {
         LYMPH_CUDA_TRY(cudaMemcpyAsync(b->d_probs, h.data(), h.size(), cudaMemcpyHostToDevice, b->stream));
         return LYMPH_OK;
     }
+    int64_t bytes = 0;   // of the blocks a step reads
+    for (const lymph_ctx* c : b->ctx) bytes += c->n_blocks * c->nd * c->nd * (b->precision == LYMPH_FP64 ? 8 : 4);
     std::vector<BatchProblem> h(b->ctx.size());
     for (size_t i = 0; i < b->ctx.size(); ++i) {
         lymph_ctx* c = b->ctx[i];
@@ -238,7 +276,7 @@ int refresh_problems(lymph_batch* b) {
         P.a.dt2 = c->dt * c->dt;
         P.a.status = b->d_status;
         P.a.n_poly = c->n_poly;
-        P.a.prefetch = 1;
+        P.a.prefetch = !b->high || (bytes >= BATCH_PREFETCH_MIN && (b->precision == LYMPH_FP64 || c->p <= 3));
         P.buf[0] = c->d_buf[0];
         P.buf[1] = c->d_buf[1];
         P.cur0 = c->cur;
@@ -254,10 +292,21 @@ void launch_shape(lymph_batch* b, const BatchProblem* probs, int off, int* queue
         kernel<<<b->grid, BATCH_THREADS, 0, b->stream>>>(probs, b->d_items, b->n_items, queue, b->d_step_idx, off,
                                                          b->d_gvals, g_stride);
     };
+    auto shape = [&](auto v) {
+        constexpr int V = decltype(v)::value;
+        if (b->absorbing) return go(k_step_batch<KT, V, BATCH_MINB, true, true>);
+        if constexpr (sizeof(KT) == 8) {
+            if (b->grid <= 3 * b->sms) return go(k_step_batch<KT, V, 3, true, false>);
+            if constexpr (V != 0) {
+                if (!b->high) return go(k_step_batch<KT, V, BATCH_MINB, false, false>);
+            }
+        }
+        go(k_step_batch<KT, V, BATCH_MINB, true, false>);
+    };
     switch (b->shape) {
-        case 1: go(k_step_batch<KT, 1>); break;
-        case 2: go(k_step_batch<KT, 2>); break;
-        default: go(k_step_batch<KT, 0>); break;
+        case 1: shape(std::integral_constant<int, 1>()); break;
+        case 2: shape(std::integral_constant<int, 2>()); break;
+        default: shape(std::integral_constant<int, 0>()); break;
     }
 }
 
@@ -424,6 +473,8 @@ int lymph_batch_create(lymph_ctx* const* ctxs, int32_t n, lymph_batch** out) {
             b->items_natural.push_back(make_int2(i, P));
         }
         per_p[c->p] += c->n_blocks;
+        b->high = b->high || c->p >= 3;
+        b->absorbing = b->absorbing || c->n_abs > 0;
     }
     for (auto& kv : per_p) key << "_p" << kv.first << "b" << kv.second;
     b->key = key.str();
