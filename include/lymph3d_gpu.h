@@ -482,7 +482,7 @@ int lymph_batch_run(lymph_batch* batch, int64_t n_steps, const double* gvals, fl
  * LYMPH_FP64 / LYMPH_MIXED also three tile shapes, the column slices per
  * degree) and keeps the fastest; the problems' states are restored
  * afterwards.  The choice is cached per batch signature in $LYMPH_TUNE_CACHE
- * (default ~/.cache/lymph3d_gb300_tune2.txt) and reused when use_cache is
+ * (default ~/.cache/lymph3d_gb300_tune3.txt) and reused when use_cache is
  * non-zero.  With tile shape 0 (the default before tuning) results equal
  * stepping each context alone bit for bit; the other shapes group each
  * row's partial sums differently: deterministic, equal up to rounding. */

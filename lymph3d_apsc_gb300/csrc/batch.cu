@@ -157,11 +157,12 @@ __global__ void k_batch_bump(int64_t* idx, int n, int* queue) {
     for (int i = 0; i < BATCH_QUEUES; ++i) queue[i] = 0;
 }
 
+constexpr int TUNE_VERSION = 3;
 std::string tune_cache_path() {
     const char* e = std::getenv("LYMPH_TUNE_CACHE");
     if (e && *e) return e;
     const char* h = std::getenv("HOME");
-    return std::string(h ? h : "/tmp") + "/.cache/lymph3d_gb300_tune2.txt";
+    return std::string(h ? h : "/tmp") + "/.cache/lymph3d_gb300_tune3.txt";
 }
 
 std::mutex g_tune_mu;
@@ -463,8 +464,10 @@ int lymph_batch_create(lymph_ctx* const* ctxs, int32_t n, lymph_batch** out) {
     // work items and their cost (bytes of blocks streamed)
     std::vector<std::pair<int64_t, int2>> cost;
     std::ostringstream key;
-    key << "sm" << b->sms << "_prec" << b->precision;
-    std::map<int, int64_t> per_p;
+    // TUNE_VERSION names the kernels the choice was measured with: to be raised with any
+    // change that moves their costs
+    key << "v" << TUNE_VERSION << "_sm" << b->sms << "_prec" << b->precision;
+    std::map<int, std::pair<int64_t, int64_t>> per_p;   // blocks, those with integer columns
     for (int i = 0; i < n; ++i) {
         lymph_ctx* c = ctxs[i];
         for (int P = 0; P < c->n_poly; ++P) {
@@ -472,11 +475,16 @@ int lymph_batch_create(lymph_ctx* const* ctxs, int32_t n, lymph_batch** out) {
             cost.push_back({nb * (int64_t)c->nd * c->nd, make_int2(i, P)});
             b->items_natural.push_back(make_int2(i, P));
         }
-        per_p[c->p] += c->n_blocks;
+        per_p[c->p].first += c->n_blocks;
+        if (c->d_Kex) per_p[c->p].second += c->n_blocks;
         b->high = b->high || c->p >= 3;
         b->absorbing = b->absorbing || c->n_abs > 0;
     }
-    for (auto& kv : per_p) key << "_p" << kv.first << "b" << kv.second;
+    for (auto& kv : per_p) {
+        key << "_p" << kv.first << "b" << kv.second.first;
+        if (kv.second.second) key << "i" << kv.second.second;
+    }
+    if (b->absorbing) key << "_abs";
     b->key = key.str();
     std::stable_sort(cost.begin(), cost.end(), [](const std::pair<int64_t, int2>& x, const std::pair<int64_t, int2>& y) { return x.first > y.first; });
     for (auto& c : cost) b->items_lpt.push_back(c.second);

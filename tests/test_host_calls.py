@@ -1,5 +1,6 @@
 """The library's host side on a fake CUDA runtime (fake_cudart.c): which calls it
 makes, and what it does when one fails.  No GPU."""
+import re
 import struct
 
 import pytest
@@ -84,3 +85,32 @@ fake.fake_clear(); s.run_steps(s.dt, 1.0, max_steps=21, kernel_timing={timed}); 
 """, tmp_path)
     log = "".join(c for c in log if c in "EKXG")
     assert log[0] == "E" and log[-1] == "E" and "K" in log
+
+
+def test_a_schedule_tuned_on_other_kernels_is_not_taken(tmp_path):
+    """Entries under the key of the kernels without integer columns, in the user's cache file
+    and in the default one of their time, leave the batch at its default schedule; a key
+    tells the blocks that are multiplied in integer columns."""
+    home = tmp_path / "home"
+    (home / ".cache").mkdir(parents=True)
+    blocks, sched, default = run(SOLVER.format(precision="FP64") + f"""
+import os
+out(int(s.n_blocks))
+old = f"sm152_prec0_p3b{{s.n_blocks}} 152 1 2\\n"
+open(os.environ["LYMPH_TUNE_CACHE"], "w").write(old)
+b = E.Batch([s]); out(b.schedule()); b.close()
+del os.environ["LYMPH_TUNE_CACHE"]; os.environ["HOME"] = {str(home)!r}
+open({str(home / ".cache" / "lymph3d_gb300_tune2.txt")!r}, "w").write(old)
+b = E.Batch([s]); out(b.schedule())
+""", tmp_path)
+    assert sched == default == [608, 0, 0]
+    keys = run("""
+import os
+for n in (3, 10):
+    s = MatrixFree(M.cube(n, agglomeration="bfs", seed=1, group=(4, 12)), 2, 1e-4)
+    s.MAKE_MATRICES_FREE()
+    b = E.Batch([s]); b.autotune(1, False); b.close()
+    out([int(s.n_blocks), open(os.environ["LYMPH_TUNE_CACHE"]).read().split()[-4]])
+""", tmp_path)
+    for (nb, key), ints in zip(keys, (False, True)):
+        assert re.search(rf"_p2b{nb}" + (rf"i{nb}$" if ints else "$"), key), key
