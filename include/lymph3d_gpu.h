@@ -475,7 +475,8 @@ typedef struct lymph_batch lymph_batch;
 int lymph_batch_create(lymph_ctx* const* ctxs, int32_t n, lymph_batch** out);
 int lymph_batch_destroy(lymph_batch* batch);
 int lymph_batch_run(lymph_batch* batch, int64_t n_steps, const double* gvals, float* ms_total);
-/* Times trial_steps steps for each candidate (1..4 persistent CTAs per SM,
+/* Times trial_steps steps (rounded up to an even number, launched as a graph
+ * like lymph_batch_run's) for each candidate (1..4 persistent CTAs per SM,
  * for LYMPH_MIXED_MF 1..what one SM holds of the lowest degree's kernel, each
  * degree's grid capped at what the SMs hold of its own kernel; items
  * largest-cost-first or problem-major; for

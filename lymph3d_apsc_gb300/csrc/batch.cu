@@ -216,6 +216,7 @@ struct lymph_batch {
     int64_t gvals_cap = 0;
     int* d_status = nullptr;
     cudaGraphExec_t graph = nullptr;
+    int64_t graph_stride = 0;   // of the time-function values it reads
     int graph_steps = 0;
     int64_t launches = 0;
     int step_nl = 2;     // kernels one batched step launches
@@ -368,16 +369,17 @@ int launch_step(lymph_batch* b, int64_t g_stride, int off, int bump) {
     return LYMPH_OK;
 }
 
-// Runs n steps with the current grid/order; the time-function values are
-// already on the device with stride g_stride per problem.
-int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, bool use_graph) {
+// Runs n steps with the current grid/order, as graphs of R (even) steps and the rest
+// launched one by one; the time-function values are already on the device with
+// stride g_stride per problem.  e0 (may be null) is recorded before the first step.
+int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, int R, cudaEvent_t e0) {
     LYMPH_TRY(refresh_problems(b));
     LYMPH_CUDA_TRY(cudaMemsetAsync(b->d_step_idx, 0, sizeof(int64_t), b->stream));
     LYMPH_CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, 2 * BATCH_QUEUES * sizeof(int), b->stream));
-    const int R = 16;
+    if (e0) LYMPH_CUDA_TRY(cudaEventRecord(e0, b->stream));
     int64_t i = 0;
-    if (use_graph && n >= R) {
-        if (b->graph && b->graph_steps != (int)g_stride) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
+    if (n >= R) {
+        if (b->graph && (b->graph_stride != g_stride || b->graph_steps != R)) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         if (!b->graph) {
             cudaGraph_t g;
             LYMPH_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
@@ -394,7 +396,8 @@ int run_loop(lymph_batch* b, int64_t n, int64_t g_stride, bool use_graph) {
             e = cudaGraphInstantiate(&b->graph, g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) { lymph_set_error(std::string("batch graph instantiate: ") + cudaGetErrorString(e)); return LYMPH_ERR_CUDA; }
-            b->graph_steps = (int)g_stride;
+            b->graph_stride = g_stride;
+            b->graph_steps = R;
         }
         for (; i + R <= n; i += R) {
             LYMPH_CUDA_TRY(cudaGraphLaunch(b->graph, b->stream));
@@ -539,7 +542,7 @@ int lymph_batch_run(lymph_batch* b, int64_t n_steps, const double* gvals, float*
     LYMPH_CUDA_TRY(cudaEventCreate(&e0));
     LYMPH_CUDA_TRY(cudaEventCreate(&e1));
     cudaEventRecord(e0, b->stream);
-    int rc = run_loop(b, n_steps, n_steps, true);
+    int rc = run_loop(b, n_steps, n_steps, 16, nullptr);
     cudaEventRecord(e1, b->stream);
     cudaEventSynchronize(e1);
     float ms = 0.0f;
@@ -575,8 +578,12 @@ int lymph_batch_autotune(lymph_batch* b, int32_t trial_steps, int32_t use_cache,
         }
         std::vector<int> curs;
         for (lymph_ctx* c : b->ctx) curs.push_back(c->cur);
-        std::vector<double> g((size_t)b->ctx.size() * (trial_steps + 1), 0.0);
-        LYMPH_TRY(upload_g(b, g.data(), trial_steps + 1));
+        // a trial runs as the loop does, in a graph: launched one by one, the matrix-free
+        // passes of small problems would be timed by the host's calls
+        const int64_t T = (int64_t)trial_steps + (trial_steps & 1);
+        const int R = (int)std::min<int64_t>(T, 16);
+        std::vector<double> g(b->ctx.size() * (size_t)T, 0.0);
+        LYMPH_TRY(upload_g(b, g.data(), T));
         float best = 1e30f;
         int bg = b->grid, bo = b->order, bs = b->shape;
         const int n_shapes = b->precision == LYMPH_MIXED_MF ? 1 : BATCH_SHAPES;
@@ -592,9 +599,8 @@ int lymph_batch_autotune(lymph_batch* b, int32_t trial_steps, int32_t use_cache,
                 b->order = ord;
                 b->grid = mult * b->sms;
                 LYMPH_TRY(upload_items(b));
-                LYMPH_TRY(run_loop(b, 1, trial_steps + 1, false));  // warm-up
-                cudaEventRecord(e0, b->stream);
-                LYMPH_TRY(run_loop(b, trial_steps, trial_steps + 1, false));
+                LYMPH_TRY(run_loop(b, T, T, R, nullptr));  // makes the graph and warms up
+                LYMPH_TRY(run_loop(b, T, T, R, e0));
                 cudaEventRecord(e1, b->stream);
                 cudaEventSynchronize(e1);
                 float ms = 0.0f;

@@ -114,3 +114,16 @@ for n in (3, 10):
 """, tmp_path)
     for (nb, key), ints in zip(keys, (False, True)):
         assert re.search(rf"_p2b{nb}" + (rf"i{nb}$" if ints else "$"), key), key
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED_MF"])
+def test_the_tuner_times_what_runs(tmp_path, precision):
+    """A trial's timed steps are one launch of a graph, as in Batch.run, with no launch of the
+    host's between its two events."""
+    log, = run(SOLVER.format(precision=precision) + """
+b = E.Batch([s]); fake.fake_clear(); b.autotune(3, False); out(calls())
+""", tmp_path)
+    trials = re.sub(r"\[.*?\]", "", log)                  # without what is captured
+    timed = re.findall(r"E([^E]*)E", trials)
+    assert len(timed) >= 8 and set(timed) == {"G"}
+    assert "K" not in trials and "X" not in trials
