@@ -93,13 +93,16 @@ static_assert(Deg<1>::ND * kBatchShapes[2][1] <= BATCH_THREADS && Deg<2>::ND * k
 // FP64 with a grid of at most three CTAs per SM, which the tuner takes where the items are
 // few, has 64 registers (24 problems of 2^3..4^3 x 6: 2.81 -> 2.33 ms), and in the shapes
 // without integer columns at p = 2 a kernel of p = 1 and 2 alone (5 problems of 20^3..26^3
-// at p = 1, tuned: 18.7 -> 18.0 ms, at p = 2 42.9 -> 40.0).
+// at p = 1, tuned: 18.7 -> 18.0 ms, at p = 2 42.9 -> 40.0).  In those shapes the FP64 kernel
+// of all degrees keeps the damping's code: what it spills lies in that code, and without it
+// the compiler has fewer loads in flight (8 problems of 20^3..26^3, tuned: 124.9 against
+// 122.5 ms, 64 of 3^3..8^3 27.3 against 27.0; in shape 0 46.0 without, 46.3 with at p = 2).
 template <typename KT, int V, int MINB, bool HIGH, bool ABS>
 __global__ void __launch_bounds__(BATCH_THREADS, MINB)
 k_step_batch(const BatchProblem* __restrict__ probs, const int2* __restrict__ items, int n_items, int* queue,
              const int64_t* step_idx, int off, const double* gvals, int64_t g_stride) {
     constexpr bool SHARED = sizeof(KT) == 4;
-    constexpr int CHAIN = 4;
+    constexpr int CHAIN = SHARED || V == 0 ? 4 : 16;
     __shared__ __align__(16) char smem[BatchSmem<KT, V, HIGH>::bytes];
     __shared__ int s_item;
     __shared__ __align__(8) char s_args[SHARED ? sizeof(StepArgs) : 8];
@@ -296,14 +299,20 @@ void launch_shape(lymph_batch* b, const BatchProblem* probs, int off, int* queue
     };
     auto shape = [&](auto v) {
         constexpr int V = decltype(v)::value;
-        if (b->absorbing) return go(k_step_batch<KT, V, BATCH_MINB, true, true>);
         if constexpr (sizeof(KT) == 8) {
-            if (b->grid <= 3 * b->sms) return go(k_step_batch<KT, V, 3, true, false>);
-            if constexpr (V != 0) {
-                if (!b->high) return go(k_step_batch<KT, V, BATCH_MINB, false, false>);
+            if (!b->absorbing) {
+                if (b->grid <= 3 * b->sms) return go(k_step_batch<KT, V, 3, true, false>);
+                if constexpr (V == 0) {
+                    return go(k_step_batch<KT, V, BATCH_MINB, true, false>);
+                } else {
+                    if (!b->high) return go(k_step_batch<KT, V, BATCH_MINB, false, false>);
+                }
             }
+            go(k_step_batch<KT, V, BATCH_MINB, true, true>);
+        } else {
+            if (b->absorbing) go(k_step_batch<KT, V, BATCH_MINB, true, true>);
+            else go(k_step_batch<KT, V, BATCH_MINB, true, false>);
         }
-        go(k_step_batch<KT, V, BATCH_MINB, true, false>);
     };
     switch (b->shape) {
         case 1: shape(std::integral_constant<int, 1>()); break;
