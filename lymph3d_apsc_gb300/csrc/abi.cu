@@ -417,6 +417,8 @@ int lymph_create(const lymph_mesh_desc* m, const lymph_params* prm, lymph_ctx** 
         static std::atomic<uint64_t> next_uid{1};
         c->uid = next_uid++;
     }
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
     MeshHash hash(m);
     int rc = LYMPH_OK;
     auto fail = [&](int code) { lymph_destroy(c); return code; };

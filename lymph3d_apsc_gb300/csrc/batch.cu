@@ -281,6 +281,7 @@ int refresh_problems(lymph_batch* b) {
         P.a.dt2 = c->dt * c->dt;
         P.a.status = b->d_status;
         P.a.n_poly = c->n_poly;
+        P.a.early = 0;
         P.a.prefetch = !b->high || (bytes >= BATCH_PREFETCH_MIN && (b->precision == LYMPH_FP64 || c->p <= 3));
         P.buf[0] = c->d_buf[0];
         P.buf[1] = c->d_buf[1];

@@ -71,6 +71,7 @@ struct lymph_ctx {
     double alpha = 10.0, theta = -1.0, dt = 1e-3;
     // sizes
     int n_node = 0, n_tet = 0, n_poly = 0, n_mat = 0;
+    int sms = 1;                    // SMs of the context's device
     uint64_t mesh_hash = 0;         // FNV-1a of the mesh descriptor's arrays (checkpoints carry it)
     std::vector<void*> arenas;      // device allocations that hold the arrays below but for the few noted in lymph_destroy
     uint64_t uid = 0;               // unique per context in the process (caches keyed by context)

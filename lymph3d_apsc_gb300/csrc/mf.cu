@@ -887,6 +887,7 @@ void lymph_mf_batch_problem(const lymph_ctx* c, int* status, void* out) {
     s.status = status;
     s.n_poly = c->n_poly;
     s.prefetch = 0;
+    s.early = 0;
     MfBatchProblem pb;
     pb.a = mf_args(c, s);
     pb.buf[0] = c->d_buf[0];

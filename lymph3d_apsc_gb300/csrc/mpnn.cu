@@ -609,7 +609,7 @@ int set_graph(lymph_mpnn* n, int n_nodes, const int32_t* wp, const int32_t* wi, 
 
 namespace {
 
-constexpr int SS_BLOCKS = 304;  // 2 x 152 SMs
+constexpr int SS_BLOCKS = 304;  // two per SM of the GB300; fixed, so that the sums have one order on every device
 
 // d1 = u1 - u0, d2 = u1 - 2 u0 + um elementwise, and per-CTA partial sums of
 // squares of u1, d1, d2 into part[3 * blockIdx.x + 0..2] (fixed order).

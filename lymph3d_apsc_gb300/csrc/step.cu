@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(Shape<PD>::T, PD == 2 && INT ? 8 : Shape<PD>::
     step_poly<PD, KT, MODE, Shape<PD>::S, INT, false, ABS, PD == 3 ? 8 : 16, PD == 2 && sizeof(KT) == 8 && !INT ? 2 : 0>(A, blockIdx.x, smem);
 }
 
-// The same for at most SMALL_POLY polyhedra without absorbing faces, p <= 3.
+// The same for at most one polyhedron per SM without absorbing faces, p <= 3.
 template <int PD, typename KT, bool INT = int_columns(PD, sizeof(KT))>
 __global__ void __launch_bounds__(Shape<PD>::T, 2) k_step_small(StepArgs A) {
     __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
@@ -290,9 +290,9 @@ template <int PD, typename KT, int MODE, bool INT>
 int launch_step_i(lymph_ctx* c, const StepArgs& A) {
     // p = 1 in one wave of 8 to 16 CTAs per SM: an early launch unbalances the SMs and a
     // late one comes too late (48 steps of 1,728 polyhedra: 475 us in FP32, plain 390 us)
-    const bool plain = PD == 1 && c->n_poly > 8 * 152 && c->n_poly <= 16 * 152;
+    const bool plain = PD == 1 && c->n_poly > 8 * c->sms && c->n_poly <= 16 * c->sms;
     if constexpr (MODE == MODE_STEP && PD <= 3) {
-        if (c->n_poly <= SMALL_POLY && !A.abs_idx) {
+        if (c->n_poly <= c->sms && !A.abs_idx) {
             constexpr size_t bytes = SmallSmem<PD, KT>::bytes;
             LYMPH_CUDA_TRY(cudaFuncSetAttribute(k_step_small<PD, KT, INT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)bytes));
@@ -366,6 +366,7 @@ StepArgs base_args(lymph_ctx* c) {
     A.step_off = 0; A.g = 0.0; A.u32_out = nullptr;
     A.u0 = nullptr; A.un = nullptr; A.out = nullptr; A.partial = c->d_partial; A.dt = c->dt; A.dt2 = c->dt * c->dt; A.status = c->d_status;
     A.n_poly = c->n_poly;
+    A.early = trigger_early(c->p, c->n_poly, c->sms);
     A.prefetch = c->n_blocks * c->nd * c->nd * (c->precision == LYMPH_FP64 ? 8 : 4) <= STEP_PREFETCH_MAX;
     A.abs_idx = c->n_abs > 0 ? c->d_abs_idx : nullptr;
     A.Dabs = c->d_Dabs;
@@ -564,7 +565,7 @@ int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double
 // 345 -> 405 us), and p = 1 at any size (46,767, 16 steps: 4.06 -> 4.25 ms).
 bool lymph_dev_int_columns(const lymph_ctx* c) {
     if (c->precision != LYMPH_FP64) return false;
-    return c->p >= 3 || (c->p == 2 && c->n_poly >= 4 * 152 && c->n_blocks >= 8 * (int64_t)c->n_poly);
+    return c->p >= 3 || (c->p == 2 && c->n_poly >= 4 * c->sms && c->n_blocks >= 8 * (int64_t)c->n_poly);
 }
 
 // The exponents of the assembled FP64 blocks that the integer columns need.

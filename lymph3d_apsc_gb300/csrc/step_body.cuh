@@ -143,6 +143,7 @@ struct StepArgs {
     int* status;
     int n_poly;
     int prefetch;              // whether a step prefetches its rows' heads
+    int early;                 // whether it lets the next step's CTAs be placed before it sums (trigger_early)
 };
 
 // Programmatic dependent launch: a step kernel starts while the one before it
@@ -157,7 +158,7 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // others idle (48 steps of 512 polyhedra in FP64: p = 3 1.70 against 1.26 ms, p = 4
 // 6.0 against 4.3 ms with FP64 products alone; of 125 polyhedra at p = 4: 1.17
 // against 1.34 ms, of 1,000 at p = 1 374 against 433 us).
-__device__ __forceinline__ bool trigger_early(int p) { return gridDim.x <= (p == 1 ? 8u : 1u) * 152u; }
+inline bool trigger_early(int p, int n_poly, int sms) { return n_poly <= (p == 1 ? 8 : 1) * sms; }
 
 // Launches a step kernel that may start before the stream's previous kernel ends.
 template <typename K, typename A>
@@ -344,7 +345,6 @@ __device__ __forceinline__ void finish_poly(const StepArgs& A, int P, double y, 
 // 48 steps of 125 hexahedra: p = 1 in FP64 267 -> 240 us, p = 2 346 -> 335 (FP64-pipe
 // bound), p = 3 627 -> 591, in FP32 263 -> 239, 285 -> 265, 371 -> 337; 100 FP64 steps
 // of 90 polyhedra (10 blocks a row): 605 -> 503, 852 -> 803, 1,856 -> 1,615 us.
-constexpr int SMALL_POLY = 152;
 constexpr int SMALL_STAGE = 88 * 1024;   // bytes of staged blocks per CTA
 template <int PD, typename KT> struct SmallSmem {
     static constexpr int ND = Deg<PD>::ND, NP = Deg<PD>::NP;
@@ -438,7 +438,7 @@ __device__ __forceinline__ void step_poly(const StepArgs& A, int P, char* smem, 
             prefetch_inside(A.Minv + (int64_t)P * Deg<PD>::NP * Deg<PD>::NP, (int64_t)Deg<PD>::NP * Deg<PD>::NP * 8);
         }
         pdl_wait();
-        if (trigger_early(PD)) pdl_trigger();
+        if (A.early) pdl_trigger();
     }
 
     constexpr int NI = SZ::NI, C0 = SZ::C0, NC = SZ::NC, JF = CPT - NI;

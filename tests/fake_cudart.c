@@ -1,6 +1,7 @@
 /* A stand-in for the CUDA runtime's entry points that the library calls, preloaded by
  * tests of its host side: device memory is host memory, kernels do nothing, and each
- * call is noted as one letter.  fake_fail_launch(n) makes the n-th kernel launch from
+ * call is noted as one letter; FAKE_SMS in the environment is the device's number of
+ * SMs (152).  fake_fail_launch(n) makes the n-th kernel launch from
  * then on fail as a launch can. */
 #include <stdlib.h>
 #include <string.h>
@@ -66,7 +67,11 @@ int __cudaLaunchKernel(void* k, dim3_ g, dim3_ b, void** a, size_t s, void* st) 
     (void)k; (void)g; (void)b; (void)a; (void)s; (void)st;
     return launch('K');
 }
+static size_t dyn_;
+size_t fake_dynamic_smem(void) { size_t d = dyn_; dyn_ = 0; return d; }   /* the largest since the last call */
 int cudaLaunchKernelExC(const void* cfg, const void* f, void** a) {
-    (void)cfg; (void)f; (void)a;
+    const size_t d = *(const size_t*)((const char*)cfg + 2 * sizeof(dim3_));   /* cudaLaunchConfig_t: grid, block, dynamic shared memory */
+    (void)f; (void)a;
+    if (d > dyn_) dyn_ = d;
     return launch('X');
 }

@@ -127,3 +127,20 @@ b = E.Batch([s]); fake.fake_clear(); b.autotune(3, False); out(calls())
     timed = re.findall(r"E([^E]*)E", trials)
     assert len(timed) >= 8 and set(timed) == {"G"}
     assert "K" not in trials and "X" not in trials
+
+
+@pytest.mark.parametrize("sms,staged,ints", [(152, True, True), (100, False, True), (200, True, False)])
+def test_rules_in_ctas_per_sm_ask_the_device(tmp_path, sms, staged, ints):
+    """125 polyhedra take the kernel that stages their rows in dynamic shared memory up to one
+    polyhedron per SM, 737 of p = 2 the integer columns from four per SM on."""
+    got = run("""
+import os, re
+fake.fake_dynamic_smem.restype = ctypes.c_size_t
+s = MatrixFree(M.cube(5, agglomeration="hex"), 2, 1e-4)
+s.MAKE_MATRICES_FREE(); fake.fake_dynamic_smem(); s.run_steps(s.dt, 1.0, max_steps=3)
+out(fake.fake_dynamic_smem() > 0)
+s = MatrixFree(M.cube(10, agglomeration="bfs", seed=1, group=(4, 12)), 2, 1e-4)
+s.MAKE_MATRICES_FREE(); b = E.Batch([s]); b.autotune(1, False)
+out(re.search(r"i\\d+", open(os.environ["LYMPH_TUNE_CACHE"]).read()) is not None)
+""", tmp_path, FAKE_SMS=str(sms))
+    assert got == [staged, ints]
