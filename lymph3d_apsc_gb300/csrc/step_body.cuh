@@ -13,14 +13,16 @@ namespace stepk {
 //
 // The GB300 retires 2 FP64 multiply-adds per clock and SM, which holds a product
 // with FP64 blocks at two thirds of the copy bandwidth, while its integer pipe idles.
-// At p = 3 and 4, and at p = 2 where it pays (lymph_dev_int_columns), 60 % of each row's columns (the last ones, c >= C0) are therefore
-// multiplied there: a block entry and a coefficient are doubles as before, their
-// mantissas multiply to the product's top 64 bits (relative error below 2^-61; an
-// FP64 product rounds to 2^-53), and the product, shifted by the exponents, adds up
-// exactly in a 128-bit accumulator whose top stands at the largest product any
-// block of the row could have.  A term loses bits only below 2^-117 of that.  The
-// sum is rounded to FP64 once per 16 blocks, so the row's error falls (K u of
-// random, graded and near-constant states: by 40 % in the mean).
+// At p = 3 and 4, and at p = 2 where it pays (lymph_dev_int_columns), 60 % of each row's
+// columns (the last ones, c >= C0) are therefore multiplied there: a block entry and a
+// coefficient are doubles as before, their mantissas multiply to the product's top 64
+// bits (three dropped parts of less than a unit each of at least 2^62: truncated towards
+// zero by less than 3 2^-62 of it, where an FP64 product rounds by 2^-53), and the
+// product, shifted by the exponents, adds up exactly in a 128-bit accumulator whose top
+// stands at the largest product any block of the row could have.  A term loses bits only
+// below 2^-117 of that.  The sum is converted to FP64 once per 16 blocks (acc_value: its
+// two words and their sum are rounded), so the row's error falls (K u of random, graded
+// and near-constant states: by 40 % in the mean).
 // 16 steps of 46,767 polyhedra at p = 3: 56.0 -> 38.0 ms (61 -> 90 % of the copy
 // bandwidth); 24 steps of a mesh of 17^3 cubes at p = 4: 18.8 -> 13.2 ms.
 constexpr bool int_columns(int p, size_t elem) { return p >= 3 && elem == 8; }
