@@ -224,37 +224,47 @@ inline int np_of(int p) { return (p + 1) * (p + 2) * (p + 3) / 6; }
 // COMPUTE_ERROR_L2_MATRIX_FREE's body for polyhedron P
 // (src/matrix_free.f90:1388-1418): sum_i du_i^T M du_i with du = uh - uex,
 // M the Np x Np modal mass matrix, rows and columns in the reference's order.
-// One CTA of L2_THREADS threads per polyhedron; the result is returned in thread 0.
-// M comes into shared memory in coalesced reads (a thread per polyhedron read
-// it at a stride of Np^2 doubles), a thread forms one row's t = M du, and one
-// thread per component adds the rows up in order.
+// A CTA takes as many polyhedra as its threads hold rows of: a thread forms one row's
+// t = M du, one per component adds the rows up in order and one per polyhedron the
+// components, M in shared memory from coalesced reads.  The FP64 pipe takes 64 cycles
+// for a warp's operation whatever lanes it has (46,861 polyhedra at p = 1, the call: 77 us
+// with a CTA or a warp per polyhedron, 53 packed, 63 with a thread per polyhedron, which
+// reads M at a stride: 19,760 at p = 3 307 us, 111 with a CTA each, 97 packed).
 constexpr int L2_THREADS = 128;
 static_assert(3 * MAX_NP <= L2_THREADS, "one thread per row");
-__device__ __forceinline__ double l2_partial_poly(int P, int NP, const double* __restrict__ Mm,
-                                                  const double* __restrict__ uh, const double* __restrict__ uex) {
-    __shared__ double s_M[MAX_NP * MAX_NP], s_du[3 * MAX_NP], s_t[3 * MAX_NP];
-    const int ND = 3 * NP, tid = threadIdx.x;
-    const double* M = Mm + (int64_t)P * NP * NP;
-    for (int i = tid; i < NP * NP; i += L2_THREADS) s_M[i] = M[i];
-    if (tid < ND) s_du[tid] = uh[(int64_t)P * ND + tid] - uex[(int64_t)P * ND + tid];
+__host__ __device__ constexpr int l2_polys(int NP) { return L2_THREADS / (3 * NP); }   // per CTA
+constexpr int L2_MASS = 10 * 4 * 4 > MAX_NP * MAX_NP ? 10 * 4 * 4 : MAX_NP * MAX_NP;
+static_assert(l2_polys(4) * 4 * 4 <= L2_MASS && l2_polys(10) * 10 * 10 <= L2_MASS && l2_polys(20) * 20 * 20 <= L2_MASS,
+              "the mass matrices of a CTA's polyhedra");
+inline unsigned l2_grid(int n_poly, int NP) { return (unsigned)((n_poly + l2_polys(NP) - 1) / l2_polys(NP)); }
+// partial[P] for the polyhedra of this block of l2_grid
+__device__ __forceinline__ void l2_partials(int n_poly, int NP, const double* __restrict__ Mm, const double* __restrict__ uh,
+                                            const double* __restrict__ uex, double* partial) {
+    __shared__ double s_M[L2_MASS], s_du[L2_THREADS], s_t[L2_THREADS], s_e[L2_THREADS];
+    const int tid = threadIdx.x, ND = 3 * NP, N = l2_polys(NP), P0 = blockIdx.x * N, n = n_poly - P0 < N ? n_poly - P0 : N;
+    const int64_t m0 = (int64_t)P0 * NP * NP, u0 = (int64_t)P0 * ND;
+    for (int i = tid; i < n * NP * NP; i += L2_THREADS) s_M[i] = Mm[m0 + i];
+    if (tid < n * ND) s_du[tid] = uh[u0 + tid] - uex[u0 + tid];
     __syncthreads();
-    if (tid < ND) {
-        const int i = tid / NP, rr = tid - i * NP;
+    if (tid < n * ND) {
+        const int k = tid / ND, r = tid - k * ND, i = r / NP, rr = r - i * NP;
+        const double *M = s_M + (k * NP + rr) * NP, *du = s_du + k * ND + i * NP;
         double t = 0.0;
-        for (int c = 0; c < NP; ++c) t = fma(s_M[rr * NP + c], s_du[i * NP + c], t);
+        for (int c = 0; c < NP; ++c) t = fma(M[c], du[c], t);
         s_t[tid] = t;
     }
     __syncthreads();
-    double e = 0.0;
-    if (tid < 3)
+    if (tid < 3 * n) {
+        double e = 0.0;
         for (int rr = 0; rr < NP; ++rr) e = fma(s_du[tid * NP + rr], s_t[tid * NP + rr], e);
-    double err = 0.0;
-    if (tid < 32) {
-        err = err + __shfl_sync(0xffffffffu, e, 0);
-        err = err + __shfl_sync(0xffffffffu, e, 1);
-        err = err + __shfl_sync(0xffffffffu, e, 2);
+        s_e[tid] = e;
     }
-    return err;
+    __syncthreads();
+    if (tid < n) {
+        double err = 0.0;
+        for (int i = 0; i < 3; ++i) err = err + s_e[3 * tid + i];
+        partial[P0 + tid] = err;
+    }
 }
 
 // Deterministic sum of v[0..n) by one CTA of 1024 threads: a fixed strided

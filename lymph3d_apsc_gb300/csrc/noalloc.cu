@@ -57,11 +57,10 @@ int scratch_address(double** out) {
 // The context path's arithmetic (the same device functions, common.cuh):
 // per polyhedron sum_i du_i^T M du_i (COMPUTE_ERROR_L2_MATRIX_FREE's body),
 // then the fixed-order sum.
-__global__ void __launch_bounds__(L2_THREADS) k_l2_partial_noalloc(int NP, const double* __restrict__ Mm,
+__global__ void __launch_bounds__(L2_THREADS) k_l2_partial_noalloc(int n_poly, int NP, const double* __restrict__ Mm,
                                                                    const double* __restrict__ uh,
                                                                    const double* __restrict__ uex, double* partial) {
-    const double e = l2_partial_poly(blockIdx.x, NP, Mm, uh, uex);
-    if (threadIdx.x == 0) partial[blockIdx.x] = e;
+    l2_partials(n_poly, NP, Mm, uh, uex, partial);
 }
 
 __global__ void __launch_bounds__(1024) k_sum_noalloc(int64_t n, const double* __restrict__ v, double* out) {
@@ -89,7 +88,7 @@ extern "C" int lymph_error_l2_noalloc(const double* d_mass_modal, const double* 
     LYMPH_TRY(scratch_address(&scratch));
     // every partial is overwritten and the total is written once, so nothing
     // left over from an earlier call is read
-    k_l2_partial_noalloc<<<n_poly, L2_THREADS>>>(Np, d_mass_modal, d_uh, d_uex, scratch);
+    k_l2_partial_noalloc<<<l2_grid(n_poly, Np), L2_THREADS>>>(n_poly, Np, d_mass_modal, d_uh, d_uex, scratch);
     LYMPH_CUDA_TRY(cudaGetLastError());
     k_sum_noalloc<<<1, 1024>>>(n_poly, scratch, scratch + NOALLOC_MAX_POLY);
     LYMPH_CUDA_TRY(cudaGetLastError());

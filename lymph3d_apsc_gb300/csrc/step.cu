@@ -46,11 +46,13 @@ __global__ void __launch_bounds__(Shape<PD>::T, 2) k_step_small(StepArgs A) {
 __global__ void k_bump(int64_t* idx, int n) { *idx += n; }
 
 // COMPUTE_ERROR_L2_MATRIX_FREE body per polyhedron: sum_i du_i^T M du_i.
-__global__ void __launch_bounds__(L2_THREADS) k_l2_partial(int NP, const double* __restrict__ Mm,
+__global__ void __launch_bounds__(L2_THREADS) k_l2_partial(int n_poly, int NP, const double* __restrict__ Mm,
                                                            const double* __restrict__ uh, const double* __restrict__ uex,
                                                            double* partial) {
-    const double e = l2_partial_poly(blockIdx.x, NP, Mm, uh, uex);
-    if (threadIdx.x == 0) partial[blockIdx.x] = e;
+    l2_partials(n_poly, NP, Mm, uh, uex, partial);
+}
+void launch_l2(lymph_ctx* c, const double* M, const double* uh, const double* uex) {
+    k_l2_partial<<<l2_grid(c->n_poly, c->Np), L2_THREADS, 0, c->stream>>>(c->n_poly, c->Np, M, uh, uex, c->d_partial);
 }
 
 // ---- COMPUTE_ERROR_DG_MATRIX_FREE ----
@@ -534,7 +536,7 @@ int lymph_dev_error_dg(lymph_ctx* c, const double* uh, const double* uex, double
 // Leapfrog energy terms: d_out[0] = |ub - ua|^2_M (rho-weighted mass),
 // d_out[1] = ub . K ua.
 int lymph_dev_energy(lymph_ctx* c, const double* ua, const double* ub, double* d_out) {
-    k_l2_partial<<<c->n_poly, L2_THREADS, 0, c->stream>>>(c->Np, c->d_M, ub, ua, c->d_partial);
+    launch_l2(c, c->d_M, ub, ua);
     k_sum<<<1, 1024, 0, c->stream>>>(c->n_poly, c->d_partial, d_out);
     StepArgs A = base_args(c);
     A.u0 = ua;
@@ -547,7 +549,7 @@ int lymph_dev_energy(lymph_ctx* c, const double* ua, const double* ub, double* d
 }
 
 int lymph_dev_error_l2(lymph_ctx* c, const double* uh, const double* uex, double* d_out) {
-    k_l2_partial<<<c->n_poly, L2_THREADS, 0, c->stream>>>(c->Np, c->d_Mm, uh, uex, c->d_partial);
+    launch_l2(c, c->d_Mm, uh, uex);
     k_sum<<<1, 1024, 0, c->stream>>>(c->n_poly, c->d_partial, d_out);
     c->launches += 2;
     LYMPH_CUDA_TRY(cudaGetLastError());
