@@ -24,13 +24,14 @@ using namespace stepk;
 
 // One CTA per polyhedron.  Without the code of absorbing faces (ABS) p = 1 takes 32 registers
 // instead of 38 with FP32 blocks, so 21 CTAs fit an SM instead of 17: 48 steps of 46,861
-// polyhedra 5.08 -> 4.42 ms, of 3,013 466 -> 430 us.  The integer columns of p = 2 keep few values
+// polyhedra 5.08 -> 4.42 ms, of 3,013 466 -> 430 us; the bound of 20 holds every mode to
+// that (30 products of the power iteration 8.89 -> 8.34 ms).  The integer columns of p = 2 keep few values
 // per thread and wait for their loads: 8 CTAs per SM (32 registers) instead of 6 take
 // 46,861 polyhedra from 46.2 to 37.8 ms, 737 from 0.89 to 0.87 (45.7 and 1.02 with FP64 products).
 // The FP64 products of p = 2 load two blocks at once (8,000 hexahedra 5.47 -> 5.42 ms, 2,197
 // 1.65 -> 1.62): left to itself the compiler loads one once the damping's code is gone.
 template <int PD, typename KT, int MODE, bool INT, bool ABS>
-__global__ void __launch_bounds__(Shape<PD>::T, PD == 2 && INT ? 8 : Shape<PD>::MINB) k_step(StepArgs A) {
+__global__ void __launch_bounds__(Shape<PD>::T, PD == 1 && sizeof(KT) == 4 ? 20 : (PD == 2 && INT ? 8 : Shape<PD>::MINB)) k_step(StepArgs A) {
     __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
     step_poly<PD, KT, MODE, Shape<PD>::S, INT, false, ABS, PD == 3 ? 8 : 16, PD == 2 && sizeof(KT) == 8 && !INT ? 2 : 0>(A, blockIdx.x, smem);
 }
