@@ -144,3 +144,18 @@ s.MAKE_MATRICES_FREE(); b = E.Batch([s]); b.autotune(1, False)
 out(re.search(r"i\\d+", open(os.environ["LYMPH_TUNE_CACHE"]).read()) is not None)
 """, tmp_path, FAKE_SMS=str(sms))
     assert got == [staged, ints]
+
+
+@pytest.mark.parametrize("n", [2, 6, 8])
+def test_the_mesh_hash_of_every_size(tmp_path, n):
+    """48, 1,296 and 3,072 tetrahedra: ids of one and of two bytes, negative neighbours, the
+    hash formed in place and by a thread: FNV-1a over the bytes of the arrays."""
+    path = tmp_path / "c.ckpt"
+    run(f"""
+m = M.cube({n}, bc="reference", agglomeration="tet", jitter=0.1)
+s = MatrixFree(m, 1, 1e-4); s.MAKE_MATRICES_FREE(); s.save_checkpoint({str(path)!r}, 0.5, 3)
+""", tmp_path)
+    m = M.cube(n, bc="reference", agglomeration="tet", jitter=0.1)
+    parts = [struct.pack("<4i", m.n_node, m.n_tet, m.n_poly, len(m.mat))]
+    parts += [a.tobytes() for a in (m.coords, m.tet_vert, m.tet_poly, m.tet_mat, m.neigh, m.fun_tag, m.mat)]
+    assert struct.pack("<Q", _fnv(*parts)) in path.read_bytes()[:128]
