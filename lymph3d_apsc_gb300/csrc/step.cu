@@ -30,9 +30,13 @@ using namespace stepk;
 // 46,861 polyhedra from 46.2 to 37.8 ms, 737 from 0.89 to 0.87 (45.7 and 1.02 with FP64 products).
 // The FP64 products of p = 2 load two blocks at once (8,000 hexahedra 5.47 -> 5.42 ms, 2,197
 // 1.65 -> 1.62): left to itself the compiler loads one once the damping's code is gone.
+// At p = 3 in FP64 6 CTAs' arrays of 20,752 bytes just fill the 132 KB division of an SM's
+// memory; with 1,600 bytes more each the next larger one is taken and meshes of 1 to 3
+// waves gain (1,296 tetrahedra 2.09 -> 2.01 ms, 1,331 hexahedra 2.62 -> 2.53; larger ones 0-1 %).
+constexpr size_t step_pad(int p, bool ints) { return p == 3 && ints ? 1600 : 0; }
 template <int PD, typename KT, int MODE, bool INT, bool ABS>
 __global__ void __launch_bounds__(Shape<PD>::T, PD == 1 && sizeof(KT) == 4 ? 20 : (PD == 2 && INT ? 8 : Shape<PD>::MINB)) k_step(StepArgs A) {
-    __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes];
+    __shared__ __align__(16) char smem[SmemSize<PD, KT, Shape<PD>::S, INT>::bytes + step_pad(PD, INT)];
     step_poly<PD, KT, MODE, Shape<PD>::S, INT, false, ABS, PD == 3 ? 8 : 16, PD == 2 && sizeof(KT) == 8 && !INT ? 2 : 0>(A, blockIdx.x, smem);
 }
 
